@@ -66,9 +66,9 @@ def build():
 
 def reference_root(arg=None):
     """The reference tree's root: an explicit argument, else the DN_REFERENCE_ROOT environment variable;
-    None when neither names an existing directory."""
+    None when neither names a directory that holds the reference's sources."""
     root = arg or os.environ.get("DN_REFERENCE_ROOT")
-    return root if root and os.path.isdir(root) else None
+    return root if root and os.path.isfile(os.path.join(root, "src", "DoonEngine", "voxel.c")) else None
 
 
 def build_reference(ref_root=None):

@@ -163,15 +163,17 @@ __global__ void __launch_bounds__(128, DN_PACKET_MIN_BLOCKS) k_light_packet_batc
     packet_loop<true, POOL>(nullptr, &a, warps[threadIdx.x >> 5]);
 }
 
-// the opaque-chunk marks (mark_opaque_word) of every map of a lighting launch: block i marks map i
+// the opaque-chunk marks (mark_opaque_cells) of every map of a lighting launch: MARK_BLOCKS blocks per map
+constexpr uint32_t MARK_BLOCKS = 16;
 __global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* l)
 {
     __shared__ uint32_t opq[8];
-    const BatchLightMap& e = l[blockIdx.x];
+    const BatchLightMap& e = l[blockIdx.x / MARK_BLOCKS];
     opaque_materials(e.mats, opq);
-    const uint64_t nwords = ((uint64_t)e.m.sx * e.m.sy * e.m.sz + 15) / 16;
-    for (uint64_t wi = threadIdx.x; wi < nwords; wi += blockDim.x)
-        mark_opaque_word(const_cast<uint32_t*>(e.m.tbits), e.m.tword, e.m.rec, wi, opq);
+    const uint64_t pairs = WalkGrid(e.m.sx, e.m.sy, e.m.sz).words / 2u;
+    const uint32_t per = blockDim.x / 32u;
+    for (uint64_t w = (blockIdx.x % MARK_BLOCKS) * per + threadIdx.x / 32u; w < pairs; w += MARK_BLOCKS * per)
+        mark_opaque_cells(e.m, w, opq);
 }
 
 // the diffuse paths of the voxels k_light_packet_batch lit, as per-lane path streams over every map's queue
@@ -358,7 +360,7 @@ struct FramePlan {
 static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, bool packets)
 {
     COUNT_LAUNCH();
-    k_mark_opaque_batch<<<la.nmaps, 256, 0, s>>>(la.maps);
+    k_mark_opaque_batch<<<la.nmaps * MARK_BLOCKS, 256, 0, s>>>(la.maps);
     CK(cudaGetLastError());
     COUNT_LAUNCH();
     const unsigned grid = (unsigned)(g_numSMs * (int)b->tuning.blocksPerSM);
@@ -571,9 +573,10 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
             a.tword = g->tword; a.tbits = g->tbits; a.treq = g->treq; a.tvis = g->tvis; a.ttouch = g->ttouch; a.tlast = g->tlast;
             a.tpend = g->tpend; a.tpendSlot = g->tpendSlot; a.rec = g->rec;
             a.reqs = g->reqs; a.reqCap = g->reqCap; a.st = g->st; a.ntiles = g->ntiles;
+            a.sx = g->sx; a.sy = g->sy; a.sz = g->sz;
             a.op = it.sync.op; a.split = it.sync.split; a.frameNum = it.sync.frameNum;
             syncStart[is] = blocksS;
-            blocksS += (uint32_t)((g->ntiles + 255) / 256);
+            blocksS += (uint32_t)((WalkGrid(g->sx, g->sy, g->sz).cells + 255) / 256);
             is++;
         }
         if (it.phases & DN_BATCH_LIGHT) {

@@ -152,18 +152,38 @@ uint32_t vol_array_bit(DNgpuVolume* g, const void* field)
     return 0u;
 }
 
+static uint64_t walk_words(const DNgpuVolume* g) { return WalkGrid(g->sx, g->sy, g->sz).words; }
+
+// a new map's walk grid: every tile absent (0), every border cell 1
+__global__ void __launch_bounds__(256) k_walk_border(uint32_t* tbits, uint32_t sx, uint32_t sy, uint32_t sz)
+{
+    const WalkGrid wg(sx, sy, sz);
+    const uint64_t cell = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    bool border = true;
+    if (cell >= wg.first && cell < wg.cells) {
+        const uint32_t i = (uint32_t)(cell - wg.first), row = (uint32_t)wg.row, plane = (uint32_t)wg.plane;
+        const uint32_t z = i / plane, y = (i - z * plane) / row, x = i - z * plane - y * row;
+        border = !(x < sx && y < sy && z < sz);
+    }
+    const unsigned b = __ballot_sync(0xFFFFFFFFu, border);
+    const uint32_t lane = threadIdx.x & 31u;
+    if (lane < 2u && cell - lane < wg.cells) tbits[(cell - lane) / 16u + lane] = spread_bits(lane ? b >> 16 : b);
+}
+
 static int alloc_tiles(DNgpuVolume* g)
 {
     uint64_t n = g->ntiles;
     int rc;
     dn_new_generation(g);
     if ((rc = valloc(g, g->tword, n)) || (rc = valloc(g, g->treq, n)) || (rc = valloc(g, g->tvis, n)) ||
-        (rc = valloc(g, g->tbits, (n + 31) / 32 * 2)) ||
+        (rc = valloc(g, g->tbits, walk_words(g))) ||
         (rc = valloc(g, g->ttouch, n)) || (rc = valloc(g, g->tlast, n)) || (rc = valloc(g, g->tpend, n)) ||
         (rc = valloc(g, g->tpendSlot, n)))
         return rc;
     CK(cudaMemsetAsync(g->tword, 0, n * 4, g->stream));
-    CK(cudaMemsetAsync(g->tbits, 0, (n + 31) / 32 * 8, g->stream));
+    COUNT_LAUNCH();
+    k_walk_border<<<(uint32_t)((walk_words(g) * 16 + 255) / 256), 256, 0, g->stream>>>(g->tbits, g->sx, g->sy, g->sz);
+    CK(cudaGetLastError());
     CK(cudaMemsetAsync(g->treq, 0, n, g->stream));
     CK(cudaMemsetAsync(g->tvis, 0, n, g->stream));
     CK(cudaMemsetAsync(g->ttouch, 0, n, g->stream));
@@ -321,7 +341,7 @@ static int persistent_arrays(DNgpuVolume* g, PersistentArray* out)
     out[k++] = {(void**)&g->treq, n};
     out[k++] = {(void**)&g->tvis, n};
     out[k++] = {(void**)&g->ttouch, n};
-    out[k++] = {(void**)&g->tbits, (n + 31) / 32 * 8};
+    out[k++] = {(void**)&g->tbits, walk_words(g) * 4};
     out[k++] = {(void**)&g->tlast, n * 4};
     out[k++] = {(void**)&g->tpend, n * 4};
     out[k++] = {(void**)&g->tpendSlot, n * 4};
@@ -539,7 +559,7 @@ static int restore_copies(DNgpuVolume* g)
     if (!rc) rc = valloc(g, g->treq, g->ntiles, cs);
     if (!rc) rc = valloc(g, g->tvis, g->ntiles, cs);
     if (!rc) rc = valloc(g, g->ttouch, g->ntiles, cs);
-    if (!rc) rc = valloc(g, g->tbits, (g->ntiles + 31) / 32 * 2, cs);
+    if (!rc) rc = valloc(g, g->tbits, walk_words(g), cs);
     if (!rc) rc = valloc(g, g->tlast, g->ntiles, cs);
     if (!rc) rc = valloc(g, g->tpend, g->ntiles, cs);
     if (!rc) rc = valloc(g, g->tpendSlot, g->ntiles, cs);
@@ -653,14 +673,15 @@ __global__ void __launch_bounds__(128, DN_PACKET_MIN_BLOCKS) k_light_packet(cons
     packet_loop<false>(&a, nullptr, warps[threadIdx.x >> 5]);
 }
 
-// the opaque-chunk marks of one map for a lighting launch with the given materials (mark_opaque_word)
-__global__ void __launch_bounds__(256) k_mark_opaque(uint32_t* tbits, const uint32_t* tword, const ChunkRec* rec,
-                                                     uint64_t nwords, const __grid_constant__ MaterialTable t)
+// the opaque-chunk marks of one map for a lighting launch with the given materials (mark_opaque_cells)
+__global__ void __launch_bounds__(256) k_mark_opaque(const __grid_constant__ DevMap m, uint64_t nwords,
+                                                     const __grid_constant__ MaterialTable t)
 {
     __shared__ uint32_t opq[8];
     opaque_materials(t.m, opq);
-    for (uint64_t wi = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; wi < nwords; wi += (uint64_t)gridDim.x * blockDim.x)
-        mark_opaque_word(tbits, tword, rec, wi, opq);
+    const uint64_t stride = (uint64_t)gridDim.x * (blockDim.x / 32u);
+    for (uint64_t w = (uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u; w < nwords / 2u; w += stride)
+        mark_opaque_cells(m, w, opq);
 }
 
 // The diffuse paths of the voxels k_light_packet lit, as per-lane path streams over the whole request list:
@@ -680,12 +701,11 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a)
     MaterialTable table;                // on the stack: a launch argument, copied at the launch
     memcpy(table.m, a.mats, sizeof(table.m));
     {
-        const uint64_t nwords = (g->ntiles + 15) / 16;
-        const uint64_t blocks = (nwords + 255) / 256;
-        const uint32_t maxBlocks = (uint32_t)(g->numSMs > 0 ? g->numSMs * 4 : 512);
+        const uint64_t nwords = walk_words(g);
+        const uint64_t blocks = (nwords / 2 + 7) / 8;
+        const uint32_t maxBlocks = (uint32_t)(g->numSMs > 0 ? g->numSMs * 8 : 1024);
         COUNT_LAUNCH();
-        k_mark_opaque<<<(uint32_t)(blocks < maxBlocks ? blocks : maxBlocks), 256, 0, g->stream>>>(
-            g->tbits, g->tword, g->rec, nwords, table);
+        k_mark_opaque<<<(uint32_t)(blocks < maxBlocks ? blocks : maxBlocks), 256, 0, g->stream>>>(dev_map(g), nwords, table);
         CK(cudaGetLastError());
     }
     if (g_lightKernel == 2 && a.p.specBounceLimit <= PK_MAX_SPEC_SEGMENTS) {
@@ -853,7 +873,8 @@ __global__ void __launch_bounds__(512) k_pack_stage(const dn_tile_op* ops, uint3
 __global__ void __launch_bounds__(256) k_compact(const __grid_constant__ CompactArgs a)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < a.ntiles; base += stride) compact_tiles(a, base);
+    const uint64_t cells = WalkGrid(a.sx, a.sy, a.sz).cells;
+    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < cells; base += stride) compact_tiles(a, base);
 }
 
 __global__ void k_clamp_requests(DevState* st, uint64_t cap)
@@ -1016,8 +1037,9 @@ static int sync_tiles(DNgpuVolume* g, const dn_sync_params* p)
     a.tword = g->tword; a.tbits = g->tbits; a.treq = g->treq; a.tvis = g->tvis; a.ttouch = g->ttouch; a.tlast = g->tlast;
     a.tpend = g->tpend; a.tpendSlot = g->tpendSlot; a.rec = g->rec;
     a.reqs = g->reqs; a.reqCap = g->reqCap; a.st = g->st; a.ntiles = g->ntiles;
+    a.sx = g->sx; a.sy = g->sy; a.sz = g->sz;
     a.op = p->op; a.split = p->split; a.frameNum = p->frameNum;
-    uint64_t blocks = (g->ntiles + 255) / 256;
+    uint64_t blocks = (WalkGrid(g->sx, g->sy, g->sz).cells + 255) / 256;
     uint32_t maxBlocks = (uint32_t)(g->numSMs > 0 ? g->numSMs * 8 : 1024);
     COUNT_LAUNCH();
     k_compact<<<(uint32_t)(blocks < maxBlocks ? blocks : maxBlocks), 256, 0, g->stream>>>(a);

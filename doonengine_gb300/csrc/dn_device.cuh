@@ -152,7 +152,11 @@ struct DevMap {
     uint32_t sx, sy, sz;
     uint32_t stepCap;                    // D16: cells a traversal segment may visit (step_cap of the size)
     const uint32_t* __restrict__ tword;  // state << 30 | slot
-    const uint32_t* __restrict__ tbits;  // 2 bits per tile: 0 absent, 1 unloaded, 2 loaded
+    // walk grid: 2 bits per chunk cell of the map and of a border one cell thick: 0 absent, 1 unloaded or
+    // border, 2 loaded, 3 loaded and opaque (during lighting).  Cell (x, y, z) is at bit
+    // w0 + 2x + y * w1 + z * w2; a row's border cell also starts the next row, a plane's border row the next plane
+    const uint32_t* __restrict__ tbits;
+    uint32_t w0, w1, w2;
     uint8_t* treq;
     uint8_t* ttouch;
     uint8_t* tvis;

@@ -49,7 +49,7 @@ struct DNgpuVolume {
     uint32_t sx, sy, sz;
     uint64_t ntiles;
     uint32_t* tword; uint8_t* treq; uint8_t* tvis; uint8_t* ttouch;
-    uint32_t* tbits;                    // 2 bits per tile: 0 absent, 1 unloaded, 2 loaded (16 tiles per word)
+    uint32_t* tbits;                    // walk grid (WalkGrid): 2 bits per cell, 16 cells per word
     uint32_t* tlast; uint32_t* tpend; uint32_t* tpendSlot;
     dn::ChunkRec* rec; uint32_t* nsamples; uint32_t slotCap;
     uint2* vox; float4* diff; float4* spec; uint64_t voxCap;
@@ -150,12 +150,29 @@ static inline bool map_evicted(DNgpuVolume* g)
     return false;
 }
 
+// The walk grid of a map: its tiles in rows of sx + 1 cells and planes of sy + 1 rows, with a plane, a row and
+// a cell before the first tile and a plane, a row and a cell behind the last.  The extra cells are the border
+// (state 1): every cell one step outside the map, diagonal steps included, is one of them.
+struct WalkGrid {
+    uint64_t row, plane, first, cells, words;
+    __host__ __device__ WalkGrid(uint32_t sx, uint32_t sy, uint32_t sz)
+    {
+        row = (uint64_t)sx + 1u;
+        plane = row * ((uint64_t)sy + 1u);
+        first = plane + row + 1u;
+        cells = first + plane * ((uint64_t)sz + 1u);
+        words = (cells + 31u) / 32u * 2u;    // a warp writes two words
+    }
+};
+
 static inline dn::DevMap dev_map(const DNgpuVolume* g)
 {
     dn::DevMap m;
     m.sx = g->sx; m.sy = g->sy; m.sz = g->sz;
     const uint64_t cap = 256ull * ((uint64_t)g->sx + g->sy + g->sz) + 4096ull;   // step_cap (dn_device.cuh)
     m.stepCap = cap > (1ull << 23) ? (1u << 23) : (uint32_t)cap;
+    const WalkGrid wg(g->sx, g->sy, g->sz);
+    m.w0 = (uint32_t)(2u * wg.first); m.w1 = (uint32_t)(2u * wg.row); m.w2 = (uint32_t)(2u * wg.plane);
     m.tword = g->tword; m.tbits = g->tbits; m.treq = g->treq; m.ttouch = g->ttouch; m.tvis = g->tvis;
     m.rec = g->rec; m.vox = g->vox; m.diff = g->diff; m.spec = g->spec;
     m.degen = nullptr;                   // set by the launch: the draw's or the lighting's counter
@@ -199,9 +216,20 @@ __device__ __forceinline__ void flush_counters(unsigned long long* stats, const 
     }
 }
 
+// spreads the 16 low bits of x to the even bit positions of a word
+__device__ __forceinline__ uint32_t spread_bits(uint32_t x)
+{
+    x &= 0xFFFFu;
+    x = (x | (x << 8)) & 0x00FF00FFu;
+    x = (x | (x << 4)) & 0x0F0F0F0Fu;
+    x = (x | (x << 2)) & 0x33333333u;
+    x = (x | (x << 1)) & 0x55555555u;
+    return x;
+}
+
 // ------------------------------------------------- opaque chunks of a lighting launch
 
-// The lighting step (seg_step) reads the 2-bit tile map; before each lighting launch a loaded chunk whose
+// The lighting rays (dn_walk.cuh) read the walk grid; before each lighting launch a loaded chunk whose
 // voxels all use materials that are opaque under the launch's materials is marked 3 instead of 2.  A ray
 // that reaches an occupied voxel of such a chunk ends there without reading the voxel's word and material
 // (its pool index is formed when the segment is shaded).  The next sync rewrites the map with 0 / 1 / 2.
@@ -216,22 +244,32 @@ __device__ __forceinline__ void opaque_materials(const dn::Material* mats, uint3
     __syncthreads();
 }
 
-// word wi of the map's 2-bit tile map (16 tiles): every loaded tile to 3 (all materials opaque) or 2
-__device__ __forceinline__ void mark_opaque_word(uint32_t* tbits, const uint32_t* tword, const dn::ChunkRec* rec,
-                                                 uint64_t wi, const uint32_t* opq)
+// Cells [32 * w, 32 * w + 32) of the walk grid, one per lane: every loaded tile to 3 (all its materials
+// opaque) or 2.  A lane per cell: its record's material set is two 16-byte loads, and the warp's votes form the
+// two words.  (One thread per word, 16 tiles and up to 128 dependent loads in a row, took 16 us on any map.)
+__device__ __forceinline__ void mark_opaque_cells(const dn::DevMap& m, uint64_t w, const uint32_t* opq)
 {
-    const uint32_t w = tbits[wi];
-    uint32_t out = w;
-    for (uint32_t k = 0; k < 16; k++) {
-        if (((w >> (2 * k)) & 2u) == 0u) continue;
-        const uint32_t slot = __ldg(&tword[wi * 16 + k]) & dn::SLOT_MASK;
-        const uint32_t* ms = rec[slot].matSet;
-        uint32_t other = 0;
-#pragma unroll
-        for (int j = 0; j < 8; j++) other |= __ldg(&ms[j]) & ~opq[j];
-        out = (out & ~(3u << (2 * k))) | ((other ? 2u : 3u) << (2 * k));
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t* tbits = const_cast<uint32_t*>(m.tbits);
+    const uint2 words = *(const uint2*)&tbits[2u * w];
+    const uint32_t st = ((lane < 16u ? words.x : words.y) >> (2u * (lane & 15u))) & 3u;
+    bool opaque = false;
+    if (st >= 2u) {
+        const uint64_t i = 32u * w + lane - m.w0 / 2u;
+        const uint32_t row = m.w1 / 2u, plane = m.w2 / 2u;
+        const uint32_t z = (uint32_t)i / plane, y = ((uint32_t)i - z * plane) / row, x = (uint32_t)i - z * plane - y * row;
+        const uint32_t slot = __ldg(&m.tword[x + m.sx * (y + m.sy * z)]) & dn::SLOT_MASK;
+        const uint4* ms = (const uint4*)m.rec[slot].matSet;
+        const uint4 a = __ldg(&ms[0]), b = __ldg(&ms[1]);
+        opaque = ((a.x & ~opq[0]) | (a.y & ~opq[1]) | (a.z & ~opq[2]) | (a.w & ~opq[3]) |
+                  (b.x & ~opq[4]) | (b.y & ~opq[5]) | (b.z & ~opq[6]) | (b.w & ~opq[7])) == 0u;
     }
-    if (out != w) tbits[wi] = out;
+    const unsigned b0 = __ballot_sync(0xFFFFFFFFu, (st == 1u) || opaque);
+    const unsigned b1 = __ballot_sync(0xFFFFFFFFu, st >= 2u);
+    if (lane < 2u) {
+        const uint32_t n = (spread_bits(lane ? b0 >> 16 : b0)) | (spread_bits(lane ? b1 >> 16 : b1) << 1);
+        if (n != (lane ? words.y : words.x)) tbits[2u * w + lane] = n;
+    }
 }
 
 // ------------------------------------------------------------------ draw
@@ -428,17 +466,6 @@ __device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Mater
 
 // -------------------------------------------------------------- sync
 
-// spreads the 16 low bits of x to the even bit positions of a word
-__device__ __forceinline__ uint32_t spread_bits(uint32_t x)
-{
-    x &= 0xFFFFu;
-    x = (x | (x << 8)) & 0x00FF00FFu;
-    x = (x | (x << 4)) & 0x0F0F0F0Fu;
-    x = (x | (x << 2)) & 0x33333333u;
-    x = (x | (x << 1)) & 0x55555555u;
-    return x;
-}
-
 struct CompactArgs {
     uint32_t* tword; uint8_t* treq; uint8_t* tvis; uint8_t* ttouch; uint32_t* tlast;
     uint32_t* tbits;
@@ -447,18 +474,28 @@ struct CompactArgs {
     uint32_t* reqs; uint64_t reqCap;
     DevState* st;
     uint64_t ntiles;
+    uint32_t sx, sy, sz;
     uint32_t op, split, frameNum;
 };
 
-// Tiles [base, base + blockDim.x) of one map: the per-tile loop of DN_sync_gpu (voxel.c:738-762) with the
-// request rule of _DN_request_chunk_lighting (1463-1489) and the state machine of _DN_stream_to_gpu
-// (1491-1536).  blockDim.x is a multiple of 32 and base a multiple of 32.
+// Walk-grid cells [base, base + blockDim.x) of one map: for each cell that is a tile, the per-tile loop of
+// DN_sync_gpu (voxel.c:738-762) with the request rule of _DN_request_chunk_lighting (1463-1489) and the state
+// machine of _DN_stream_to_gpu (1491-1536); and the cells' words of the walk grid.  The threads follow the grid
+// and not the tiles, so that a warp's 32 cells are two whole words.  blockDim.x and base are multiples of 32.
 __device__ __forceinline__ void compact_tiles(const CompactArgs& a, uint64_t base)
 {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t t = base + threadIdx.x;
+    const WalkGrid wg(a.sx, a.sy, a.sz);
+    const uint64_t cell = base + threadIdx.x;
+    // tile of the cell; a.ntiles: a border cell or behind the grid
+    uint64_t t = a.ntiles;
+    if (cell >= wg.first && cell < wg.cells) {
+        const uint32_t i = (uint32_t)(cell - wg.first), row = (uint32_t)wg.row, plane = (uint32_t)wg.plane;
+        const uint32_t z = i / plane, y = (i - z * plane) / row, x = i - z * plane - y * row;
+        if (x < a.sx && y < a.sy && z < a.sz) t = (uint64_t)x + (uint64_t)a.sx * (y + (uint64_t)a.sy * z);
+    }
     uint32_t groups = 0;
-    uint32_t finalSt = 0;
+    uint32_t finalSt = 1;
     if (t < a.ntiles) {
         const uint32_t w = a.tword[t];
         const uint32_t st = w >> 30;
@@ -501,12 +538,12 @@ __device__ __forceinline__ void compact_tiles(const CompactArgs& a, uint64_t bas
         a.tvis[t] = (uint8_t)vis;
         a.tlast[t] = lu;
     }
-    // the 2-bit tile map read by the chunk-level DDA step: 32 tiles per warp, two words
+    // 32 cells per warp, two words of the walk grid
     {
         const unsigned b0 = __ballot_sync(0xFFFFFFFFu, finalSt == 1u);
         const unsigned b1 = __ballot_sync(0xFFFFFFFFu, finalSt == 2u);
-        if (lane == 0 && base + threadIdx.x - lane < a.ntiles) {
-            const uint64_t wi = (base + threadIdx.x) >> 4;
+        if (lane == 0 && cell < wg.cells) {
+            const uint64_t wi = cell >> 4;
             a.tbits[wi] = spread_bits(b0 & 0xFFFFu) | (spread_bits(b1 & 0xFFFFu) << 1);
             a.tbits[wi + 1] = spread_bits(b0 >> 16) | (spread_bits(b1 >> 16) << 1);
         }

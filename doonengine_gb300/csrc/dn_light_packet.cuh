@@ -57,11 +57,12 @@ constexpr uint32_t PK_POOL_ALT = PK_POOL_FAN == 64u ? 128u : 64u;   // the batch
 // Work units per request group in a one-map launch: a warp takes 32 / PK_PARTS voxels of a group at a time,
 // so that the launch does not end with a few warps finishing whole groups while the others have left.  Per
 // warp exit times on the large map's frame 11 with whole groups: the last warp left 2.7 ms after 90 % of
-// them had, 16 % of the warps' time idle; units of 16, 8 and 4 voxels measured +8 %, +12 % and +13 %.  A
-// many-map launch keeps whole groups: its queue is long enough that the tail is small, and smaller units
-// measured slower there (the setup of a unit runs on a fraction of the lanes).
+// them had, 16 % of the warps' time idle.  Units of 8 voxels against 4: the 64x32x64 map 14.9 against 15.5 ms
+// per frame, 16x16x16 maps 0.70 against 0.79 (with K = 16 a unit of 4 fills half a pool).  A many-map launch
+// keeps whole groups: its queue is long enough that the tail is small, and smaller units measured slower there
+// (the setup of a unit runs on a fraction of the lanes).
 #ifndef DN_PK_PARTS
-#define DN_PK_PARTS 8
+#define DN_PK_PARTS 4
 #endif
 constexpr uint32_t PK_PARTS = DN_PK_PARTS;
 static_assert(PK_PARTS == 1u || PK_PARTS == 2u || PK_PARTS == 4u || PK_PARTS == 8u,
@@ -189,9 +190,9 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
         const uint32_t perPool = K < POOL ? POOL / K : 1u;
 
         // per-lane ray state
-        Seg s;
-        uint32_t hs = 0, hitIdx = 0;
-        bool live = false, stepping = false;
+        Ray s;
+        s.mode = RM_IDLE;
+        bool live = false;
         uint32_t rid = 0, ncon = 0;       // the lane's ray: index in its fan array; contributions so far
         bool isSpec = false;
         int vi = -1;                      // the ray's voxel
@@ -232,7 +233,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                             jd.jA = pv.talbedo; jd.jB = pv.pos0; jd.jU = tm.reflectType; jd.b = 0; ncon = 0;
                             const f3 P = mk(p.spherePts[kk][0], p.spherePts[kk][1], p.spherePts[kk][2]);
                             const f3 sd = adds(normalize(add(muls(pv.refl, (float)tm.shininess), P)), EPS);
-                            seg_begin(s, pv.pos0, sd, rcp3(sd));
+                            ray_begin(s, m, pv.pos0, sd, rcp3(sd), false, c);
                         } else {
                             // shadow ray: voxels of the pool in slot order, K rays each (1 on the first sample)
                             isSpec = false;
@@ -246,13 +247,11 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                                 if (rid < off + n) { vi = v; kk = ((firstMask >> v) & 1u) ? 64u : rid - off; break; }
                                 off += n;
                             }
-                            seg_begin(s, W.v[vi].pos0, mk(sdir[kk][0], sdir[kk][1], sdir[kk][2]),
-                                      mk(sinv[kk][0], sinv[kk][1], sinv[kk][2]));
+                            ray_begin(s, m, W.v[vi].pos0, mk(sdir[kk][0], sdir[kk][1], sdir[kk][2]),
+                                      mk(sinv[kk][0], sinv[kk][1], sinv[kk][2]), false, c);
                         }
                         c.rays++;
                         live = true;
-                        stepping = true;
-                        hs = 0;
                     }
                     next = (next + (uint32_t)__popc(need)) < total ? next + (uint32_t)__popc(need) : total;
                 }
@@ -261,30 +260,28 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                 // step until 'batch' lanes have an ended segment (or none is left stepping); the live lanes
                 // do not change while stepping, so one vote per step tells both
                 for (;;) {
-                    const unsigned st = __ballot_sync(0xFFFFFFFFu, stepping);
+                    const unsigned st = __ballot_sync(0xFFFFFFFFu, ray_stepping(s));
                     if (!st || (uint32_t)__popc(liveMask & ~st) >= batch) break;
-                    if (stepping) {
-                        const uint32_t rr = seg_step(s, m, mats, p.sunStrength, c, hitIdx);
-                        if (rr) { stepping = false; hs = rr; }
-                    }
+                    if (ray_stepping(s)) walk_round(s, m, mats, p.sunStrength, c);
                 }
                 // shade the ended segments
-                if (!live || stepping) continue;
+                if (!live || ray_stepping(s)) continue;
+                const bool hit = s.mode == RM_HIT;
                 if (isSpec) {
                     // specular_ray body after step_map (voxelLighting.comp:98-144)
                     const PacketVoxel& pv = W.v[vi];
                     bool more = false, add_ = false;
                     f3 sc = mk(0.0f, 0.0f, 0.0f);
-                    if (hs == 1u) {
-                        hit_position(s);
+                    if (hit) {
+                        const f3 hpos = ray_hit_position(s);
                         Voxel hv;
-                        decompress(m, hit_index(s, hitIdx), hv);
-                        const i3 hp{f2i(truncf(s.pos.x)), f2i(truncf(s.pos.y)), f2i(truncf(s.pos.z))};
+                        decompress(m, ray_hit_index(s, m), hv);
+                        const i3 hp{f2i(truncf(hpos.x)), f2i(truncf(hpos.y)), f2i(truncf(hpos.z))};
                         if (in_map(m, hp)) {
                             uint8_t* vp = &m.tvis[map_index(m, hp)];
                             if (*vp == 0) *vp = 1;
                         }
-                        const f3 d = vabs(sub(vfloor(muls(s.pos, 8.0f)), vfloor(muls(jd.jB, 8.0f))));
+                        const f3 d = vabs(sub(vfloor(muls(hpos, 8.0f)), vfloor(muls(jd.jB, 8.0f))));
                         if (!(dot(d, d) <= 1.0f)) {
                             const Material& hm = mats[hv.material];
                             const f3 hd = muls(hv.diff, 1.0f - hm.specular);
@@ -303,13 +300,11 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                                     jd.jA.y = jd.jA.y * (hv.albedo.y * s.cmul * hm.specular);
                                     jd.jA.z = jd.jA.z * (hv.albedo.z * s.cmul * hm.specular);
                                     jd.jU = hm.reflectType;
-                                    jd.jB = s.pos;
+                                    jd.jB = hpos;
                                     const f3 nd = reflect(s.dir, hv.normal);
                                     jd.b++;
                                     if (jd.b < p.specBounceLimit) {
-                                        const TState keep = s.ts;
-                                        seg_begin(s, s.pos, nd, rcp3(nd));
-                                        s.ts = keep;   // one ray job: bounces keep the transparency state
+                                        ray_begin(s, m, hpos, nd, rcp3(nd), true, c);
                                         c.rays++;
                                         more = true;
                                     }
@@ -333,17 +328,13 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                         W.con[rid][ncon][0] = sc.x; W.con[rid][ncon][1] = sc.y; W.con[rid][ncon][2] = sc.z;
                         ncon++;
                     }
-                    hs = 0;
-                    if (more) stepping = true;
-                    else { W.ncon[rid] = (uint8_t)ncon; live = false; }
+                    if (!more) { W.ncon[rid] = (uint8_t)ncon; live = false; }
                 } else {
                     // shadow_ray: an unoccluded ray adds sunStrength * colorMult + colorAdd
-                    const bool miss = hs == 2u;
                     W.sh[rid][0] = sun.x * s.cmul + s.cadd.x;
                     W.sh[rid][1] = sun.y * s.cmul + s.cadd.y;
                     W.sh[rid][2] = sun.z * s.cmul + s.cadd.z;
-                    W.shHas[rid] = miss ? 1 : 0;
-                    hs = 0;
+                    W.shHas[rid] = hit ? 0 : 1;
                     live = false;
                 }
             }

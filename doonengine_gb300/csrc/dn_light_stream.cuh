@@ -7,10 +7,9 @@
  *   light rays (K fixed shadow rays, or one along the sun on the first
  *   sample), then numDiffuse diffuse paths (each up to diffuseBounceLimit
  *   segments), then the running average and the write-out.
- * All lanes share one loop whose body is one traversal step of each lane's
- * current ray segment (seg_step: the two-level DDA flattened into one loop), so lanes
- * on different rays, different jobs or different voxels still execute
- * together.  When a segment ends, the lane waits; the per-segment work
+ * All lanes share one loop whose body is one round of each lane's current ray
+ * segment (walk_round, dn_walk.cuh), so lanes on different rays, different jobs
+ * or different voxels still execute together.  When a segment ends, the lane waits; the per-segment work
  * (shading the finished segment, choosing and setting up the next one,
  * finishing a voxel, fetching the next voxel) runs for all waiting lanes at
  * once when at least `batch` lanes wait (or no lane is still stepping).
@@ -21,7 +20,7 @@
  * 32 voxels.
  */
 #pragma once
-#include "dn_device.cuh"
+#include "dn_walk.cuh"
 
 namespace dn {
 
@@ -57,193 +56,7 @@ struct LightTables {
     float sinv[65][3];
 };
 
-// traversal state of one ray segment (flattened two-level DDA, refraction off).  Both levels step with
-// the same delta and step signs, so one set of DDA registers (cpos, cside, clastMin) holds the level being
-// walked; entering a chunk saves the chunk-level registers (opos, oside, olastMin) and leaving restores
-// them.  The reference keeps the side distances before the last step as a vector (lastSideDist) but only
-// ever uses its minimum (voxelShared.comp:338, 445), so that minimum is kept instead, formed in the same
-// order (min3).
-struct Seg {
-    f3 pos, dir, inv;
-    i3 cpos, opos, step;
-    f3 cside, oside, cp;
-    float clastMin, olastMin;
-    const ChunkRec* rec;
-    uint32_t flags;      // bit0 inner level, bit1 ignore (current level), bit2 saved outer ignore, bit3 requested,
-                         // bit4 degenerate direction (D16), bit5 the current chunk's materials are all opaque,
-                         // bit6 the segment ended on a voxel of such a chunk (hitIdx holds its local index),
-                         // bit7 the segment ended on a voxel and pos is not yet its hit position,
-                         // bits 8-31 cells visited by the segment (D16 cell cap)
-    f3 cadd;
-    float cmul;
-    TState ts;
-};
-
-__device__ __forceinline__ void seg_begin(Seg& s, f3 pos, f3 dir, f3 inv)
-{
-    // step_map's set-up (voxelShared.comp:421-433) with first voxel ignored
-    s.pos = pos; s.dir = dir; s.inv = inv;
-    s.cadd = mk(0.0f, 0.0f, 0.0f);
-    s.cmul = 1.0f;
-    s.ts.lastVoxID = 255u; s.ts.lastVoxRefract = 1.0f;   // D13: fresh per ray job (spec / diffuse bounces keep it)
-    f3 delta;
-    init_dda(dir, inv, pos, s.cpos, delta, s.step, s.cside);
-    s.clastMin = 0.0f;   // min3 of the zero vector
-    s.flags = 2u;        // ignore the first voxel
-    // D16: a zero or NaN direction component traverses nothing; the first step ends the segment as a miss
-    // (a position outside the map) and counts it
-    if (!finite_dir(inv)) { s.cpos.x = -1; s.flags = 2u | 16u; }
-}
-
-// Enters the loaded chunk of chunk cell idx (tile state cst >= 2) from the chunk level
-// (voxelShared.comp:441-449): saves the chunk-level DDA state and starts the voxel-level DDA at the entry point.
-__device__ __forceinline__ void seg_enter(Seg& s, const DevMap& m, Counters& c, uint32_t idx, uint32_t cst, f3 delta,
-                                          i3 step)
-{
-    c.outer++;
-    c.entered++;
-    if (m.ttouch[idx] == 0) m.ttouch[idx] = 1;
-    const float tt = s.clastMin - EPS;
-    const f3 up = add(s.pos, muls(s.dir, tt));
-    f3 cp = mk((up.x - (float)s.cpos.x) * 8.0f, (up.y - (float)s.cpos.y) * 8.0f, (up.z - (float)s.cpos.z) * 8.0f);
-    const float lo = EPS, hi_ = 8.0f - EPS;
-    // cp is finite here (a finite origin and direction, D16), so fminf / fmaxf give GLSL clamp's values and
-    // the floors below are 0..7: a plain conversion, and fl itself for (float)cpos
-    cp.x = fminf(fmaxf(cp.x, lo), hi_); cp.y = fminf(fmaxf(cp.y, lo), hi_); cp.z = fminf(fmaxf(cp.z, lo), hi_);
-    s.cp = cp;
-    s.opos = s.cpos; s.oside = s.cside; s.olastMin = s.clastMin;
-    const f3 fl = vfloor(cp);
-    s.cpos.x = (int32_t)fl.x; s.cpos.y = (int32_t)fl.y; s.cpos.z = (int32_t)fl.z;
-    const f3 sg = mk((float)step.x, (float)step.y, (float)step.z);
-    s.cside.x = (sg.x * (fl.x - cp.x) + sg.x * 0.5f + 0.5f) * delta.x;
-    s.cside.y = (sg.y * (fl.y - cp.y) + sg.y * 0.5f + 0.5f) * delta.y;
-    s.cside.z = (sg.z * (fl.z - cp.z) + sg.z * 0.5f + 0.5f) * delta.z;
-    s.clastMin = 0.0f;
-    s.rec = &m.rec[__ldg(&m.tword[idx]) & SLOT_MASK];
-    // inner level; the chunk inherits ignoreFirst; bit5: the chunk is marked opaque
-    s.flags = (s.flags & ~(4u | 32u)) | 1u | ((s.flags & 2u) << 1) | (cst == 3u ? 32u : 0u);
-}
-
-// Advances one traversal step.  Returns 0 while the segment continues, 1 on an opaque hit (hit_position()
-// moves s.pos to the hit; hitIdx = pool index of the voxel, or its local index in s.rec when flags bit 6 is
-// set -- hit_index() gives the pool index), 2 when it leaves the map.  The common case (a chunk cell that is not loaded, or a
-// voxel cell that is empty) runs one code path for both levels; entering a chunk, leaving it, reaching a voxel
-// and leaving the map are the divergent events.  In a chunk marked 3 in the tile map (every material of its
-// voxels opaque under the launch's materials, mark_opaque_word) the first occupied voxel ends the ray without
-// its word, rank or material being read: the reference would find it opaque (voxelShared.comp:360-364).
-__device__ __forceinline__ uint32_t seg_step(Seg& s, const DevMap& m, const Material* mats, const float* sunStrength,
-                                             Counters& c, uint32_t& hitIdx)
-{
-    const f3 delta = vabs(s.inv);
-    const i3 step = s.step;
-    const bool inner = (s.flags & 1u) != 0u;
-    const uint32_t bx = inner ? 8u : m.sx, by = inner ? 8u : m.sy, bz = inner ? 8u : m.sz;
-    const bool inb = (uint32_t)s.cpos.x < bx && (uint32_t)s.cpos.y < by && (uint32_t)s.cpos.z < bz;
-    // D16: every visited cell (each outer or inner iteration of step_map / step_chunk) counts; a segment
-    // that reached the cap ends as a miss
-    if (inb) {
-        if (s.flags >= (m.stepCap << 8)) return 2u;   // (flags >> 8) >= stepCap: the low byte holds state bits
-        s.flags += 256u;
-    }
-    const uint32_t idx = (uint32_t)s.cpos.x + bx * ((uint32_t)s.cpos.y + by * (uint32_t)s.cpos.z);
-    uint32_t w = 0;
-    if (inb) w = __ldg(inner ? &s.rec->mask[idx >> 5] : &m.tbits[idx >> 4]);
-    // chunk level: 2-bit state (0 absent, 1 unloaded, 2 loaded); voxel level: occupancy bit -- one shift
-    // brings either to the low bits (cst is only read at the chunk level)
-    const uint32_t bits = w >> (inner ? (idx & 31u) : ((idx & 15u) << 1));
-    const uint32_t cst = bits & 3u;
-    const bool occ = inb && (inner ? (((bits & 1u) != 0u) && !(s.flags & 2u)) : (cst >= 2u));
-    if (!inb || occ) {
-        if (!inner) {
-            if (!inb) {
-                if (s.flags & 16u) count_degenerate(m);
-                return 2u;
-            }
-            seg_enter(s, m, c, idx, cst, delta, step);
-            return 0u;
-        }
-        if (!inb) {
-            // the chunk was crossed without a hit: back to the chunk level, which then iterates
-            s.cpos = s.opos; s.cside = s.oside; s.clastMin = s.olastMin;
-            s.flags = (s.flags & ~3u) | ((s.flags >> 1) & 2u);
-        } else {
-            c.inner++;
-            c.hits++;
-            if (s.flags & 32u) {
-                hitIdx = idx;
-                s.flags |= 64u | 128u;   // the hit position is formed when shading needs it (hit_position)
-                return 1u;
-            }
-            const uint32_t vi = __ldg(&s.rec->voxBase) + vox_rank(s.rec, idx);
-            const uint2 vw = __ldg(&m.vox[vi]);
-            const uint32_t material = vw.x >> 24;
-            const Material& mat = mats[material];
-            if (mat.opacity == 1.0f) {
-                hitIdx = vi;
-                s.flags |= 128u;
-                return 1u;
-            }
-            const uint32_t thisID = (vw.y & 0xFFFFFF00u) | material;
-            if (s.ts.lastVoxID != thisID) {
-                const f3 alb = mk((float)((vw.y >> 24) & 0xFF) * INV255, (float)((vw.y >> 16) & 0xFF) * INV255,
-                                  (float)((vw.y >> 8) & 0xFF) * INV255);
-                const float k = s.cmul * mat.opacity;
-                s.cadd.x = s.cadd.x + k * alb.x * sunStrength[0];
-                s.cadd.y = s.cadd.y + k * alb.y * sunStrength[1];
-                s.cadd.z = s.cadd.z + k * alb.z * sunStrength[2];
-                s.cmul = s.cmul * (1.0f - mat.opacity);
-                s.ts.lastVoxID = thisID;
-                s.ts.lastVoxRefract = mat.refractIndex;
-            }
-        }
-    } else {
-        // an empty cell, either level, without branches: the counters, and at the voxel level the end of a
-        // run of transparent voxels (lastVoxID 255 always comes with refract 1, so writing both is the
-        // reference's reset); an unloaded chunk cell requests its chunk once per ray
-        c.inner += inner ? 1u : 0u;
-        c.outer += inner ? 0u : 1u;
-        s.ts.lastVoxID = inner ? 255u : s.ts.lastVoxID;
-        s.ts.lastVoxRefract = inner ? 1.0f : s.ts.lastVoxRefract;
-        if (!inner && !(s.flags & 8u) && cst != 0u) {
-            if (m.treq[idx] == 0) m.treq[idx] = 1;
-            s.flags |= 8u;
-        }
-    }
-    // iterate_DDA on the current level (voxelShared.comp:309-317).  With a finite direction (D16) every side
-    // distance is finite and non-negative (never -0), so fminf gives GLSL min's value (y < x ? y : x) and
-    // adding delta only on the stepped axes gives exactly side + (mask ? 1 : 0) * delta.
-    const float gyz = fminf(s.cside.y, s.cside.z), gzx = fminf(s.cside.z, s.cside.x), gxy = fminf(s.cside.x, s.cside.y);
-    s.clastMin = fminf(gxy, s.cside.z);   // min3(lastSideDist) of the next step
-    const bool mx = s.cside.x <= gyz;
-    const bool my = s.cside.y <= gzx;
-    const bool mz = s.cside.z <= gxy;
-    if (mx) s.cside.x = s.cside.x + delta.x;
-    if (my) s.cside.y = s.cside.y + delta.y;
-    if (mz) s.cside.z = s.cside.z + delta.z;
-    s.cpos.x += (int32_t)mx * step.x; s.cpos.y += (int32_t)my * step.y; s.cpos.z += (int32_t)mz * step.z;
-    s.flags &= ~2u;
-    return 0u;
-}
-
 __device__ __forceinline__ f3 rcp3(f3 d) { return mk(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z)); }
-
-// the pool index of the voxel a segment ended on (seg_step's hitIdx)
-__device__ __forceinline__ uint32_t hit_index(const Seg& s, uint32_t hitIdx)
-{
-    return (s.flags & 64u) ? __ldg(&s.rec->voxBase) + vox_rank(s.rec, hitIdx) : hitIdx;
-}
-
-// the hit position of a segment that ended on a voxel (voxelShared.comp:362-364), formed when shading needs
-// it: shadow rays never do.  The segment's state is unchanged since the hit.
-__device__ __forceinline__ void hit_position(Seg& s)
-{
-    if (s.flags & 128u) {
-        const float t = s.clastMin + EPS;
-        const f3 cp = add(s.cp, muls(s.dir, t));
-        s.pos = add(mk((float)s.opos.x, (float)s.opos.y, (float)s.opos.z), muls(cp, INV_CHUNK));
-        s.flags &= ~128u;
-    }
-}
 
 // per-lane job state of the voxel being lit
 struct Job {
@@ -303,31 +116,34 @@ __device__ __forceinline__ f3 diffuse_dir(const Job& j, const dn_light_params& p
 // which left the direct light in the diffuse output slot); the final write replaces that slot with the
 // voxel's new diffuse lighting and leaves the specular slot and the lit-voxel count alone.
 template <bool DIFFONLY = false>
-__device__ __forceinline__ bool advance(Job& j, Seg& s, uint32_t& hitState, uint32_t hitIdx, const DevMap& m,
-                                        const dn_light_params& p, const Material* mats, const float (*sdir)[3],
-                                        const float (*sinv)[3], float4* out, Counters& c, uint32_t& lit)
+__device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const dn_light_params& p,
+                                        const Material* mats, const float (*sdir)[3], const float (*sinv)[3],
+                                        float4* out, Counters& c, uint32_t& lit)
 {
     const bool rngSin = p.rngMode == 1u;
     const f3 sun = mk(p.sunStrength[0], p.sunStrength[1], p.sunStrength[2]);
     const f3 sunDir = mk(p.sunDir[0], p.sunDir[1], p.sunDir[2]);
-    if (hitState) {
-        const bool hit = hitState == 1u;
-        hitState = 0;
+    if (s.mode == RM_HIT || s.mode == RM_MISS) {
+        const bool hit = s.mode == RM_HIT;
+        s.mode = RM_IDLE;
         Voxel hv;
-        if (hit) hit_position(s);
-        if (hit) decompress(m, hit_index(s, hitIdx), hv);
+        f3 hpos = s.pos;
+        if (hit) {
+            hpos = ray_hit_position(s);
+            decompress(m, ray_hit_index(s, m), hv);
+        }
         // the diffuse-only kernel's jobs never reach the specular and shadow phases: with DIFFONLY their
         // code is left out of it (a smaller kernel: fewer instruction-fetch stalls)
         if (!DIFFONLY && j.phase == PH_SPEC) {
             // specular_ray body after step_map (voxelLighting.comp:98-144)
             bool done = true;
             if (hit) {
-                const i3 hp{f2i(truncf(s.pos.x)), f2i(truncf(s.pos.y)), f2i(truncf(s.pos.z))};
+                const i3 hp{f2i(truncf(hpos.x)), f2i(truncf(hpos.y)), f2i(truncf(hpos.z))};
                 if (in_map(m, hp)) {
                     uint8_t* vp = &m.tvis[map_index(m, hp)];
                     if (*vp == 0) *vp = 1;
                 }
-                const f3 d = vabs(sub(vfloor(muls(s.pos, 8.0f)), vfloor(muls(j.jB, 8.0f))));
+                const f3 d = vabs(sub(vfloor(muls(hpos, 8.0f)), vfloor(muls(j.jB, 8.0f))));
                 if (!(dot(d, d) <= 1.0f)) {
                     const Material& hm = mats[hv.material];
                     const f3 hd = muls(hv.diff, 1.0f - hm.specular);
@@ -345,13 +161,11 @@ __device__ __forceinline__ bool advance(Job& j, Seg& s, uint32_t& hitState, uint
                             j.jA.y = j.jA.y * (hv.albedo.y * s.cmul * hm.specular);
                             j.jA.z = j.jA.z * (hv.albedo.z * s.cmul * hm.specular);
                             j.jU = hm.reflectType;
-                            j.jB = s.pos;
+                            j.jB = hpos;
                             const f3 nd = reflect(s.dir, hv.normal);
                             j.b++;
                             if (j.b < p.specBounceLimit) {
-                                const TState keep = s.ts;
-                                seg_begin(s, s.pos, nd, rcp3(nd));   // next bounce
-                                s.ts = keep;      // one ray job: bounces keep the transparency state
+                                ray_begin(s, m, hpos, nd, rcp3(nd), true, c);   // next bounce
                                 c.rays++;
                                 return true;
                             }
@@ -383,7 +197,7 @@ __device__ __forceinline__ bool advance(Job& j, Seg& s, uint32_t& hitState, uint
             if (hit) {
                 j.jB = hv.normal;
                 j.jU = hv.material;
-                const f3 d = vabs(sub(vfloor(muls(j.pos0, 8.0f)), vfloor(muls(s.pos, 8.0f))));
+                const f3 d = vabs(sub(vfloor(muls(j.pos0, 8.0f)), vfloor(muls(hpos, 8.0f))));
                 if (!(dot(d, d) < 1.0f)) {
                     const Material& hm = mats[hv.material];
                     if (hm.emissive) {
@@ -398,9 +212,7 @@ __device__ __forceinline__ bool advance(Job& j, Seg& s, uint32_t& hitState, uint
                         j.b++;
                         if (j.b < p.diffuseBounceLimit) {
                             const f3 nd = diffuse_dir(j, p, mats, rngSin);
-                            const TState keep = s.ts;
-                            seg_begin(s, s.pos, nd, rcp3(nd));
-                            s.ts = keep;
+                            ray_begin(s, m, hpos, nd, rcp3(nd), true, c);
                             c.rays++;
                             return true;
                         }
@@ -424,7 +236,7 @@ __device__ __forceinline__ bool advance(Job& j, Seg& s, uint32_t& hitState, uint
                 j.b = 0; j.jA = j.talbedo; j.jB = j.pos0; j.jU = tm.reflectType;
                 const f3 P = mk(p.spherePts[j.k][0], p.spherePts[j.k][1], p.spherePts[j.k][2]);
                 const f3 sd = adds(normalize(add(muls(j.refl, (float)tm.shininess), P)), EPS);
-                seg_begin(s, j.pos0, sd, rcp3(sd));
+                ray_begin(s, m, j.pos0, sd, rcp3(sd), false, c);
                 c.rays++;
                 return true;
             }
@@ -437,7 +249,7 @@ __device__ __forceinline__ bool advance(Job& j, Seg& s, uint32_t& hitState, uint
             const uint32_t n = j.firstSample ? 1u : p.K;
             if (j.k < n) {
                 const uint32_t q = j.firstSample ? 64u : j.k;
-                seg_begin(s, j.pos0, mk(sdir[q][0], sdir[q][1], sdir[q][2]), mk(sinv[q][0], sinv[q][1], sinv[q][2]));
+                ray_begin(s, m, j.pos0, mk(sdir[q][0], sdir[q][1], sdir[q][2]), mk(sinv[q][0], sinv[q][1], sinv[q][2]), false, c);
                 c.rays++;
                 return true;
             }
@@ -459,7 +271,7 @@ __device__ __forceinline__ bool advance(Job& j, Seg& s, uint32_t& hitState, uint
                     j.jU = j.tmat;
                 }
                 const f3 nd = diffuse_dir(j, p, mats, rngSin);
-                seg_begin(s, j.pos0, nd, rcp3(nd));
+                ray_begin(s, m, j.pos0, nd, rcp3(nd), false, c);
                 c.rays++;
                 return true;
             }
@@ -625,14 +437,13 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
         else if constexpr (DIFFONLY) return one->gtab->mats;
         else return sh->mats;
     };
-    Seg s;
-    bool rayActive = false;
-    uint32_t hitState = 0, hitIdx = 0;
+    Ray s;
+    s.mode = RM_IDLE;
     Counters c{0, 0, 0, 0, 0};
     uint32_t lit = 0;
     while (true) {
-        const unsigned waiting = __ballot_sync(0xFFFFFFFFu, !rayActive && j.phase != PH_DONE);
-        const unsigned stepping = __ballot_sync(0xFFFFFFFFu, rayActive);
+        const unsigned waiting = __ballot_sync(0xFFFFFFFFu, !ray_stepping(s) && j.phase != PH_DONE);
+        const unsigned stepping = __ballot_sync(0xFFFFFFFFu, ray_stepping(s));
         if (waiting == 0u && stepping == 0u) break;
         if (stepping == 0u || (uint32_t)__popc(waiting) >= batch) {
             for (int round = 0; round < 4; round++) {
@@ -679,25 +490,20 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
                     winNext += took;
                 }
                 // shade the finished segment and set up the next one (or finish the voxel)
-                if (!rayActive && j.phase != PH_DONE && j.phase != PH_FETCH) {
+                if (!ray_stepping(s) && j.phase != PH_DONE && j.phase != PH_FETCH) {
                     if constexpr (MANY) {
                         if (j.map != lmi) { le = &many->maps[j.map]; lmi = j.map; }
-                        rayActive = advance<DIFFONLY>(j, s, hitState, hitIdx, le->m, le->p, le->mats, le->sdir, le->sinv, le->out,
-                                                      c, lit);
+                        advance<DIFFONLY>(j, s, le->m, le->p, le->mats, le->sdir, le->sinv, le->out, c, lit);
                     } else if constexpr (DIFFONLY) {
-                        rayActive = advance<true>(j, s, hitState, hitIdx, one->m, one->p, MATS(), one->gtab->sdir,
-                                                  one->gtab->sinv, one->out, c, lit);
+                        advance<true>(j, s, one->m, one->p, MATS(), one->gtab->sdir, one->gtab->sinv, one->out, c, lit);
                     } else {
-                        rayActive = advance(j, s, hitState, hitIdx, one->m, one->p, sh->mats, sh->sdir, sh->sinv, one->out, c, lit);
+                        advance(j, s, one->m, one->p, sh->mats, sh->sdir, sh->sinv, one->out, c, lit);
                     }
                 }
                 if (__ballot_sync(0xFFFFFFFFu, j.phase == PH_FETCH) == 0u) break;
             }
         }
-        if (rayActive) {
-            const uint32_t r = seg_step(s, M(), MATS(), P().sunStrength, c, hitIdx);
-            if (r) { rayActive = false; hitState = r; }
-        }
+        if (ray_stepping(s)) walk_round(s, M(), MATS(), P().sunStrength, c);
     }
     flush_counters(MANY ? many->stats : one->stats, c, 0, lit);
 }

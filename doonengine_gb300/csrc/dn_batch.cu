@@ -60,7 +60,7 @@ struct DNgpuBatch {
     // the lighting launch of the last frame (autotuning re-runs it) and the generations of its maps
     BatchLightArgs lastLight;
     bool lastLightValid;
-    bool lastPackets;
+    bool lastPackets, lastFar;
     std::vector<std::pair<DNgpuVolume*, uint64_t>> lastLightGens;
 };
 
@@ -83,18 +83,16 @@ __global__ void k_batch_reset(const CompactArgs* s, uint32_t ns)
     if (i < ns) s[i].st->w[ST_REQ] = 0;
 }
 
+template <bool FAR>
 __global__ void __launch_bounds__(256, DN_DRAW_MIN_BLOCKS) k_draw_batch(const BatchDrawEntry* d, const uint32_t* start, uint32_t nd,
                                                     unsigned long long* stats)
 {
-    __shared__ Material smat[256];
     const uint32_t mi = find_range(start, nd, blockIdx.x);
     const BatchDrawEntry& e = d[mi];
-    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 256; i += blockDim.x * blockDim.y) smat[i] = e.mats[i];
-    __syncthreads();
     const uint32_t local = blockIdx.x - start[mi];
     const uint32_t bx = local % e.gridX, by = local / e.gridX;
     Counters c;
-    const uint32_t primary = draw_pixel(e.d, smat, bx * blockDim.x + threadIdx.x, by * blockDim.y + threadIdx.y, c);
+    const uint32_t primary = draw_pixel<FAR>(e.d, e.mats, bx * blockDim.x + threadIdx.x, by * blockDim.y + threadIdx.y, c);
     flush_counters(stats, c, primary, 0);
 }
 
@@ -148,10 +146,11 @@ __global__ void k_batch_prep(BatchLightMap* l, uint32_t nl, const CompactArgs* s
     if (threadIdx.x == 0) reqStart[nl] = carry;
 }
 
+template <bool FAR>
 __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream_batch(const __grid_constant__ BatchLightArgs a)
 {
     __shared__ Job jobs[128];
-    stream_loop<true>(nullptr, &a, nullptr, jobs[threadIdx.x]);
+    stream_loop<true, false, FAR>(nullptr, &a, nullptr, jobs[threadIdx.x]);
 }
 
 // POOL: rays per fan kind per pool (the rays a warp pulls from a request group at a time); the autotuner
@@ -180,7 +179,7 @@ __global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* 
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse_batch(const __grid_constant__ BatchLightArgs a)
 {
     __shared__ Job jobs[128];
-    stream_loop<true, true>(nullptr, &a, nullptr, jobs[threadIdx.x]);
+    stream_loop<true, true, false>(nullptr, &a, nullptr, jobs[threadIdx.x]);
 }
 
 __global__ void k_commit_batch(const BatchLightMap* l, const uint32_t* reqStart, uint32_t nl)
@@ -228,7 +227,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     b->tuning.streamBatch = b->tuning.kernel == 2u ? g_packetBatch : g_streamBatch;
     b->tuning.blocksPerSM = DN_STREAM_MIN_BLOCKS; b->tuning.useGraph = 1;
     b->tuning.poolRays = PK_POOL_FAN; b->tuning.diffuseBatch = g_streamBatch;
-    b->lastPackets = false;
+    b->lastPackets = b->lastFar = false;
     b->graph = nullptr;
     b->lastLightValid = false;
     int rc = DN_CUDA_OK;
@@ -252,7 +251,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     }
     if (!rc) {
         int perSM = 0, perSM2 = 0, perSM3 = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_stream_batch, 128, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_stream_batch<false>, 128, 0);
         int perSMAlt = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM2, k_light_packet_batch<PK_POOL_FAN>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMAlt, k_light_packet_batch<PK_POOL_ALT>, 128, 0);
@@ -354,10 +353,11 @@ struct FramePlan {
     uint32_t drawBlocks, syncBlocks;
     bool hostImages;
     bool packets;               // lighting as warp packets (dn_light_packet.cuh)
+    bool far;                   // a map of the frame is far: the kernels' FAR forms, ray streams for lighting
 };
 
 // packets: the lighting kernel of dn_light_packet.cuh (every map's specBounceLimit within its limit)
-static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, bool packets)
+static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, bool packets, bool far)
 {
     COUNT_LAUNCH();
     k_mark_opaque_batch<<<la.nmaps * MARK_BLOCKS, 256, 0, s>>>(la.maps);
@@ -366,7 +366,8 @@ static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, 
     const unsigned grid = (unsigned)(g_numSMs * (int)b->tuning.blocksPerSM);
     if (packets && b->tuning.poolRays == PK_POOL_ALT) k_light_packet_batch<PK_POOL_ALT><<<grid, 128, 0, s>>>(la);
     else if (packets) k_light_packet_batch<PK_POOL_FAN><<<grid, 128, 0, s>>>(la);
-    else k_light_stream_batch<<<grid, 128, 0, s>>>(la);
+    else if (far) k_light_stream_batch<true><<<grid, 128, 0, s>>>(la);
+    else k_light_stream_batch<false><<<grid, 128, 0, s>>>(la);
     CK(cudaGetLastError());
     if (packets) {
         // the diffuse paths: a second pass over the same queue
@@ -398,8 +399,10 @@ static int issue_frame(DNgpuBatch* b, const dn_batch_item* items, uint32_t n, co
     }
     if (t.nd) {
         COUNT_LAUNCH();
-        k_draw_batch<<<f.drawBlocks, dim3(8, 32), 0, s>>>((const BatchDrawEntry*)(d + t.oDraw),
-                                                         (const uint32_t*)(d + t.oDrawStart), t.nd, b->bst->stats);
+        const BatchDrawEntry* de = (const BatchDrawEntry*)(d + t.oDraw);
+        const uint32_t* ds = (const uint32_t*)(d + t.oDrawStart);
+        if (f.far) k_draw_batch<true><<<f.drawBlocks, dim3(8, 32), 0, s>>>(de, ds, t.nd, b->bst->stats);
+        else k_draw_batch<false><<<f.drawBlocks, dim3(8, 32), 0, s>>>(de, ds, t.nd, b->bst->stats);
         CK(cudaGetLastError());
     }
     if (f.hostImages) {
@@ -436,7 +439,7 @@ static int issue_frame(DNgpuBatch* b, const dn_batch_item* items, uint32_t n, co
         la.workCounter = b->workCounter;
         la.stats = b->bst->lstats;
         la.batch = b->tuning.streamBatch;
-        int rc = issue_light(b, la, s, f.packets);
+        int rc = issue_light(b, la, s, f.packets, f.far);
         if (rc) return rc;
         COUNT_LAUNCH();
         k_commit_batch<<<(unsigned)(g_numSMs * 4), 256, 0, s>>>(la.maps, la.reqStart, t.nl);
@@ -504,8 +507,11 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
     uint32_t maxSpec = 0;
     for (uint32_t i = 0; i < n; i++)
         if ((items[i].phases & DN_BATCH_LIGHT) && items[i].light.specBounceLimit > maxSpec) maxSpec = items[i].light.specBounceLimit;
-    f.packets = b->tuning.kernel == 2u && maxSpec <= PK_MAX_SPEC_SEGMENTS;
+    f.far = false;
+    for (uint32_t i = 0; i < n; i++) f.far = f.far || map_far(items[i].map);
+    f.packets = b->tuning.kernel == 2u && maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far;
     b->lastPackets = f.packets;
+    b->lastFar = f.far;
     if (f.t.size > b->tabCap) {
         // growing waits for the stream, frees pinned memory (which waits for the device) and renews the
         // graph, a stall of up to two frames: the first table is large enough for about 370 maps per frame
@@ -753,8 +759,8 @@ extern "C" int dn_cuda_batch_autotune(DNgpuBatch* b, dn_batch_tuning* chosen)
     }
     const dn_batch_tuning keep = b->tuning;
     dn_batch_tuning best = keep;
-    // packets were possible in the last frame only if every lit map's specBounceLimit allowed them
-    const bool packetsOk = b->lastPackets || keep.kernel != 2u;
+    // packets were possible in the last frame only if every lit map's specBounceLimit allowed them and no map is far
+    const bool packetsOk = b->lastPackets || (keep.kernel != 2u && !b->lastFar);
     float bestMs = 3.4e38f;
     int rc = DN_CUDA_OK;
     // times the last frame's lighting launch under tuning t (best of two runs)
@@ -767,7 +773,7 @@ extern "C" int dn_cuda_batch_autotune(DNgpuBatch* b, dn_batch_tuning* chosen)
             cudaError_t e = cudaMemsetAsync(b->workCounter, 0, 4, b->stream);
             if (e == cudaSuccess) e = cudaEventRecord(e0, b->stream);
             if (e != cudaSuccess) { rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "autotune: %s", cudaGetErrorString(e)); break; }
-            rc = issue_light(b, la, b->stream, t.kernel == 2u && packetsOk);
+            rc = issue_light(b, la, b->stream, t.kernel == 2u && packetsOk, b->lastFar);
             if (rc) break;
             e = cudaEventRecord(e1, b->stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);

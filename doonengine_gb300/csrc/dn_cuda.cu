@@ -629,19 +629,18 @@ extern "C" int dn_cuda_reserve(DNgpuVolume* g, uint32_t slotCap, uint64_t voxelC
 
 // ------------------------------------------------------------------ draw
 
+template <bool FAR>
 __global__ void __launch_bounds__(256, DN_DRAW_MIN_BLOCKS) k_draw(const __grid_constant__ DrawArgs a)
 {
-    __shared__ Material smat[256];
-    for (int i = threadIdx.x + threadIdx.y * blockDim.x; i < 256; i += blockDim.x * blockDim.y) smat[i] = a.mats[i];
-    __syncthreads();
     Counters c;
-    const uint32_t primary = draw_pixel(a.d, smat, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, c);
+    const uint32_t primary = draw_pixel<FAR>(a.d, a.mats, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, c);
     flush_counters(a.d.stats, c, primary, 0);
 }
 
 // -------------------------------------------------------------- lighting
 
 // The lighting launch as persistent per-lane ray streams (dn_light_stream.cuh).
+template <bool FAR>
 __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream(const __grid_constant__ StreamArgs a)
 {
     __shared__ StreamShared sh;
@@ -651,7 +650,7 @@ __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream(cons
     // shadow directions are identical for every voxel of the launch
     for (int k = threadIdx.x; k < 65; k += blockDim.x) shadow_dir(a.p, k, sh.sdir[k], sh.sinv[k]);
     __syncthreads();
-    stream_loop<false>(&a, nullptr, &sh, jobs[threadIdx.x]);
+    stream_loop<false, false, FAR>(&a, nullptr, &sh, jobs[threadIdx.x]);
 }
 
 // The lighting launch with specular and shadow fans traced as warp packets (dn_light_packet.cuh).
@@ -689,12 +688,12 @@ __global__ void __launch_bounds__(256) k_mark_opaque(const __grid_constant__ Dev
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const __grid_constant__ StreamArgs a)
 {
     __shared__ Job jobs[128];
-    stream_loop<false, true>(&a, nullptr, nullptr, jobs[threadIdx.x]);
+    stream_loop<false, true, false>(&a, nullptr, nullptr, jobs[threadIdx.x]);
 }
 
 // launches the lighting kernel g_lightKernel selects (1 ray streams, 2 warp packets followed by the
-// diffuse-path kernel; packets need specBounceLimit <= PK_MAX_SPEC_SEGMENTS and fall back to streams
-// otherwise) with its batch threshold
+// diffuse-path kernel; packets need specBounceLimit <= PK_MAX_SPEC_SEGMENTS and a map that is not
+// far, and fall back to streams otherwise) with its batch threshold
 static int launch_light(DNgpuVolume* g, StreamArgs& a)
 {
     int perSM = 0;
@@ -708,7 +707,7 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a)
         k_mark_opaque<<<(uint32_t)(blocks < maxBlocks ? blocks : maxBlocks), 256, 0, g->stream>>>(dev_map(g), nwords, table);
         CK(cudaGetLastError());
     }
-    if (g_lightKernel == 2 && a.p.specBounceLimit <= PK_MAX_SPEC_SEGMENTS) {
+    if (g_lightKernel == 2 && a.p.specBounceLimit <= PK_MAX_SPEC_SEGMENTS && !map_far(g)) {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_packet, 128, 0));
         if (perSM < 1) perSM = 1;
         a.batch = g_packetBatch;
@@ -725,11 +724,14 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a)
         COUNT_LAUNCH();
         k_light_diffuse<<<g->numSMs * perSM, 128, 0, g->stream>>>(a);
     } else {
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_stream, 128, 0));
+        const bool far = map_far(g);
+        CK(far ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_stream<true>, 128, 0)
+               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_stream<false>, 128, 0));
         if (perSM < 1) perSM = 1;
         a.batch = g_streamBatch;
         COUNT_LAUNCH();
-        k_light_stream<<<g->numSMs * perSM, 128, 0, g->stream>>>(a);
+        if (far) k_light_stream<true><<<g->numSMs * perSM, 128, 0, g->stream>>>(a);
+        else k_light_stream<false><<<g->numSMs * perSM, 128, 0, g->stream>>>(a);
     }
     CK(cudaGetLastError());
     return DN_CUDA_OK;
@@ -1298,7 +1300,8 @@ static int launch_draw(DNgpuVolume* g, const dn_draw_params* p, const dn_materia
     dim3 block(DN_DRAW_BX, DN_DRAW_BY);
     dim3 grid((p->width + DN_DRAW_BX - 1) / DN_DRAW_BX, (p->height + DN_DRAW_BY - 1) / DN_DRAW_BY);
     COUNT_LAUNCH();
-    k_draw<<<grid, block, 0, g->stream>>>(*a);
+    if (map_far(g)) k_draw<true><<<grid, block, 0, g->stream>>>(*a);
+    else k_draw<false><<<grid, block, 0, g->stream>>>(*a);
     CK(cudaGetLastError());
     return DN_CUDA_OK;
 }

@@ -6,7 +6,7 @@
  */
 #pragma once
 #include "dn_cuda.h"
-#include "dn_device.cuh"
+#include "dn_walk.cuh"
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -80,10 +80,10 @@ struct DNgpuVolume {
 
 
 #ifndef DN_DRAW_MIN_BLOCKS
-// resident 256-thread draw blocks per SM the register allocation must allow: 3 (80 registers, a few spills)
-// against 2 at 96 registers; measured +0.9 % on the batched workload and +1.2 % on the streaming one, where
-// the draw is a quarter of the frame (4: 64 registers, more spills, no gain)
-#define DN_DRAW_MIN_BLOCKS 3
+// resident 256-thread draw blocks per SM the register allocation must allow: 4 (64 registers, 16 bytes of spills).
+// A 1080p draw of the 64x32x64 map: 335 us, 3 blocks 369, 5 blocks 323; a 257x143 draw 14.0, 13.0, 14.6; edited
+// frames at 720p 211, 215, 214
+#define DN_DRAW_MIN_BLOCKS 4
 #endif
 
 extern int g_device;
@@ -165,14 +165,18 @@ struct WalkGrid {
     }
 };
 
+// maps whose rays the FAR forms of the kernels walk (dn_walk.cuh)
+static inline bool map_far(const DNgpuVolume* g) { return (uint64_t)g->sx + g->sy + g->sz > dn::FAR_SUM; }
+
 static inline dn::DevMap dev_map(const DNgpuVolume* g)
 {
     dn::DevMap m;
     m.sx = g->sx; m.sy = g->sy; m.sz = g->sz;
-    const uint64_t cap = 256ull * ((uint64_t)g->sx + g->sy + g->sz) + 4096ull;   // step_cap (dn_device.cuh)
+    const uint64_t cap = 256ull * ((uint64_t)g->sx + g->sy + g->sz) + 4096ull;   // D16
     m.stepCap = cap > (1ull << 23) ? (1u << 23) : (uint32_t)cap;
     const WalkGrid wg(g->sx, g->sy, g->sz);
     m.w0 = (uint32_t)(2u * wg.first); m.w1 = (uint32_t)(2u * wg.row); m.w2 = (uint32_t)(2u * wg.plane);
+    m.wk = m.w0 - dn::CODE_BITS * (1u + m.w1 + m.w2);
     m.tword = g->tword; m.tbits = g->tbits; m.treq = g->treq; m.ttouch = g->ttouch; m.tvis = g->tvis;
     m.rec = g->rec; m.vox = g->vox; m.diff = g->diff; m.spec = g->spec;
     m.degen = nullptr;                   // set by the launch: the draw's or the lighting's counter
@@ -198,22 +202,23 @@ __device__ __forceinline__ uint32_t lane_id()
     return l;
 }
 
+// Adds a thread's counters to the launch's.  Every thread of the block calls it, at its end: the sums go through
+// shared memory, so that a launch makes one atomic per counter and block.  (One per warp made 450,000 atomics on
+// one line per 1080p draw, more than the L2 takes in the time of the draw itself.)
 __device__ __forceinline__ void flush_counters(unsigned long long* stats, const dn::Counters& c, uint32_t primary, uint32_t lit)
 {
-    // warp-reduce then one atomic per counter per warp
-    uint32_t v[7] = {c.rays, primary, c.outer, c.entered, c.inner, c.hits, lit};
-    const unsigned full = __activemask();
+    __shared__ unsigned long long sum[7];
+    const uint32_t tid = threadIdx.x + threadIdx.y * blockDim.x;
+    if (tid < 7u) sum[tid] = 0;
+    __syncthreads();
+    const uint32_t v[7] = {c.rays, primary, c.outer, c.entered, c.inner, c.hits, lit};
 #pragma unroll
     for (int k = 0; k < 7; k++) {
-        uint32_t x = v[k];
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(full, x, o);
-        v[k] = x;
+        const uint32_t x = __reduce_add_sync(0xFFFFFFFFu, v[k]);
+        if (lane_id() == 0u && x) atomicAdd(&sum[k], (unsigned long long)x);
     }
-    int leader = __ffs(full) - 1;
-    if ((int)lane_id() == leader) {
-#pragma unroll
-        for (int k = 0; k < 7; k++) if (v[k]) atomicAdd(&stats[k], (unsigned long long)v[k]);
-    }
+    __syncthreads();
+    if (tid < 7u && sum[tid]) atomicAdd(&stats[tid], sum[tid]);
 }
 
 // spreads the 16 low bits of x to the even bit positions of a word
@@ -319,19 +324,15 @@ __device__ __forceinline__ void raster_sample(const float* tex, uint32_t w, uint
         out[k] = w00 * __ldg(t00 + k) + w10 * __ldg(t10 + k) + w01 * __ldg(t01 + k) + w11 * __ldg(t11 + k);
 }
 
-// One primary ray (voxelDraw.comp:24-147): pixel (x, y) of the image described by a; smat holds the map's
+// One primary ray (voxelDraw.comp:24-147): pixel (x, y) of the image described by a; mats: the map's
 // materials.  Returns 1 when a primary ray was traced.
-__device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Material* smat, uint32_t x, uint32_t y,
+template <bool FAR>
+__device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Material* mats, uint32_t x, uint32_t y,
                                                dn::Counters& cnt)
 {
     using namespace dn;
     const dn_draw_params& p = a.p;
-    RayCtx c;
-    c.m = &a.m; c.mats = smat;
-    c.sunStrength = mk(p.sunStrength[0], p.sunStrength[1], p.sunStrength[2]);
-    c.emissive = p.emissiveStrength;
-    c.refraction = true;   // voxelDraw.comp:65
-    c.c = Counters{0, 0, 0, 0, 0};
+    cnt = Counters{0, 0, 0, 0, 0};
     uint32_t primary = 0;
     if (x < p.width && y < p.height) {
         const uint64_t pix = (uint64_t)y * p.width + x;
@@ -346,7 +347,7 @@ __device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Mater
             const float sx = (float)x / (float)p.width * 2.0f - 1.0f;
             const float sy = (float)y / (float)p.height * 2.0f - 1.0f;
             f3 rayPos = mk(p.origin[0], p.origin[1], p.origin[2]);
-            c.orgRayPos = rayPos;
+            const f3 orgRayPos = rayPos;
             const float (*M)[4] = p.dirMat;
             f3 rd = mk(M[0][0] * sx + M[1][0] * sy + M[2][0] * 0.0f + M[3][0] * 1.0f,
                        M[0][1] * sx + M[1][1] * sy + M[2][1] * 0.0f + M[3][1] * 1.0f,
@@ -398,25 +399,17 @@ __device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Mater
                 fc = background(rayDir);
             } else {
                 if (tNear > 0.0f) rayPos = add(rayPos, muls(rayDir, tNear + EPS));
-                // normal_AABB, voxelShared.comp:276-284
-                f3 cc = muls(add(mk(0.0f, 0.0f, 0.0f), mapMax), 0.5f);
-                f3 pp = sub(rayPos, cc);
-                f3 dd = muls(sub(mapMax, mk(0.0f, 0.0f, 0.0f)), 0.5f);
-                const float bias = 1.0f + EPS;
-                f3 q = mk(pp.x / dd.x * bias, pp.y / dd.y * bias, pp.z / dd.z * bias);
-                f3 hitNormal = normalize(mk(truncf(q.x), truncf(q.y), truncf(q.z)));
-                TState ts{255u, 1.0f};
-                Voxel fv;
-                fv.normal = mk(0.0f, 0.0f, 0.0f); fv.material = 0; fv.albedo = fv.normal; fv.spec = fv.normal; fv.diff = fv.normal;
-                f3 cadd; float cmul; HitInfo hi;
+                f3 hitNormal;
+                f3 cadd; float cmul; PrimaryHit hi;
                 primary = 1;
-                if (step_map(c, ts, rayDir, inv, rayPos, false, maxDepth, hitNormal, fv, cadd, cmul, hi)) {
+                if (trace_primary<FAR>(a.m, mats, mk(p.sunStrength[0], p.sunStrength[1], p.sunStrength[2]), orgRayPos, rayPos, rayDir,
+                                  inv, maxDepth, hitNormal, cadd, cmul, hi, cnt)) {
                     i3 mp{f2i(floorf(rayPos.x)), f2i(floorf(rayPos.y)), f2i(floorf(rayPos.z))};
                     if (in_map(a.m, mp)) {
                         uint8_t* vp = &a.m.tvis[map_index(a.m, mp)];
                         if (*vp == 0) *vp = 1;
                     }
-                    f3 dv = sub(rayPos, c.orgRayPos);
+                    f3 dv = sub(rayPos, orgRayPos);
                     depth = sqrtf(dot(dv, dv));
                     if (maxDepth > 0.0f && depth > maxDepth) {
                         // the rasterised scene is in front of the voxel (voxelDraw.comp:127-131): the pixel shows
@@ -425,12 +418,14 @@ __device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Mater
                         depth = maxDepth;
                     } else {
                         // voxel_color, voxelDraw.comp:32-61
-                        const Material& mt = smat[fv.material];
+                        Voxel fv;
+                        decompress(a.m, hi.voxel, fv);
+                        const Material& mt = mats[fv.material];
                         f3 sp = muls(fv.spec, mt.specular);
                         f3 df = muls(fv.diff, 1.0f - mt.specular);
                         switch (p.viewMode) {
                         case 0: {
-                            f3 solid = mt.emissive ? muls(fv.albedo, c.emissive) : add(mul(df, fv.albedo), sp);
+                            f3 solid = mt.emissive ? muls(fv.albedo, p.emissiveStrength) : add(mul(df, fv.albedo), sp);
                             fc = add(muls(solid, cmul), cadd);
                             break;
                         }
@@ -441,9 +436,8 @@ __device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Mater
                         case 5: fc = vabs(hitNormal); break;
                         default: fc = mk(0.0f, 0.0f, 0.0f); break;
                         }
-                        const uint32_t tx = hi.tile % a.m.sx, ty = (hi.tile / a.m.sx) % a.m.sy, tz = hi.tile / (a.m.sx * a.m.sy);
-                        const uint32_t gx = tx * 8u + (uint32_t)hi.local.x, gy = ty * 8u + (uint32_t)hi.local.y,
-                                       gz = tz * 8u + (uint32_t)hi.local.z;
+                        const uint32_t gx = (uint32_t)hi.cell.x * 8u + (hi.local & 7u), gy = (uint32_t)hi.cell.y * 8u + ((hi.local >> 3) & 7u),
+                                       gz = (uint32_t)hi.cell.z * 8u + (hi.local >> 6);
                         hitIdx = gx + (a.m.sx * 8u) * (gy + (a.m.sy * 8u) * gz);
                         if (hitNormal.x > 0.0f) face = 0; else if (hitNormal.x < 0.0f) face = 1;
                         else if (hitNormal.y > 0.0f) face = 2; else if (hitNormal.y < 0.0f) face = 3;
@@ -460,7 +454,6 @@ __device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Mater
         if (a.hit) a.hit[pix] = hitIdx;
         if (a.face) a.face[pix] = face;
     }
-    cnt = c.c;
     return primary;
 }
 

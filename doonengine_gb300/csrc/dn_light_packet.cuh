@@ -12,7 +12,7 @@
  * `batch` lanes have one.  Each ray's contributions go to shared memory; when the pool is empty, each
  * voxel's sums are formed by one lane walking its rays (and their segments) in ray order, so every sum
  * is accumulated in exactly the reference's order.  The kernel writes each voxel's specular lighting and
- * leaves its direct light for the diffuse kernel (dn_light_stream.cuh, stream_loop<.., true>), which traces
+ * leaves its direct light for the diffuse kernel (dn_light_stream.cuh, stream_loop<.., true, false>), which traces
  * the diffuse paths (numDiffuse per voxel, up to diffuseBounceLimit segments each) as per-lane path
  * streams over all request groups and finishes each voxel as the reference's lighting main does (running
  * average, clamps, voxelLighting.comp:238-288).
@@ -233,7 +233,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                             jd.jA = pv.talbedo; jd.jB = pv.pos0; jd.jU = tm.reflectType; jd.b = 0; ncon = 0;
                             const f3 P = mk(p.spherePts[kk][0], p.spherePts[kk][1], p.spherePts[kk][2]);
                             const f3 sd = adds(normalize(add(muls(pv.refl, (float)tm.shininess), P)), EPS);
-                            ray_begin(s, m, pv.pos0, sd, rcp3(sd), false, c);
+                            ray_begin<false>(s, m, pv.pos0, sd, rcp3(sd), false, c);
                         } else {
                             // shadow ray: voxels of the pool in slot order, K rays each (1 on the first sample)
                             isSpec = false;
@@ -247,7 +247,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                                 if (rid < off + n) { vi = v; kk = ((firstMask >> v) & 1u) ? 64u : rid - off; break; }
                                 off += n;
                             }
-                            ray_begin(s, m, W.v[vi].pos0, mk(sdir[kk][0], sdir[kk][1], sdir[kk][2]),
+                            ray_begin<false>(s, m, W.v[vi].pos0, mk(sdir[kk][0], sdir[kk][1], sdir[kk][2]),
                                       mk(sinv[kk][0], sinv[kk][1], sinv[kk][2]), false, c);
                         }
                         c.rays++;
@@ -262,7 +262,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                 for (;;) {
                     const unsigned st = __ballot_sync(0xFFFFFFFFu, ray_stepping(s));
                     if (!st || (uint32_t)__popc(liveMask & ~st) >= batch) break;
-                    if (ray_stepping(s)) walk_round(s, m, mats, p.sunStrength, c);
+                    if (ray_stepping(s)) walk_round<false>(s, m, mats, p.sunStrength, c);
                 }
                 // shade the ended segments
                 if (!live || ray_stepping(s)) continue;
@@ -273,7 +273,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                     bool more = false, add_ = false;
                     f3 sc = mk(0.0f, 0.0f, 0.0f);
                     if (hit) {
-                        const f3 hpos = ray_hit_position(s);
+                        const f3 hpos = ray_hit_position<false>(s);
                         Voxel hv;
                         decompress(m, ray_hit_index(s, m), hv);
                         const i3 hp{f2i(truncf(hpos.x)), f2i(truncf(hpos.y)), f2i(truncf(hpos.z))};
@@ -304,7 +304,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                                     const f3 nd = reflect(s.dir, hv.normal);
                                     jd.b++;
                                     if (jd.b < p.specBounceLimit) {
-                                        ray_begin(s, m, hpos, nd, rcp3(nd), true, c);
+                                        ray_begin<false>(s, m, hpos, nd, rcp3(nd), true, c);
                                         c.rays++;
                                         more = true;
                                     }

@@ -115,7 +115,7 @@ __device__ __forceinline__ f3 diffuse_dir(const Job& j, const dn_light_params& p
 // DIFFONLY: the voxel's diffuse paths only (its specular and direct light came from the ray-fan kernel,
 // which left the direct light in the diffuse output slot); the final write replaces that slot with the
 // voxel's new diffuse lighting and leaves the specular slot and the lit-voxel count alone.
-template <bool DIFFONLY = false>
+template <bool DIFFONLY, bool FAR>
 __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const dn_light_params& p,
                                         const Material* mats, const float (*sdir)[3], const float (*sinv)[3],
                                         float4* out, Counters& c, uint32_t& lit)
@@ -129,7 +129,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
         Voxel hv;
         f3 hpos = s.pos;
         if (hit) {
-            hpos = ray_hit_position(s);
+            hpos = ray_hit_position<FAR>(s);
             decompress(m, ray_hit_index(s, m), hv);
         }
         // the diffuse-only kernel's jobs never reach the specular and shadow phases: with DIFFONLY their
@@ -165,7 +165,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                             const f3 nd = reflect(s.dir, hv.normal);
                             j.b++;
                             if (j.b < p.specBounceLimit) {
-                                ray_begin(s, m, hpos, nd, rcp3(nd), true, c);   // next bounce
+                                ray_begin<FAR>(s, m, hpos, nd, rcp3(nd), true, c);   // next bounce
                                 c.rays++;
                                 return true;
                             }
@@ -212,7 +212,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                         j.b++;
                         if (j.b < p.diffuseBounceLimit) {
                             const f3 nd = diffuse_dir(j, p, mats, rngSin);
-                            ray_begin(s, m, hpos, nd, rcp3(nd), true, c);
+                            ray_begin<FAR>(s, m, hpos, nd, rcp3(nd), true, c);
                             c.rays++;
                             return true;
                         }
@@ -236,7 +236,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                 j.b = 0; j.jA = j.talbedo; j.jB = j.pos0; j.jU = tm.reflectType;
                 const f3 P = mk(p.spherePts[j.k][0], p.spherePts[j.k][1], p.spherePts[j.k][2]);
                 const f3 sd = adds(normalize(add(muls(j.refl, (float)tm.shininess), P)), EPS);
-                ray_begin(s, m, j.pos0, sd, rcp3(sd), false, c);
+                ray_begin<FAR>(s, m, j.pos0, sd, rcp3(sd), false, c);
                 c.rays++;
                 return true;
             }
@@ -249,7 +249,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
             const uint32_t n = j.firstSample ? 1u : p.K;
             if (j.k < n) {
                 const uint32_t q = j.firstSample ? 64u : j.k;
-                ray_begin(s, m, j.pos0, mk(sdir[q][0], sdir[q][1], sdir[q][2]), mk(sinv[q][0], sinv[q][1], sinv[q][2]), false, c);
+                ray_begin<FAR>(s, m, j.pos0, mk(sdir[q][0], sdir[q][1], sdir[q][2]), mk(sinv[q][0], sinv[q][1], sinv[q][2]), false, c);
                 c.rays++;
                 return true;
             }
@@ -271,7 +271,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                     j.jU = j.tmat;
                 }
                 const f3 nd = diffuse_dir(j, p, mats, rngSin);
-                ray_begin(s, m, j.pos0, nd, rcp3(nd), false, c);
+                ray_begin<FAR>(s, m, j.pos0, nd, rcp3(nd), false, c);
                 c.rays++;
                 return true;
             }
@@ -410,8 +410,8 @@ __device__ __forceinline__ void shadow_dir(const dn_light_params& p, int k, floa
 // queue over the requests of many maps (many); each lane reads its current voxel's map, parameters,
 // materials and shadow directions from that map's entry of the device table.  DIFFONLY: the
 // diffuse paths of the voxels the ray-fan kernel lit (advance<true>); one map's materials are read from
-// its device tables (one->gtab) and sh is not used.
-template <bool MANY, bool DIFFONLY = false>
+// its device tables (one->gtab) and sh is not used.  FAR: maps above FAR_SUM chunks (dn_walk.cuh).
+template <bool MANY, bool DIFFONLY, bool FAR>
 __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLightArgs* many, const StreamShared* sh,
                                             Job& j)
 {
@@ -493,17 +493,17 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
                 if (!ray_stepping(s) && j.phase != PH_DONE && j.phase != PH_FETCH) {
                     if constexpr (MANY) {
                         if (j.map != lmi) { le = &many->maps[j.map]; lmi = j.map; }
-                        advance<DIFFONLY>(j, s, le->m, le->p, le->mats, le->sdir, le->sinv, le->out, c, lit);
+                        advance<DIFFONLY, FAR>(j, s, le->m, le->p, le->mats, le->sdir, le->sinv, le->out, c, lit);
                     } else if constexpr (DIFFONLY) {
-                        advance<true>(j, s, one->m, one->p, MATS(), one->gtab->sdir, one->gtab->sinv, one->out, c, lit);
+                        advance<true, FAR>(j, s, one->m, one->p, MATS(), one->gtab->sdir, one->gtab->sinv, one->out, c, lit);
                     } else {
-                        advance(j, s, one->m, one->p, sh->mats, sh->sdir, sh->sinv, one->out, c, lit);
+                        advance<false, FAR>(j, s, one->m, one->p, sh->mats, sh->sdir, sh->sinv, one->out, c, lit);
                     }
                 }
                 if (__ballot_sync(0xFFFFFFFFu, j.phase == PH_FETCH) == 0u) break;
             }
         }
-        if (ray_stepping(s)) walk_round(s, M(), MATS(), P().sunStrength, c);
+        if (ray_stepping(s)) walk_round<FAR>(s, M(), MATS(), P().sunStrength, c);
     }
     flush_counters(MANY ? many->stats : one->stats, c, 0, lit);
 }

@@ -1,9 +1,13 @@
-"""The lighting rays' walk at the sizes where its grid can go wrong: maps of one chunk, one chunk thick, and with
-rows, planes and cell counts around the 16 cells of a grid word and the 32 of a warp -- opaque, and with every third
-material see-through (chunks entered whose voxels the walk goes on through).  Against the oracle: hits and counters
-equal, lighting bit for bit."""
+"""The rays' walk through the map (primary and lighting) at the sizes where its grid can go wrong: maps of one chunk, one
+chunk thick, and with rows, planes and cell counts around the 16 cells of a grid word and the 32 of a warp -- opaque,
+and with every third material see-through (chunks entered whose voxels the walk goes on through) -- and a map so long
+that its rays' coordinates are integers (the kernels' FAR forms).  Against the oracle: hits and counters equal,
+lighting bit for bit."""
+import numpy as np
 import pytest
 
+import doonengine_gb300 as dn
+from oracle import oracle as O
 from parity_util import Pair
 
 pytestmark = pytest.mark.gpu
@@ -25,8 +29,46 @@ def test_walk_matches_oracle(gpu_ready, size, glass):
             pair.sync()
             _, differ = pair.light(num_diffuse=2)
             assert differ == 0
-        st, oc = pair.vol.stats(), pair.om.counters()
-        for k_gpu, k_or in COUNTERS:
-            assert st[k_gpu] == oc[k_or], (k_gpu, st[k_gpu], oc[k_or])
+        check_counters(pair)
     finally:
         pair.close()
+
+
+@pytest.mark.parametrize("glass", [False, True])
+@pytest.mark.parametrize("length", [262141, 262143, 262200])
+def test_long_map_matches_oracle(gpu_ready, length, glass):
+    """1 x 2 chunks across; 262144 chunks along all axes together is the last map with coded coordinates"""
+    dn.init()
+    pair = Pair.__new__(Pair)
+    pair.vol, pair.om = dn.Volume((1, 2, length), 64), O.OracleMap((1, 2, length))
+    pair.cfg, pair.W, pair.H, pair.frame = {}, 48, 24, 0
+    pair.img = dn.Image(pair.W, pair.H)
+    try:
+        vol = pair.vol
+        vol.palette(5, 16, 2, 0.1, 0.9, 0.5)
+        rng = np.random.default_rng(5)
+        z0 = length - 30        # near the far end: rays leave the map within the border's reach
+        for z in range(z0, z0 + 24):
+            for _ in range(40):
+                vol.set_voxel((0, 0, z), (int(rng.integers(8)), int(rng.integers(4)), int(rng.integers(8))),
+                              int(rng.integers(16)), tuple(rng.normal(size=3)), tuple(int(x) for x in rng.integers(0, 256, 3)))
+        if glass:
+            for m in range(0, 14, 3):
+                vol.set_material(m, opacity=0.4, refract=1.3, specular=0.3, reflect_type=1, shininess=2)
+        vol.camera(0.3, 0.6, (z0 - 2.0) / length, 20.0, 8.0, 90.0)
+        vol.s.numDirectRays = 3
+        for _ in range(4):
+            pair.draw()
+            pair.sync()
+            _, differ = pair.light()
+            assert differ == 0
+        assert pair.vol.stats()["litVoxels"] > 0
+        check_counters(pair)
+    finally:
+        pair.close()
+
+
+def check_counters(pair):
+    st, oc = pair.vol.stats(), pair.om.counters()
+    for k_gpu, k_or in COUNTERS:
+        assert st[k_gpu] == oc[k_or], (k_gpu, st[k_gpu], oc[k_or])

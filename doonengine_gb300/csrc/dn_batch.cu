@@ -150,7 +150,8 @@ template <bool FAR>
 __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream_batch(const __grid_constant__ BatchLightArgs a)
 {
     __shared__ Job jobs[128];
-    stream_loop<true, false, FAR>(nullptr, &a, nullptr, jobs[threadIdx.x]);
+    __shared__ TintT<128> tint;
+    stream_loop<true, false, FAR>(nullptr, &a, nullptr, jobs[threadIdx.x], tint);
 }
 
 // POOL: rays per fan kind per pool (the rays a warp pulls from a request group at a time); the autotuner
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream_batc
 template <uint32_t POOL>
 __global__ void __launch_bounds__(128, DN_PACKET_MIN_BLOCKS) k_light_packet_batch(const __grid_constant__ BatchLightArgs a)
 {
-    __shared__ PacketWarpT<POOL> warps[4];
+    __shared__ PacketWarpT<POOL, PK_VOXELS> warps[4];
     packet_loop<true, POOL>(nullptr, &a, warps[threadIdx.x >> 5]);
 }
 
@@ -179,7 +180,8 @@ __global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* 
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse_batch(const __grid_constant__ BatchLightArgs a)
 {
     __shared__ Job jobs[128];
-    stream_loop<true, true, false>(nullptr, &a, nullptr, jobs[threadIdx.x]);
+    __shared__ TintT<128> tint;
+    stream_loop<true, true, false>(nullptr, &a, nullptr, jobs[threadIdx.x], tint);
 }
 
 __global__ void k_commit_batch(const BatchLightMap* l, const uint32_t* reqStart, uint32_t nl)

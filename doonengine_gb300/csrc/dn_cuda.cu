@@ -95,7 +95,7 @@ extern "C" uint64_t dn_cuda_alloc_count(void) { return __atomic_load_n(&g_allocs
 // of ray fans; DN_STREAM_BATCH lanes, 1..32), read once at init
 int g_lightKernel = 2;
 uint32_t g_streamBatch = 24;
-uint32_t g_packetBatch = 12;   // lanes with an ended segment before the packet kernel shades (measured best)
+uint32_t g_packetBatch = 16;   // lanes with an ended segment before the packet kernel shades (12 and 20 within 1 %)
 
 static void noalloc_forget(void);
 
@@ -646,11 +646,12 @@ __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream(cons
     __shared__ StreamShared sh;
     // per-voxel job state lives in shared memory: it is touched only when a segment ends
     __shared__ Job jobs[128];
+    __shared__ TintT<128> tint;
     for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.mats[i] = a.mats[i];
     // shadow directions are identical for every voxel of the launch
     for (int k = threadIdx.x; k < 65; k += blockDim.x) shadow_dir(a.p, k, sh.sdir[k], sh.sinv[k]);
     __syncthreads();
-    stream_loop<false, false, FAR>(&a, nullptr, &sh, jobs[threadIdx.x]);
+    stream_loop<false, false, FAR>(&a, nullptr, &sh, jobs[threadIdx.x], tint);
 }
 
 // The lighting launch with specular and shadow fans traced as warp packets (dn_light_packet.cuh).
@@ -665,9 +666,8 @@ __global__ void k_light_tables(const __grid_constant__ MaterialTable t, const __
 
 __global__ void __launch_bounds__(128, DN_PACKET_MIN_BLOCKS) k_light_packet(const __grid_constant__ StreamArgs a)
 {
-    // shared memory holds only the four warps' pools (31 KB per block with 128-ray pools): 6 blocks fit
-    // the 196 KB carveout, leaving about 60 KB of L1 for the map's masks and voxels; the tables are read
-    // from a.gtab
+    // shared memory holds only the four warps' pools (25 KB per block with 128-ray pools): 7 blocks take 175 KB, the
+    // rest of the SM's 256 KB is L1 for the map's masks and voxels; the tables are read from a.gtab
     __shared__ PacketWarp warps[4];
     packet_loop<false>(&a, nullptr, warps[threadIdx.x >> 5]);
 }
@@ -688,7 +688,8 @@ __global__ void __launch_bounds__(256) k_mark_opaque(const __grid_constant__ Dev
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const __grid_constant__ StreamArgs a)
 {
     __shared__ Job jobs[128];
-    stream_loop<false, true, false>(&a, nullptr, nullptr, jobs[threadIdx.x]);
+    __shared__ TintT<128> tint;
+    stream_loop<false, true, false>(&a, nullptr, nullptr, jobs[threadIdx.x], tint);
 }
 
 // launches the lighting kernel g_lightKernel selects (1 ray streams, 2 warp packets followed by the

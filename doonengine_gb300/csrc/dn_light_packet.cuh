@@ -3,23 +3,31 @@
  *
  * Every lit voxel casts two fans of K rays from one point: K specular rays around its reflection
  * direction (voxelLighting.comp:83-146, each up to specBounceLimit segments) and K shadow rays around the
- * sun direction (D8).  A warp takes one work unit -- 32 / PK_PARTS voxels of a request group (a group is 32
- * voxels of one chunk) in a one-map launch, a whole group in a many-map launch -- and traces the fans of
- * PK_POOL_FAN / K of its voxels at a time as one pool: the pool's rays are numbered (specular fans first,
- * then the shadow rays), and a lane whose ray has ended takes the pool's next ray, so consecutive rays of
- * a fan run side by side and the lanes of a warp walk nearly the same cells (a fan's shadow rays are
- * almost parallel, its specular rays share their origin and lobe).  Ended segments are shaded once
- * `batch` lanes have one.  Each ray's contributions go to shared memory; when the pool is empty, each
- * voxel's sums are formed by one lane walking its rays (and their segments) in ray order, so every sum
- * is accumulated in exactly the reference's order.  The kernel writes each voxel's specular lighting and
- * leaves its direct light for the diffuse kernel (dn_light_stream.cuh, stream_loop<.., true, false>), which traces
- * the diffuse paths (numDiffuse per voxel, up to diffuseBounceLimit segments each) as per-lane path
- * streams over all request groups and finishes each voxel as the reference's lighting main does (running
- * average, clamps, voxelLighting.comp:238-288).
+ * sun direction (D8).  A warp takes one work unit -- 16, 8 or 4 voxels of a request group (a group is 32
+ * voxels of one chunk) -- and traces the fans of PK_POOL_FAN / K of its voxels at a time as one pool: the
+ * pool's rays are numbered (specular fans first, then the shadow rays), and a lane whose ray has ended takes
+ * the pool's next ray, so consecutive rays of a fan run side by side and the lanes of a warp walk nearly the
+ * same cells (a fan's shadow rays are almost parallel, its specular rays share their origin and lobe).  The
+ * specular directions of a whole pool are formed before its first ray, by full warps.  Ended segments are
+ * shaded once `batch` lanes have one.  Each ray's contributions go to shared memory; when the pool is empty,
+ * each sum of a voxel's lighting is formed by one lane walking its rays (and their segments) in ray order, so
+ * every sum is accumulated in exactly the reference's order.  The kernel writes each voxel's specular
+ * lighting and leaves its direct light for the diffuse kernel (dn_light_stream.cuh,
+ * stream_loop<.., true, false>), which traces the diffuse paths (numDiffuse per voxel, up to
+ * diffuseBounceLimit segments each) as per-lane path streams over all request groups and finishes each voxel
+ * as the reference's lighting main does (running average, clamps, voxelLighting.comp:238-288).
  *
  * Results, traversal side effects (requested / touched / visible flags) and counters are those of the
  * one-voxel-per-lane form (dn_light_stream.cuh): the same rays are traced with the same
  * operations; only the assignment of rays to lanes differs.
+ *
+ * Bound by issue and by load latency at 28 warps per SM.  Between segments a lane keeps only its ray's number:
+ * what a bounce needs besides (multiplier, sky flag) is in the ray's shared-memory slot and two flag bits, and
+ * the light of see-through voxels is in shared memory for the rays that meet one (TintT), so the kernel takes
+ * 70 registers instead of 80.  Measured with the directions formed by full warps, the table-free sums (a lane
+ * per component) and the three unit sizes, us per frame or call, before -> after: 64x32x64 map at 1080p, K = 32:
+ * 14200 -> 12240; 16x16x16 at 640x360, K = 16: 661 -> 507; glass 2970 -> 2597; twelve maps batched
+ * 15230 -> 12010; eight maps served 2259 -> 1459.
  */
 #pragma once
 #include "dn_light_stream.cuh"
@@ -27,59 +35,64 @@
 namespace dn {
 
 #ifndef DN_PACKET_MIN_BLOCKS
-#define DN_PACKET_MIN_BLOCKS 6   // 6 blocks of 4 warps per SM (measured best on the large map: 5 and 4 are slower)
+// 7 blocks of 4 warps per SM (70 registers).  The 64x32x64 map, us per frame: 12440; 6 blocks 12800, 8 (64
+// registers, spills, little L1 left) 12990
+#define DN_PACKET_MIN_BLOCKS 7
 #endif
 
 // specBounceLimit handled here (the reference's default is 2); larger limits use the stream kernel
 constexpr uint32_t PK_MAX_SPEC_SEGMENTS = 2;
 
-// per-voxel data of the warp's request group (shared memory, written by the voxel's lane)
+// per-voxel data of the warp's unit (shared memory, written by the voxel's lane)
 struct PacketVoxel {
-    f3 pos0, tnormal, talbedo, refl;
-    f3 spec;                 // specular sum / K (after the specular pass)
-    f3 direct;               // shadow sum / n (after the shadow pass)
-    uint32_t tmat, key, vidx, flags;   // flags: 1 valid, 2 first sample, 4 specular pass, 8 diffuse passes
-    float indirect;
+    f3 pos0, talbedo, refl;
+    uint32_t tmat, flags;    // flags: 1 valid, 2 first sample, 4 specular pass, 8 diffuse passes
 };
 enum : uint32_t { PV_VALID = 1u, PV_FIRST = 2u, PV_SPEC = 4u, PV_DIFF = 8u };
 
-// rays per fan kind in one pool (voxels per pool = PK_POOL_FAN / K): the pool's specular contributions,
-// shadow contributions and counts live in shared memory, 38 B per pooled ray.  Larger pools shorten the
-// tail that a pool's longest rays leave; the shared memory they take comes out of L1 (the SM's 256 KB
-// split).  Measured on the large map at 6 blocks per SM with the tables in global memory: 64 rays
-// 3.38 G rays/s, 96 3.55, 128 3.64-3.66 (31 KB per block, 60 KB of L1), 160 3.60, 192 (5 blocks) 3.40.
+// rays per fan kind in one pool (voxels per pool = PK_POOL_FAN / K): the pool's specular slots, shadow
+// contributions and counts live in shared memory, 38 B per pooled ray.  Larger pools shorten the tail that a
+// pool's longest rays leave; the shared memory they take comes out of L1 (the SM's 256 KB split).  Measured, us per
+// frame of the 64x32x64 map (K = 32), of a 16x16x16 map (K = 16) and of twelve maps batched: 128 rays 12444, 513,
+// 12750; 96 rays 12299, 537, 13388; 192 rays 14361, 542, 13659.
 #ifndef DN_PK_POOL_FAN
 #define DN_PK_POOL_FAN 128
 #endif
 constexpr uint32_t PK_POOL_FAN = DN_PK_POOL_FAN;
 constexpr uint32_t PK_POOL_ALT = PK_POOL_FAN == 64u ? 128u : 64u;   // the batched autotuner's other pool size
 
-// Work units per request group in a one-map launch: a warp takes 32 / PK_PARTS voxels of a group at a time,
-// so that the launch does not end with a few warps finishing whole groups while the others have left.  Per
-// warp exit times on the large map's frame 11 with whole groups: the last warp left 2.7 ms after 90 % of
-// them had, 16 % of the warps' time idle.  Units of 8 voxels against 4: the 64x32x64 map 14.9 against 15.5 ms
-// per frame, 16x16x16 maps 0.70 against 0.79 (with K = 16 a unit of 4 fills half a pool).  A many-map launch
-// keeps whole groups: its queue is long enough that the tail is small, and smaller units measured slower there
-// (the setup of a unit runs on a fraction of the lanes).
-#ifndef DN_PK_PARTS
-#define DN_PK_PARTS 4
+// Work units: 16 voxels of a request group at a time while more than PK_MID voxels per warp of the launch are left in
+// the queue, 8 down to PK_TAIL, then 4.  Large units have fewer pool tails, small ones spread the end of a launch.
+// One size for all, us per frame of the 64x32x64 map, the 16x16x16 map, the glass map and twelve maps batched: 16 voxels
+// 12336, 514, 2885, 12105; 8 voxels 12444, 513, 2685, 12750; 4 voxels 12675, 573, 2720, 14115; these three 12243, 507,
+// 2597, 12014 (a middle of 128 or 256 voxels per warp, a tail of 4 or 16: within 2 %).
+#ifndef DN_PK_MID
+#define DN_PK_MID 192
 #endif
-constexpr uint32_t PK_PARTS = DN_PK_PARTS;
-static_assert(PK_PARTS == 1u || PK_PARTS == 2u || PK_PARTS == 4u || PK_PARTS == 8u,
-              "a unit is 32, 16, 8 or 4 voxels of a group");
+#ifndef DN_PK_TAIL
+#define DN_PK_TAIL 8
+#endif
+constexpr uint32_t PK_MID = DN_PK_MID, PK_TAIL = DN_PK_TAIL;
+constexpr uint32_t PK_VOXELS = 16;
 
-template <uint32_t POOL>
+template <uint32_t POOL, uint32_t VOXELS>
 struct PacketWarpT {
-    PacketVoxel v[32];
-    float con[POOL][PK_MAX_SPEC_SEGMENTS][3];   // specular contributions of each pooled ray, in segment order
-    float sh[POOL][3];                          // shadow contribution of each pooled ray
+    PacketVoxel v[VOXELS];
+    // a pooled specular ray's direction and its reciprocal until a lane takes the ray, then the contributions of its
+    // (at most two) segments; while the second segment runs, the upper three hold the first one's multiplier
+    float con[2 * 3][POOL];
+    float sh[3][POOL];                          // shadow contribution of each pooled ray
     uint8_t ncon[POOL];                         // contributions of each specular ray
     uint8_t shHas[POOL];                        // the shadow ray was unoccluded
+    uint8_t specList[VOXELS], fanList[VOXELS], firstList[VOXELS];   // the pool's voxels by what they cast
+    TintT<32> tint;
 };
-using PacketWarp = PacketWarpT<PK_POOL_FAN>;
+using PacketWarp = PacketWarpT<PK_POOL_FAN, PK_VOXELS>;
+static_assert(PK_MAX_SPEC_SEGMENTS == 2, "con holds two segments' contributions");
 
-// sets up voxel (req, lane) of the group (voxel_setup of dn_light_stream.cuh); invalid slots get zero output
-__device__ __forceinline__ void packet_setup(PacketVoxel& pv, uint32_t req, uint32_t lane, const DevMap& m,
+// sets up voxel (req, vlane) of the group (voxel_setup of dn_light_stream.cuh) and writes the outputs that no ray
+// decides: zero for invalid slots and for light the voxel does not cast rays for
+__device__ __forceinline__ void packet_setup(PacketVoxel& pv, uint32_t req, uint32_t vlane, const DevMap& m,
                                              const dn_light_params& p, const Material* mats, const uint32_t* reqs,
                                              const uint32_t* nsamples, float4* out)
 {
@@ -87,56 +100,52 @@ __device__ __forceinline__ void packet_setup(PacketVoxel& pv, uint32_t req, uint
     const uint32_t word = reqs[req];
     const uint32_t tile = word >> 4, group = word & 15u;
     const uint32_t tw = __ldg(&m.tword[tile]);
-    const uint32_t vn = group * 32u + lane;
+    const uint32_t vn = group * 32u + vlane;
+    const uint64_t o = ((uint64_t)req * 32u + vlane) * 2u;
     i3 cp; uint32_t li;
     const ChunkRec* rc = &m.rec[tw & SLOT_MASK];
     if ((tw >> 30) != 2u || vn >= __ldg(&rc->nvox) || !select_voxel(rc, vn, cp, li)) {
-        const uint64_t o = ((uint64_t)req * 32u + lane) * 2u;
         out[o] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         out[o + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         return;
     }
     const i3 mp{__ldg(&rc->pos[0]), __ldg(&rc->pos[1]), __ldg(&rc->pos[2])};
-    pv.vidx = __ldg(&rc->voxBase) + vn;
-    const uint2 w = __ldg(&m.vox[pv.vidx]);
-    pv.tnormal = mk(((float)((w.x >> 16) & 0xFF) * INV255 - 0.5f) * 2.0f, ((float)((w.x >> 8) & 0xFF) * INV255 - 0.5f) * 2.0f,
-                    ((float)(w.x & 0xFF) * INV255 - 0.5f) * 2.0f);
+    const uint2 w = __ldg(&m.vox[__ldg(&rc->voxBase) + vn]);
+    const f3 tnormal = voxel_normal(w);
     pv.tmat = w.x >> 24;
     pv.talbedo = mk((float)((w.y >> 24) & 0xFF) * INV255, (float)((w.y >> 16) & 0xFF) * INV255,
                     (float)((w.y >> 8) & 0xFF) * INV255);
     const uint32_t samples = __ldg(&nsamples[tw & SLOT_MASK]);
-    const uint32_t ns = samples < p.maxDiffuse ? samples : p.maxDiffuse;
-    pv.indirect = (float)ns;
-    const bool first = (pv.indirect == 0.0f);
-    const uint32_t gx = (uint32_t)(mp.x * 8 + cp.x), gy = (uint32_t)(mp.y * 8 + cp.y), gz = (uint32_t)(mp.z * 8 + cp.z);
-    pv.key = rng_key(__float_as_uint(p.time), p.mapId, gx + (m.sx * 8u) * (gy + (m.sy * 8u) * gz));
+    const bool first = (samples < p.maxDiffuse ? samples : p.maxDiffuse) == 0u;
     f3 rp;
     rp.x = INV_CHUNK * (float)cp.x + (float)mp.x + HALF_INV_CHUNK;
     rp.y = INV_CHUNK * (float)cp.y + (float)mp.y + HALF_INV_CHUNK;
     rp.z = INV_CHUNK * (float)cp.z + (float)mp.z + HALF_INV_CHUNK;
     const float off = HALF_INV_CHUNK - EPS;
-    pv.pos0 = add(rp, muls(pv.tnormal, off));
+    pv.pos0 = add(rp, muls(tnormal, off));
     const Material& tm = mats[pv.tmat];
     const f3 viewDir = sub(pv.pos0, mk(p.camPos[0], p.camPos[1], p.camPos[2]));
-    const bool doSpec = tm.specular > 0.0f && dot(viewDir, pv.tnormal) < 0.0f && tm.reflectType <= 1u;
+    // no specular segments (specBounceLimit 0): the sum stays zero
+    const bool doSpec = tm.specular > 0.0f && dot(viewDir, tnormal) < 0.0f && tm.reflectType <= 1u && p.specBounceLimit > 0u;
     const bool doDiff = tm.specular < 1.0f;
-    if (doSpec) pv.refl = reflect(normalize(viewDir), pv.tnormal);
-    pv.spec = mk(0.0f, 0.0f, 0.0f);
-    pv.direct = pv.spec;
+    if (doSpec) pv.refl = reflect(normalize(viewDir), tnormal);
+    if (!doDiff) out[o] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (!doSpec) out[o + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     pv.flags = PV_VALID | (first ? PV_FIRST : 0u) | (doSpec ? PV_SPEC : 0u) | (doDiff ? PV_DIFF : 0u);
 }
 
-// The work units of one launch (a part of a request group, or a whole group in a many-map launch).  Per
-// unit: (1) pools of PK_POOL_FAN/K voxels (at least one): every ray of their specular fans, first-sample
-// shadow rays and shadow fans is traced by whichever lane is free -- a lane takes the pool's next ray as
-// soon as its own ended, and the shading of ended segments runs once `batch` lanes have one, so no lane
-// waits for the slowest ray of a fan; each ray's contributions go to shared memory, and when the pool is
-// empty every voxel's sums are formed in the reference's order; (2) the write-out of each voxel's
-// specular lighting and direct light (its diffuse paths run in k_light_diffuse).
+// The work units of one launch (a part of a request group).  Per unit: (1) the setup of its voxels; (2) pools of
+// PK_POOL_FAN/K voxels (at least one): the directions of all its specular rays, by whole warps; then every ray of
+// the specular fans, the shadow fans and the first-sample shadow rays is traced by whichever lane is free -- a lane
+// takes the pool's next ray as soon as its own ended, the shading of ended specular segments runs once `batch` lanes
+// have one, so no lane waits for the slowest ray of a fan; each ray's contributions go to shared memory, and when
+// the pool is empty every voxel's sums are formed in the reference's order and written (its diffuse paths run in
+// k_light_diffuse, which reads the direct light left in the voxel's diffuse slot).
 template <bool MANY, uint32_t POOL = PK_POOL_FAN>
-__device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLightArgs* many, PacketWarpT<POOL>& W)
+__device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLightArgs* many, PacketWarpT<POOL, PK_VOXELS>& W)
 {
     const uint32_t lane = lane_id_s();
+    const uint32_t below = (1u << lane) - 1u;
     uint32_t nreq = 0;
     if constexpr (MANY) nreq = *(volatile const uint32_t*)&many->reqStart[many->nmaps];
     else nreq = *(volatile const uint32_t*)one->nreqPtr;
@@ -144,15 +153,21 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
     const uint32_t batch = MANY ? many->batch : one->batch;
     Counters c{0, 0, 0, 0, 0};
     uint32_t lit = 0;
+    // the queue's groups: `big` ones in 2 units each, up to `mid` in 4, the rest in 8
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    const uint32_t lastMid = warps * PK_MID / 32u, lastTail = warps * PK_TAIL / 32u;
+    const uint32_t big = nreq > lastMid ? nreq - lastMid : 0u, mid = nreq > lastTail ? nreq - lastTail : 0u;
+    const uint32_t bigUnits = big * 2u, midUnits = bigUnits + (mid - big) * 4u, units = midUnits + (nreq - mid) * 8u;
     for (;;) {
         uint32_t u = 0;
         if (lane == 0) u = atomicAdd(counter, 1u);
         u = __shfl_sync(0xFFFFFFFFu, u, 0);
-        constexpr uint32_t parts = MANY ? 1u : PK_PARTS;
-        if (u >= nreq * parts) break;
-        // unit u: lanes [part * 32 / parts, (part + 1) * 32 / parts) of request group r
-        const uint32_t r = u / parts;
-        const bool mine = lane / (32u / parts) == u % parts;
+        if (u >= units) break;
+        // unit u: voxels [first, first + count) of request group r
+        uint32_t r, first, count;
+        if (u < bigUnits) { r = u >> 1; count = 16; first = (u & 1u) * 16u; }
+        else if (u < midUnits) { r = big + ((u - bigUnits) >> 2); count = 8; first = ((u - bigUnits) & 3u) * 8u; }
+        else { r = mid + ((u - midUnits) >> 3); count = 4; first = ((u - midUnits) & 7u) * 4u; }
         // the group's map (warp-uniform)
         const BatchLightMap* e = nullptr;
         uint32_t req = r;
@@ -171,235 +186,202 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
         const float (*sdir)[3] = MANY ? e->sdir : one->gtab->sdir;
         const float (*sinv)[3] = MANY ? e->sinv : one->gtab->sinv;
         float4* out = MANY ? e->out : one->out;
-        const f3 sun = mk(p.sunStrength[0], p.sunStrength[1], p.sunStrength[2]);
-        const f3 sunDir = mk(p.sunDir[0], p.sunDir[1], p.sunDir[2]);
         const uint32_t K = p.K;
+        const uint32_t overK = (65536u + K - 1u) / K;   // q / K = q * overK >> 16 for every q < 1024 (K <= 64)
 
-        if (mine) packet_setup(W.v[lane], req, lane, m, p, mats, MANY ? e->reqs : one->reqs, MANY ? e->nsamples : one->nsamples, out);
-        else W.v[lane].flags = 0;   // another unit's voxel: its warp sets it up and writes it
-        __syncwarp();
-        const uint32_t myFlags = W.v[lane].flags;
-        const uint32_t specAll = __ballot_sync(0xFFFFFFFFu, (myFlags & (PV_VALID | PV_SPEC)) == (PV_VALID | PV_SPEC));
-        const uint32_t specMask = p.specBounceLimit > 0u ? specAll : 0u;
-        // no specular segments: the sum stays zero and is still divided by K
-        if (!specMask && ((specAll >> lane) & 1u)) W.v[lane].spec = divs(mk(0.0f, 0.0f, 0.0f), (float)K);
-        const uint32_t diffMask = __ballot_sync(0xFFFFFFFFu, (myFlags & (PV_VALID | PV_DIFF)) == (PV_VALID | PV_DIFF));
+        uint32_t myFlags = 0;
+        if (lane < count) {
+            packet_setup(W.v[lane], req, first + lane, m, p, mats, MANY ? e->reqs : one->reqs, MANY ? e->nsamples : one->nsamples, out);
+            myFlags = W.v[lane].flags;
+        }
+        lit += myFlags & PV_VALID;
+        const uint32_t specMask = __ballot_sync(0xFFFFFFFFu, (myFlags & PV_SPEC) != 0u);
+        const uint32_t diffMask = __ballot_sync(0xFFFFFFFFu, (myFlags & PV_DIFF) != 0u);
         const uint32_t firstMask = diffMask & __ballot_sync(0xFFFFFFFFu, (myFlags & PV_FIRST) != 0u);
-        const uint32_t workMask = specMask | diffMask;
-        const uint32_t nWork = (uint32_t)__popc(workMask);
-        const uint32_t perPool = K < POOL ? POOL / K : 1u;
+        uint32_t todo = specMask | diffMask;
 
-        // per-lane ray state
         Ray s;
         s.mode = RM_IDLE;
-        bool live = false;
-        uint32_t rid = 0, ncon = 0;       // the lane's ray: index in its fan array; contributions so far
-        bool isSpec = false;
-        int vi = -1;                      // the ray's voxel
-        Job jd;                           // specular: jA mult, jB last position, jU reflect type, b bounce
-
-        // ---- (1) pools of specular and shadow fans
-        for (uint32_t base = 0; base < nWork; base += perPool) {
-            // the pool's voxels: slots j < np of workMask, from bit 'base' on; ray layout:
-            // [specular rays of voxel 0, 1, ...] then [shadow rays of voxel 0, 1, ...]
-            uint32_t rest = workMask;
-            for (uint32_t t = 0; t < base; t++) rest &= rest - 1u;
-            const uint32_t np = (nWork - base) < perPool ? (nWork - base) : perPool;
-            uint32_t poolMask = 0, rm = rest;
-            for (uint32_t t = 0; t < np; t++) { poolMask |= rm & (0u - rm); rm &= rm - 1u; }
-            const uint32_t nSpecRays = (uint32_t)__popc(poolMask & specMask) * K;
-            const uint32_t nFanVox = (uint32_t)__popc(poolMask & diffMask & ~firstMask);
-            const uint32_t nFirst = (uint32_t)__popc(poolMask & firstMask);
-            const uint32_t nShRays = nFanVox * K + nFirst;   // shadow rays in voxel order (1 or K per voxel)
-            const uint32_t total = nSpecRays + nShRays;
+        uint32_t q = 0;       // the lane's ray: its number in the pool
+        while (todo) {
+            // the pool's voxels: the lowest perPool bits left; its rays: K per specular voxel, then K per fan voxel,
+            // then one per first-sample voxel
+            const uint32_t perPool = K < POOL ? POOL * overK >> 16 : 1u;
+            const bool mine = ((todo >> lane) & 1u) && (uint32_t)__popc(todo & below) < perPool;
+            const uint32_t poolMask = __ballot_sync(0xFFFFFFFFu, mine);
+            todo &= ~poolMask;
+            const uint32_t specs = poolMask & specMask, fans = poolMask & diffMask & ~firstMask, firsts = poolMask & firstMask;
+            __syncwarp();   // the last pool's sums have been read
+            if ((specs >> lane) & 1u) W.specList[__popc(specs & below)] = (uint8_t)lane;
+            if ((fans >> lane) & 1u) W.fanList[__popc(fans & below)] = (uint8_t)lane;
+            if ((firsts >> lane) & 1u) W.firstList[__popc(firsts & below)] = (uint8_t)lane;
+            __syncwarp();
+            const uint32_t nSpec = (uint32_t)__popc(specs) * K, nFan = (uint32_t)__popc(fans) * K;
+            const uint32_t total = nSpec + nFan + (uint32_t)__popc(firsts);
+            // specular directions (voxelLighting.comp:83-97) and their reciprocals, a ray per lane
+            for (uint32_t i = lane; i < nSpec; i += 32u) {
+                const uint32_t j = i * overK >> 16, k = i - j * K;
+                const PacketVoxel& pv = W.v[W.specList[j]];
+                const f3 P = mk(p.spherePts[k][0], p.spherePts[k][1], p.spherePts[k][2]);
+                const f3 d = adds(normalize(add(muls(pv.refl, (float)mats[pv.tmat].shininess), P)), EPS);
+                const f3 inv = rcp3(d);
+                W.con[0][i] = d.x; W.con[1][i] = d.y; W.con[2][i] = d.z;
+                W.con[3][i] = inv.x; W.con[4][i] = inv.y; W.con[5][i] = inv.z;
+            }
+            __syncwarp();
             uint32_t next = 0;
-            for (int guard = 0; guard < (1 << 30); guard++) {
+            for (;;) {
                 // lanes without a ray take the pool's next rays in order
-                const unsigned need = __ballot_sync(0xFFFFFFFFu, !live);
+                const unsigned need = __ballot_sync(0xFFFFFFFFu, s.mode == RM_IDLE);
                 if (next < total && need) {
-                    const uint32_t rank = __popc(need & ((1u << lane) - 1u));
-                    if (!live && next + rank < total) {
-                        const uint32_t q = next + rank;
-                        if (q < nSpecRays) {
-                            // specular ray kk of the pool's (q / K)-th specular voxel
-                            isSpec = true;
-                            rid = q;
-                            const uint32_t kk = q % K;
-                            uint32_t mm = poolMask & specMask;
-                            for (uint32_t t = 0; t < q / K; t++) mm &= mm - 1u;
-                            vi = __ffs(mm) - 1;
-                            const PacketVoxel& pv = W.v[vi];
-                            const Material& tm = mats[pv.tmat];
-                            jd.jA = pv.talbedo; jd.jB = pv.pos0; jd.jU = tm.reflectType; jd.b = 0; ncon = 0;
-                            const f3 P = mk(p.spherePts[kk][0], p.spherePts[kk][1], p.spherePts[kk][2]);
-                            const f3 sd = adds(normalize(add(muls(pv.refl, (float)tm.shininess), P)), EPS);
-                            ray_begin<false>(s, m, pv.pos0, sd, rcp3(sd), false, c);
+                    const uint32_t mineq = next + (uint32_t)__popc(need & below);
+                    if (s.mode == RM_IDLE && mineq < total) {
+                        q = mineq;
+                        uint32_t vi;
+                        f3 d, inv;
+                        if (q < nSpec) {
+                            vi = W.specList[q * overK >> 16];
+                            d = mk(W.con[0][q], W.con[1][q], W.con[2][q]);
+                            inv = mk(W.con[3][q], W.con[4][q], W.con[5][q]);
                         } else {
-                            // shadow ray: voxels of the pool in slot order, K rays each (1 on the first sample)
-                            isSpec = false;
-                            rid = q - nSpecRays;
-                            uint32_t mm = poolMask & diffMask, off = 0, kk = 0;
-                            vi = -1;
-                            while (mm) {
-                                const int v = __ffs(mm) - 1;
-                                mm &= mm - 1u;
-                                const uint32_t n = ((firstMask >> v) & 1u) ? 1u : K;
-                                if (rid < off + n) { vi = v; kk = ((firstMask >> v) & 1u) ? 64u : rid - off; break; }
-                                off += n;
+                            const uint32_t f = q - nSpec;
+                            uint32_t k = 64u;
+                            if (f < nFan) {
+                                const uint32_t j = f * overK >> 16;
+                                vi = W.fanList[j];
+                                k = f - j * K;
+                            } else {
+                                vi = W.firstList[f - nFan];
                             }
-                            ray_begin<false>(s, m, W.v[vi].pos0, mk(sdir[kk][0], sdir[kk][1], sdir[kk][2]),
-                                      mk(sinv[kk][0], sinv[kk][1], sinv[kk][2]), false, c);
+                            d = mk(sdir[k][0], sdir[k][1], sdir[k][2]);
+                            inv = mk(sinv[k][0], sinv[k][1], sinv[k][2]);
                         }
                         c.rays++;
-                        live = true;
+                        ray_begin<false>(s, m, W.v[vi].pos0, d, inv, false, c, W.tint, lane);
                     }
-                    next = (next + (uint32_t)__popc(need)) < total ? next + (uint32_t)__popc(need) : total;
+                    next = min(next + (uint32_t)__popc(need), total);
                 }
-                const unsigned liveMask = __ballot_sync(0xFFFFFFFFu, live);
-                if (!liveMask) break;
+                const unsigned live = __ballot_sync(0xFFFFFFFFu, s.mode != RM_IDLE);
+                if (!live) break;
                 // step until 'batch' lanes have an ended segment (or none is left stepping); the live lanes
-                // do not change while stepping, so one vote per step tells both
+                // do not change while stepping, so one vote per round tells both
                 for (;;) {
                     const unsigned st = __ballot_sync(0xFFFFFFFFu, ray_stepping(s));
-                    if (!st || (uint32_t)__popc(liveMask & ~st) >= batch) break;
-                    if (ray_stepping(s)) walk_round<false>(s, m, mats, p.sunStrength, c);
+                    if (!st || (uint32_t)__popc(live & ~st) >= batch) break;
+                    if (ray_stepping(s)) walk_round<false>(s, m, mats, p.sunStrength, c, W.tint, lane);
                 }
                 // shade the ended segments
-                if (!live || ray_stepping(s)) continue;
+                if (s.mode == RM_IDLE || ray_stepping(s)) continue;
+                const f3 sun = mk(p.sunStrength[0], p.sunStrength[1], p.sunStrength[2]);
+                f3 cadd;
+                float cmul;
+                ray_tint(s, W.tint, lane, cadd, cmul);
                 const bool hit = s.mode == RM_HIT;
-                if (isSpec) {
-                    // specular_ray body after step_map (voxelLighting.comp:98-144)
-                    const PacketVoxel& pv = W.v[vi];
-                    bool more = false, add_ = false;
-                    f3 sc = mk(0.0f, 0.0f, 0.0f);
-                    if (hit) {
-                        const f3 hpos = ray_hit_position<false>(s);
-                        Voxel hv;
-                        decompress(m, ray_hit_index(s, m), hv);
-                        const i3 hp{f2i(truncf(hpos.x)), f2i(truncf(hpos.y)), f2i(truncf(hpos.z))};
-                        if (in_map(m, hp)) {
-                            uint8_t* vp = &m.tvis[map_index(m, hp)];
-                            if (*vp == 0) *vp = 1;
-                        }
-                        const f3 d = vabs(sub(vfloor(muls(hpos, 8.0f)), vfloor(muls(jd.jB, 8.0f))));
-                        if (!(dot(d, d) <= 1.0f)) {
-                            const Material& hm = mats[hv.material];
-                            const f3 hd = muls(hv.diff, 1.0f - hm.specular);
-                            add_ = true;
-                            if (hm.emissive) {
-                                sc.x = ((hv.albedo.x * p.emissiveStrength * s.cmul + s.cadd.x) * jd.jA.x) * pv.talbedo.x;
-                                sc.y = ((hv.albedo.y * p.emissiveStrength * s.cmul + s.cadd.y) * jd.jA.y) * pv.talbedo.y;
-                                sc.z = ((hv.albedo.z * p.emissiveStrength * s.cmul + s.cadd.z) * jd.jA.z) * pv.talbedo.z;
-                            } else {
-                                const f3 hc = mul(hd, hv.albedo);
-                                sc.x = (hc.x * s.cmul + s.cadd.x) * jd.jA.x;
-                                sc.y = (hc.y * s.cmul + s.cadd.y) * jd.jA.y;
-                                sc.z = (hc.z * s.cmul + s.cadd.z) * jd.jA.z;
-                                if (hm.specular != 0.0f) {
-                                    jd.jA.x = jd.jA.x * (hv.albedo.x * s.cmul * hm.specular);
-                                    jd.jA.y = jd.jA.y * (hv.albedo.y * s.cmul * hm.specular);
-                                    jd.jA.z = jd.jA.z * (hv.albedo.z * s.cmul * hm.specular);
-                                    jd.jU = hm.reflectType;
-                                    jd.jB = hpos;
-                                    const f3 nd = reflect(s.dir, hv.normal);
-                                    jd.b++;
-                                    if (jd.b < p.specBounceLimit) {
-                                        ray_begin<false>(s, m, hpos, nd, rcp3(nd), true, c);
-                                        c.rays++;
-                                        more = true;
-                                    }
-                                }
-                            }
-                        }
-                    } else if (dot(s.dir, sunDir) > 0.99f) {
-                        add_ = true;
-                        sc.x = sun.x * s.cmul + s.cadd.x;
-                        sc.y = sun.y * s.cmul + s.cadd.y;
-                        sc.z = sun.z * s.cmul + s.cadd.z;
-                    } else {
-                        const f3 sky = (jd.jU == 1u) ? sky_color(mk(p.skyBot[0], p.skyBot[1], p.skyBot[2]),
-                                                                mk(p.skyTop[0], p.skyTop[1], p.skyTop[2]), s.dir) : sun;
-                        add_ = true;
-                        sc.x = (sky.x * s.cmul + s.cadd.x) * jd.jA.x;
-                        sc.y = (sky.y * s.cmul + s.cadd.y) * jd.jA.y;
-                        sc.z = (sky.z * s.cmul + s.cadd.z) * jd.jA.z;
-                    }
-                    if (add_ && ncon < PK_MAX_SPEC_SEGMENTS) {   // at most one per segment; the host checks the limit
-                        W.con[rid][ncon][0] = sc.x; W.con[rid][ncon][1] = sc.y; W.con[rid][ncon][2] = sc.z;
-                        ncon++;
-                    }
-                    if (!more) { W.ncon[rid] = (uint8_t)ncon; live = false; }
-                } else {
+                s.mode = RM_IDLE;
+                if (q >= nSpec) {
                     // shadow_ray: an unoccluded ray adds sunStrength * colorMult + colorAdd
-                    W.sh[rid][0] = sun.x * s.cmul + s.cadd.x;
-                    W.sh[rid][1] = sun.y * s.cmul + s.cadd.y;
-                    W.sh[rid][2] = sun.z * s.cmul + s.cadd.z;
-                    W.shHas[rid] = hit ? 0 : 1;
-                    live = false;
+                    const uint32_t f = q - nSpec;
+                    W.sh[0][f] = sun.x * cmul + cadd.x;
+                    W.sh[1][f] = sun.y * cmul + cadd.y;
+                    W.sh[2][f] = sun.z * cmul + cadd.z;
+                    W.shHas[f] = hit ? 0 : 1;
+                    continue;
                 }
-            }
-            __syncwarp();
-            // the pool's sums in the reference's order: lane 2j sums voxel j's specular rays (ray, then
-            // segment order), lane 2j+1 its shadow rays; pools of more than 16 voxels (small K) take a
-            // second round
-            for (uint32_t j = lane >> 1; j < np; j += 16u) {
-                {
-                    uint32_t mm = poolMask;
-                    for (uint32_t t = 0; t < j; t++) mm &= mm - 1u;
-                    const int v = __ffs(mm) - 1;
-                    f3 acc = mk(0.0f, 0.0f, 0.0f);
-                    if ((lane & 1u) == 0u) {
-                        if ((specMask >> v) & 1u) {
-                            const uint32_t r0 = (uint32_t)__popc(poolMask & specMask & ((1u << v) - 1u)) * K;
-                            for (uint32_t k2 = 0; k2 < K; k2++) {
-                                const uint32_t n = W.ncon[r0 + k2];
-                                for (uint32_t jj = 0; jj < n; jj++) {
-                                    acc.x = acc.x + W.con[r0 + k2][jj][0];
-                                    acc.y = acc.y + W.con[r0 + k2][jj][1];
-                                    acc.z = acc.z + W.con[r0 + k2][jj][2];
-                                }
-                            }
-                            W.v[v].spec = divs(acc, (float)K);
-                        }
-                    } else if ((diffMask >> v) & 1u) {
-                        uint32_t r0 = 0, mm2 = poolMask & diffMask & ((1u << v) - 1u);
-                        while (mm2) {
-                            const int u = __ffs(mm2) - 1;
-                            mm2 &= mm2 - 1u;
-                            r0 += ((firstMask >> u) & 1u) ? 1u : K;
-                        }
-                        const uint32_t n = ((firstMask >> v) & 1u) ? 1u : K;
-                        for (uint32_t k2 = 0; k2 < n; k2++)
-                            if (W.shHas[r0 + k2]) {
-                                acc.x = acc.x + W.sh[r0 + k2][0];
-                                acc.y = acc.y + W.sh[r0 + k2][1];
-                                acc.z = acc.z + W.sh[r0 + k2][2];
-                            }
-                        W.v[v].direct = divs(acc, (float)n);
+                // specular_ray body after step_map (voxelLighting.comp:98-144).  A bounced segment started at the
+                // last hit position (its origin) and left the multiplier in con and its material's sky flag in s.flags
+                const PacketVoxel& pv = W.v[W.specList[q * overK >> 16]];
+                const bool bounced = (s.flags & RF_BOUNCED) != 0u;
+                const f3 mult = bounced ? mk(W.con[3][q], W.con[4][q], W.con[5][q]) : pv.talbedo;
+                bool more = false, add_ = true;
+                f3 sc;
+                if (hit) {
+                    const f3 hpos = ray_hit_position<false>(s);
+                    Voxel hv;
+                    decompress(m, ray_hit_index(s, m), hv);
+                    const i3 hp{f2i(truncf(hpos.x)), f2i(truncf(hpos.y)), f2i(truncf(hpos.z))};
+                    if (in_map(m, hp)) {
+                        uint8_t* vp = &m.tvis[map_index(m, hp)];
+                        if (*vp == 0) *vp = 1;
                     }
+                    const f3 d = vabs(sub(vfloor(muls(hpos, 8.0f)), vfloor(muls(s.pos, 8.0f))));
+                    add_ = !(dot(d, d) <= 1.0f);
+                    if (add_) {
+                        const Material& hm = mats[hv.material];
+                        const f3 hd = muls(hv.diff, 1.0f - hm.specular);
+                        if (hm.emissive) {
+                            sc.x = ((hv.albedo.x * p.emissiveStrength * cmul + cadd.x) * mult.x) * pv.talbedo.x;
+                            sc.y = ((hv.albedo.y * p.emissiveStrength * cmul + cadd.y) * mult.y) * pv.talbedo.y;
+                            sc.z = ((hv.albedo.z * p.emissiveStrength * cmul + cadd.z) * mult.z) * pv.talbedo.z;
+                        } else {
+                            const f3 hc = mul(hd, hv.albedo);
+                            sc.x = (hc.x * cmul + cadd.x) * mult.x;
+                            sc.y = (hc.y * cmul + cadd.y) * mult.y;
+                            sc.z = (hc.z * cmul + cadd.z) * mult.z;
+                            if (hm.specular != 0.0f && !bounced && p.specBounceLimit > 1u) {
+                                // the bounce
+                                more = true;
+                                W.con[3][q] = mult.x * (hv.albedo.x * cmul * hm.specular);
+                                W.con[4][q] = mult.y * (hv.albedo.y * cmul * hm.specular);
+                                W.con[5][q] = mult.z * (hv.albedo.z * cmul * hm.specular);
+                                const f3 nd = reflect(s.dir, hv.normal);
+                                ray_begin<false>(s, m, hpos, nd, rcp3(nd), true, c, W.tint, lane);
+                                s.flags |= RF_BOUNCED | (hm.reflectType == 1u ? RF_SKY : 0u);
+                                c.rays++;
+                            }
+                        }
+                    }
+                } else if (dot(s.dir, mk(p.sunDir[0], p.sunDir[1], p.sunDir[2])) > 0.99f) {
+                    sc.x = sun.x * cmul + cadd.x;
+                    sc.y = sun.y * cmul + cadd.y;
+                    sc.z = sun.z * cmul + cadd.z;
+                } else {
+                    const bool reflectsSky = bounced ? (s.flags & RF_SKY) != 0u : mats[pv.tmat].reflectType == 1u;
+                    const f3 sky = reflectsSky ? sky_color(mk(p.skyBot[0], p.skyBot[1], p.skyBot[2]),
+                                                           mk(p.skyTop[0], p.skyTop[1], p.skyTop[2]), s.dir) : sun;
+                    sc.x = (sky.x * cmul + cadd.x) * mult.x;
+                    sc.y = (sky.y * cmul + cadd.y) * mult.y;
+                    sc.z = (sky.z * cmul + cadd.z) * mult.z;
                 }
+                if (add_) {
+                    const uint32_t at = bounced ? 3u : 0u;
+                    W.con[at][q] = sc.x; W.con[at + 1u][q] = sc.y; W.con[at + 2u][q] = sc.z;
+                }
+                if (!more) W.ncon[q] = (uint8_t)((bounced ? 1u : 0u) + (add_ ? 1u : 0u));
             }
             __syncwarp();
+            // the pool's sums in the reference's order (ray, then segment), a component of a voxel's specular or
+            // direct light per lane, written as the voxel's lighting (voxelLighting.comp:266-288, FP32)
+            const uint32_t nSpecSums = (uint32_t)__popc(specs) * 3u, nFanSums = (uint32_t)__popc(fans) * 3u;
+            const uint32_t nSums = nSpecSums + nFanSums + (uint32_t)__popc(firsts) * 3u;
+            for (uint32_t i = lane; i < nSums; i += 32u) {
+                float acc = 0.0f;
+                if (i < nSpecSums) {
+                    const uint32_t j = i / 3u, comp = i - 3u * j, v = W.specList[j];
+                    for (uint32_t k = j * K; k < j * K + K; k++) {
+                        const uint32_t n = W.ncon[k];
+                        if (n > 0u) acc = acc + W.con[comp][k];
+                        if (n > 1u) acc = acc + W.con[3u + comp][k];
+                    }
+                    acc = acc / (float)K;
+                    float* o = (float*)&out[((uint64_t)req * 32u + first + v) * 2u + 1u];
+                    o[comp] = gmin(gmax(acc, 0.0f), 1.0f);
+                    if (comp == 0u) o[3] = 0.0f;
+                } else {
+                    const uint32_t i2 = i - nSpecSums;
+                    const bool fan = i2 < nFanSums;
+                    const uint32_t i3 = fan ? i2 : i2 - nFanSums, j = i3 / 3u, comp = i3 - 3u * j;
+                    const uint32_t v = fan ? W.fanList[j] : W.firstList[j];
+                    const uint32_t k0 = fan ? j * K : nFan + j, n = fan ? K : 1u;
+                    for (uint32_t k = k0; k < k0 + n; k++)
+                        if (W.shHas[k]) acc = acc + W.sh[comp][k];
+                    acc = acc / (float)n;
+                    float* o = (float*)&out[((uint64_t)req * 32u + first + v) * 2u];
+                    o[comp] = acc;
+                    if (comp == 0u) o[3] = 0.0f;
+                }
+            }
         }
-
-        // ---- (2) write the voxel's specular lighting (voxelLighting.comp:266-288, FP32).  Its diffuse paths
-        // run in the diffuse kernel that follows (k_light_diffuse: per-lane path streams, so that one long
-        // path does not hold the other 31 lanes), which reads the direct light left here in the diffuse slot
-        // and replaces it with the voxel's new diffuse lighting; a voxel without diffuse paths gets zero.
-        __syncwarp();
-        if (myFlags & PV_VALID) {
-            const PacketVoxel& pv = W.v[lane];
-            const f3 sp = (myFlags & PV_SPEC) ? pv.spec : mk(0.0f, 0.0f, 0.0f);
-            const float4 outS = make_float4(gmin(gmax(sp.x, 0.0f), 1.0f), gmin(gmax(sp.y, 0.0f), 1.0f),
-                                            gmin(gmax(sp.z, 0.0f), 1.0f), 0.0f);
-            const float4 outD = (myFlags & PV_DIFF) ? make_float4(pv.direct.x, pv.direct.y, pv.direct.z, 0.0f)
-                                                    : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            const uint64_t o = ((uint64_t)req * 32u + lane) * 2u;
-            out[o] = outD;
-            out[o + 1] = outS;
-            lit++;
-        }
-        __syncwarp();
+        __syncwarp();   // the unit's voxels are read no more
     }
     flush_counters(MANY ? many->stats : one->stats, c, 0, lit);
 }

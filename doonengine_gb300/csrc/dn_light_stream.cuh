@@ -116,7 +116,7 @@ __device__ __forceinline__ f3 diffuse_dir(const Job& j, const dn_light_params& p
 // which left the direct light in the diffuse output slot); the final write replaces that slot with the
 // voxel's new diffuse lighting and leaves the specular slot and the lit-voxel count alone.
 template <bool DIFFONLY, bool FAR>
-__device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const dn_light_params& p,
+__device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const DevMap& m, const dn_light_params& p,
                                         const Material* mats, const float (*sdir)[3], const float (*sinv)[3],
                                         float4* out, Counters& c, uint32_t& lit)
 {
@@ -127,7 +127,9 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
         const bool hit = s.mode == RM_HIT;
         s.mode = RM_IDLE;
         Voxel hv;
-        f3 hpos = s.pos;
+        f3 hpos = s.pos, cadd;
+        float cmul;
+        ray_tint(s, tint, threadIdx.x, cadd, cmul);
         if (hit) {
             hpos = ray_hit_position<FAR>(s);
             decompress(m, ray_hit_index(s, m), hv);
@@ -148,24 +150,24 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                     const Material& hm = mats[hv.material];
                     const f3 hd = muls(hv.diff, 1.0f - hm.specular);
                     if (hm.emissive) {
-                        j.spec.x = j.spec.x + ((hv.albedo.x * p.emissiveStrength * s.cmul + s.cadd.x) * j.jA.x) * j.talbedo.x;
-                        j.spec.y = j.spec.y + ((hv.albedo.y * p.emissiveStrength * s.cmul + s.cadd.y) * j.jA.y) * j.talbedo.y;
-                        j.spec.z = j.spec.z + ((hv.albedo.z * p.emissiveStrength * s.cmul + s.cadd.z) * j.jA.z) * j.talbedo.z;
+                        j.spec.x = j.spec.x + ((hv.albedo.x * p.emissiveStrength * cmul + cadd.x) * j.jA.x) * j.talbedo.x;
+                        j.spec.y = j.spec.y + ((hv.albedo.y * p.emissiveStrength * cmul + cadd.y) * j.jA.y) * j.talbedo.y;
+                        j.spec.z = j.spec.z + ((hv.albedo.z * p.emissiveStrength * cmul + cadd.z) * j.jA.z) * j.talbedo.z;
                     } else {
                         const f3 hc = mul(hd, hv.albedo);
-                        j.spec.x = j.spec.x + (hc.x * s.cmul + s.cadd.x) * j.jA.x;
-                        j.spec.y = j.spec.y + (hc.y * s.cmul + s.cadd.y) * j.jA.y;
-                        j.spec.z = j.spec.z + (hc.z * s.cmul + s.cadd.z) * j.jA.z;
+                        j.spec.x = j.spec.x + (hc.x * cmul + cadd.x) * j.jA.x;
+                        j.spec.y = j.spec.y + (hc.y * cmul + cadd.y) * j.jA.y;
+                        j.spec.z = j.spec.z + (hc.z * cmul + cadd.z) * j.jA.z;
                         if (hm.specular != 0.0f) {
-                            j.jA.x = j.jA.x * (hv.albedo.x * s.cmul * hm.specular);
-                            j.jA.y = j.jA.y * (hv.albedo.y * s.cmul * hm.specular);
-                            j.jA.z = j.jA.z * (hv.albedo.z * s.cmul * hm.specular);
+                            j.jA.x = j.jA.x * (hv.albedo.x * cmul * hm.specular);
+                            j.jA.y = j.jA.y * (hv.albedo.y * cmul * hm.specular);
+                            j.jA.z = j.jA.z * (hv.albedo.z * cmul * hm.specular);
                             j.jU = hm.reflectType;
                             j.jB = hpos;
                             const f3 nd = reflect(s.dir, hv.normal);
                             j.b++;
                             if (j.b < p.specBounceLimit) {
-                                ray_begin<FAR>(s, m, hpos, nd, rcp3(nd), true, c);   // next bounce
+                                ray_begin<FAR>(s, m, hpos, nd, rcp3(nd), true, c, tint, threadIdx.x);   // next bounce
                                 c.rays++;
                                 return true;
                             }
@@ -173,22 +175,22 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                     }
                 }
             } else if (dot(s.dir, sunDir) > 0.99f) {
-                j.spec.x = j.spec.x + (sun.x * s.cmul + s.cadd.x);
-                j.spec.y = j.spec.y + (sun.y * s.cmul + s.cadd.y);
-                j.spec.z = j.spec.z + (sun.z * s.cmul + s.cadd.z);
+                j.spec.x = j.spec.x + (sun.x * cmul + cadd.x);
+                j.spec.y = j.spec.y + (sun.y * cmul + cadd.y);
+                j.spec.z = j.spec.z + (sun.z * cmul + cadd.z);
             } else {
                 const f3 sc = (j.jU == 1u) ? sky_color(mk(p.skyBot[0], p.skyBot[1], p.skyBot[2]),
                                                       mk(p.skyTop[0], p.skyTop[1], p.skyTop[2]), s.dir) : sun;
-                j.spec.x = j.spec.x + (sc.x * s.cmul + s.cadd.x) * j.jA.x;
-                j.spec.y = j.spec.y + (sc.y * s.cmul + s.cadd.y) * j.jA.y;
-                j.spec.z = j.spec.z + (sc.z * s.cmul + s.cadd.z) * j.jA.z;
+                j.spec.x = j.spec.x + (sc.x * cmul + cadd.x) * j.jA.x;
+                j.spec.y = j.spec.y + (sc.y * cmul + cadd.y) * j.jA.y;
+                j.spec.z = j.spec.z + (sc.z * cmul + cadd.z) * j.jA.z;
             }
             if (done) { j.k++; j.b = 0; }
         } else if (!DIFFONLY && j.phase == PH_SHADOW) {
             if (!hit) {
-                j.acc.x = j.acc.x + (sun.x * s.cmul + s.cadd.x);
-                j.acc.y = j.acc.y + (sun.y * s.cmul + s.cadd.y);
-                j.acc.z = j.acc.z + (sun.z * s.cmul + s.cadd.z);
+                j.acc.x = j.acc.x + (sun.x * cmul + cadd.x);
+                j.acc.y = j.acc.y + (sun.y * cmul + cadd.y);
+                j.acc.z = j.acc.z + (sun.z * cmul + cadd.z);
             }
             j.k++;
         } else if (j.phase == PH_DIFF) {
@@ -201,18 +203,18 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                 if (!(dot(d, d) < 1.0f)) {
                     const Material& hm = mats[hv.material];
                     if (hm.emissive) {
-                        j.acc.x = j.acc.x + j.jA.x * (hv.albedo.x * p.emissiveStrength * s.cmul + s.cadd.x);
-                        j.acc.y = j.acc.y + j.jA.y * (hv.albedo.y * p.emissiveStrength * s.cmul + s.cadd.y);
-                        j.acc.z = j.acc.z + j.jA.z * (hv.albedo.z * p.emissiveStrength * s.cmul + s.cadd.z);
+                        j.acc.x = j.acc.x + j.jA.x * (hv.albedo.x * p.emissiveStrength * cmul + cadd.x);
+                        j.acc.y = j.acc.y + j.jA.y * (hv.albedo.y * p.emissiveStrength * cmul + cadd.y);
+                        j.acc.z = j.acc.z + j.jA.z * (hv.albedo.z * p.emissiveStrength * cmul + cadd.z);
                     } else {
-                        j.jA.x = j.jA.x * (hv.albedo.x * s.cmul + s.cadd.x);
-                        j.jA.y = j.jA.y * (hv.albedo.y * s.cmul + s.cadd.y);
-                        j.jA.z = j.jA.z * (hv.albedo.z * s.cmul + s.cadd.z);
+                        j.jA.x = j.jA.x * (hv.albedo.x * cmul + cadd.x);
+                        j.jA.y = j.jA.y * (hv.albedo.y * cmul + cadd.y);
+                        j.jA.z = j.jA.z * (hv.albedo.z * cmul + cadd.z);
                         j.jC = s.dir;
                         j.b++;
                         if (j.b < p.diffuseBounceLimit) {
                             const f3 nd = diffuse_dir(j, p, mats, rngSin);
-                            ray_begin<FAR>(s, m, hpos, nd, rcp3(nd), true, c);
+                            ray_begin<FAR>(s, m, hpos, nd, rcp3(nd), true, c, tint, threadIdx.x);
                             c.rays++;
                             return true;
                         }
@@ -220,9 +222,9 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                 }
             } else {
                 const float k = gmax(dot(s.dir, sunDir), 0.0f);
-                j.acc.x = j.acc.x + (j.jA.x * k * sun.x * s.cmul + s.cadd.x);
-                j.acc.y = j.acc.y + (j.jA.y * k * sun.y * s.cmul + s.cadd.y);
-                j.acc.z = j.acc.z + (j.jA.z * k * sun.z * s.cmul + s.cadd.z);
+                j.acc.x = j.acc.x + (j.jA.x * k * sun.x * cmul + cadd.x);
+                j.acc.y = j.acc.y + (j.jA.y * k * sun.y * cmul + cadd.y);
+                j.acc.z = j.acc.z + (j.jA.z * k * sun.z * cmul + cadd.z);
             }
             if (pathDone) { j.acc = add(j.acc, j.direct); j.i++; j.b = 0; }
         }
@@ -236,7 +238,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                 j.b = 0; j.jA = j.talbedo; j.jB = j.pos0; j.jU = tm.reflectType;
                 const f3 P = mk(p.spherePts[j.k][0], p.spherePts[j.k][1], p.spherePts[j.k][2]);
                 const f3 sd = adds(normalize(add(muls(j.refl, (float)tm.shininess), P)), EPS);
-                ray_begin<FAR>(s, m, j.pos0, sd, rcp3(sd), false, c);
+                ray_begin<FAR>(s, m, j.pos0, sd, rcp3(sd), false, c, tint, threadIdx.x);
                 c.rays++;
                 return true;
             }
@@ -249,7 +251,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
             const uint32_t n = j.firstSample ? 1u : p.K;
             if (j.k < n) {
                 const uint32_t q = j.firstSample ? 64u : j.k;
-                ray_begin<FAR>(s, m, j.pos0, mk(sdir[q][0], sdir[q][1], sdir[q][2]), mk(sinv[q][0], sinv[q][1], sinv[q][2]), false, c);
+                ray_begin<FAR>(s, m, j.pos0, mk(sdir[q][0], sdir[q][1], sdir[q][2]), mk(sinv[q][0], sinv[q][1], sinv[q][2]), false, c, tint, threadIdx.x);
                 c.rays++;
                 return true;
             }
@@ -271,7 +273,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, const DevMap& m, const d
                     j.jU = j.tmat;
                 }
                 const f3 nd = diffuse_dir(j, p, mats, rngSin);
-                ray_begin<FAR>(s, m, j.pos0, nd, rcp3(nd), false, c);
+                ray_begin<FAR>(s, m, j.pos0, nd, rcp3(nd), false, c, tint, threadIdx.x);
                 c.rays++;
                 return true;
             }
@@ -413,7 +415,7 @@ __device__ __forceinline__ void shadow_dir(const dn_light_params& p, int k, floa
 // its device tables (one->gtab) and sh is not used.  FAR: maps above FAR_SUM chunks (dn_walk.cuh).
 template <bool MANY, bool DIFFONLY, bool FAR>
 __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLightArgs* many, const StreamShared* sh,
-                                            Job& j)
+                                            Job& j, TintT<128>& tint)
 {
     const uint32_t lane = lane_id_s();
     const uint32_t batch = MANY ? many->batch : one->batch;
@@ -493,17 +495,17 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
                 if (!ray_stepping(s) && j.phase != PH_DONE && j.phase != PH_FETCH) {
                     if constexpr (MANY) {
                         if (j.map != lmi) { le = &many->maps[j.map]; lmi = j.map; }
-                        advance<DIFFONLY, FAR>(j, s, le->m, le->p, le->mats, le->sdir, le->sinv, le->out, c, lit);
+                        advance<DIFFONLY, FAR>(j, s, tint, le->m, le->p, le->mats, le->sdir, le->sinv, le->out, c, lit);
                     } else if constexpr (DIFFONLY) {
-                        advance<true, FAR>(j, s, one->m, one->p, MATS(), one->gtab->sdir, one->gtab->sinv, one->out, c, lit);
+                        advance<true, FAR>(j, s, tint, one->m, one->p, MATS(), one->gtab->sdir, one->gtab->sinv, one->out, c, lit);
                     } else {
-                        advance<false, FAR>(j, s, one->m, one->p, sh->mats, sh->sdir, sh->sinv, one->out, c, lit);
+                        advance<false, FAR>(j, s, tint, one->m, one->p, sh->mats, sh->sdir, sh->sinv, one->out, c, lit);
                     }
                 }
                 if (__ballot_sync(0xFFFFFFFFu, j.phase == PH_FETCH) == 0u) break;
             }
         }
-        if (ray_stepping(s)) walk_round<FAR>(s, M(), MATS(), P().sunStrength, c);
+        if (ray_stepping(s)) walk_round<FAR>(s, M(), MATS(), P().sunStrength, c, tint, threadIdx.x);
     }
     flush_counters(MANY ? many->stats : one->stats, c, 0, lit);
 }

@@ -54,7 +54,8 @@ enum : uint32_t {
     RM_HIT = 5,           // ended on a voxel
     RM_MISS = 6           // left the map
 };
-enum : uint32_t { RF_REQUESTED = 1u, RF_IGNORE = 2u, RF_OPAQUE = 4u };
+enum : uint32_t { RF_REQUESTED = 1u, RF_IGNORE = 2u, RF_OPAQUE = 4u, RF_TINT = 8u,
+                  RF_BOUNCED = 16u, RF_SKY = 32u };   // the last two: the packet kernel's
 
 struct Ray {
     f3 pos, dir, delta;      // origin, direction, |1 / direction|
@@ -62,9 +63,15 @@ struct Ray {
     f3 side; float last, v;  // voxel level: the same; v codes the cell and the steps left (voxel_code)
     uint32_t slot;           // record of the entered chunk
     uint32_t mode, flags;
-    f3 cadd; float cmul;     // light of the see-through voxels crossed
-    uint32_t lastId, lastAt; // the last see-through voxel's identity, and the lane's voxel-cell count there
     uint32_t seg;            // FAR: cells visited by the segment
+};
+
+// What see-through voxels did to a lane's ray, in shared memory (one column per lane): most rays meet none, and
+// the six registers buy a third more resident warps.  Valid while the ray's RF_TINT is set.
+template <int LANES>
+struct TintT {
+    float add[3][LANES], mul[LANES];            // light gained, and the share that still passes
+    uint32_t lastId[LANES], lastAt[LANES];      // the last see-through voxel's identity, and the lane's voxel-cell count there
 };
 
 __device__ __forceinline__ bool ray_stepping(const Ray& r) { return r.mode - RM_OUTER < 4u; }
@@ -184,14 +191,13 @@ __device__ __forceinline__ void ray_request(Ray& r, const DevMap& m, i3 cell)
 
 // Starts a segment (step_map's set-up, voxelShared.comp:421-433, first voxel ignored).  keep: a bounce of the
 // same ray job, which keeps the transparency state (D13).
-template <bool FAR>
-__device__ __forceinline__ void ray_begin(Ray& r, const DevMap& m, f3 pos, f3 dir, f3 inv, bool keep, Counters& c)
+template <bool FAR, class Tint>
+__device__ __forceinline__ void ray_begin(Ray& r, const DevMap& m, f3 pos, f3 dir, f3 inv, bool keep, Counters& c, Tint& t,
+                                          uint32_t col)
 {
     r.pos = pos; r.dir = dir; r.delta = vabs(inv);
-    r.cadd = mk(0.0f, 0.0f, 0.0f);
-    r.cmul = 1.0f;
-    if (!keep) { r.lastId = 255u; r.lastAt = 0xFFFFFFFFu; }
-    r.flags = 0;
+    r.flags = keep ? r.flags & RF_TINT : 0u;
+    if (r.flags) { t.add[0][col] = 0.0f; t.add[1][col] = 0.0f; t.add[2][col] = 0.0f; t.mul[col] = 1.0f; }
     r.seg = 0;
     r.olast = 0.0f;
     const f3 fl = vfloor(pos);
@@ -212,7 +218,7 @@ __device__ __forceinline__ void ray_begin(Ray& r, const DevMap& m, f3 pos, f3 di
     const uint32_t st = cell_state<FAR>(m, r.cell);
     if (st >= 2u) {
         r.mode = st;
-        r.flags = RF_IGNORE;
+        r.flags |= RF_IGNORE;
         return;
     }
     c.outer++;
@@ -222,9 +228,9 @@ __device__ __forceinline__ void ray_begin(Ray& r, const DevMap& m, f3 pos, f3 di
 }
 
 // one round: see the file comment
-template <bool FAR>
+template <bool FAR, class Tint>
 __device__ __forceinline__ void walk_round(Ray& r, const DevMap& m, const Material* mats, const float* sunStrength,
-                                           Counters& c)
+                                           Counters& c, Tint& t, uint32_t col)
 {
     const f3 sg = mk(copysignf(1.0f, r.dir.x), copysignf(1.0f, r.dir.y), copysignf(1.0f, r.dir.z));
     // FAR: counts k visited cells at a level; false (the segment ends as a miss, D16) when the cap comes before the last
@@ -260,9 +266,9 @@ __device__ __forceinline__ void walk_round(Ray& r, const DevMap& m, const Materi
     }
     bool occ = false;
     if ((r.mode == RM_ENTER || r.mode == RM_ENTER_OPAQUE) && visit(c.outer, 1u)) {
-        const uint32_t t = map_index(m, cell_ints<FAR>(r.cell));
-        r.slot = __ldg(&m.tword[t]) & SLOT_MASK;
-        if (m.ttouch[t] == 0) m.ttouch[t] = 1;
+        const uint32_t tile = map_index(m, cell_ints<FAR>(r.cell));
+        r.slot = __ldg(&m.tword[tile]) & SLOT_MASK;
+        if (m.ttouch[tile] == 0) m.ttouch[tile] = 1;
         c.entered++;
         const f3 cp = chunk_entry(r.pos, r.dir, r.olast, cell_pos<FAR>(r.cell));
         const f3 fl = vfloor(cp);
@@ -273,7 +279,7 @@ __device__ __forceinline__ void walk_round(Ray& r, const DevMap& m, const Materi
         r.v = voxel_code(sg, fl);
         const uint32_t op = r.mode == RM_ENTER_OPAQUE ? RF_OPAQUE : 0u;
         if (!(r.flags & RF_IGNORE)) occ = voxel_occupied(&m.rec[r.slot], r.v);
-        r.flags = (r.flags & RF_REQUESTED) | op;
+        r.flags = (r.flags & ~(RF_IGNORE | RF_OPAQUE)) | op;
         r.mode = RM_INNER;
         visit(c.inner, 1u);
     }
@@ -302,7 +308,8 @@ __device__ __forceinline__ void walk_round(Ray& r, const DevMap& m, const Materi
         } else if (occ) {
             c.hits++;
             // whether the voxel cell before this one was see-through (no empty voxel cell in between)
-            const bool run = r.lastAt + 1u == c.inner;
+            const bool tinted = (r.flags & RF_TINT) != 0u;
+            const bool run = tinted && t.lastAt[col] + 1u == c.inner;
             bool opaque = (r.flags & RF_OPAQUE) != 0u;
             if (!opaque) {
                 const ChunkRec* rc = &m.rec[r.slot];
@@ -313,25 +320,39 @@ __device__ __forceinline__ void walk_round(Ray& r, const DevMap& m, const Materi
                 opaque = mat.opacity == 1.0f;
                 if (!opaque) {
                     const uint32_t thisID = (vw.y & 0xFFFFFF00u) | material;
-                    if ((run ? r.lastId : 255u) != thisID) {
+                    if (!tinted) {
+                        t.add[0][col] = 0.0f; t.add[1][col] = 0.0f; t.add[2][col] = 0.0f; t.mul[col] = 1.0f;
+                        r.flags |= RF_TINT;
+                    }
+                    if (!run || t.lastId[col] != thisID) {
                         const f3 alb = mk((float)((vw.y >> 24) & 0xFF) * INV255, (float)((vw.y >> 16) & 0xFF) * INV255,
                                           (float)((vw.y >> 8) & 0xFF) * INV255);
-                        const float k = r.cmul * mat.opacity;
-                        r.cadd.x = r.cadd.x + k * alb.x * sunStrength[0];
-                        r.cadd.y = r.cadd.y + k * alb.y * sunStrength[1];
-                        r.cadd.z = r.cadd.z + k * alb.z * sunStrength[2];
-                        r.cmul = r.cmul * (1.0f - mat.opacity);
-                        r.lastId = thisID;
+                        const float mul = t.mul[col];
+                        const float k = mul * mat.opacity;
+                        t.add[0][col] = t.add[0][col] + k * alb.x * sunStrength[0];
+                        t.add[1][col] = t.add[1][col] + k * alb.y * sunStrength[1];
+                        t.add[2][col] = t.add[2][col] + k * alb.z * sunStrength[2];
+                        t.mul[col] = mul * (1.0f - mat.opacity);
+                        t.lastId[col] = thisID;
                     }
-                    r.lastAt = c.inner;
+                    t.lastAt[col] = c.inner;
                 }
             }
             if (opaque) {
                 r.mode = RM_HIT;
-                if (run) r.lastAt = c.inner;   // a bounce goes on from this cell with the same state
+                if (run) t.lastAt[col] = c.inner;   // a bounce goes on from this cell with the same state
             }
         }
     }
+}
+
+// the light a ray gained from see-through voxels, and the share that still passes
+template <class Tint>
+__device__ __forceinline__ void ray_tint(const Ray& r, const Tint& t, uint32_t col, f3& add, float& mul)
+{
+    add = mk(0.0f, 0.0f, 0.0f);
+    mul = 1.0f;
+    if (r.flags & RF_TINT) { add = mk(t.add[0][col], t.add[1][col], t.add[2][col]); mul = t.mul[col]; }
 }
 
 // the pool index of the voxel a ray ended on (RM_HIT)

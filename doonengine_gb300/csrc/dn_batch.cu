@@ -4,7 +4,7 @@
  * A frame of a batch is a fixed handful of device operations whatever the number of maps:
  *   1. one host-to-device copy of the frame's table (per-map parameters, image pointers, materials);
  *   2. k_batch_reset: zero the request counters of the maps whose per-tile pass runs;
- *   3. k_draw_batch: every pixel of every image (blocks of 8x32 pixels; a block belongs to one map);
+ *   3. k_draw_batch: every pixel of every image (blocks of 16x8 pixels; a block belongs to one map);
  *   4. k_compact_batch: the per-tile sync pass over every tile of every map (blocks of 256 tiles);
  *   5. k_batch_prep: clamp the request counts, lay the maps' request lists end to end as one queue (an
  *      exclusive prefix over the counts) and compute each map's shadow directions;
@@ -31,7 +31,7 @@ using namespace dn;
 struct BatchDrawEntry {
     DrawMap d;
     const Material* mats;
-    uint32_t gridX;             // blocks of 8 pixels across
+    uint32_t gridX;             // blocks across
 };
 
 struct DNgpuBatch {
@@ -84,7 +84,7 @@ __global__ void k_batch_reset(const CompactArgs* s, uint32_t ns)
 }
 
 template <bool FAR>
-__global__ void __launch_bounds__(256, DN_DRAW_MIN_BLOCKS) k_draw_batch(const BatchDrawEntry* d, const uint32_t* start, uint32_t nd,
+__global__ void __launch_bounds__(DN_DRAW_BX * DN_DRAW_BY, DN_DRAW_WARPS * 32 / (DN_DRAW_BX * DN_DRAW_BY)) k_draw_batch(const BatchDrawEntry* d, const uint32_t* start, uint32_t nd,
                                                     unsigned long long* stats)
 {
     const uint32_t mi = find_range(start, nd, blockIdx.x);
@@ -403,8 +403,8 @@ static int issue_frame(DNgpuBatch* b, const dn_batch_item* items, uint32_t n, co
         COUNT_LAUNCH();
         const BatchDrawEntry* de = (const BatchDrawEntry*)(d + t.oDraw);
         const uint32_t* ds = (const uint32_t*)(d + t.oDrawStart);
-        if (f.far) k_draw_batch<true><<<f.drawBlocks, dim3(8, 32), 0, s>>>(de, ds, t.nd, b->bst->stats);
-        else k_draw_batch<false><<<f.drawBlocks, dim3(8, 32), 0, s>>>(de, ds, t.nd, b->bst->stats);
+        if (f.far) k_draw_batch<true><<<f.drawBlocks, dim3(DN_DRAW_BX, DN_DRAW_BY), 0, s>>>(de, ds, t.nd, b->bst->stats);
+        else k_draw_batch<false><<<f.drawBlocks, dim3(DN_DRAW_BX, DN_DRAW_BY), 0, s>>>(de, ds, t.nd, b->bst->stats);
         CK(cudaGetLastError());
     }
     if (f.hostImages) {
@@ -568,9 +568,9 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
             e.d.face = it.faceOut ? (it.hostImage ? g->dface : it.faceOut) : nullptr;
             e.d.stats = b->bst->stats;
             e.mats = mats;
-            e.gridX = (it.draw.width + 7) / 8;
+            e.gridX = (it.draw.width + DN_DRAW_BX - 1) / DN_DRAW_BX;
             drawStart[id] = blocksD;
-            blocksD += e.gridX * ((it.draw.height + 31) / 32);
+            blocksD += e.gridX * ((it.draw.height + DN_DRAW_BY - 1) / DN_DRAW_BY);
             key.push_back((uint64_t)(uintptr_t)it.colorOut); key.push_back((uint64_t)(uintptr_t)it.hitOut);
             key.push_back((uint64_t)(uintptr_t)it.faceOut); key.push_back(((uint64_t)it.draw.width << 32) | it.draw.height);
             id++;

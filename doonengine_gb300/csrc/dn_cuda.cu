@@ -629,8 +629,8 @@ extern "C" int dn_cuda_reserve(DNgpuVolume* g, uint32_t slotCap, uint64_t voxelC
 
 // ------------------------------------------------------------------ draw
 
-template <bool FAR>
-__global__ void __launch_bounds__(256, DN_DRAW_MIN_BLOCKS) k_draw(const __grid_constant__ DrawArgs a)
+template <bool FAR, int WARPS>
+__global__ void __launch_bounds__(DN_DRAW_BX * DN_DRAW_BY, WARPS * 32 / (DN_DRAW_BX * DN_DRAW_BY)) k_draw(const __grid_constant__ DrawArgs a)
 {
     Counters c;
     const uint32_t primary = draw_pixel<FAR>(a.d, a.mats, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, c);
@@ -1292,17 +1292,14 @@ static int launch_draw(DNgpuVolume* g, const dn_draw_params* p, const dn_materia
     a->d.p = *p;
     a->d.color = color; a->d.hit = hit; a->d.face = face; a->d.stats = g->st->stats;
     memcpy(a->mats, materials, sizeof(a->mats));
-#ifndef DN_DRAW_BX
-// 8 x 32 pixels per block: 16 x 16 and 32 x 8 measured equal or slower (large map: draw + sync 0.78 ms
-// per frame with 8 x 32, 0.81 with 16 x 16, 0.89 with 32 x 8)
-#define DN_DRAW_BX 8
-#define DN_DRAW_BY 32
-#endif
     dim3 block(DN_DRAW_BX, DN_DRAW_BY);
     dim3 grid((p->width + DN_DRAW_BX - 1) / DN_DRAW_BX, (p->height + DN_DRAW_BY - 1) / DN_DRAW_BY);
     COUNT_LAUNCH();
-    if (map_far(g)) k_draw<true><<<grid, block, 0, g->stream>>>(*a);
-    else k_draw<false><<<grid, block, 0, g->stream>>>(*a);
+    // an image whose warps are all resident at 24 per SM takes the build for 24 (74 registers, no spills): a 257x143
+    // draw 13.1 us against 14.0
+    if (map_far(g)) k_draw<true, DN_DRAW_WARPS><<<grid, block, 0, g->stream>>>(*a);
+    else if (grid.x * grid.y * (DN_DRAW_BX * DN_DRAW_BY / 32u) <= 24u * (unsigned)g->numSMs) k_draw<false, 24><<<grid, block, 0, g->stream>>>(*a);
+    else k_draw<false, DN_DRAW_WARPS><<<grid, block, 0, g->stream>>>(*a);
     CK(cudaGetLastError());
     return DN_CUDA_OK;
 }

@@ -79,11 +79,17 @@ struct DNgpuVolume {
 
 
 
-#ifndef DN_DRAW_MIN_BLOCKS
-// resident 256-thread draw blocks per SM the register allocation must allow: 4 (64 registers, 16 bytes of spills).
-// A 1080p draw of the 64x32x64 map: 335 us, 3 blocks 369, 5 blocks 323; a 257x143 draw 14.0, 13.0, 14.6; edited
-// frames at 720p 211, 215, 214
-#define DN_DRAW_MIN_BLOCKS 4
+// The draw's blocks: 16 x 8 pixels (a warp 16 x 2, whose rays stay together and whose rows are whole 32-byte sectors
+// of the image), 32 warps per SM (64 registers, 16 bytes of spills).  us per 1080p draw of the 64x32x64 map, 257x143
+// draw, edited 720p frame, 234x149 draw through glass: 309, 12.4, 192, 42; blocks of 8 x 32 335, 13.1, 197, 47; 8 x 8
+// 308, 13.1, 191, 48; 32 x 4 332, 12.9, 195, 40; 16 x 2 294, 12.9, 191, 47; 28 warps per SM 341, 12.4, 197, 42; 40 warps
+// 311, 12.3, 194, 42.
+#ifndef DN_DRAW_WARPS
+#define DN_DRAW_WARPS 32
+#endif
+#ifndef DN_DRAW_BX
+#define DN_DRAW_BX 16
+#define DN_DRAW_BY 8
 #endif
 
 extern int g_device;

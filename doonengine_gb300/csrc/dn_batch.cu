@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256) k_compact_batch(const CompactArgs* s, con
 }
 
 // blocks [0, nl): shadow directions of light map blockIdx.x.  Block nl: clamp the request count of every
-// synced map to its capacity (dn_cuda_sync's k_clamp_requests), then the exclusive prefix of the light
+// synced map to its capacity (the list's words behind it were not written), then the exclusive prefix of the light
 // maps' counts into reqStart[0..nl] and a zero work counter.
 __global__ void k_batch_prep(BatchLightMap* l, uint32_t nl, const CompactArgs* s, uint32_t ns, uint32_t* reqStart,
                              uint32_t* workCounter)
@@ -119,7 +119,7 @@ __global__ void k_batch_prep(BatchLightMap* l, uint32_t nl, const CompactArgs* s
     }
     __shared__ uint32_t warpSum[32];
     __shared__ uint32_t carry;
-    if (threadIdx.x == 0) { carry = 0; *workCounter = 0; }
+    if (threadIdx.x == 0) { carry = 0; workCounter[0] = workCounter[1] = 0; }
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint32_t base = 0; base < nl; base += blockDim.x) {
@@ -167,13 +167,11 @@ __global__ void __launch_bounds__(128, DN_PACKET_MIN_BLOCKS) k_light_packet_batc
 constexpr uint32_t MARK_BLOCKS = 16;
 __global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* l)
 {
-    __shared__ uint32_t opq[8];
     const BatchLightMap& e = l[blockIdx.x / MARK_BLOCKS];
-    opaque_materials(e.mats, opq);
     const uint64_t pairs = WalkGrid(e.m.sx, e.m.sy, e.m.sz).words / 2u;
     const uint32_t per = blockDim.x / 32u;
     for (uint64_t w = (blockIdx.x % MARK_BLOCKS) * per + threadIdx.x / 32u; w < pairs; w += MARK_BLOCKS * per)
-        mark_opaque_cells(e.m, w, opq);
+        mark_opaque_cells(e.m, w, e.opaque);
 }
 
 // the diffuse paths of the voxels k_light_packet_batch lit, as per-lane path streams over every map's queue
@@ -239,7 +237,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->copiesDone, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->tableFree, cudaEventDisableTiming);
     if (e != cudaSuccess) rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "stream / event: %s", cudaGetErrorString(e));
-    if (!rc) rc = dalloc(&b->workCounter, 1);
+    if (!rc) rc = dalloc(&b->workCounter, 2);
     if (!rc) rc = dalloc(&b->bst, 1);
     if (!rc) rc = dalloc(&b->lsave, 8);
     if (!rc) {
@@ -375,7 +373,6 @@ static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, 
         // the diffuse paths: a second pass over the same queue
         BatchLightArgs ld = la;
         ld.batch = b->tuning.diffuseBatch;
-        CK(cudaMemsetAsync(la.workCounter, 0, 4, s));
         COUNT_LAUNCH();
         k_light_diffuse_batch<<<(unsigned)(g_numSMs * b->maxBlocksDiffuse), 128, 0, s>>>(ld);
         CK(cudaGetLastError());
@@ -596,6 +593,7 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
             e.nreqPtr = &g->st->w[ST_REQ]; e.reqCap = g->reqCap;
             e.p = it.light;
             e.mats = mats;
+            e.opaque = opaque_set(it.materials);
             e.diffOut = g->diff; e.specOut = g->spec; e.samplesOut = g->nsamples;
             il++;
         }
@@ -772,7 +770,7 @@ extern "C" int dn_cuda_batch_autotune(DNgpuBatch* b, dn_batch_tuning* chosen)
         la.batch = t.streamBatch;
         float ms = 3.4e38f;
         for (int rep = 0; rep < 2 && !rc; rep++) {
-            cudaError_t e = cudaMemsetAsync(b->workCounter, 0, 4, b->stream);
+            cudaError_t e = cudaMemsetAsync(b->workCounter, 0, 8, b->stream);
             if (e == cudaSuccess) e = cudaEventRecord(e0, b->stream);
             if (e != cudaSuccess) { rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "autotune: %s", cudaGetErrorString(e)); break; }
             rc = issue_light(b, la, b->stream, t.kernel == 2u && packetsOk, b->lastFar);

@@ -9,7 +9,7 @@
  *   pool    vox[i] (uint2: normal word, linear albedo word), diff[i] / spec[i] (float4, FP32)
  *   frame   reqs[] ((tile << 4) | group), lightOut[] (scratch: new lighting per request lane)
  * Kernels per frame: k_draw (primary rays); k_pack_stage (or k_sync_stage for records packed on the host)
- * + k_compact (DN_sync_gpu); k_mark_opaque + k_light_tables + k_light_packet + k_light_diffuse (or
+ * + k_compact (DN_sync_gpu); k_light_prep + k_light_packet + k_light_diffuse (or
  * k_light_stream) + k_commit (DN_update_lighting).
  */
 #include "dn_internal.cuh"
@@ -647,40 +647,46 @@ __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream(cons
     // per-voxel job state lives in shared memory: it is touched only when a segment ends
     __shared__ Job jobs[128];
     __shared__ TintT<128> tint;
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.mats[i] = a.mats[i];
-    // shadow directions are identical for every voxel of the launch
-    for (int k = threadIdx.x; k < 65; k += blockDim.x) shadow_dir(a.p, k, sh.sdir[k], sh.sinv[k]);
+    for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.mats[i] = a.gtab->mats[i];
+    for (int i = threadIdx.x; i < 65 * 3; i += blockDim.x) {
+        (&sh.sdir[0][0])[i] = (&a.gtab->sdir[0][0])[i];
+        (&sh.sinv[0][0])[i] = (&a.gtab->sinv[0][0])[i];
+    }
     __syncthreads();
     stream_loop<false, false, FAR>(&a, nullptr, &sh, jobs[threadIdx.x], tint);
 }
 
-// The lighting launch with specular and shadow fans traced as warp packets (dn_light_packet.cuh).
-// the launch's materials and shadow directions into the volume's device tables, which k_light_packet
-// reads through L1 (a kernel, not a copy from host memory, so that the launch sequence can be captured)
-__global__ void k_light_tables(const __grid_constant__ MaterialTable t, const __grid_constant__ dn_light_params p,
-                               LightTables* out)
+// What a lighting launch reads, before it: block 0 writes the launch's materials and shadow directions to the
+// volume's device tables (a kernel, not a copy from host memory, so that the launch sequence can be captured), zeroes
+// the queue positions and clamps the request count to the list; the others set the opaque-chunk marks.  (Four
+// launches before: two of them waited only for their own start.)
+__global__ void __launch_bounds__(256) k_light_prep(const __grid_constant__ DevMap m, uint64_t nwords,
+                                                    const __grid_constant__ OpaqueSet opaque,
+                                                    const __grid_constant__ MaterialTable t,
+                                                    const __grid_constant__ dn_light_params p, LightTables* tab, DevState* st,
+                                                    uint64_t reqCap)
 {
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) out->mats[i] = t.m[i];
-    for (int k = threadIdx.x; k < 65; k += blockDim.x) shadow_dir(p, k, out->sdir[k], out->sinv[k]);
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i < 256; i += blockDim.x) tab->mats[i] = t.m[i];
+        for (int k = threadIdx.x; k < 65; k += blockDim.x) shadow_dir(p, k, tab->sdir[k], tab->sinv[k]);
+        if (threadIdx.x == 0) {
+            st->work[0] = st->work[1] = 0;
+            if (st->w[ST_REQ] > reqCap) st->w[ST_REQ] = (uint32_t)reqCap;
+        }
+        return;
+    }
+    const uint64_t stride = (uint64_t)(gridDim.x - 1u) * (blockDim.x / 32u);
+    for (uint64_t w = (uint64_t)(blockIdx.x - 1u) * (blockDim.x / 32u) + threadIdx.x / 32u; w < nwords / 2u; w += stride)
+        mark_opaque_cells(m, w, opaque);
 }
 
+// The lighting launch with specular and shadow fans traced as warp packets (dn_light_packet.cuh).
 __global__ void __launch_bounds__(128, DN_PACKET_MIN_BLOCKS) k_light_packet(const __grid_constant__ StreamArgs a)
 {
     // shared memory holds only the four warps' pools (25 KB per block with 128-ray pools): 7 blocks take 175 KB, the
     // rest of the SM's 256 KB is L1 for the map's masks and voxels; the tables are read from a.gtab
     __shared__ PacketWarp warps[4];
     packet_loop<false>(&a, nullptr, warps[threadIdx.x >> 5]);
-}
-
-// the opaque-chunk marks of one map for a lighting launch with the given materials (mark_opaque_cells)
-__global__ void __launch_bounds__(256) k_mark_opaque(const __grid_constant__ DevMap m, uint64_t nwords,
-                                                     const __grid_constant__ MaterialTable t)
-{
-    __shared__ uint32_t opq[8];
-    opaque_materials(t.m, opq);
-    const uint64_t stride = (uint64_t)gridDim.x * (blockDim.x / 32u);
-    for (uint64_t w = (uint64_t)blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u; w < nwords / 2u; w += stride)
-        mark_opaque_cells(m, w, opq);
 }
 
 // The diffuse paths of the voxels k_light_packet lit, as per-lane path streams over the whole request list:
@@ -695,44 +701,40 @@ __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const
 // launches the lighting kernel g_lightKernel selects (1 ray streams, 2 warp packets followed by the
 // diffuse-path kernel; packets need specBounceLimit <= PK_MAX_SPEC_SEGMENTS and a map that is not
 // far, and fall back to streams otherwise) with its batch threshold
-static int launch_light(DNgpuVolume* g, StreamArgs& a)
+static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materials)
 {
-    int perSM = 0;
-    MaterialTable table;                // on the stack: a launch argument, copied at the launch
-    memcpy(table.m, a.mats, sizeof(table.m));
+    // resident blocks per SM, the same on every device this library is built for
+    auto resident = [](auto* k) {
+        int n = 0;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 128, 0) == cudaSuccess && n > 0 ? n : 1;
+    };
     {
+        MaterialTable table;            // on the stack: a launch argument, copied at the launch
+        memcpy(table.m, materials, sizeof(table.m));
         const uint64_t nwords = walk_words(g);
         const uint64_t blocks = (nwords / 2 + 7) / 8;
         const uint32_t maxBlocks = (uint32_t)(g->numSMs > 0 ? g->numSMs * 8 : 1024);
         COUNT_LAUNCH();
-        k_mark_opaque<<<(uint32_t)(blocks < maxBlocks ? blocks : maxBlocks), 256, 0, g->stream>>>(dev_map(g), nwords, table);
+        k_light_prep<<<1u + (uint32_t)(blocks < maxBlocks ? blocks : maxBlocks), 256, 0, g->stream>>>(
+            dev_map(g), nwords, opaque_set(materials), table, a.p, g->dtab, g->st, g->reqCap);
         CK(cudaGetLastError());
     }
+    a.gtab = g->dtab;
     if (g_lightKernel == 2 && a.p.specBounceLimit <= PK_MAX_SPEC_SEGMENTS && !map_far(g)) {
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_packet, 128, 0));
-        if (perSM < 1) perSM = 1;
+        static const int packets = resident(k_light_packet), paths = resident(k_light_diffuse);
         a.batch = g_packetBatch;
-        a.gtab = g->dtab;
         COUNT_LAUNCH();
-        k_light_tables<<<1, 256, 0, g->stream>>>(table, a.p, g->dtab);
-        COUNT_LAUNCH();
-        k_light_packet<<<g->numSMs * perSM, 128, 0, g->stream>>>(a);
+        k_light_packet<<<g->numSMs * packets, 128, 0, g->stream>>>(a);
         CK(cudaGetLastError());
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_diffuse, 128, 0));
-        if (perSM < 1) perSM = 1;
-        CK(cudaMemsetAsync(a.workCounter, 0, 4, g->stream));
         a.batch = g_streamBatch;
         COUNT_LAUNCH();
-        k_light_diffuse<<<g->numSMs * perSM, 128, 0, g->stream>>>(a);
+        k_light_diffuse<<<g->numSMs * paths, 128, 0, g->stream>>>(a);
     } else {
-        const bool far = map_far(g);
-        CK(far ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_stream<true>, 128, 0)
-               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_stream<false>, 128, 0));
-        if (perSM < 1) perSM = 1;
+        static const int streams = resident(k_light_stream<false>), farStreams = resident(k_light_stream<true>);
         a.batch = g_streamBatch;
         COUNT_LAUNCH();
-        if (far) k_light_stream<true><<<g->numSMs * perSM, 128, 0, g->stream>>>(a);
-        else k_light_stream<false><<<g->numSMs * perSM, 128, 0, g->stream>>>(a);
+        if (map_far(g)) k_light_stream<true><<<g->numSMs * farStreams, 128, 0, g->stream>>>(a);
+        else k_light_stream<false><<<g->numSMs * streams, 128, 0, g->stream>>>(a);
     }
     CK(cudaGetLastError());
     return DN_CUDA_OK;
@@ -878,11 +880,6 @@ __global__ void __launch_bounds__(256) k_compact(const __grid_constant__ Compact
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t cells = WalkGrid(a.sx, a.sy, a.sz).cells;
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < cells; base += stride) compact_tiles(a, base);
-}
-
-__global__ void k_clamp_requests(DevState* st, uint64_t cap)
-{
-    if (st->w[ST_REQ] > cap) st->w[ST_REQ] = (uint32_t)cap;
 }
 
 static int stage_reserve(DNgpuVolume* g, size_t total, unsigned char** host, int* which);
@@ -1032,7 +1029,8 @@ static int dn_stage_chunks(DNgpuVolume* g, const dn_pack_params* pk, const dn_ti
     return DN_CUDA_OK;
 }
 
-// the per-tile pass of a sync after its staging (compact_tiles), then the request count's clamp
+// the per-tile pass of a sync after its staging (compact_tiles); the request count may pass the list's capacity (the
+// words behind it were not written): its readers clamp it
 static int sync_tiles(DNgpuVolume* g, const dn_sync_params* p)
 {
     CK(cudaMemsetAsync(&g->st->w[ST_REQ], 0, 4, g->stream));
@@ -1046,9 +1044,6 @@ static int sync_tiles(DNgpuVolume* g, const dn_sync_params* p)
     uint32_t maxBlocks = (uint32_t)(g->numSMs > 0 ? g->numSMs * 8 : 1024);
     COUNT_LAUNCH();
     k_compact<<<(uint32_t)(blocks < maxBlocks ? blocks : maxBlocks), 256, 0, g->stream>>>(a);
-    CK(cudaGetLastError());
-    COUNT_LAUNCH();
-    k_clamp_requests<<<1, 1, 0, g->stream>>>(g->st, g->reqCap);
     CK(cudaGetLastError());
     return DN_CUDA_OK;
 }
@@ -1129,17 +1124,14 @@ extern "C" int dn_cuda_light(DNgpuVolume* g, const dn_light_params* p, const dn_
     if (!g || !p || !materials) return dn_set_err(DN_CUDA_ERR_ARG, "null argument");
     if (p->K < 1 || p->K > 64) return dn_set_err(DN_CUDA_ERR_ARG, "K = %u", p->K);
     CK(cudaSetDevice(g->device));
-    CK(cudaMemsetAsync(&g->st->w[ST_WORK], 0, 4, g->stream));
-    static thread_local StreamArgs* a = nullptr;
-    if (!a) a = new StreamArgs();
+    StreamArgs args, *a = &args;
     a->m = dev_map(g);
     a->m.degen = &g->st->lstats[S_DEGEN];
-    a->reqs = g->reqs; a->workCounter = &g->st->w[ST_WORK]; a->nreqPtr = &g->st->w[ST_REQ];
+    a->reqs = g->reqs; a->workCounter = g->st->work; a->nreqPtr = &g->st->w[ST_REQ];
     a->nsamples = g->nsamples; a->out = g->lightOut; a->stats = g->st->lstats;
     a->batch = g_streamBatch;
     a->p = *p;
-    memcpy(a->mats, materials, sizeof(a->mats));
-    int rc = launch_light(g, *a);
+    int rc = launch_light(g, *a, materials);
     if (rc) return rc;
     COUNT_LAUNCH();
     k_commit<<<g->numSMs * 4, 256, 0, g->stream>>>(dev_map(g), g->reqs, &g->st->w[ST_REQ], g->lightOut, g->diff, g->spec,
@@ -1203,12 +1195,11 @@ static int noalloc_scratch(int device, float4** out)
 
 // the call's request count, or 0 and the capacity flag when the list exceeds the limit; the work counter
 // of the lighting launch starts at zero
-__global__ void k_noalloc_guard(DevState* st, uint32_t limit)
+__global__ void k_noalloc_guard(DevState* st, uint32_t limit, uint64_t reqCap)
 {
-    const uint32_t n = st->w[ST_REQ];
+    const uint32_t n = st->w[ST_REQ] > reqCap ? (uint32_t)reqCap : st->w[ST_REQ];
     st->w[ST_LIMITED] = n <= limit ? n : 0u;
     if (n > limit) atomicOr(&st->w[ST_ERR], ERRF_NOALLOC_CAPACITY);
-    st->w[ST_WORK] = 0;
 }
 
 extern "C" uint32_t dn_cuda_light_noalloc_set_limit(uint32_t groups)
@@ -1229,17 +1220,16 @@ extern "C" int dn_cuda_light_noalloc(DNgpuVolume* g, const dn_light_params* p, c
     int rc = noalloc_scratch(g->device, &scratch);
     if (rc) return rc;
     COUNT_LAUNCH();
-    k_noalloc_guard<<<1, 1, 0, g->stream>>>(g->st, __atomic_load_n(&g_noallocLimit, __ATOMIC_RELAXED));
+    k_noalloc_guard<<<1, 1, 0, g->stream>>>(g->st, __atomic_load_n(&g_noallocLimit, __ATOMIC_RELAXED), g->reqCap);
     CK(cudaGetLastError());
     StreamArgs a;                       // launch arguments on the stack: no host allocation either
     a.m = dev_map(g);
     a.m.degen = &g->st->lstats[S_DEGEN];
-    a.reqs = g->reqs; a.workCounter = &g->st->w[ST_WORK]; a.nreqPtr = &g->st->w[ST_LIMITED];
+    a.reqs = g->reqs; a.workCounter = g->st->work; a.nreqPtr = &g->st->w[ST_LIMITED];
     a.nsamples = g->nsamples; a.out = scratch; a.stats = g->st->lstats;
     a.batch = g_streamBatch;
     a.p = *p;
-    memcpy(a.mats, materials, sizeof(a.mats));
-    rc = launch_light(g, a);
+    rc = launch_light(g, a, materials);
     if (rc) return rc;
     COUNT_LAUNCH();
     k_commit<<<g->numSMs * 4, 256, 0, g->stream>>>(dev_map(g), g->reqs, &g->st->w[ST_LIMITED], scratch, g->diff, g->spec,
@@ -1341,6 +1331,7 @@ extern "C" int dn_cuda_finish(DNgpuVolume* g, uint64_t* numRequests)
     CK(cudaSetDevice(g->device));
     CK(cudaMemcpyAsync(g->hst, g->st, sizeof(DevState), cudaMemcpyDeviceToHost, g->stream));
     CK(cudaStreamSynchronize(g->stream));
+    if (g->hst->w[ST_REQ] > g->reqCap) g->hst->w[ST_REQ] = (uint32_t)g->reqCap;
     if (numRequests) *numRequests = g->hst->w[ST_REQ];
     if (g->hst->w[ST_ERR]) {
         uint32_t e = g->hst->w[ST_ERR];
@@ -1536,7 +1527,7 @@ extern "C" int dn_cuda_flush_l2(void* stream, size_t bytes)
 
 extern "C" const char* dn_cuda_kernel_names(void)
 {
-    return "k_draw;k_light_stream;k_light_packet;k_light_diffuse;k_light_tables;k_mark_opaque;k_commit;k_sync_stage;k_pack_stage;k_compact;k_clamp_requests;k_flush;"
+    return "k_draw;k_light_stream;k_light_packet;k_light_diffuse;k_light_prep;k_commit;k_sync_stage;k_pack_stage;k_compact;k_walk_border;k_flush;"
            "k_draw_batch;k_compact_batch;k_batch_reset;k_batch_prep;k_mark_opaque_batch;k_light_stream_batch;k_light_packet_batch;"
            "k_light_diffuse_batch;k_commit_batch;k_batch_gather;"
            "k_shape_count;k_shape_write";

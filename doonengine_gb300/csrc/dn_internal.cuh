@@ -26,15 +26,16 @@ int dn_set_err(int code, const char* fmt, ...);
 
 // ST_LIMITED: the request count a dn_cuda_light_noalloc launch lights (its own count, or 0 when the
 // list exceeds the fixed scratch; k_noalloc_guard writes it)
-enum { ST_REQ = 0, ST_WORK = 1, ST_ERR = 2, ST_LIMITED = 3 };
+enum { ST_REQ = 0, ST_ERR = 2, ST_LIMITED = 3 };
 // error flag bits of ST_ERR (reported by dn_cuda_finish / dn_cuda_batch_finish)
 enum : uint32_t { ERRF_TILE = 1u, ERRF_RECORD = 2u, ERRF_REQUESTS = 4u, ERRF_NOALLOC_CAPACITY = 0x100u };
 enum { S_RAYS = 0, S_PRIMARY, S_OUTER, S_ENTERED, S_INNER, S_HITS, S_LIT, S_DEGEN, S_COUNT };
 
 struct DevState {
-    uint32_t w[4];                      // nreq, work counter, error flags, noalloc request count
+    uint32_t w[4];                      // nreq, -, error flags, noalloc request count
     unsigned long long stats[8];        // draw kernels
     unsigned long long lstats[8];       // lighting kernels
+    uint32_t work[2];                   // queue positions of the lighting kernels: fans (or streams), diffuse paths
 };
 
 struct DNgpuBatch;
@@ -245,20 +246,23 @@ __device__ __forceinline__ uint32_t spread_bits(uint32_t x)
 // that reaches an occupied voxel of such a chunk ends there without reading the voxel's word and material
 // (its pool index is formed when the segment is shaded).  The next sync rewrites the map with 0 / 1 / 2.
 
-// opq[8] (shared memory): bit m set when material m is opaque (opacity exactly 1, voxelShared.comp:360)
-__device__ __forceinline__ void opaque_materials(const dn::Material* mats, uint32_t* opq)
+// bit m set when material m is opaque (opacity exactly 1, voxelShared.comp:360)
+struct OpaqueSet { uint32_t w[8]; };
+static inline OpaqueSet opaque_set(const dn_material* mats)
 {
-    if (threadIdx.x < 8) opq[threadIdx.x] = 0;
-    __syncthreads();
-    for (uint32_t m = threadIdx.x; m < 256; m += blockDim.x)
-        if (mats[m].opacity == 1.0f) atomicOr(&opq[m >> 5], 1u << (m & 31u));
-    __syncthreads();
+    OpaqueSet o;
+    for (int k = 0; k < 8; k++) {
+        uint32_t w = 0;
+        for (int b = 0; b < 32; b++) w |= (mats[32 * k + b].opacity == 1.0f ? 1u : 0u) << b;
+        o.w[k] = w;
+    }
+    return o;
 }
 
 // Cells [32 * w, 32 * w + 32) of the walk grid, one per lane: every loaded tile to 3 (all its materials
 // opaque) or 2.  A lane per cell: its record's material set is two 16-byte loads, and the warp's votes form the
 // two words.  (One thread per word, 16 tiles and up to 128 dependent loads in a row, took 16 us on any map.)
-__device__ __forceinline__ void mark_opaque_cells(const dn::DevMap& m, uint64_t w, const uint32_t* opq)
+__device__ __forceinline__ void mark_opaque_cells(const dn::DevMap& m, uint64_t w, const OpaqueSet& op)
 {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t* tbits = const_cast<uint32_t*>(m.tbits);
@@ -272,8 +276,8 @@ __device__ __forceinline__ void mark_opaque_cells(const dn::DevMap& m, uint64_t 
         const uint32_t slot = __ldg(&m.tword[x + m.sx * (y + m.sy * z)]) & dn::SLOT_MASK;
         const uint4* ms = (const uint4*)m.rec[slot].matSet;
         const uint4 a = __ldg(&ms[0]), b = __ldg(&ms[1]);
-        opaque = ((a.x & ~opq[0]) | (a.y & ~opq[1]) | (a.z & ~opq[2]) | (a.w & ~opq[3]) |
-                  (b.x & ~opq[4]) | (b.y & ~opq[5]) | (b.z & ~opq[6]) | (b.w & ~opq[7])) == 0u;
+        opaque = ((a.x & ~op.w[0]) | (a.y & ~op.w[1]) | (a.z & ~op.w[2]) | (a.w & ~op.w[3]) |
+                  (b.x & ~op.w[4]) | (b.y & ~op.w[5]) | (b.z & ~op.w[6]) | (b.w & ~op.w[7])) == 0u;
     }
     const unsigned b0 = __ballot_sync(0xFFFFFFFFu, (st == 1u) || opaque);
     const unsigned b1 = __ballot_sync(0xFFFFFFFFu, st >= 2u);

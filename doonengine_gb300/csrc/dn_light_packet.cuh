@@ -62,7 +62,8 @@ constexpr uint32_t PK_POOL_FAN = DN_PK_POOL_FAN;
 constexpr uint32_t PK_POOL_ALT = PK_POOL_FAN == 64u ? 128u : 64u;   // the batched autotuner's other pool size
 
 // Work units: 16 voxels of a request group at a time while more than PK_MID voxels per warp of the launch are left in
-// the queue, 8 down to PK_TAIL, then 4.  Large units have fewer pool tails, small ones spread the end of a launch.
+// the queue, 8 down to PK_TAIL, then 4; 2 or 1 in a launch that has no more voxels than twice its warps or its warps.
+// Large units have fewer pool tails, small ones spread the end of a launch.
 // One size for all, us per frame of the 64x32x64 map, the 16x16x16 map, the glass map and twelve maps batched: 16 voxels
 // 12336, 514, 2885, 12105; 8 voxels 12444, 513, 2685, 12750; 4 voxels 12675, 573, 2720, 14115; these three 12243, 507,
 // 2597, 12014 (a middle of 128 or 256 voxels per warp, a tail of 4 or 16: within 2 %).
@@ -134,6 +135,32 @@ __device__ __forceinline__ void packet_setup(PacketVoxel& pv, uint32_t req, uint
     pv.flags = PV_VALID | (first ? PV_FIRST : 0u) | (doSpec ? PV_SPEC : 0u) | (doDiff ? PV_DIFF : 0u);
 }
 
+// Unit u of a queue of nreq request groups: voxels [first, first + count) of group r; false when there is none.  The
+// queue is five stretches, of units of 16, 8, 4, 2 and 1 voxels.  (Formed again for every unit: kept over the loop,
+// the stretches' bounds cost the many-map kernel spills.)
+__device__ __forceinline__ bool packet_unit(uint32_t u, uint32_t nreq, uint32_t& r, uint32_t& first, uint32_t& count)
+{
+    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
+    uint32_t from = 0;
+#pragma unroll 1
+    for (uint32_t i = 0; i < 5u; i++) {
+        // voxels per warp of the launch that the next stretches take
+        const uint32_t left = i == 0u ? PK_MID : i == 1u ? PK_TAIL : i == 2u ? (nreq * 16u <= warps ? 2u : 0u)
+                            : i == 3u ? (nreq * 32u <= warps ? 1u : 0u) : 0u;
+        const uint32_t after = warps * left / 32u, to = nreq > after ? nreq - after : 0u;
+        const uint32_t units = (to - from) << (i + 1u);
+        if (u < units) {
+            count = 16u >> i;
+            r = from + (u >> (i + 1u));
+            first = (u & ((2u << i) - 1u)) * count;
+            return true;
+        }
+        u -= units;
+        from = to;
+    }
+    return false;
+}
+
 // The work units of one launch (a part of a request group).  Per unit: (1) the setup of its voxels; (2) pools of
 // PK_POOL_FAN/K voxels (at least one): the directions of all its specular rays, by whole warps; then every ray of
 // the specular fans, the shadow fans and the first-sample shadow rays is traced by whichever lane is free -- a lane
@@ -153,21 +180,13 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
     const uint32_t batch = MANY ? many->batch : one->batch;
     Counters c{0, 0, 0, 0, 0};
     uint32_t lit = 0;
-    // the queue's groups: `big` ones in 2 units each, up to `mid` in 4, the rest in 8
-    const uint32_t warps = gridDim.x * (blockDim.x / 32u);
-    const uint32_t lastMid = warps * PK_MID / 32u, lastTail = warps * PK_TAIL / 32u;
-    const uint32_t big = nreq > lastMid ? nreq - lastMid : 0u, mid = nreq > lastTail ? nreq - lastTail : 0u;
-    const uint32_t bigUnits = big * 2u, midUnits = bigUnits + (mid - big) * 4u, units = midUnits + (nreq - mid) * 8u;
     for (;;) {
         uint32_t u = 0;
         if (lane == 0) u = atomicAdd(counter, 1u);
         u = __shfl_sync(0xFFFFFFFFu, u, 0);
-        if (u >= units) break;
         // unit u: voxels [first, first + count) of request group r
         uint32_t r, first, count;
-        if (u < bigUnits) { r = u >> 1; count = 16; first = (u & 1u) * 16u; }
-        else if (u < midUnits) { r = big + ((u - bigUnits) >> 2); count = 8; first = ((u - bigUnits) & 3u) * 8u; }
-        else { r = mid + ((u - midUnits) >> 3); count = 4; first = ((u - midUnits) & 7u) * 4u; }
+        if (!packet_unit(u, nreq, r, first, count)) break;
         // the group's map (warp-uniform)
         const BatchLightMap* e = nullptr;
         uint32_t req = r;

@@ -20,12 +20,15 @@
  * 32 voxels.
  */
 #pragma once
-#include "dn_walk.cuh"
+#include "dn_internal.cuh"
 
 namespace dn {
 
 #ifndef DN_STREAM_MIN_BLOCKS
 #define DN_STREAM_MIN_BLOCKS 4   // 4 blocks of 4 warps per SM (measured best: leaves L1 room for the tile map)
+#endif
+#ifndef DN_WINDOW_WARPS
+#define DN_WINDOW_WARPS 1
 #endif
 #ifndef DN_DIFF_MIN_BLOCKS
 #define DN_DIFF_MIN_BLOCKS 6     // the diffuse-path kernel (k_light_diffuse): 6 blocks of 4 warps per SM
@@ -36,20 +39,19 @@ enum : uint32_t { PH_FETCH = 0, PH_SPEC = 1, PH_SHADOW = 2, PH_DIFF = 3, PH_FINA
 struct StreamArgs {
     DevMap m;
     const uint32_t* reqs;
-    uint32_t* workCounter;
+    uint32_t* workCounter;            // [2], DevState::work
     const uint32_t* nreqPtr;
     const uint32_t* nsamples;
     float4* out;
     unsigned long long* stats;
     uint32_t batch;
     dn_light_params p;
-    Material mats[256];
-    const struct LightTables* gtab;   // device copy of mats and the shadow directions (k_light_packet)
+    const struct LightTables* gtab;   // the launch's materials and shadow directions (k_light_prep)
 };
 
 struct MaterialTable { Material m[256]; };
 
-// per-launch tables k_light_packet reads through L1: the materials and the shadow directions
+// per-launch tables the lighting kernels read through L1: the materials and the shadow directions
 struct LightTables {
     Material mats[256];
     float sdir[65][3];   // shadow directions k < K, [64]: the first-sample direction sunDir + EPS
@@ -377,6 +379,7 @@ struct BatchLightMap {
     uint64_t reqCap;
     dn_light_params p;
     const Material* mats;       // the map's 256 materials
+    OpaqueSet opaque;           // those that are opaque
     float4* diffOut;            // committed lighting and sample counts (k_commit_batch)
     float4* specOut;
     uint32_t* samplesOut;
@@ -422,8 +425,12 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
     uint32_t nreq = 0;
     if constexpr (MANY) nreq = *(volatile const uint32_t*)&many->reqStart[many->nmaps];
     else nreq = *(volatile const uint32_t*)one->nreqPtr;
-    uint32_t* const counter = MANY ? many->workCounter : one->workCounter;
-    uint32_t winMap = 0, winReq = 0, winNext = 32;     // warp-uniform voxel window: map, request, next lane in it
+    uint32_t* const counter = (MANY ? many->workCounter : one->workCounter) + (DIFFONLY ? 1 : 0);
+    uint32_t winMap = 0, winReq = 0, winNext = 32, winEnd = 32;   // warp-uniform voxel window: map, request, next voxel, end
+    // a window is a whole request group, or a part of one when the launch has fewer groups than warps: its few paths
+    // then run on all SMs, and a path waits for fewer others
+    uint32_t parts = 0;   // log2 of the windows per group
+    while (parts < 5u && (nreq << (parts + 1u)) <= gridDim.x * (blockDim.x / 32u) * DN_WINDOW_WARPS) parts++;
     bool exhausted = false;
     j.phase = PH_FETCH;
     j.map = 0;
@@ -453,15 +460,18 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
                 for (int guard = 0; guard < 64; guard++) {
                     const unsigned need = __ballot_sync(0xFFFFFFFFu, j.phase == PH_FETCH);
                     if (need == 0u) break;
-                    if (winNext >= 32u) {
+                    if (winNext >= winEnd) {
                         uint32_t r = 0;
                         if (!exhausted && lane == 0) r = atomicAdd(counter, 1u);
                         r = __shfl_sync(0xFFFFFFFFu, r, 0);
-                        if (exhausted || r >= nreq) {
+                        if (exhausted || r >= nreq << parts) {
                             exhausted = true;
                             if (j.phase == PH_FETCH) j.phase = PH_DONE;
                             break;
                         }
+                        winNext = (r & ((1u << parts) - 1u)) << (5u - parts);
+                        winEnd = winNext + (32u >> parts);
+                        r >>= parts;
                         if constexpr (MANY) {
                             // the map whose request range holds r: reqStart[map] <= r < reqStart[map + 1]
                             uint32_t lo = 0, hi = many->nmaps;
@@ -474,10 +484,9 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
                         } else {
                             winReq = r;
                         }
-                        winNext = 0;
                     }
                     const uint32_t rank = __popc(need & ((1u << lane) - 1u));
-                    if (j.phase == PH_FETCH && winNext + rank < 32u) {
+                    if (j.phase == PH_FETCH && winNext + rank < winEnd) {
                         if constexpr (MANY) {
                             const BatchLightMap& e = many->maps[winMap];
                             if (winMap != lmi) { le = &e; lmi = winMap; }
@@ -488,7 +497,7 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
                                                   one->out);
                         }
                     }
-                    const uint32_t took = (uint32_t)__popc(need) < 32u - winNext ? (uint32_t)__popc(need) : 32u - winNext;
+                    const uint32_t took = (uint32_t)__popc(need) < winEnd - winNext ? (uint32_t)__popc(need) : winEnd - winNext;
                     winNext += took;
                 }
                 // shade the finished segment and set up the next one (or finish the voxel)

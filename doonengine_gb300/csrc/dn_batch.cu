@@ -60,7 +60,8 @@ struct DNgpuBatch {
     // the lighting launch of the last frame (autotuning re-runs it) and the generations of its maps
     BatchLightArgs lastLight;
     bool lastLightValid;
-    bool lastPackets, lastFar;
+    uint32_t lastSegs;          // the packet build the last frame's maps can take (its segments; 0: ray streams only)
+    bool lastFar;
     std::vector<std::pair<DNgpuVolume*, uint64_t>> lastLightGens;
 };
 
@@ -156,11 +157,11 @@ __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream_batc
 
 // POOL: rays per fan kind per pool (the rays a warp pulls from a request group at a time); the autotuner
 // picks PK_POOL_FAN or PK_POOL_ALT (dn_batch_tuning.poolRays)
-template <uint32_t POOL>
-__global__ void __launch_bounds__(128, DN_PACKET_MIN_BLOCKS) k_light_packet_batch(const __grid_constant__ BatchLightArgs a)
+template <uint32_t POOL, uint32_t SEGS>
+__global__ void __launch_bounds__(128, packet_blocks(SEGS)) k_light_packet_batch(const __grid_constant__ BatchLightArgs a)
 {
-    __shared__ PacketWarpT<POOL, PK_VOXELS> warps[4];
-    packet_loop<true, POOL>(nullptr, &a, warps[threadIdx.x >> 5]);
+    __shared__ PacketWarpT<POOL, SEGS> warps[4];
+    packet_loop<true, POOL, SEGS>(nullptr, &a, warps[threadIdx.x >> 5]);
 }
 
 // the opaque-chunk marks (mark_opaque_cells) of every map of a lighting launch: MARK_BLOCKS blocks per map
@@ -227,7 +228,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     b->tuning.streamBatch = b->tuning.kernel == 2u ? g_packetBatch : g_streamBatch;
     b->tuning.blocksPerSM = DN_STREAM_MIN_BLOCKS; b->tuning.useGraph = 1;
     b->tuning.poolRays = PK_POOL_FAN; b->tuning.diffuseBatch = g_streamBatch;
-    b->lastPackets = b->lastFar = false;
+    b->lastSegs = 0; b->lastFar = false;
     b->graph = nullptr;
     b->lastLightValid = false;
     int rc = DN_CUDA_OK;
@@ -253,8 +254,8 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
         int perSM = 0, perSM2 = 0, perSM3 = 0;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_stream_batch<false>, 128, 0);
         int perSMAlt = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM2, k_light_packet_batch<PK_POOL_FAN>, 128, 0);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMAlt, k_light_packet_batch<PK_POOL_ALT>, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM2, k_light_packet_batch<PK_POOL_FAN, 2>, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMAlt, k_light_packet_batch<PK_POOL_ALT, 2>, 128, 0);
         b->maxBlocksPacketAlt = perSMAlt < 1 ? 1 : perSMAlt;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM3, k_light_diffuse_batch, 128, 0);
         if (e != cudaSuccess) rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "occupancy: %s", cudaGetErrorString(e));
@@ -352,20 +353,23 @@ struct FramePlan {
     TableLayout t;
     uint32_t drawBlocks, syncBlocks;
     bool hostImages;
-    bool packets;               // lighting as warp packets (dn_light_packet.cuh)
+    uint32_t packets;           // lighting as warp packets (dn_light_packet.cuh): the build's segments, or 0
     bool far;                   // a map of the frame is far: the kernels' FAR forms, ray streams for lighting
 };
 
-// packets: the lighting kernel of dn_light_packet.cuh (every map's specBounceLimit within its limit)
-static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, bool packets, bool far)
+// packets: the segments of the build of dn_light_packet.cuh to run (every map's specBounceLimit within its limit), 0
+// for the ray streams
+static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, uint32_t packets, bool far)
 {
     COUNT_LAUNCH();
     k_mark_opaque_batch<<<la.nmaps * MARK_BLOCKS, 256, 0, s>>>(la.maps);
     CK(cudaGetLastError());
     COUNT_LAUNCH();
     const unsigned grid = (unsigned)(g_numSMs * (int)b->tuning.blocksPerSM);
-    if (packets && b->tuning.poolRays == PK_POOL_ALT) k_light_packet_batch<PK_POOL_ALT><<<grid, 128, 0, s>>>(la);
-    else if (packets) k_light_packet_batch<PK_POOL_FAN><<<grid, 128, 0, s>>>(la);
+    if (packets == 4u) k_light_packet_batch<64, 4><<<grid, 128, 0, s>>>(la);
+    else if (packets == 8u) k_light_packet_batch<64, 8><<<grid, 128, 0, s>>>(la);
+    else if (packets && b->tuning.poolRays == PK_POOL_ALT) k_light_packet_batch<PK_POOL_ALT, 2><<<grid, 128, 0, s>>>(la);
+    else if (packets) k_light_packet_batch<PK_POOL_FAN, 2><<<grid, 128, 0, s>>>(la);
     else if (far) k_light_stream_batch<true><<<grid, 128, 0, s>>>(la);
     else k_light_stream_batch<false><<<grid, 128, 0, s>>>(la);
     CK(cudaGetLastError());
@@ -508,8 +512,8 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
         if ((items[i].phases & DN_BATCH_LIGHT) && items[i].light.specBounceLimit > maxSpec) maxSpec = items[i].light.specBounceLimit;
     f.far = false;
     for (uint32_t i = 0; i < n; i++) f.far = f.far || map_far(items[i].map);
-    f.packets = b->tuning.kernel == 2u && maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far;
-    b->lastPackets = f.packets;
+    f.packets = b->tuning.kernel == 2u && maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far ? packet_segments(maxSpec) : 0u;
+    b->lastSegs = maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far ? packet_segments(maxSpec) : 0u;
     b->lastFar = f.far;
     if (f.t.size > b->tabCap) {
         // growing waits for the stream, frees pinned memory (which waits for the device) and renews the
@@ -543,7 +547,7 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
     std::vector<uint64_t> key;
     key.reserve(4 + (size_t)n * 10);
     key.push_back(n); key.push_back(b->tabGen); key.push_back(b->tuning.streamBatch); key.push_back(b->tuning.blocksPerSM);
-    key.push_back(b->tuning.kernel);
+    key.push_back(b->tuning.kernel); key.push_back(((uint64_t)f.packets << 1) | (f.far ? 1u : 0u));
     for (uint32_t i = 0; i < n; i++) {
         const dn_batch_item& it = items[i];
         DNgpuVolume* g = it.map;
@@ -759,8 +763,8 @@ extern "C" int dn_cuda_batch_autotune(DNgpuBatch* b, dn_batch_tuning* chosen)
     }
     const dn_batch_tuning keep = b->tuning;
     dn_batch_tuning best = keep;
-    // packets were possible in the last frame only if every lit map's specBounceLimit allowed them and no map is far
-    const bool packetsOk = b->lastPackets || (keep.kernel != 2u && !b->lastFar);
+    // packets are possible when every lit map's specBounceLimit allows them and no map is far
+    const bool packetsOk = b->lastSegs != 0u;
     float bestMs = 3.4e38f;
     int rc = DN_CUDA_OK;
     // times the last frame's lighting launch under tuning t (best of two runs)
@@ -773,7 +777,7 @@ extern "C" int dn_cuda_batch_autotune(DNgpuBatch* b, dn_batch_tuning* chosen)
             cudaError_t e = cudaMemsetAsync(b->workCounter, 0, 8, b->stream);
             if (e == cudaSuccess) e = cudaEventRecord(e0, b->stream);
             if (e != cudaSuccess) { rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "autotune: %s", cudaGetErrorString(e)); break; }
-            rc = issue_light(b, la, b->stream, t.kernel == 2u && packetsOk, b->lastFar);
+            rc = issue_light(b, la, b->stream, t.kernel == 2u ? b->lastSegs : 0u, b->lastFar);
             if (rc) break;
             e = cudaEventRecord(e1, b->stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);

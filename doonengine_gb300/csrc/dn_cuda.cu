@@ -681,12 +681,13 @@ __global__ void __launch_bounds__(256) k_light_prep(const __grid_constant__ DevM
 }
 
 // The lighting launch with specular and shadow fans traced as warp packets (dn_light_packet.cuh).
-__global__ void __launch_bounds__(128, DN_PACKET_MIN_BLOCKS) k_light_packet(const __grid_constant__ StreamArgs a)
+template <uint32_t POOL, uint32_t SEGS>
+__global__ void __launch_bounds__(128, packet_blocks(SEGS)) k_light_packet(const __grid_constant__ StreamArgs a)
 {
     // shared memory holds only the four warps' pools (25 KB per block with 128-ray pools): 7 blocks take 175 KB, the
     // rest of the SM's 256 KB is L1 for the map's masks and voxels; the tables are read from a.gtab
-    __shared__ PacketWarp warps[4];
-    packet_loop<false>(&a, nullptr, warps[threadIdx.x >> 5]);
+    __shared__ PacketWarpT<POOL, SEGS> warps[4];
+    packet_loop<false, POOL, SEGS>(&a, nullptr, warps[threadIdx.x >> 5]);
 }
 
 // The diffuse paths of the voxels k_light_packet lit, as per-lane path streams over the whole request list:
@@ -721,10 +722,15 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materi
     }
     a.gtab = g->dtab;
     if (g_lightKernel == 2 && a.p.specBounceLimit <= PK_MAX_SPEC_SEGMENTS && !map_far(g)) {
-        static const int packets = resident(k_light_packet), paths = resident(k_light_diffuse);
+        static const int packets2 = resident(k_light_packet<PK_POOL_FAN, 2>), packets4 = resident(k_light_packet<64, 4>),
+                         packets8 = resident(k_light_packet<64, 8>), paths = resident(k_light_diffuse);
         a.batch = g_packetBatch;
         COUNT_LAUNCH();
-        k_light_packet<<<g->numSMs * packets, 128, 0, g->stream>>>(a);
+        switch (packet_segments(a.p.specBounceLimit)) {
+        case 2: k_light_packet<PK_POOL_FAN, 2><<<g->numSMs * packets2, 128, 0, g->stream>>>(a); break;
+        case 4: k_light_packet<64, 4><<<g->numSMs * packets4, 128, 0, g->stream>>>(a); break;
+        default: k_light_packet<64, 8><<<g->numSMs * packets8, 128, 0, g->stream>>>(a); break;
+        }
         CK(cudaGetLastError());
         a.batch = g_streamBatch;
         COUNT_LAUNCH();

@@ -40,8 +40,18 @@ namespace dn {
 #define DN_PACKET_MIN_BLOCKS 7
 #endif
 
-// specBounceLimit handled here (the reference's default is 2); larger limits use the stream kernel
-constexpr uint32_t PK_MAX_SPEC_SEGMENTS = 2;
+// specBounceLimit handled here (the reference's default is 2); larger limits use the stream kernel.  A pooled ray
+// keeps one contribution per segment, so there are builds for at most 2, 4 and 8 segments: 128-ray pools for 2,
+// 64-ray pools for more.  Four lighting updates of a 16x12x16 map with limit 4, K = 16 and 4 paths per voxel, read
+// back: 6.8 ms, 18.8 with the ray streams.
+constexpr uint32_t PK_MAX_SPEC_SEGMENTS = 8;
+__host__ __device__ constexpr uint32_t packet_segments(uint32_t specBounceLimit)
+{
+    return specBounceLimit <= 2u ? 2u : specBounceLimit <= 4u ? 4u : 8u;
+}
+
+// resident blocks the register allocation of a build must allow (8-segment pools take 34 KB per block)
+constexpr int packet_blocks(uint32_t segs) { return segs <= 4u ? DN_PACKET_MIN_BLOCKS : 6; }
 
 // per-voxel data of the warp's unit (shared memory, written by the voxel's lane)
 struct PacketVoxel {
@@ -76,20 +86,18 @@ constexpr uint32_t PK_POOL_ALT = PK_POOL_FAN == 64u ? 128u : 64u;   // the batch
 constexpr uint32_t PK_MID = DN_PK_MID, PK_TAIL = DN_PK_TAIL;
 constexpr uint32_t PK_VOXELS = 16;
 
-template <uint32_t POOL, uint32_t VOXELS>
+template <uint32_t POOL, uint32_t SEGS>
 struct PacketWarpT {
-    PacketVoxel v[VOXELS];
+    PacketVoxel v[PK_VOXELS];
     // a pooled specular ray's direction and its reciprocal until a lane takes the ray, then the contributions of its
-    // (at most two) segments; while the second segment runs, the upper three hold the first one's multiplier
-    float con[2 * 3][POOL];
+    // segments; while segment b > 0 runs, its place holds the ray's multiplier
+    float con[3 * SEGS][POOL];
     float sh[3][POOL];                          // shadow contribution of each pooled ray
     uint8_t ncon[POOL];                         // contributions of each specular ray
     uint8_t shHas[POOL];                        // the shadow ray was unoccluded
-    uint8_t specList[VOXELS], fanList[VOXELS], firstList[VOXELS];   // the pool's voxels by what they cast
+    uint8_t specList[PK_VOXELS], fanList[PK_VOXELS], firstList[PK_VOXELS];   // the pool's voxels by what they cast
     TintT<32> tint;
 };
-using PacketWarp = PacketWarpT<PK_POOL_FAN, PK_VOXELS>;
-static_assert(PK_MAX_SPEC_SEGMENTS == 2, "con holds two segments' contributions");
 
 // sets up voxel (req, vlane) of the group (voxel_setup of dn_light_stream.cuh) and writes the outputs that no ray
 // decides: zero for invalid slots and for light the voxel does not cast rays for
@@ -168,9 +176,10 @@ __device__ __forceinline__ bool packet_unit(uint32_t u, uint32_t nreq, uint32_t&
 // have one, so no lane waits for the slowest ray of a fan; each ray's contributions go to shared memory, and when
 // the pool is empty every voxel's sums are formed in the reference's order and written (its diffuse paths run in
 // k_light_diffuse, which reads the direct light left in the voxel's diffuse slot).
-template <bool MANY, uint32_t POOL = PK_POOL_FAN>
-__device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLightArgs* many, PacketWarpT<POOL, PK_VOXELS>& W)
+template <bool MANY, uint32_t POOL, uint32_t SEGS>
+__device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLightArgs* many, PacketWarpT<POOL, SEGS>& W)
 {
+    static_assert(SEGS >= 2u && POOL >= 64u, "a slot holds a direction and its reciprocal, a pool one voxel's rays");
     const uint32_t lane = lane_id_s();
     const uint32_t below = (1u << lane) - 1u;
     uint32_t nreq = 0;
@@ -309,8 +318,9 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                 // specular_ray body after step_map (voxelLighting.comp:98-144).  A bounced segment started at the
                 // last hit position (its origin) and left the multiplier in con and its material's sky flag in s.flags
                 const PacketVoxel& pv = W.v[W.specList[q * overK >> 16]];
-                const bool bounced = (s.flags & RF_BOUNCED) != 0u;
-                const f3 mult = bounced ? mk(W.con[3][q], W.con[4][q], W.con[5][q]) : pv.talbedo;
+                const uint32_t b = s.flags >> RF_BOUNCES, at = SEGS == 2u ? (b ? 3u : 0u) : 3u * b;
+                const uint32_t in = SEGS == 2u ? 3u : at, up = SEGS == 2u ? 3u : at + 3u;   // this multiplier, the next one
+                const f3 mult = b ? mk(W.con[in][q], W.con[in + 1u][q], W.con[in + 2u][q]) : pv.talbedo;
                 bool more = false, add_ = true;
                 f3 sc;
                 if (hit) {
@@ -336,15 +346,15 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                             sc.x = (hc.x * cmul + cadd.x) * mult.x;
                             sc.y = (hc.y * cmul + cadd.y) * mult.y;
                             sc.z = (hc.z * cmul + cadd.z) * mult.z;
-                            if (hm.specular != 0.0f && !bounced && p.specBounceLimit > 1u) {
+                            if (hm.specular != 0.0f && (SEGS == 2u ? !b && p.specBounceLimit > 1u : b + 1u < SEGS && b + 1u < p.specBounceLimit)) {
                                 // the bounce
                                 more = true;
-                                W.con[3][q] = mult.x * (hv.albedo.x * cmul * hm.specular);
-                                W.con[4][q] = mult.y * (hv.albedo.y * cmul * hm.specular);
-                                W.con[5][q] = mult.z * (hv.albedo.z * cmul * hm.specular);
+                                W.con[up][q] = mult.x * (hv.albedo.x * cmul * hm.specular);
+                                W.con[up + 1u][q] = mult.y * (hv.albedo.y * cmul * hm.specular);
+                                W.con[up + 2u][q] = mult.z * (hv.albedo.z * cmul * hm.specular);
                                 const f3 nd = reflect(s.dir, hv.normal);
                                 ray_begin<false>(s, m, hpos, nd, rcp3(nd), true, c, W.tint, lane);
-                                s.flags |= RF_BOUNCED | (hm.reflectType == 1u ? RF_SKY : 0u);
+                                s.flags |= ((SEGS == 2u ? 1u : b + 1u) << RF_BOUNCES) | (hm.reflectType == 1u ? RF_SKY : 0u);
                                 c.rays++;
                             }
                         }
@@ -354,7 +364,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                     sc.y = sun.y * cmul + cadd.y;
                     sc.z = sun.z * cmul + cadd.z;
                 } else {
-                    const bool reflectsSky = bounced ? (s.flags & RF_SKY) != 0u : mats[pv.tmat].reflectType == 1u;
+                    const bool reflectsSky = b ? (s.flags & RF_SKY) != 0u : mats[pv.tmat].reflectType == 1u;
                     const f3 sky = reflectsSky ? sky_color(mk(p.skyBot[0], p.skyBot[1], p.skyBot[2]),
                                                            mk(p.skyTop[0], p.skyTop[1], p.skyTop[2]), s.dir) : sun;
                     sc.x = (sky.x * cmul + cadd.x) * mult.x;
@@ -362,10 +372,9 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                     sc.z = (sky.z * cmul + cadd.z) * mult.z;
                 }
                 if (add_) {
-                    const uint32_t at = bounced ? 3u : 0u;
                     W.con[at][q] = sc.x; W.con[at + 1u][q] = sc.y; W.con[at + 2u][q] = sc.z;
                 }
-                if (!more) W.ncon[q] = (uint8_t)((bounced ? 1u : 0u) + (add_ ? 1u : 0u));
+                if (!more) W.ncon[q] = (uint8_t)((SEGS == 2u ? (b ? 1u : 0u) : b) + (add_ ? 1u : 0u));
             }
             __syncwarp();
             // the pool's sums in the reference's order (ray, then segment), a component of a voxel's specular or
@@ -380,6 +389,8 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                         const uint32_t n = W.ncon[k];
                         if (n > 0u) acc = acc + W.con[comp][k];
                         if (n > 1u) acc = acc + W.con[3u + comp][k];
+                        if constexpr (SEGS > 2u)
+                            for (uint32_t b = 2; b < n; b++) acc = acc + W.con[3u * b + comp][k];
                     }
                     acc = acc / (float)K;
                     float* o = (float*)&out[((uint64_t)req * 32u + first + v) * 2u + 1u];

@@ -55,7 +55,8 @@ enum : uint32_t {
     RM_MISS = 6           // left the map
 };
 enum : uint32_t { RF_REQUESTED = 1u, RF_IGNORE = 2u, RF_OPAQUE = 4u, RF_TINT = 8u,
-                  RF_BOUNCED = 16u, RF_SKY = 32u };   // the last two: the packet kernel's
+                  RF_SKY = 16u };           // the packet kernel's, as the bits from RF_BOUNCES on
+constexpr uint32_t RF_BOUNCES = 8;            // the ray's segments before this one
 
 struct Ray {
     f3 pos, dir, delta;      // origin, direction, |1 / direction|

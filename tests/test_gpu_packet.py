@@ -1,0 +1,76 @@
+"""The packet kernel's builds: specular rays of more segments than two (4- and 8-segment slots; 9 runs the ray streams) at
+the fan sizes where a pool holds many voxels, one and a fraction of one; and a batch whose maps need different builds
+and whose limit changes while its frame is replayed as a graph."""
+import numpy as np
+import pytest
+
+import doonengine_gb300 as dn
+from doonengine_gb300 import configs
+from parity_util import Pair
+from test_gpu_walk import check_counters
+
+pytestmark = pytest.mark.gpu
+
+
+def mirrors(vol):
+    for m in range(0, 14):
+        vol.set_material(m, specular=0.4 + 0.04 * m, reflect_type=m % 2, shininess=2 + m % 5)
+
+
+@pytest.mark.parametrize("limit,K", [(2, 64), (3, 1), (3, 33), (4, 5), (4, 64), (5, 16), (8, 7), (8, 64), (9, 16)])
+def test_specular_segments_match_oracle(gpu_ready, limit, K):
+    pair = Pair("tiny", K=K)
+    try:
+        pair.vol.s.specBounceLimit = limit
+        mirrors(pair.vol)
+        for _ in range(3):
+            pair.draw()
+            pair.sync()
+            _, differ = pair.light()
+            assert differ == 0
+        check_counters(pair)
+    finally:
+        pair.close()
+
+
+def test_batched_limits_match_plain(gpu_ready):
+    def build():
+        out = []
+        for i, limit in enumerate((2, 3, 7)):
+            v, cfg = configs.build_volume("tiny", seed=40 + i)
+            mirrors(v)
+            v.s.specBounceLimit = limit
+            out.append(v)
+        return out
+
+    dn.init()
+    plain, batched = build(), build()
+    W, H = 96, 64
+    images = [dn.Image(W, H) for _ in plain]
+    batch = dn.Batch(batched)
+    try:
+        for frame in range(6):
+            # the last three frames repeat the composition (a replayed graph) with other limits
+            if frame == 3:
+                for vs in (plain, batched):
+                    vs[2].s.specBounceLimit = 2
+            if frame == 5:
+                for vs in (plain, batched):
+                    vs[0].s.specBounceLimit = 9
+            for v, im in zip(plain, images):
+                v.draw(im, *v.view_proj(H / W))
+                v.sync()
+                v.update_lighting(1, 1000, 1.0 + frame)
+            batch.run([dn.Batch.item(v, im, *v.view_proj(H / W), sync=(2, 1), light=(1, 1000, 1.0 + frame))
+                       for v, im in zip(batched, images)])
+            assert batch.finish()
+            for a, b in zip(plain, batched):
+                assert a.finish()
+                for x, y in zip(a.export_lighting(), b.export_lighting()):
+                    assert np.array_equal(x, y)
+    finally:
+        batch.close()
+        for im in images:
+            im.close()
+        for v in plain + batched:
+            v.close()

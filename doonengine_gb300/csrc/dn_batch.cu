@@ -20,6 +20,7 @@
 #include "dn_internal.cuh"
 #include "dn_light_stream.cuh"
 #include "dn_light_packet.cuh"
+#include "dn_light_path.cuh"
 #include <string.h>
 #include <stddef.h>
 #include <new>
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream_batc
 {
     __shared__ Job jobs[128];
     __shared__ TintT<128> tint;
-    stream_loop<true, false, FAR>(nullptr, &a, nullptr, jobs[threadIdx.x], tint);
+    stream_loop<true, FAR>(nullptr, &a, nullptr, jobs[threadIdx.x], tint);
 }
 
 // POOL: rays per fan kind per pool (the rays a warp pulls from a request group at a time); the autotuner
@@ -178,9 +179,9 @@ __global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* 
 // the diffuse paths of the voxels k_light_packet_batch lit, as per-lane path streams over every map's queue
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse_batch(const __grid_constant__ BatchLightArgs a)
 {
-    __shared__ Job jobs[128];
+    __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
-    stream_loop<true, true, false>(nullptr, &a, nullptr, jobs[threadIdx.x], tint);
+    path_loop<true>(nullptr, &a, jobs[threadIdx.x], tint);
 }
 
 __global__ void k_commit_batch(const BatchLightMap* l, const uint32_t* reqStart, uint32_t nl)

@@ -15,6 +15,7 @@
 #include "dn_internal.cuh"
 #include "dn_light_stream.cuh"
 #include "dn_light_packet.cuh"
+#include "dn_light_path.cuh"
 #include <stdio.h>
 #include <string.h>
 #include <stdlib.h>
@@ -653,7 +654,7 @@ __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream(cons
         (&sh.sinv[0][0])[i] = (&a.gtab->sinv[0][0])[i];
     }
     __syncthreads();
-    stream_loop<false, false, FAR>(&a, nullptr, &sh, jobs[threadIdx.x], tint);
+    stream_loop<false, FAR>(&a, nullptr, &sh, jobs[threadIdx.x], tint);
 }
 
 // What a lighting launch reads, before it: block 0 writes the launch's materials and shadow directions to the
@@ -690,13 +691,12 @@ __global__ void __launch_bounds__(128, packet_blocks(SEGS)) k_light_packet(const
     packet_loop<false, POOL, SEGS>(&a, nullptr, warps[threadIdx.x >> 5]);
 }
 
-// The diffuse paths of the voxels k_light_packet lit, as per-lane path streams over the whole request list:
-// a lane whose voxel's paths are done takes the next voxel, so no lane waits for another lane's long path.
+// the diffuse paths of the voxels k_light_packet lit (dn_light_path.cuh)
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const __grid_constant__ StreamArgs a)
 {
-    __shared__ Job jobs[128];
+    __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
-    stream_loop<false, true, false>(&a, nullptr, nullptr, jobs[threadIdx.x], tint);
+    path_loop<false>(&a, nullptr, jobs[threadIdx.x], tint);
 }
 
 // launches the lighting kernel g_lightKernel selects (1 ray streams, 2 warp packets followed by the

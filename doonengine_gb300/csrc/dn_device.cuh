@@ -229,24 +229,30 @@ __device__ __forceinline__ f3 sky_color(f3 bot, f3 top, f3 dir)
     return mk(bot.x * (1.0f - a) + top.x * a, bot.y * (1.0f - a) + top.y * a, bot.z * (1.0f - a) + top.z * a);
 }
 
-// n-th set bit of a chunk mask -> local position; false if n >= popcount
+// n-th set bit of a chunk mask -> local position; false if n >= popcount.  The partial counts name the quarter of the
+// mask, a binary search over popcounts the bit in its word.
 __device__ __forceinline__ bool select_voxel(const ChunkRec* r, uint32_t n, i3& out, uint32_t& li)
 {
-    uint32_t count = 0;
-    for (uint32_t w = 0; w < 16; w++) {
-        uint32_t bits = __ldg(&r->mask[w]);
-        uint32_t c = __popc(bits);
-        if (count + c > n) {
-            for (uint32_t k = n - count; k > 0; k--) bits &= bits - 1u;   // drop the k lowest set bits
-            uint32_t b = (uint32_t)(__ffs(bits) - 1);
-            uint32_t pos = w * 32u + b;
-            li = pos;
-            out.x = (int32_t)(pos & 7u); out.y = (int32_t)((pos >> 3) & 7u); out.z = (int32_t)(pos >> 6);
-            return true;
-        }
-        count += c;
+    const uint32_t p0 = __ldg(&r->partial[0]), p1 = __ldg(&r->partial[1]), p2 = __ldg(&r->partial[2]);
+    uint32_t w = 0, count = 0;
+    if (n >= p2) { w = 12; count = p2; }
+    else if (n >= p1) { w = 8; count = p1; }
+    else if (n >= p0) { w = 4; count = p0; }
+    const uint4 q = __ldg((const uint4*)&r->mask[w]);
+    uint32_t bits = q.x, c = (uint32_t)__popc(q.x);
+    if (n - count >= c) { count += c; w++; bits = q.y; c = (uint32_t)__popc(q.y); }
+    if (n - count >= c) { count += c; w++; bits = q.z; c = (uint32_t)__popc(q.z); }
+    if (n - count >= c) { count += c; w++; bits = q.w; c = (uint32_t)__popc(q.w); }
+    uint32_t k = n - count, b = 0;
+    if (k >= c) return false;
+#pragma unroll
+    for (uint32_t s = 16; s > 0; s >>= 1) {
+        const uint32_t low = (uint32_t)__popc((bits >> b) & ((1u << s) - 1u));
+        if (k >= low) { k -= low; b += s; }
     }
-    return false;
+    li = w * 32u + b;
+    out.x = (int32_t)(li & 7u); out.y = (int32_t)((li >> 3) & 7u); out.z = (int32_t)(li >> 6);
+    return true;
 }
 
 } // namespace dn

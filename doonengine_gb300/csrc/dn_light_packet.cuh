@@ -12,8 +12,8 @@
  * shaded once `batch` lanes have one.  Each ray's contributions go to shared memory; when the pool is empty,
  * each sum of a voxel's lighting is formed by one lane walking its rays (and their segments) in ray order, so
  * every sum is accumulated in exactly the reference's order.  The kernel writes each voxel's specular
- * lighting and leaves its direct light for the diffuse kernel (dn_light_stream.cuh,
- * stream_loop<.., true, false>), which traces the diffuse paths (numDiffuse per voxel, up to
+ * lighting and leaves its direct light for the diffuse kernel (path_loop,
+ * dn_light_path.cuh), which traces the diffuse paths (numDiffuse per voxel, up to
  * diffuseBounceLimit segments each) as per-lane path streams over all request groups and finishes each voxel
  * as the reference's lighting main does (running average, clamps, voxelLighting.comp:238-288).
  *

@@ -1,0 +1,248 @@
+/*
+ * dn_light_path.cuh -- the diffuse paths of a lighting update (voxelLighting.comp:148-214, 238-288).
+ *
+ * The packet kernel (dn_light_packet.cuh) leaves each voxel's direct light in its diffuse output slot; this kernel
+ * traces the voxel's numDiffuse paths of up to diffuseBounceLimit segments, forms the running average and replaces
+ * the slot.  Every lane owns one voxel and walks its paths in the reference's order; a lane whose voxel is done takes
+ * the next one of its warp's window, so that a long path holds no other lane.  The paths of a warp have nothing in
+ * common, so the walk's rounds run with about a third of the lanes, and what a segment's end needs runs for all
+ * waiting lanes at once when `batch` of them wait (or none is left stepping).
+ *
+ * The code between segments is one sequence -- finish, fetch, choose the direction, begin -- with each part in one
+ * place: as branches of one advance function, with the direction and the ray's start inlined at three ends, the
+ * kernel was 54 KB and waited for instructions a quarter of the time (2.7 of 10.9 cycles per instruction).
+ * With this loop and voxels found by their partial counts, us per frame or call, before -> after: 23x11x37 map with 2
+ * paths per voxel 575 -> 464; 16x16x16 map 520 -> 461; glass 2653 -> 2435; twelve maps batched 11806 -> 10142; 64x32x64
+ * map at 1080p 12324 -> 11826.
+ */
+#pragma once
+#include "dn_light_stream.cuh"
+
+// 7 blocks of 4 warps per SM; 6 and 8 within 1 %
+#ifndef DN_DIFF_MIN_BLOCKS
+#define DN_DIFF_MIN_BLOCKS 7
+#endif
+
+namespace dn {
+
+// per-lane voxel and path (shared memory, touched between segments only; an odd number of words per lane)
+struct PathJob {
+    f3 pos0, tnormal, direct;
+    f3 acc, carry, normal;       // the voxel's sum; the path's colour so far; the normal the next direction starts from
+    uint32_t material;           // of the last hit
+    uint32_t key, vidx, req, vlane;
+    float indirect;              // weight of the lighting so far (0: the voxel's first sample)
+    uint32_t b, i;               // bounce, path
+    uint32_t pad;
+};
+static_assert(sizeof(PathJob) % 8 == 4, "odd number of words");
+
+// The voxel's new diffuse lighting from its paths' sum (voxelLighting.comp:266-278, FP32)
+__device__ __forceinline__ void path_write(const PathJob& j, const DevMap& m, const dn_light_params& p, float4* out)
+{
+    const float4 prev = __ldg(&m.diff[j.vidx]);
+    const float den = j.indirect + (float)p.numDiffuse;
+    const f3 d = mk((prev.x * j.indirect + j.acc.x) / den, (prev.y * j.indirect + j.acc.y) / den,
+                    (prev.z * j.indirect + j.acc.z) / den);
+    out[((uint64_t)j.req * 32u + j.vlane) * 2u] = make_float4(gmin(gmax(d.x, 0.0f), 1.0f), gmin(gmax(d.y, 0.0f), 1.0f),
+                                                             gmin(gmax(d.z, 0.0f), 1.0f), 0.0f);
+}
+
+// Sets up voxel (req, vlane); false when the slot holds no voxel with diffuse paths, or its lighting needs no ray and
+// is written here.
+__device__ __forceinline__ bool path_setup(PathJob& j, uint32_t req, uint32_t vlane, const DevMap& m, const dn_light_params& p,
+                                           const Material* mats, const uint32_t* reqs, const uint32_t* nsamples, float4* out)
+{
+    const uint32_t word = reqs[req];
+    const uint32_t tile = word >> 4, group = word & 15u;
+    const uint32_t tw = __ldg(&m.tword[tile]);
+    const uint32_t vn = group * 32u + vlane;
+    i3 cp; uint32_t li;
+    const ChunkRec* rc = &m.rec[tw & SLOT_MASK];
+    if ((tw >> 30) != 2u || vn >= __ldg(&rc->nvox) || !select_voxel(rc, vn, cp, li)) return false;
+    const i3 mp{__ldg(&rc->pos[0]), __ldg(&rc->pos[1]), __ldg(&rc->pos[2])};
+    j.req = req; j.vlane = vlane;
+    j.vidx = __ldg(&rc->voxBase) + vn;
+    const uint2 w = __ldg(&m.vox[j.vidx]);
+    if (!(mats[w.x >> 24].specular < 1.0f)) return false;
+    j.tnormal = voxel_normal(w);
+    const uint32_t samples = __ldg(&nsamples[tw & SLOT_MASK]);
+    j.indirect = (float)(samples < p.maxDiffuse ? samples : p.maxDiffuse);
+    const uint32_t gx = (uint32_t)(mp.x * 8 + cp.x), gy = (uint32_t)(mp.y * 8 + cp.y), gz = (uint32_t)(mp.z * 8 + cp.z);
+    j.key = rng_key(__float_as_uint(p.time), p.mapId, gx + (m.sx * 8u) * (gy + (m.sy * 8u) * gz));
+    f3 rp;
+    rp.x = INV_CHUNK * (float)cp.x + (float)mp.x + HALF_INV_CHUNK;
+    rp.y = INV_CHUNK * (float)cp.y + (float)mp.y + HALF_INV_CHUNK;
+    rp.z = INV_CHUNK * (float)cp.z + (float)mp.z + HALF_INV_CHUNK;
+    const float off = HALF_INV_CHUNK - EPS;
+    j.pos0 = add(rp, muls(j.tnormal, off));
+    const float4 d = out[((uint64_t)req * 32u + vlane) * 2u];
+    j.direct = mk(d.x, d.y, d.z);
+    j.acc = mk(0.0f, 0.0f, 0.0f);
+    j.i = 0;
+    if (p.numDiffuse == 0u || p.diffuseBounceLimit == 0u) {
+        const f3 amb = mk(p.ambient[0], p.ambient[1], p.ambient[2]);
+        for (uint32_t i = 0; i < p.numDiffuse; i++) j.acc = add(add(j.acc, amb), j.direct);
+        path_write(j, m, p, out);
+        return false;
+    }
+    return true;
+}
+
+// direction of the path's next segment (voxelLighting.comp:160-168); last: the segment before it
+__device__ __forceinline__ f3 path_dir(const PathJob& j, f3 last, const dn_light_params& p, const Material* mats)
+{
+    const bool rngSin = p.rngMode == 1u;
+    const uint32_t at = j.i * 16u + j.b;
+    const float seed = p.time * (float)(j.i + 1u);
+    bool lobe = false;
+    f3 base = j.normal;
+    if (j.b > 0u) {
+        const Material& hm = mats[j.material];
+        const float r = rngSin ? srand1(seed + (float)p.diffuseBounceLimit + (float)j.b) : hrand(j.key, 2u, at << 8);
+        lobe = (r + 1.0f) * 0.5f < hm.specular;
+        if (lobe) base = muls(reflect(last, j.normal), (float)hm.shininess);
+    }
+    f3 d = base;
+    if (lobe || j.indirect != 0.0f) {
+        const f3 rs = rngSin ? sphere_sin(lobe ? p.time + (float)j.b : seed + (float)j.b) : sphere_hash(j.key, lobe ? 3u : 1u, at);
+        d = add(base, rs);
+    }
+    d = normalize(d);
+    return lobe ? d : adds(d, EPS);
+}
+
+// The persistent loop of the launch: one map (one) or a queue over the requests of many maps (many), each lane then
+// reading its voxel's map through that map's entry of the device table.
+template <bool MANY>
+__device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLightArgs* many, PathJob& j, TintT<128>& tint)
+{
+    const uint32_t lane = lane_id_s(), col = threadIdx.x;
+    const uint32_t batch = MANY ? many->batch : one->batch;
+    uint32_t nreq = 0;
+    if constexpr (MANY) nreq = *(volatile const uint32_t*)&many->reqStart[many->nmaps];
+    else nreq = *(volatile const uint32_t*)one->nreqPtr;
+    uint32_t* const counter = (MANY ? many->workCounter : one->workCounter) + 1;
+    uint32_t winMap = 0, winReq = 0, winNext = 32, winEnd = 32;   // warp-uniform voxel window: map, request, next voxel, end
+    const uint32_t parts = window_parts(nreq);
+    bool exhausted = false;
+    const BatchLightMap* le = nullptr;
+    if constexpr (MANY) le = &many->maps[0];
+    auto M = [&]() -> const DevMap& { if constexpr (MANY) return le->m; else return one->m; };
+    auto P = [&]() -> const dn_light_params& { if constexpr (MANY) return le->p; else return one->p; };
+    auto MATS = [&]() -> const Material* { if constexpr (MANY) return le->mats; else return one->gtab->mats; };
+    auto OUT = [&]() -> float4* { if constexpr (MANY) return le->out; else return one->out; };
+    Ray s;
+    s.mode = RM_IDLE;
+    bool own = false, done = false;    // the lane has a voxel; no voxel is left for it
+    Counters c{0, 0, 0, 0, 0};
+    for (;;) {
+        const unsigned waiting = __ballot_sync(0xFFFFFFFFu, !ray_stepping(s) && !done);
+        const unsigned stepping = __ballot_sync(0xFFFFFFFFu, ray_stepping(s));
+        if ((waiting | stepping) == 0u) break;
+        if (stepping == 0u || (uint32_t)__popc(waiting) >= batch) {
+            bool start = false;        // the lane's next segment starts
+            f3 org = mk(0.0f, 0.0f, 0.0f);
+            if (s.mode == RM_HIT || s.mode == RM_MISS) {
+                // diffuse_ray body after step_map (voxelLighting.comp:176-201)
+                f3 cadd;
+                float cmul;
+                ray_tint(s, tint, col, cadd, cmul);
+                if (s.mode == RM_HIT) {
+                    org = ray_hit_position<false>(s);
+                    const uint2 w = __ldg(&M().vox[ray_hit_index(s, M())]);
+                    const f3 albedo = mk((float)((w.y >> 24) & 0xFF) * INV255, (float)((w.y >> 16) & 0xFF) * INV255,
+                                         (float)((w.y >> 8) & 0xFF) * INV255);
+                    j.normal = voxel_normal(w);
+                    j.material = w.x >> 24;
+                    const f3 d = vabs(sub(vfloor(muls(j.pos0, 8.0f)), vfloor(muls(org, 8.0f))));
+                    if (!(dot(d, d) < 1.0f)) {
+                        if (MATS()[j.material].emissive) {
+                            const float e = P().emissiveStrength;
+                            j.acc.x = j.acc.x + j.carry.x * (albedo.x * e * cmul + cadd.x);
+                            j.acc.y = j.acc.y + j.carry.y * (albedo.y * e * cmul + cadd.y);
+                            j.acc.z = j.acc.z + j.carry.z * (albedo.z * e * cmul + cadd.z);
+                        } else {
+                            j.carry.x = j.carry.x * (albedo.x * cmul + cadd.x);
+                            j.carry.y = j.carry.y * (albedo.y * cmul + cadd.y);
+                            j.carry.z = j.carry.z * (albedo.z * cmul + cadd.z);
+                            j.b++;
+                            start = j.b < P().diffuseBounceLimit;
+                        }
+                    }
+                } else {
+                    const float k = gmax(dot(s.dir, mk(P().sunDir[0], P().sunDir[1], P().sunDir[2])), 0.0f);
+                    j.acc.x = j.acc.x + (j.carry.x * k * P().sunStrength[0] * cmul + cadd.x);
+                    j.acc.y = j.acc.y + (j.carry.y * k * P().sunStrength[1] * cmul + cadd.y);
+                    j.acc.z = j.acc.z + (j.carry.z * k * P().sunStrength[2] * cmul + cadd.z);
+                }
+                s.mode = RM_IDLE;
+                if (!start) {
+                    j.acc = add(j.acc, j.direct);
+                    j.i++;
+                    if (j.i >= P().numDiffuse) {
+                        path_write(j, M(), P(), OUT());
+                        own = false;
+                    }
+                }
+            }
+            // voxels for the lanes without one
+            for (;;) {
+                const unsigned need = __ballot_sync(0xFFFFFFFFu, !own && !done);
+                if (need == 0u) break;
+                if (winNext >= winEnd) {
+                    uint32_t r = 0;
+                    if (!exhausted && lane == 0) r = atomicAdd(counter, 1u);
+                    r = __shfl_sync(0xFFFFFFFFu, r, 0);
+                    if (exhausted || r >= nreq << parts) {
+                        exhausted = true;
+                        if (!own) done = true;
+                        break;
+                    }
+                    winNext = (r & ((1u << parts) - 1u)) << (5u - parts);
+                    winEnd = winNext + (32u >> parts);
+                    r >>= parts;
+                    winReq = r;
+                    if constexpr (MANY) {
+                        // the map whose request range holds r: reqStart[map] <= r < reqStart[map + 1]
+                        uint32_t lo = 0, hi = many->nmaps;
+                        while (hi - lo > 1u) {
+                            const uint32_t mid = (lo + hi) >> 1;
+                            if (__ldg(&many->reqStart[mid]) <= r) lo = mid; else hi = mid;
+                        }
+                        winMap = lo;
+                        winReq = r - __ldg(&many->reqStart[lo]);
+                    }
+                }
+                const uint32_t rank = __popc(need & ((1u << lane) - 1u));
+                if (!own && !done && winNext + rank < winEnd) {
+                    if constexpr (MANY) {
+                        le = &many->maps[winMap];
+                        own = path_setup(j, winReq, winNext + rank, le->m, le->p, le->mats, le->reqs, le->nsamples, le->out);
+                    } else {
+                        own = path_setup(j, winReq, winNext + rank, one->m, one->p, MATS(), one->reqs, one->nsamples, one->out);
+                    }
+                }
+                const uint32_t took = (uint32_t)__popc(need) < winEnd - winNext ? (uint32_t)__popc(need) : winEnd - winNext;
+                winNext += took;
+            }
+            // the next segment: a bounce, or a path's first
+            if (own && !ray_stepping(s)) {
+                if (!start) {
+                    j.acc = add(j.acc, mk(P().ambient[0], P().ambient[1], P().ambient[2]));
+                    j.carry = mk(1.0f, 1.0f, 1.0f);
+                    j.normal = adds(j.tnormal, EPS);
+                    j.b = 0;
+                    org = j.pos0;
+                }
+                const f3 d = path_dir(j, s.dir, P(), MATS());
+                ray_begin<false>(s, M(), org, d, rcp3(d), start, c, tint, col);
+                c.rays++;
+            }
+        }
+        if (ray_stepping(s)) walk_round<false>(s, M(), MATS(), P().sunStrength, c, tint, col);
+    }
+    flush_counters(MANY ? many->stats : one->stats, c, 0, 0);
+}
+
+} // namespace dn

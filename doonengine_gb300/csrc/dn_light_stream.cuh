@@ -27,12 +27,6 @@ namespace dn {
 #ifndef DN_STREAM_MIN_BLOCKS
 #define DN_STREAM_MIN_BLOCKS 4   // 4 blocks of 4 warps per SM (measured best: leaves L1 room for the tile map)
 #endif
-#ifndef DN_WINDOW_WARPS
-#define DN_WINDOW_WARPS 1
-#endif
-#ifndef DN_DIFF_MIN_BLOCKS
-#define DN_DIFF_MIN_BLOCKS 6     // the diffuse-path kernel (k_light_diffuse): 6 blocks of 4 warps per SM
-#endif
 
 enum : uint32_t { PH_FETCH = 0, PH_SPEC = 1, PH_SHADOW = 2, PH_DIFF = 3, PH_FINAL = 4, PH_DONE = 5 };
 
@@ -114,10 +108,7 @@ __device__ __forceinline__ f3 diffuse_dir(const Job& j, const dn_light_params& p
 
 // Consumes the finished segment (hitState 1 hit / 2 miss) and sets up the next segment of this lane's
 // voxel; returns true when a segment was started.  Leaves the job in PH_FETCH when the voxel is done.
-// DIFFONLY: the voxel's diffuse paths only (its specular and direct light came from the ray-fan kernel,
-// which left the direct light in the diffuse output slot); the final write replaces that slot with the
-// voxel's new diffuse lighting and leaves the specular slot and the lit-voxel count alone.
-template <bool DIFFONLY, bool FAR>
+template <bool FAR>
 __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const DevMap& m, const dn_light_params& p,
                                         const Material* mats, const float (*sdir)[3], const float (*sinv)[3],
                                         float4* out, Counters& c, uint32_t& lit)
@@ -136,9 +127,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
             hpos = ray_hit_position<FAR>(s);
             decompress(m, ray_hit_index(s, m), hv);
         }
-        // the diffuse-only kernel's jobs never reach the specular and shadow phases: with DIFFONLY their
-        // code is left out of it (a smaller kernel: fewer instruction-fetch stalls)
-        if (!DIFFONLY && j.phase == PH_SPEC) {
+        if (j.phase == PH_SPEC) {
             // specular_ray body after step_map (voxelLighting.comp:98-144)
             bool done = true;
             if (hit) {
@@ -188,7 +177,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
                 j.spec.z = j.spec.z + (sc.z * cmul + cadd.z) * j.jA.z;
             }
             if (done) { j.k++; j.b = 0; }
-        } else if (!DIFFONLY && j.phase == PH_SHADOW) {
+        } else if (j.phase == PH_SHADOW) {
             if (!hit) {
                 j.acc.x = j.acc.x + (sun.x * cmul + cadd.x);
                 j.acc.y = j.acc.y + (sun.y * cmul + cadd.y);
@@ -233,7 +222,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
     }
     // start the next segment of this voxel
     for (int guard = 0; guard < 8; guard++) {
-        if (!DIFFONLY && j.phase == PH_SPEC) {
+        if (j.phase == PH_SPEC) {
             if (j.k < p.K) {
                 if (p.specBounceLimit == 0u) { j.k++; continue; }
                 const Material& tm = mats[j.tmat];
@@ -249,7 +238,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
             j.k = 0;
             continue;
         }
-        if (!DIFFONLY && j.phase == PH_SHADOW) {
+        if (j.phase == PH_SHADOW) {
             const uint32_t n = j.firstSample ? 1u : p.K;
             if (j.k < n) {
                 const uint32_t q = j.firstSample ? 64u : j.k;
@@ -294,10 +283,8 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
                                             gmin(gmax(j.acc.z, 0.0f), 1.0f), 0.0f);
             const uint64_t o = ((uint64_t)j.req * 32u + j.vlane) * 2u;
             out[o] = outD;
-            if constexpr (!DIFFONLY) {
-                out[o + 1] = outS;
-                lit++;
-            }
+            out[o + 1] = outS;
+            lit++;
             j.phase = PH_FETCH;
         }
         return false;
@@ -306,9 +293,6 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
 }
 
 // Sets up voxel (req, vlane); returns false (and writes zero outputs) when the slot holds no voxel.
-// DIFFONLY: false (writing nothing) also for a voxel without diffuse paths; otherwise the job starts at its
-// diffuse paths with the direct light the ray-fan kernel left in the voxel's diffuse output slot.
-template <bool DIFFONLY = false>
 __device__ __forceinline__ bool voxel_setup(Job& j, uint32_t req, uint32_t vlane, const DevMap& m, const dn_light_params& p,
                                             const Material* mats, const uint32_t* reqs, const uint32_t* nsamples, float4* out)
 {
@@ -320,11 +304,9 @@ __device__ __forceinline__ bool voxel_setup(Job& j, uint32_t req, uint32_t vlane
     i3 cp; uint32_t li;
     const ChunkRec* rc = &m.rec[tw & SLOT_MASK];
     if ((tw >> 30) != 2u || vn >= __ldg(&rc->nvox) || !select_voxel(rc, vn, cp, li)) {
-        if constexpr (!DIFFONLY) {
-            const uint64_t o = ((uint64_t)req * 32u + vlane) * 2u;
-            out[o] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            out[o + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        }
+        const uint64_t o = ((uint64_t)req * 32u + vlane) * 2u;
+        out[o] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        out[o + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         return false;
     }
     const i3 mp{__ldg(&rc->pos[0]), __ldg(&rc->pos[1]), __ldg(&rc->pos[2])};
@@ -349,15 +331,6 @@ __device__ __forceinline__ bool voxel_setup(Job& j, uint32_t req, uint32_t vlane
     j.pos0 = add(rp, muls(j.tnormal, off));
     const Material& tm = mats[j.tmat];
     j.doDiff = tm.specular < 1.0f;
-    if constexpr (DIFFONLY) {
-        if (!j.doDiff) return false;
-        const float4 d = out[((uint64_t)req * 32u + vlane) * 2u];
-        j.direct = mk(d.x, d.y, d.z);
-        j.spec = mk(0.0f, 0.0f, 0.0f); j.acc = j.spec;
-        j.k = 0; j.b = 0; j.i = 0;
-        j.phase = PH_DIFF;
-        return true;
-    }
     const f3 viewDir = sub(j.pos0, mk(p.camPos[0], p.camPos[1], p.camPos[2]));
     j.doSpec = tm.specular > 0.0f && dot(viewDir, j.tnormal) < 0.0f && tm.reflectType <= 1u;
     if (j.doSpec) j.refl = reflect(normalize(viewDir), j.tnormal);
@@ -410,13 +383,21 @@ __device__ __forceinline__ void shadow_dir(const dn_light_params& p, int k, floa
     i3[0] = __frcp_rn(d.x); i3[1] = __frcp_rn(d.y); i3[2] = __frcp_rn(d.z);
 }
 
+// A warp's window into the queue is a whole request group, or a part of one (2^-result) when the launch has fewer
+// groups than warps: its few voxels then run on all SMs, and one waits for fewer others.
+__device__ __forceinline__ uint32_t window_parts(uint32_t nreq)
+{
+    uint32_t parts = 0;
+    while (parts < 5u && (nreq << (parts + 1u)) <= gridDim.x * (blockDim.x / 32u)) parts++;
+    return parts;
+}
+
 // The persistent loop of a lighting launch.  MANY = false: one map whose arguments live in the launch's
 // parameter space (one) and whose materials and shadow directions were staged into sh.  MANY = true: a
 // queue over the requests of many maps (many); each lane reads its current voxel's map, parameters,
-// materials and shadow directions from that map's entry of the device table.  DIFFONLY: the
-// diffuse paths of the voxels the ray-fan kernel lit (advance<true>); one map's materials are read from
-// its device tables (one->gtab) and sh is not used.  FAR: maps above FAR_SUM chunks (dn_walk.cuh).
-template <bool MANY, bool DIFFONLY, bool FAR>
+// materials and shadow directions from that map's entry of the device table.  FAR: maps above FAR_SUM chunks
+// (dn_walk.cuh).
+template <bool MANY, bool FAR>
 __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLightArgs* many, const StreamShared* sh,
                                             Job& j, TintT<128>& tint)
 {
@@ -425,12 +406,9 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
     uint32_t nreq = 0;
     if constexpr (MANY) nreq = *(volatile const uint32_t*)&many->reqStart[many->nmaps];
     else nreq = *(volatile const uint32_t*)one->nreqPtr;
-    uint32_t* const counter = (MANY ? many->workCounter : one->workCounter) + (DIFFONLY ? 1 : 0);
+    uint32_t* const counter = MANY ? many->workCounter : one->workCounter;
     uint32_t winMap = 0, winReq = 0, winNext = 32, winEnd = 32;   // warp-uniform voxel window: map, request, next voxel, end
-    // a window is a whole request group, or a part of one when the launch has fewer groups than warps: its few paths
-    // then run on all SMs, and a path waits for fewer others
-    uint32_t parts = 0;   // log2 of the windows per group
-    while (parts < 5u && (nreq << (parts + 1u)) <= gridDim.x * (blockDim.x / 32u) * DN_WINDOW_WARPS) parts++;
+    const uint32_t parts = window_parts(nreq);
     bool exhausted = false;
     j.phase = PH_FETCH;
     j.map = 0;
@@ -443,7 +421,6 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
     auto P = [&]() -> const dn_light_params& { if constexpr (MANY) return le->p; else return one->p; };
     auto MATS = [&]() -> const Material* {
         if constexpr (MANY) return le->mats;
-        else if constexpr (DIFFONLY) return one->gtab->mats;
         else return sh->mats;
     };
     Ray s;
@@ -491,9 +468,9 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
                             const BatchLightMap& e = many->maps[winMap];
                             if (winMap != lmi) { le = &e; lmi = winMap; }
                             j.map = winMap;
-                            voxel_setup<DIFFONLY>(j, winReq, winNext + rank, e.m, e.p, e.mats, e.reqs, e.nsamples, e.out);
+                            voxel_setup(j, winReq, winNext + rank, e.m, e.p, e.mats, e.reqs, e.nsamples, e.out);
                         } else {
-                            voxel_setup<DIFFONLY>(j, winReq, winNext + rank, one->m, one->p, MATS(), one->reqs, one->nsamples,
+                            voxel_setup(j, winReq, winNext + rank, one->m, one->p, MATS(), one->reqs, one->nsamples,
                                                   one->out);
                         }
                     }
@@ -504,11 +481,9 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
                 if (!ray_stepping(s) && j.phase != PH_DONE && j.phase != PH_FETCH) {
                     if constexpr (MANY) {
                         if (j.map != lmi) { le = &many->maps[j.map]; lmi = j.map; }
-                        advance<DIFFONLY, FAR>(j, s, tint, le->m, le->p, le->mats, le->sdir, le->sinv, le->out, c, lit);
-                    } else if constexpr (DIFFONLY) {
-                        advance<true, FAR>(j, s, tint, one->m, one->p, MATS(), one->gtab->sdir, one->gtab->sinv, one->out, c, lit);
+                        advance<FAR>(j, s, tint, le->m, le->p, le->mats, le->sdir, le->sinv, le->out, c, lit);
                     } else {
-                        advance<false, FAR>(j, s, tint, one->m, one->p, sh->mats, sh->sdir, sh->sinv, one->out, c, lit);
+                        advance<FAR>(j, s, tint, one->m, one->p, sh->mats, sh->sdir, sh->sinv, one->out, c, lit);
                     }
                 }
                 if (__ballot_sync(0xFFFFFFFFu, j.phase == PH_FETCH) == 0u) break;

@@ -58,14 +58,8 @@ __device__ __forceinline__ f3 refract(f3 I, f3 N, float eta)
     float s = eta * d + sqrtf(k);
     return sub(muls(I, eta), muls(N, s));
 }
-// float -> int32 with saturation, NaN -> 0
-__device__ __forceinline__ int32_t f2i(float x)
-{
-    if (x != x) return 0;
-    if (x >= 2147483648.0f) return 0x7FFFFFFF;
-    if (x < -2147483648.0f) return (int32_t)0x80000000;
-    return (int32_t)x;
-}
+// float -> int32 towards zero with saturation, NaN -> 0: what PTX's cvt.rzi.s32.f32 does
+__device__ __forceinline__ int32_t f2i(float x) { return __float2int_rz(x); }
 
 // ---------------------------------------------------------------- RNG (D5)
 
@@ -159,7 +153,7 @@ struct DevMap {
     // w0 + 2x + y * w1 + z * w2; a row's border cell also starts the next row, a plane's border row the next plane
     const uint32_t* __restrict__ tbits;
     uint32_t w0, w1, w2;
-    uint32_t wk;                         // w0 less what coded cells add (dn_walk.cuh)
+    uint32_t wk, tk, sxy;                // coded cells (dn_walk.cuh): w0 and tile 0 less what the codes add; sx * sy
     uint8_t* treq;
     uint8_t* ttouch;
     uint8_t* tvis;
@@ -181,13 +175,19 @@ __device__ __forceinline__ uint32_t map_index(const DevMap& m, i3 p)
     return (uint32_t)p.x + m.sx * ((uint32_t)p.y + m.sy * (uint32_t)p.z);
 }
 
-// rank of voxel li among the set bits (get_voxel_index, voxelShared.comp:150-169)
+// rank of voxel li among the set bits (get_voxel_index, voxelShared.comp:150-169): its quarter of the mask and the
+// partial counts as two 16-byte loads that do not wait for one another, no loop over words
 __device__ __forceinline__ uint32_t vox_rank(const ChunkRec* r, uint32_t li)
 {
-    uint32_t w = li >> 5;
-    uint32_t n = (w > 3) ? __ldg(&r->partial[(w >> 2) - 1]) : 0u;
-    for (uint32_t i = w & ~3u; i < w; i++) n += __popc(__ldg(&r->mask[i]));
-    return n + __popc(__ldg(&r->mask[w]) & ((1u << (li & 31)) - 1u));
+    const uint32_t w = li >> 5, quarter = w >> 2, in = w & 3u;
+    const uint4 m = __ldg((const uint4*)&r->mask[quarter * 4u]);
+    const uint4 p = __ldg((const uint4*)r->partial);   // partial[3], nvox
+    uint32_t n = quarter == 0u ? 0u : quarter == 1u ? p.x : quarter == 2u ? p.y : p.z;
+    const uint32_t own = in == 0u ? m.x : in == 1u ? m.y : in == 2u ? m.z : m.w;
+    n += in > 0u ? __popc(m.x) : 0;
+    n += in > 1u ? __popc(m.y) : 0;
+    n += in > 2u ? __popc(m.z) : 0;
+    return n + __popc(own & ((1u << (li & 31)) - 1u));
 }
 
 __device__ __forceinline__ f3 voxel_normal(uint2 w)

@@ -184,6 +184,8 @@ static inline dn::DevMap dev_map(const DNgpuVolume* g)
     const WalkGrid wg(g->sx, g->sy, g->sz);
     m.w0 = (uint32_t)(2u * wg.first); m.w1 = (uint32_t)(2u * wg.row); m.w2 = (uint32_t)(2u * wg.plane);
     m.wk = m.w0 - dn::CODE_BITS * (1u + m.w1 + m.w2);
+    m.sxy = g->sx * g->sy;
+    m.tk = 0u - dn::CODE_BITS / 2u - dn::CODE_BITS * (g->sx + m.sxy);
     m.tword = g->tword; m.tbits = g->tbits; m.treq = g->treq; m.ttouch = g->ttouch; m.tvis = g->tvis;
     m.rec = g->rec; m.vox = g->vox; m.diff = g->diff; m.spec = g->spec;
     m.degen = nullptr;                   // set by the launch: the draw's or the lighting's counter

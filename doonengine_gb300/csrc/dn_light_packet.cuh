@@ -84,7 +84,10 @@ constexpr uint32_t PK_POOL_ALT = PK_POOL_FAN == 64u ? 128u : 64u;   // the batch
 #define DN_PK_TAIL 8
 #endif
 constexpr uint32_t PK_MID = DN_PK_MID, PK_TAIL = DN_PK_TAIL;
-constexpr uint32_t PK_VOXELS = 16;
+#ifndef DN_PK_VOX
+#define DN_PK_VOX 16
+#endif
+constexpr uint32_t PK_VOXELS = DN_PK_VOX;
 
 template <uint32_t POOL, uint32_t SEGS>
 struct PacketWarpT {
@@ -327,7 +330,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                     const f3 hpos = ray_hit_position<false>(s);
                     Voxel hv;
                     decompress(m, ray_hit_index(s, m), hv);
-                    const i3 hp{f2i(truncf(hpos.x)), f2i(truncf(hpos.y)), f2i(truncf(hpos.z))};
+                    const i3 hp{f2i(hpos.x), f2i(hpos.y), f2i(hpos.z)};
                     if (in_map(m, hp)) {
                         uint8_t* vp = &m.tvis[map_index(m, hp)];
                         if (*vp == 0) *vp = 1;

@@ -131,7 +131,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
             // specular_ray body after step_map (voxelLighting.comp:98-144)
             bool done = true;
             if (hit) {
-                const i3 hp{f2i(truncf(hpos.x)), f2i(truncf(hpos.y)), f2i(truncf(hpos.z))};
+                const i3 hp{f2i(hpos.x), f2i(hpos.y), f2i(hpos.z)};
                 if (in_map(m, hp)) {
                     uint8_t* vp = &m.tvis[map_index(m, hp)];
                     if (*vp == 0) *vp = 1;

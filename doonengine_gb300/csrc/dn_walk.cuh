@@ -89,23 +89,26 @@ __device__ __forceinline__ float min3f(float a, float b, float c)
     return d;
 }
 
-// the first side distance of one axis (init_DDA, voxelShared.comp:305): sg is +-1, fl the cell's coordinate
+// the first side distance of one axis, (s * (fl - p) + s * 0.5 + 0.5) * delta of init_DDA (voxelShared.comp:305): sg is
+// +-1, so both products are exact and one fma rounds as their sum does; fl is the cell's coordinate
 __device__ __forceinline__ float side0(float sg, float fl, float p, float delta)
 {
-    return (sg * (fl - p) + sg * 0.5f + 0.5f) * delta;
+    return (__fmaf_rn(sg, fl - p, sg * 0.5f) + 0.5f) * delta;
 }
 
 // The code of voxel cell fl of a chunk: index x + 8y + 64z below bit 10; above it the steps left on each axis
 // (7 - x upwards, x downwards) in 4-bit fields, whose top bit appears when the axis leaves the chunk.  A step
 // along an axis adds voxel_steps' constant.  All exact in a float.
-__device__ __forceinline__ float voxel_code(f3 sg, f3 fl)
-{
-    const f3 left = mk(3.5f - sg.x * (fl.x - 3.5f), 3.5f - sg.y * (fl.y - 3.5f), 3.5f - sg.z * (fl.z - 3.5f));
-    return CODE_BASE + (fl.x + 8.0f * fl.y + 64.0f * fl.z) + 1024.0f * (left.x + 16.0f * left.y + 256.0f * left.z);
-}
 __device__ __forceinline__ f3 voxel_steps(f3 sg)
 {
-    return mk(sg.x - 1024.0f, 8.0f * sg.y - 16384.0f, 64.0f * sg.z - 262144.0f);
+    return mk(sg.x - 1024.0f, __fmaf_rn(sg.y, 8.0f, -16384.0f), __fmaf_rn(sg.z, 64.0f, -262144.0f));
+}
+// CODE_BASE + x + 8y + 64z + 1024 * (left.x + 16 left.y + 256 left.z) with left = 3.5 + 3.5 s - s * fl, sorted by fl
+__device__ __forceinline__ float voxel_code(f3 sg, f3 fl)
+{
+    const float base = __fmaf_rn(sg.x, 3584.0f, __fmaf_rn(sg.y, 57344.0f, __fmaf_rn(sg.z, 917504.0f, CODE_BASE + 978432.0f)));
+    return __fmaf_rn(fl.x, __fmaf_rn(sg.x, -1024.0f, 1.0f),
+                     __fmaf_rn(fl.y, __fmaf_rn(sg.y, -16384.0f, 8.0f), __fmaf_rn(fl.z, __fmaf_rn(sg.z, -262144.0f, 64.0f), base)));
 }
 
 // Chunk cells: CODE_BASE + 2x, CODE_BASE + y, CODE_BASE + z; FAR: the integers x, y, z in the floats' bits.
@@ -116,7 +119,7 @@ template <bool FAR>
 __device__ __forceinline__ f3 cell_code(f3 fl)
 {
     if constexpr (FAR) return mk(__int_as_float((int32_t)fl.x), __int_as_float((int32_t)fl.y), __int_as_float((int32_t)fl.z));
-    return mk(CODE_BASE + 2.0f * fl.x, CODE_BASE + fl.y, CODE_BASE + fl.z);
+    return mk(__fmaf_rn(2.0f, fl.x, CODE_BASE), CODE_BASE + fl.y, CODE_BASE + fl.z);
 }
 // the coordinates of a coded cell
 template <bool FAR>
@@ -133,6 +136,13 @@ __device__ __forceinline__ i3 cell_ints(f3 c)
         p.x = (p.x - (int32_t)CODE_BITS) >> 1; p.y -= (int32_t)CODE_BITS; p.z -= (int32_t)CODE_BITS;
     }
     return p;
+}
+// the tile of a map cell
+template <bool FAR>
+__device__ __forceinline__ uint32_t cell_tile(const DevMap& m, f3 c)
+{
+    if constexpr (FAR) return map_index(m, cell_ints<FAR>(c));
+    return (__float_as_uint(c.x) >> 1) + __float_as_uint(c.y) * m.sx + __float_as_uint(c.z) * m.sxy + m.tk;
 }
 // what a step adds to a coded cell
 template <bool FAR>
@@ -159,7 +169,7 @@ __device__ __forceinline__ uint32_t cell_state(const DevMap& m, f3 c)
 // whether whole coordinates fl are a cell of the map
 __device__ __forceinline__ bool inside_map(const DevMap& m, f3 fl)
 {
-    return fl.x >= 0.0f && fl.y >= 0.0f && fl.z >= 0.0f && fl.x < (float)m.sx && fl.y < (float)m.sy && fl.z < (float)m.sz;
+    return min3f(fl.x, fl.y, fl.z) >= 0.0f && fl.x < (float)m.sx && fl.y < (float)m.sy && fl.z < (float)m.sz;
 }
 
 // whether the coded voxel of a record is occupied
@@ -267,7 +277,7 @@ __device__ __forceinline__ void walk_round(Ray& r, const DevMap& m, const Materi
     }
     bool occ = false;
     if ((r.mode == RM_ENTER || r.mode == RM_ENTER_OPAQUE) && visit(c.outer, 1u)) {
-        const uint32_t tile = map_index(m, cell_ints<FAR>(r.cell));
+        const uint32_t tile = cell_tile<FAR>(m, r.cell);
         r.slot = __ldg(&m.tword[tile]) & SLOT_MASK;
         if (m.ttouch[tile] == 0) m.ttouch[tile] = 1;
         c.entered++;
@@ -450,7 +460,7 @@ __device__ __forceinline__ bool trace_primary(const DevMap& m, const Material* m
         c.outer++;
         if (st >= 2u) {
             c.entered++;
-            const uint32_t tile = map_index(m, cell_ints<FAR>(cell));
+            const uint32_t tile = cell_tile<FAR>(m, cell);
             const ChunkRec* rec = &m.rec[__ldg(&m.tword[tile]) & SLOT_MASK];
             if (m.ttouch[tile] == 0) m.ttouch[tile] = 1;
             f3 cp = chunk_entry(pos, dir, olast, cell_pos<FAR>(cell));

@@ -1536,5 +1536,5 @@ extern "C" const char* dn_cuda_kernel_names(void)
     return "k_draw;k_light_stream;k_light_packet;k_light_diffuse;k_light_prep;k_commit;k_sync_stage;k_pack_stage;k_compact;k_walk_border;k_flush;"
            "k_draw_batch;k_compact_batch;k_batch_reset;k_batch_prep;k_mark_opaque_batch;k_light_stream_batch;k_light_packet_batch;"
            "k_light_diffuse_batch;k_commit_batch;k_batch_gather;"
-           "k_shape_count;k_shape_write";
+           "k_shape_count;k_shape_write;k_shape_once";
 }

@@ -11,6 +11,9 @@
  *   host:                   exclusive prefix over the chunks;
  *   pass 2 (k_shape_write): each edited voxel's record at its chunk's offset plus its rank among the
  *                           chunk's edited voxels in voxel order z, y, x (warp ballots + a block scan).
+ * A shape over few chunks takes one pass (k_shape_once) that writes counts and records straight into pinned host
+ * memory, each chunk's at 512 times its number, and the host closes the gaps: such a call is all latency, and this is
+ * one launch and one wait instead of two of each with three copies.
  * The host side (voxelShapes.c of this library) applies the list to the CPU map with the reference's
  * rules.  Every float operation is the reference's, in its order, with no contraction, so the distances
  * and normals are bit-identical to the reference's x86 build.  Where the reference passes floats through
@@ -161,28 +164,51 @@ __global__ void __launch_bounds__(512) k_shape_count(ShapeArgs a)
     if (threadIdx.x == 0) a.counts[c] = (uint32_t)total;
 }
 
-__global__ void __launch_bounds__(512) k_shape_write(ShapeArgs a)
+// the record of this thread's voxel, if the shape touches it, behind `first` by its rank in the chunk; the block's
+// count in total
+__device__ __forceinline__ void write_hit(const ShapeArgs& a, uint64_t first, uint32_t cls, const float n[3], uint32_t& total)
 {
     __shared__ uint32_t warpCount[16];
-    int gx, gy, gz;
-    const uint32_t c = block_voxel(a, gx, gy, gz);
-    float n[3];
-    const uint32_t cls = shape_classify(a.p, gx, gy, gz, n);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const unsigned ballot = __ballot_sync(0xFFFFFFFFu, cls != 0u);
     if (lane == 0) warpCount[warp] = (uint32_t)__popc(ballot);
     __syncthreads();
-    if (cls == 0u) return;
     uint32_t rank = (uint32_t)__popc(ballot & ((1u << lane) - 1u));
-    for (uint32_t w = 0; w < warp; w++) rank += warpCount[w];
-    const uint64_t at = a.offsets[c] + rank;
-    if (at >= a.capacity) return;     // the host sized the list from pass 1; never taken
+    total = 0;
+    for (uint32_t w = 0; w < 16u; w++) {
+        if (w < warp) rank += warpCount[w];
+        total += warpCount[w];
+    }
+    const uint64_t at = first + rank;
+    if (cls == 0u || at >= a.capacity) return;     // the host sized the list; the second is never taken
     dn_shape_hit h;
     h.local = (uint16_t)threadIdx.x;
     h.inside = cls == 1u ? 1u : 0u;
     h.pad = 0;
     h.normal[0] = n[0]; h.normal[1] = n[1]; h.normal[2] = n[2];
     a.hits[at] = h;
+}
+
+__global__ void __launch_bounds__(512) k_shape_write(ShapeArgs a)
+{
+    int gx, gy, gz;
+    const uint32_t c = block_voxel(a, gx, gy, gz);
+    float n[3];
+    const uint32_t cls = shape_classify(a.p, gx, gy, gz, n);
+    uint32_t total;
+    write_hit(a, a.offsets[c], cls, n, total);
+}
+
+// both passes of a small shape; counts and hits are pinned host memory, chunk c's hits start at 512 c
+__global__ void __launch_bounds__(512) k_shape_once(ShapeArgs a)
+{
+    int gx, gy, gz;
+    const uint32_t c = block_voxel(a, gx, gy, gz);
+    float n[3];
+    const uint32_t cls = shape_classify(a.p, gx, gy, gz, n);
+    uint32_t total;
+    write_hit(a, (uint64_t)c * 512u, cls, n, total);
+    if (threadIdx.x == 0) a.counts[c] = total;
 }
 
 // device time of the evaluation passes and voxels evaluated, since the last reset
@@ -201,8 +227,8 @@ extern "C" void dn_cuda_shape_stats(uint64_t* voxels, double* deviceMs, int rese
 namespace {
 
 // Per-thread buffers of the evaluation, grown as needed and kept between calls (a shape call then costs
-// two launches and three copies, no allocation): device counts / offsets / hits, pinned host offsets and
-// hits, a stream and four timing events.  A shape call made from inside a transform function while the
+// one launch, or two and three copies, no allocation): device counts / offsets / hits, pinned host offsets, counts
+// and hits, a stream and four timing events.  A shape call made from inside a transform function while the
 // thread's buffers are still lent out (between dn_cuda_shape_eval and dn_cuda_shape_free) uses buffers
 // of its own for that call.  The buffers are not freed at thread exit.
 struct ShapeScratch {
@@ -214,6 +240,7 @@ struct ShapeScratch {
     uint64_t* doffsets; size_t nOffsets;
     dn_shape_hit* dhits; size_t nHits;
     uint64_t* hoffsets; size_t nHOffsets;
+    uint32_t* hcounts; size_t nHCounts;
     dn_shape_hit* hhits; size_t nHHits;
 };
 thread_local ShapeScratch t_scratch = {};
@@ -254,10 +281,42 @@ int scratch_ready(ShapeScratch& sc)
     return DN_CUDA_OK;
 }
 
-// the two passes on sc; hits land in sc.hhits (pinned)
+// Shapes over at most this many chunks take one pass: the records of 32 chunks are at most 256 KB to move on the host.
+// Frames that place or cut a sphere and relight it, us, before -> after: 639x400 (24x7x8 chunks) 135 -> 123, 101x64
+// (24x4x5) 95 -> 67, 720p with spheres of up to 11 voxels radius (27 to 64 chunks) 165 -> 161.
+const int64_t SHAPE_ONCE_CHUNKS = 32;
+
+// the evaluation on sc; hits land in sc.hhits (pinned)
 int shape_eval_on(ShapeScratch& sc, const ShapeArgs& proto, int64_t nchunks, uint32_t* counts, uint64_t* total)
 {
     ShapeArgs a = proto;
+    if (nchunks <= SHAPE_ONCE_CHUNKS) {
+        int rc = grow_pinned(sc.hcounts, sc.nHCounts, (size_t)nchunks);
+        if (!rc) rc = grow_pinned(sc.hhits, sc.nHHits, (size_t)nchunks * 512u);
+        if (rc) return rc;
+        a.counts = sc.hcounts;
+        a.hits = sc.hhits;
+        a.capacity = (uint64_t)nchunks * 512u;
+        COUNT_LAUNCH();
+        CK(cudaEventRecord(sc.ev[0], sc.stream));
+        k_shape_once<<<(unsigned)nchunks, 512, 0, sc.stream>>>(a);
+        CK(cudaGetLastError());
+        CK(cudaEventRecord(sc.ev[1], sc.stream));
+        CK(cudaStreamSynchronize(sc.stream));
+        float ms = 0.0f;
+        cudaEventElapsedTime(&ms, sc.ev[0], sc.ev[1]);
+        uint64_t sum = 0;
+        for (int64_t i = 0; i < nchunks; i++) {
+            counts[i] = sc.hcounts[i];
+            if (sum != (uint64_t)i * 512u)
+                memmove(sc.hhits + sum, sc.hhits + (size_t)i * 512u, (size_t)counts[i] * sizeof(dn_shape_hit));
+            sum += counts[i];
+        }
+        g_shapeMs += (double)ms;
+        g_shapeVoxels += (unsigned long long)nchunks * 512ull;
+        *total = sum;
+        return DN_CUDA_OK;
+    }
     int rc = grow_device(sc.dcounts, sc.nCounts, (size_t)nchunks);
     if (!rc) rc = grow_device(sc.doffsets, sc.nOffsets, (size_t)nchunks);
     if (!rc) rc = grow_pinned(sc.hoffsets, sc.nHOffsets, (size_t)nchunks);
@@ -306,6 +365,7 @@ void scratch_release(ShapeScratch& sc)
     if (sc.stream) cudaStreamDestroy(sc.stream);
     cudaFree(sc.dcounts); cudaFree(sc.doffsets); cudaFree(sc.dhits);
     cudaFreeHost(sc.hoffsets);
+    cudaFreeHost(sc.hcounts);
     sc = ShapeScratch{};
 }
 

@@ -42,7 +42,7 @@ struct DNgpuBatch {
     std::vector<DNgpuVolume*> members;
     unsigned char* htab; unsigned char* dtab; size_t tabCap;
     uint64_t tabGen;
-    uint32_t* workCounter;
+    uint32_t* workCounter;      // queue positions of the fans and of the diffuse paths, and BatchLightArgs::mixed
     DevState* bst;              // counters of batched launches (device)
     DevState* hbst;             // pinned copy
     unsigned long long* lsave;  // lighting counters saved around autotuning (device)
@@ -121,7 +121,7 @@ __global__ void k_batch_prep(BatchLightMap* l, uint32_t nl, const CompactArgs* s
     }
     __shared__ uint32_t warpSum[32];
     __shared__ uint32_t carry;
-    if (threadIdx.x == 0) { carry = 0; workCounter[0] = workCounter[1] = 0; }
+    if (threadIdx.x == 0) { carry = 0; workCounter[0] = workCounter[1] = workCounter[2] = 0; }
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     for (uint32_t base = 0; base < nl; base += blockDim.x) {
@@ -162,18 +162,19 @@ template <uint32_t POOL, uint32_t SEGS>
 __global__ void __launch_bounds__(128, packet_blocks(SEGS)) k_light_packet_batch(const __grid_constant__ BatchLightArgs a)
 {
     __shared__ PacketWarpT<POOL, SEGS> warps[4];
-    packet_loop<true, POOL, SEGS>(nullptr, &a, warps[threadIdx.x >> 5]);
+    if (*a.mixed) packet_loop<true, POOL, SEGS, true>(nullptr, &a, warps[threadIdx.x >> 5]);
+    else packet_loop<true, POOL, SEGS, false>(nullptr, &a, warps[threadIdx.x >> 5]);
 }
 
 // the opaque-chunk marks (mark_opaque_cells) of every map of a lighting launch: MARK_BLOCKS blocks per map
 constexpr uint32_t MARK_BLOCKS = 16;
-__global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* l)
+__global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* l, uint32_t* mixed)
 {
     const BatchLightMap& e = l[blockIdx.x / MARK_BLOCKS];
     const uint64_t pairs = WalkGrid(e.m.sx, e.m.sy, e.m.sz).words / 2u;
     const uint32_t per = blockDim.x / 32u;
     for (uint64_t w = (blockIdx.x % MARK_BLOCKS) * per + threadIdx.x / 32u; w < pairs; w += MARK_BLOCKS * per)
-        mark_opaque_cells(e.m, w, e.opaque);
+        mark_opaque_cells(e.m, w, e.opaque, mixed);
 }
 
 // the diffuse paths of the voxels k_light_packet_batch lit, as per-lane path streams over every map's queue
@@ -181,7 +182,8 @@ __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse_batch
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
-    path_loop<true>(nullptr, &a, jobs[threadIdx.x], tint);
+    if (*a.mixed) path_loop<true, true>(nullptr, &a, jobs[threadIdx.x], tint);
+    else path_loop<true, false>(nullptr, &a, jobs[threadIdx.x], tint);
 }
 
 __global__ void k_commit_batch(const BatchLightMap* l, const uint32_t* reqStart, uint32_t nl)
@@ -239,7 +241,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->copiesDone, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->tableFree, cudaEventDisableTiming);
     if (e != cudaSuccess) rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "stream / event: %s", cudaGetErrorString(e));
-    if (!rc) rc = dalloc(&b->workCounter, 2);
+    if (!rc) rc = dalloc(&b->workCounter, 3);
     if (!rc) rc = dalloc(&b->bst, 1);
     if (!rc) rc = dalloc(&b->lsave, 8);
     if (!rc) {
@@ -363,7 +365,7 @@ struct FramePlan {
 static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, uint32_t packets, bool far)
 {
     COUNT_LAUNCH();
-    k_mark_opaque_batch<<<la.nmaps * MARK_BLOCKS, 256, 0, s>>>(la.maps);
+    k_mark_opaque_batch<<<la.nmaps * MARK_BLOCKS, 256, 0, s>>>(la.maps, la.mixed);
     CK(cudaGetLastError());
     COUNT_LAUNCH();
     const unsigned grid = (unsigned)(g_numSMs * (int)b->tuning.blocksPerSM);
@@ -441,6 +443,7 @@ static int issue_frame(DNgpuBatch* b, const dn_batch_item* items, uint32_t n, co
         la.reqStart = (const uint32_t*)(d + t.oReqStart);
         la.nmaps = t.nl;
         la.workCounter = b->workCounter;
+        la.mixed = b->workCounter + 2;
         la.stats = b->bst->lstats;
         la.batch = b->tuning.streamBatch;
         int rc = issue_light(b, la, s, f.packets, f.far);
@@ -775,7 +778,7 @@ extern "C" int dn_cuda_batch_autotune(DNgpuBatch* b, dn_batch_tuning* chosen)
         la.batch = t.streamBatch;
         float ms = 3.4e38f;
         for (int rep = 0; rep < 2 && !rc; rep++) {
-            cudaError_t e = cudaMemsetAsync(b->workCounter, 0, 8, b->stream);
+            cudaError_t e = cudaMemsetAsync(b->workCounter, 0, 12, b->stream);
             if (e == cudaSuccess) e = cudaEventRecord(e0, b->stream);
             if (e != cudaSuccess) { rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "autotune: %s", cudaGetErrorString(e)); break; }
             rc = issue_light(b, la, b->stream, t.kernel == 2u ? b->lastSegs : 0u, b->lastFar);

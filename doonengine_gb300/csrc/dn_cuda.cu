@@ -665,20 +665,21 @@ __global__ void __launch_bounds__(256) k_light_prep(const __grid_constant__ DevM
                                                     const __grid_constant__ OpaqueSet opaque,
                                                     const __grid_constant__ MaterialTable t,
                                                     const __grid_constant__ dn_light_params p, LightTables* tab, DevState* st,
-                                                    uint64_t reqCap)
+                                                    uint64_t reqCap, uint32_t turn)
 {
     if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < 256; i += blockDim.x) tab->mats[i] = t.m[i];
         for (int k = threadIdx.x; k < 65; k += blockDim.x) shadow_dir(p, k, tab->sdir[k], tab->sinv[k]);
         if (threadIdx.x == 0) {
             st->work[0] = st->work[1] = 0;
+            st->mixed[turn ^ 1u] = 0;
             if (st->w[ST_REQ] > reqCap) st->w[ST_REQ] = (uint32_t)reqCap;
         }
         return;
     }
     const uint64_t stride = (uint64_t)(gridDim.x - 1u) * (blockDim.x / 32u);
     for (uint64_t w = (uint64_t)(blockIdx.x - 1u) * (blockDim.x / 32u) + threadIdx.x / 32u; w < nwords / 2u; w += stride)
-        mark_opaque_cells(m, w, opaque);
+        mark_opaque_cells(m, w, opaque, &st->mixed[turn]);
 }
 
 // The lighting launch with specular and shadow fans traced as warp packets (dn_light_packet.cuh).
@@ -688,7 +689,8 @@ __global__ void __launch_bounds__(128, packet_blocks(SEGS)) k_light_packet(const
     // shared memory holds only the four warps' pools (25 KB per block with 128-ray pools): 7 blocks take 175 KB, the
     // rest of the SM's 256 KB is L1 for the map's masks and voxels; the tables are read from a.gtab
     __shared__ PacketWarpT<POOL, SEGS> warps[4];
-    packet_loop<false, POOL, SEGS>(&a, nullptr, warps[threadIdx.x >> 5]);
+    if (*a.mixed) packet_loop<false, POOL, SEGS, true>(&a, nullptr, warps[threadIdx.x >> 5]);
+    else packet_loop<false, POOL, SEGS, false>(&a, nullptr, warps[threadIdx.x >> 5]);
 }
 
 // the diffuse paths of the voxels k_light_packet lit (dn_light_path.cuh)
@@ -696,7 +698,8 @@ __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
-    path_loop<false>(&a, nullptr, jobs[threadIdx.x], tint);
+    if (*a.mixed) path_loop<false, true>(&a, nullptr, jobs[threadIdx.x], tint);
+    else path_loop<false, false>(&a, nullptr, jobs[threadIdx.x], tint);
 }
 
 // launches the lighting kernel g_lightKernel selects (1 ray streams, 2 warp packets followed by the
@@ -717,10 +720,12 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materi
         const uint32_t maxBlocks = (uint32_t)(g->numSMs > 0 ? g->numSMs * 8 : 1024);
         COUNT_LAUNCH();
         k_light_prep<<<1u + (uint32_t)(blocks < maxBlocks ? blocks : maxBlocks), 256, 0, g->stream>>>(
-            dev_map(g), nwords, opaque_set(materials), table, a.p, g->dtab, g->st, g->reqCap);
+            dev_map(g), nwords, opaque_set(materials), table, a.p, g->dtab, g->st, g->reqCap, g->lightTurn);
         CK(cudaGetLastError());
     }
     a.gtab = g->dtab;
+    a.mixed = &g->st->mixed[g->lightTurn];
+    g->lightTurn ^= 1u;
     if (g_lightKernel == 2 && a.p.specBounceLimit <= PK_MAX_SPEC_SEGMENTS && !map_far(g)) {
         static const int packets2 = resident(k_light_packet<PK_POOL_FAN, 2>), packets4 = resident(k_light_packet<64, 4>),
                          packets8 = resident(k_light_packet<64, 8>), paths = resident(k_light_diffuse);

@@ -35,6 +35,9 @@ struct DevState {
     uint32_t w[4];                      // nreq, -, error flags, noalloc request count
     unsigned long long stats[8];        // draw kernels
     unsigned long long lstats[8];       // lighting kernels
+    // whether a loaded chunk was not all opaque in a lighting launch: the launches take turns, each zeroing the word of
+    // the next (a launch captured and replayed never does: its word then stays set, which is always right)
+    uint32_t mixed[2];
     uint32_t work[2];                   // queue positions of the lighting kernels: fans (or streams), diffuse paths
 };
 
@@ -56,6 +59,7 @@ struct DNgpuVolume {
     uint2* vox; float4* diff; float4* spec; uint64_t voxCap;
     uint32_t* reqs; float4* lightOut; uint64_t reqCap;
     DevState* st;
+    uint32_t lightTurn;                 // the word of DevState::mixed the next lighting launch sets
     dn::LightTables* dtab;              // materials and shadow directions of the last lighting launch (k_light_packet)
     // pinned staging for sync uploads and small readbacks
     // two pinned upload buffers: a sync takes one whose last upload is done, so the host does not wait for
@@ -263,8 +267,9 @@ static inline OpaqueSet opaque_set(const dn_material* mats)
 
 // Cells [32 * w, 32 * w + 32) of the walk grid, one per lane: every loaded tile to 3 (all its materials
 // opaque) or 2.  A lane per cell: its record's material set is two 16-byte loads, and the warp's votes form the
-// two words.  (One thread per word, 16 tiles and up to 128 dependent loads in a row, took 16 us on any map.)
-__device__ __forceinline__ void mark_opaque_cells(const dn::DevMap& m, uint64_t w, const OpaqueSet& op)
+// two words.  *mixed is set when a loaded chunk is not all opaque.  (One thread per word, 16 tiles and up to 128
+// dependent loads in a row, took 16 us on any map.)
+__device__ __forceinline__ void mark_opaque_cells(const dn::DevMap& m, uint64_t w, const OpaqueSet& op, uint32_t* mixed)
 {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t* tbits = const_cast<uint32_t*>(m.tbits);
@@ -283,6 +288,7 @@ __device__ __forceinline__ void mark_opaque_cells(const dn::DevMap& m, uint64_t 
     }
     const unsigned b0 = __ballot_sync(0xFFFFFFFFu, (st == 1u) || opaque);
     const unsigned b1 = __ballot_sync(0xFFFFFFFFu, st >= 2u);
+    if (lane == 0u && (b1 & ~b0)) *mixed = 1u;
     if (lane < 2u) {
         const uint32_t n = (spread_bits(lane ? b0 >> 16 : b0)) | (spread_bits(lane ? b1 >> 16 : b1) << 1);
         if (n != (lane ? words.y : words.x)) tbits[2u * w + lane] = n;

@@ -179,7 +179,7 @@ __device__ __forceinline__ bool packet_unit(uint32_t u, uint32_t nreq, uint32_t&
 // have one, so no lane waits for the slowest ray of a fan; each ray's contributions go to shared memory, and when
 // the pool is empty every voxel's sums are formed in the reference's order and written (its diffuse paths run in
 // k_light_diffuse, which reads the direct light left in the voxel's diffuse slot).
-template <bool MANY, uint32_t POOL, uint32_t SEGS>
+template <bool MANY, uint32_t POOL, uint32_t SEGS, bool TINTED>
 __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLightArgs* many, PacketWarpT<POOL, SEGS>& W)
 {
     static_assert(SEGS >= 2u && POOL >= 64u, "a slot holds a direction and its reciprocal, a pool one voxel's rays");
@@ -288,7 +288,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                             inv = mk(sinv[k][0], sinv[k][1], sinv[k][2]);
                         }
                         c.rays++;
-                        ray_begin<false>(s, m, W.v[vi].pos0, d, inv, false, c, W.tint, lane);
+                        ray_begin<false, TINTED>(s, m, W.v[vi].pos0, d, inv, false, c, W.tint, lane);
                     }
                     next = min(next + (uint32_t)__popc(need), total);
                 }
@@ -299,14 +299,14 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                 for (;;) {
                     const unsigned st = __ballot_sync(0xFFFFFFFFu, ray_stepping(s));
                     if (!st || (uint32_t)__popc(live & ~st) >= batch) break;
-                    if (ray_stepping(s)) walk_round<false>(s, m, mats, p.sunStrength, c, W.tint, lane);
+                    if (ray_stepping(s)) walk_round<false, TINTED>(s, m, mats, p.sunStrength, c, W.tint, lane);
                 }
                 // shade the ended segments
                 if (s.mode == RM_IDLE || ray_stepping(s)) continue;
                 const f3 sun = mk(p.sunStrength[0], p.sunStrength[1], p.sunStrength[2]);
                 f3 cadd;
                 float cmul;
-                ray_tint(s, W.tint, lane, cadd, cmul);
+                ray_tint<TINTED>(s, W.tint, lane, cadd, cmul);
                 const bool hit = s.mode == RM_HIT;
                 s.mode = RM_IDLE;
                 if (q >= nSpec) {
@@ -356,7 +356,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                                 W.con[up + 1u][q] = mult.y * (hv.albedo.y * cmul * hm.specular);
                                 W.con[up + 2u][q] = mult.z * (hv.albedo.z * cmul * hm.specular);
                                 const f3 nd = reflect(s.dir, hv.normal);
-                                ray_begin<false>(s, m, hpos, nd, rcp3(nd), true, c, W.tint, lane);
+                                ray_begin<false, TINTED>(s, m, hpos, nd, rcp3(nd), true, c, W.tint, lane);
                                 s.flags |= ((SEGS == 2u ? 1u : b + 1u) << RF_BOUNCES) | (hm.reflectType == 1u ? RF_SKY : 0u);
                                 c.rays++;
                             }

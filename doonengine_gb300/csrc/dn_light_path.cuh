@@ -114,7 +114,7 @@ __device__ __forceinline__ f3 path_dir(const PathJob& j, f3 last, const dn_light
 
 // The persistent loop of the launch: one map (one) or a queue over the requests of many maps (many), each lane then
 // reading its voxel's map through that map's entry of the device table.
-template <bool MANY>
+template <bool MANY, bool TINTED>
 __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLightArgs* many, PathJob& j, TintT<128>& tint)
 {
     const uint32_t lane = lane_id_s(), col = threadIdx.x;
@@ -147,7 +147,7 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
                 // diffuse_ray body after step_map (voxelLighting.comp:176-201)
                 f3 cadd;
                 float cmul;
-                ray_tint(s, tint, col, cadd, cmul);
+                ray_tint<TINTED>(s, tint, col, cadd, cmul);
                 if (s.mode == RM_HIT) {
                     org = ray_hit_position<false>(s);
                     const uint2 w = __ldg(&M().vox[ray_hit_index(s, M())]);
@@ -236,11 +236,11 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
                     org = j.pos0;
                 }
                 const f3 d = path_dir(j, s.dir, P(), MATS());
-                ray_begin<false>(s, M(), org, d, rcp3(d), start, c, tint, col);
+                ray_begin<false, TINTED>(s, M(), org, d, rcp3(d), start, c, tint, col);
                 c.rays++;
             }
         }
-        if (ray_stepping(s)) walk_round<false>(s, M(), MATS(), P().sunStrength, c, tint, col);
+        if (ray_stepping(s)) walk_round<false, TINTED>(s, M(), MATS(), P().sunStrength, c, tint, col);
     }
     flush_counters(MANY ? many->stats : one->stats, c, 0, 0);
 }

@@ -41,6 +41,7 @@ struct StreamArgs {
     uint32_t batch;
     dn_light_params p;
     const struct LightTables* gtab;   // the launch's materials and shadow directions (k_light_prep)
+    const uint32_t* mixed;            // nonzero: a loaded chunk has see-through voxels (mark_opaque_cells)
 };
 
 struct MaterialTable { Material m[256]; };
@@ -122,7 +123,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
         Voxel hv;
         f3 hpos = s.pos, cadd;
         float cmul;
-        ray_tint(s, tint, threadIdx.x, cadd, cmul);
+        ray_tint<true>(s, tint, threadIdx.x, cadd, cmul);
         if (hit) {
             hpos = ray_hit_position<FAR>(s);
             decompress(m, ray_hit_index(s, m), hv);
@@ -158,7 +159,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
                             const f3 nd = reflect(s.dir, hv.normal);
                             j.b++;
                             if (j.b < p.specBounceLimit) {
-                                ray_begin<FAR>(s, m, hpos, nd, rcp3(nd), true, c, tint, threadIdx.x);   // next bounce
+                                ray_begin<FAR, true>(s, m, hpos, nd, rcp3(nd), true, c, tint, threadIdx.x);   // next bounce
                                 c.rays++;
                                 return true;
                             }
@@ -205,7 +206,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
                         j.b++;
                         if (j.b < p.diffuseBounceLimit) {
                             const f3 nd = diffuse_dir(j, p, mats, rngSin);
-                            ray_begin<FAR>(s, m, hpos, nd, rcp3(nd), true, c, tint, threadIdx.x);
+                            ray_begin<FAR, true>(s, m, hpos, nd, rcp3(nd), true, c, tint, threadIdx.x);
                             c.rays++;
                             return true;
                         }
@@ -229,7 +230,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
                 j.b = 0; j.jA = j.talbedo; j.jB = j.pos0; j.jU = tm.reflectType;
                 const f3 P = mk(p.spherePts[j.k][0], p.spherePts[j.k][1], p.spherePts[j.k][2]);
                 const f3 sd = adds(normalize(add(muls(j.refl, (float)tm.shininess), P)), EPS);
-                ray_begin<FAR>(s, m, j.pos0, sd, rcp3(sd), false, c, tint, threadIdx.x);
+                ray_begin<FAR, true>(s, m, j.pos0, sd, rcp3(sd), false, c, tint, threadIdx.x);
                 c.rays++;
                 return true;
             }
@@ -242,7 +243,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
             const uint32_t n = j.firstSample ? 1u : p.K;
             if (j.k < n) {
                 const uint32_t q = j.firstSample ? 64u : j.k;
-                ray_begin<FAR>(s, m, j.pos0, mk(sdir[q][0], sdir[q][1], sdir[q][2]), mk(sinv[q][0], sinv[q][1], sinv[q][2]), false, c, tint, threadIdx.x);
+                ray_begin<FAR, true>(s, m, j.pos0, mk(sdir[q][0], sdir[q][1], sdir[q][2]), mk(sinv[q][0], sinv[q][1], sinv[q][2]), false, c, tint, threadIdx.x);
                 c.rays++;
                 return true;
             }
@@ -264,7 +265,7 @@ __device__ __forceinline__ bool advance(Job& j, Ray& s, TintT<128>& tint, const 
                     j.jU = j.tmat;
                 }
                 const f3 nd = diffuse_dir(j, p, mats, rngSin);
-                ray_begin<FAR>(s, m, j.pos0, nd, rcp3(nd), false, c, tint, threadIdx.x);
+                ray_begin<FAR, true>(s, m, j.pos0, nd, rcp3(nd), false, c, tint, threadIdx.x);
                 c.rays++;
                 return true;
             }
@@ -367,6 +368,7 @@ struct BatchLightArgs {
     uint32_t* workCounter;
     unsigned long long* stats;
     uint32_t batch;
+    uint32_t* mixed;            // nonzero: a loaded chunk of a map has see-through voxels (mark_opaque_cells)
 };
 
 // shadow directions normalize(sunDir * softness + P_k) + EPS (k < K) and sunDir + EPS ([64]) with reciprocals
@@ -489,7 +491,7 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
                 if (__ballot_sync(0xFFFFFFFFu, j.phase == PH_FETCH) == 0u) break;
             }
         }
-        if (ray_stepping(s)) walk_round<FAR>(s, M(), MATS(), P().sunStrength, c, tint, threadIdx.x);
+        if (ray_stepping(s)) walk_round<FAR, true>(s, M(), MATS(), P().sunStrength, c, tint, threadIdx.x);
     }
     flush_counters(MANY ? many->stats : one->stats, c, 0, lit);
 }

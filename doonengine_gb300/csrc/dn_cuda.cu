@@ -634,7 +634,8 @@ template <bool FAR, int WARPS>
 __global__ void __launch_bounds__(DN_DRAW_BX * DN_DRAW_BY, WARPS * 32 / (DN_DRAW_BX * DN_DRAW_BY)) k_draw(const __grid_constant__ DrawArgs a)
 {
     Counters c;
-    const uint32_t primary = draw_pixel<FAR>(a.d, a.mats, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y, c);
+    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = (blockIdx.z * gridDim.y + blockIdx.y) * blockDim.y + threadIdx.y;
+    const uint32_t primary = draw_pixel<FAR>(a.d, a.mats, x, y, c);
     flush_counters(a.d.stats, c, primary, 0);
 }
 
@@ -1294,12 +1295,15 @@ static int launch_draw(DNgpuVolume* g, const dn_draw_params* p, const dn_materia
     a->d.color = color; a->d.hit = hit; a->d.face = face; a->d.stats = g->st->stats;
     memcpy(a->mats, materials, sizeof(a->mats));
     dim3 block(DN_DRAW_BX, DN_DRAW_BY);
-    dim3 grid((p->width + DN_DRAW_BX - 1) / DN_DRAW_BX, (p->height + DN_DRAW_BY - 1) / DN_DRAW_BY);
+    // rows of blocks beyond the 65535 of a grid's y go to z
+    const uint32_t bx = (uint32_t)(((uint64_t)p->width + DN_DRAW_BX - 1) / DN_DRAW_BX),
+                   by = (uint32_t)(((uint64_t)p->height + DN_DRAW_BY - 1) / DN_DRAW_BY), bz = (by + 65534u) / 65535u;
+    const dim3 grid(bx, (by + bz - 1u) / bz, bz);
     COUNT_LAUNCH();
     // an image whose warps are all resident at 24 per SM takes the build for 24 (74 registers, no spills): a 257x143
     // draw 13.1 us against 14.0
     if (map_far(g)) k_draw<true, DN_DRAW_WARPS><<<grid, block, 0, g->stream>>>(*a);
-    else if (grid.x * grid.y * (DN_DRAW_BX * DN_DRAW_BY / 32u) <= 24u * (unsigned)g->numSMs) k_draw<false, 24><<<grid, block, 0, g->stream>>>(*a);
+    else if ((uint64_t)bx * by * (DN_DRAW_BX * DN_DRAW_BY / 32u) <= 24u * (uint64_t)g->numSMs) k_draw<false, 24><<<grid, block, 0, g->stream>>>(*a);
     else k_draw<false, DN_DRAW_WARPS><<<grid, block, 0, g->stream>>>(*a);
     CK(cudaGetLastError());
     return DN_CUDA_OK;

@@ -182,8 +182,9 @@ __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse_batch
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
-    if (*a.mixed) path_loop<true, true>(nullptr, &a, jobs[threadIdx.x], tint);
-    else path_loop<true, false>(nullptr, &a, jobs[threadIdx.x], tint);
+    __shared__ uint8_t order[128];
+    if (*a.mixed) path_loop<true, true>(nullptr, &a, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
+    else path_loop<true, false>(nullptr, &a, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
 }
 
 __global__ void k_commit_batch(const BatchLightMap* l, const uint32_t* reqStart, uint32_t nl)
@@ -230,7 +231,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     b->tuning.kernel = g_lightKernel == 2 ? 2u : 1u;
     b->tuning.streamBatch = b->tuning.kernel == 2u ? g_packetBatch : g_streamBatch;
     b->tuning.blocksPerSM = DN_STREAM_MIN_BLOCKS; b->tuning.useGraph = 1;
-    b->tuning.poolRays = PK_POOL_FAN; b->tuning.diffuseBatch = g_streamBatch;
+    b->tuning.poolRays = PK_POOL_FAN; b->tuning.diffuseBatch = g_pathBatch;
     b->lastSegs = 0; b->lastFar = false;
     b->graph = nullptr;
     b->lastLightValid = false;

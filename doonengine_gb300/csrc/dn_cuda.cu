@@ -92,10 +92,11 @@ void dn_new_generation(DNgpuVolume* g) { g->gen = __atomic_add_fetch(&g_generati
 extern "C" uint64_t dn_cuda_launch_count(void) { return __atomic_load_n(&g_launches, __ATOMIC_RELAXED); }
 extern "C" uint64_t dn_cuda_alloc_count(void) { return __atomic_load_n(&g_allocs, __ATOMIC_RELAXED); }
 
-// lighting kernel selection and stream batch threshold (DN_LIGHT_KERNEL=1 per-lane ray streams, 2 warp packets
+// lighting kernel selection and the batch thresholds of ray streams and diffuse paths (DN_LIGHT_KERNEL=1 per-lane ray streams, 2 warp packets
 // of ray fans; DN_STREAM_BATCH lanes, 1..32), read once at init
 int g_lightKernel = 2;
-uint32_t g_streamBatch = 24;
+uint32_t g_streamBatch = 28;   // the ray streams': 24 takes 3-10 % more, 20 6-15 %
+uint32_t g_pathBatch = 20;     // the diffuse paths': 24 takes up to 2 % more, 28 up to 3 %, 16 the same
 uint32_t g_packetBatch = 16;   // lanes with an ended segment before the packet kernel shades (12 and 20 within 1 %)
 
 static void noalloc_forget(void);
@@ -105,7 +106,7 @@ extern "C" int dn_cuda_init(int device)
     if (const char* e = getenv("DN_LIGHT_KERNEL")) g_lightKernel = atoi(e) == 1 ? 1 : 2;
     if (const char* e = getenv("DN_STREAM_BATCH")) {
         int b = atoi(e);
-        g_streamBatch = (uint32_t)(b < 1 ? 1 : (b > 32 ? 32 : b));
+        g_streamBatch = g_pathBatch = (uint32_t)(b < 1 ? 1 : (b > 32 ? 32 : b));
     }
     if (const char* e = getenv("DN_PACKET_BATCH")) {
         int b = atoi(e);
@@ -699,8 +700,9 @@ __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
-    if (*a.mixed) path_loop<false, true>(&a, nullptr, jobs[threadIdx.x], tint);
-    else path_loop<false, false>(&a, nullptr, jobs[threadIdx.x], tint);
+    __shared__ uint8_t order[128];
+    if (*a.mixed) path_loop<false, true>(&a, nullptr, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
+    else path_loop<false, false>(&a, nullptr, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
 }
 
 // launches the lighting kernel g_lightKernel selects (1 ray streams, 2 warp packets followed by the
@@ -738,7 +740,7 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materi
         default: k_light_packet<64, 8><<<g->numSMs * packets8, 128, 0, g->stream>>>(a); break;
         }
         CK(cudaGetLastError());
-        a.batch = g_streamBatch;
+        a.batch = g_pathBatch;
         COUNT_LAUNCH();
         k_light_diffuse<<<g->numSMs * paths, 128, 0, g->stream>>>(a);
     } else {

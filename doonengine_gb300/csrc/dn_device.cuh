@@ -75,11 +75,12 @@ __device__ __forceinline__ uint32_t rng_key(uint32_t seed, uint32_t mapId, uint3
 {
     return hash32(seed ^ hash32(voxel ^ hash32(mapId + 0x632be5abu)));
 }
-__device__ __forceinline__ float hrand(uint32_t key, uint32_t stream, uint32_t idx)
+__device__ __forceinline__ float hash_unit(uint32_t key, uint32_t x)
 {
-    uint32_t h = hash32(key ^ hash32((stream << 28) ^ idx));
+    uint32_t h = hash32(key ^ hash32(x));
     return (float)(h >> 8) * (1.0f / 8388608.0f) - 1.0f;
 }
+__device__ __forceinline__ float hrand(uint32_t key, uint32_t stream, uint32_t idx) { return hash_unit(key, (stream << 28) ^ idx); }
 // deterministic sine: Cody-Waite reduction by pi/2 and Taylor polynomials on [-pi/4, pi/4]
 __device__ __forceinline__ float det_sin(float x)
 {
@@ -95,17 +96,23 @@ __device__ __forceinline__ float det_sin(float x)
     return q == 0 ? s : (q == 1 ? c : (q == 2 ? -s : -c));
 }
 __device__ __forceinline__ float srand1(float s) { float v = det_sin(s) * 43758.5453f; return (v - floorf(v)) * 2.0f - 1.0f; }
+__device__ __forceinline__ f3 sphere_try_sin(float s) { return mk(srand1(s), srand1(s * 2.0f), srand1(s * 3.0f)); }
 static __device__ __noinline__ f3 sphere_sin(float seed)
 {
 #pragma unroll 1
     for (int t = 0; t < 64; t++) {
         float s = seed;
         seed = seed + 1.0f;
-        f3 p = mk(srand1(s), srand1(s * 2.0f), srand1(s * 3.0f));
+        f3 p = sphere_try_sin(s);
         if (dot(p, p) >= 1.0f) continue;
         return p;
     }
     return mk(0.0f, 0.0f, 0.0f);
+}
+// a point of the cube from the hashes of three numbers (hrand's of one stream)
+__device__ __forceinline__ f3 sphere_try_hash(uint32_t key, uint32_t x, uint32_t y, uint32_t z)
+{
+    return mk(hash_unit(key, x), hash_unit(key, y), hash_unit(key, z));
 }
 __device__ __forceinline__ f3 sphere_hash(uint32_t key, uint32_t stream, uint32_t base)
 {

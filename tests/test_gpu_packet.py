@@ -74,3 +74,54 @@ def test_batched_limits_match_plain(gpu_ready):
             im.close()
         for v in plain + batched:
             v.close()
+
+
+@pytest.mark.parametrize("paths,bounces", [(1, 1), (3, 6)])
+@pytest.mark.parametrize("rng", [0, 1])
+def test_path_directions_match_oracle(gpu_ready, rng, paths, bounces):
+    """sphere points drawn by a warp for its lanes: both generators, first segments only and many bounces"""
+    pair = Pair("tiny", K=5)
+    try:
+        pair.vol.s.rngMode, pair.vol.s.diffuseBounceLimit = rng, bounces
+        mirrors(pair.vol)
+        for _ in range(3):
+            pair.draw()
+            pair.sync()
+            _, differ = pair.light(num_diffuse=paths)
+            assert differ == 0
+        check_counters(pair)
+    finally:
+        pair.close()
+
+
+def test_batched_generators_match_plain(gpu_ready):
+    """maps of both generators in one batch: a warp's voxels come from both"""
+    def build():
+        out = []
+        for i in range(6):
+            v, _ = configs.build_volume("tiny", map=(1 + i, 2, 2), shapes=1 + i, seed=60 + i)
+            v.s.rngMode = i % 2
+            out.append(v)
+        return out
+
+    dn.init()
+    plain, batched = build(), build()
+    images = [dn.Image(96, 64) for _ in plain]
+    batch = dn.Batch(batched)
+    try:
+        for frame in range(4):
+            for v, im in zip(plain, images):
+                v.draw(im, *v.view_proj(64 / 96))
+                v.sync()
+                v.update_lighting(2, 1000, 1.0 + frame)
+            batch.run([dn.Batch.item(v, im, *v.view_proj(64 / 96), sync=(2, 1), light=(2, 1000, 1.0 + frame))
+                       for v, im in zip(batched, images)])
+            assert batch.finish()
+            for a, b in zip(plain, batched):
+                assert a.finish()
+                for x, y in zip(a.export_lighting(), b.export_lighting()):
+                    assert np.array_equal(x, y)
+    finally:
+        batch.close()
+        for x in images + plain + batched:
+            x.close()

@@ -672,6 +672,7 @@ __global__ void __launch_bounds__(256) k_light_prep(const __grid_constant__ DevM
     if (blockIdx.x == 0) {
         for (int i = threadIdx.x; i < 256; i += blockDim.x) tab->mats[i] = t.m[i];
         for (int k = threadIdx.x; k < 65; k += blockDim.x) shadow_dir(p, k, tab->sdir[k], tab->sinv[k]);
+        for (int i = threadIdx.x; i < 64 * 3; i += blockDim.x) (&tab->pts[0][0])[i] = (&p.spherePts[0][0])[i];
         if (threadIdx.x == 0) {
             st->work[0] = st->work[1] = 0;
             st->mixed[turn ^ 1u] = 0;

@@ -51,6 +51,7 @@ struct LightTables {
     Material mats[256];
     float sdir[65][3];   // shadow directions k < K, [64]: the first-sample direction sunDir + EPS
     float sinv[65][3];
+    float pts[64][3];    // the specular fan's offsets
 };
 
 __device__ __forceinline__ f3 rcp3(f3 d) { return mk(__frcp_rn(d.x), __frcp_rn(d.y), __frcp_rn(d.z)); }

@@ -11,9 +11,10 @@
  *   host:                   exclusive prefix over the chunks;
  *   pass 2 (k_shape_write): each edited voxel's record at its chunk's offset plus its rank among the
  *                           chunk's edited voxels in voxel order z, y, x (warp ballots + a block scan).
- * A shape over few chunks takes one pass (k_shape_once) that writes counts and records straight into pinned host
- * memory, each chunk's at 512 times its number, and the host closes the gaps: such a call is all latency, and this is
- * one launch and one wait instead of two of each with three copies.
+ * Both read and write pinned host memory: a call moves nothing but its edits, and three copies with their waits cost
+ * more than that (sphere of radius 8: 74 -> 54 us; 12: 120 -> 100; 24, 8 MB of edits: 540 either way).
+ * A shape over few chunks takes one pass (k_shape_once) that writes each chunk's records at 512 times its number, and the
+ * host closes the gaps: such a call is all latency, and this is one launch and one wait instead of two of each.
  * The host side (voxelShapes.c of this library) applies the list to the CPU map with the reference's
  * rules.  Every float operation is the reference's, in its order, with no contraction, so the distances
  * and normals are bit-identical to the reference's x86 build.  Where the reference passes floats through
@@ -227,8 +228,7 @@ extern "C" void dn_cuda_shape_stats(uint64_t* voxels, double* deviceMs, int rese
 namespace {
 
 // Per-thread buffers of the evaluation, grown as needed and kept between calls (a shape call then costs
-// one launch, or two and three copies, no allocation): device counts / offsets / hits, pinned host offsets, counts
-// and hits, a stream and four timing events.  A shape call made from inside a transform function while the
+// one launch or two, no allocation): pinned offsets, counts and hits, a stream and four timing events.  A shape call made from inside a transform function while the
 // thread's buffers are still lent out (between dn_cuda_shape_eval and dn_cuda_shape_free) uses buffers
 // of its own for that call.  The buffers are not freed at thread exit.
 struct ShapeScratch {
@@ -236,27 +236,11 @@ struct ShapeScratch {
     int device;
     cudaStream_t stream;
     cudaEvent_t ev[4];
-    uint32_t* dcounts; size_t nCounts;
-    uint64_t* doffsets; size_t nOffsets;
-    dn_shape_hit* dhits; size_t nHits;
     uint64_t* hoffsets; size_t nHOffsets;
     uint32_t* hcounts; size_t nHCounts;
     dn_shape_hit* hhits; size_t nHHits;
 };
 thread_local ShapeScratch t_scratch = {};
-
-template <class T> int grow_device(T*& p, size_t& cap, size_t need)
-{
-    if (need <= cap && p) return DN_CUDA_OK;
-    if (p) cudaFree(p);
-    p = nullptr;
-    cap = 0;
-    const size_t n = need < 1024 ? 1024 : need + need / 2;
-    COUNT_ALLOC();
-    CK(cudaMalloc((void**)&p, n * sizeof(T)));
-    cap = n;
-    return DN_CUDA_OK;
-}
 
 template <class T> int grow_pinned(T*& p, size_t& cap, size_t need)
 {
@@ -317,36 +301,32 @@ int shape_eval_on(ShapeScratch& sc, const ShapeArgs& proto, int64_t nchunks, uin
         *total = sum;
         return DN_CUDA_OK;
     }
-    int rc = grow_device(sc.dcounts, sc.nCounts, (size_t)nchunks);
-    if (!rc) rc = grow_device(sc.doffsets, sc.nOffsets, (size_t)nchunks);
+    int rc = grow_pinned(sc.hcounts, sc.nHCounts, (size_t)nchunks);
     if (!rc) rc = grow_pinned(sc.hoffsets, sc.nHOffsets, (size_t)nchunks);
     if (rc) return rc;
-    a.counts = sc.dcounts;
+    a.counts = sc.hcounts;
     COUNT_LAUNCH();
     CK(cudaEventRecord(sc.ev[0], sc.stream));
     k_shape_count<<<(unsigned)nchunks, 512, 0, sc.stream>>>(a);
     CK(cudaGetLastError());
     CK(cudaEventRecord(sc.ev[1], sc.stream));
-    CK(cudaMemcpyAsync(counts, sc.dcounts, (size_t)nchunks * 4, cudaMemcpyDeviceToHost, sc.stream));
     CK(cudaStreamSynchronize(sc.stream));
+    memcpy(counts, sc.hcounts, (size_t)nchunks * 4);
     float msCount = 0.0f, msWrite = 0.0f;
     cudaEventElapsedTime(&msCount, sc.ev[0], sc.ev[1]);
     uint64_t sum = 0;
     for (int64_t i = 0; i < nchunks; i++) { sc.hoffsets[i] = sum; sum += counts[i]; }
     if (sum) {
-        rc = grow_device(sc.dhits, sc.nHits, (size_t)sum);
-        if (!rc) rc = grow_pinned(sc.hhits, sc.nHHits, (size_t)sum);
+        rc = grow_pinned(sc.hhits, sc.nHHits, (size_t)sum);
         if (rc) return rc;
-        CK(cudaMemcpyAsync(sc.doffsets, sc.hoffsets, (size_t)nchunks * 8, cudaMemcpyHostToDevice, sc.stream));
-        a.offsets = sc.doffsets;
-        a.hits = sc.dhits;
+        a.offsets = sc.hoffsets;
+        a.hits = sc.hhits;
         a.capacity = sum;
         COUNT_LAUNCH();
         CK(cudaEventRecord(sc.ev[2], sc.stream));
         k_shape_write<<<(unsigned)nchunks, 512, 0, sc.stream>>>(a);
         CK(cudaGetLastError());
         CK(cudaEventRecord(sc.ev[3], sc.stream));
-        CK(cudaMemcpyAsync(sc.hhits, sc.dhits, (size_t)sum * sizeof(dn_shape_hit), cudaMemcpyDeviceToHost, sc.stream));
         CK(cudaStreamSynchronize(sc.stream));
         cudaEventElapsedTime(&msWrite, sc.ev[2], sc.ev[3]);
     } else if (!sc.hhits) {
@@ -363,7 +343,6 @@ void scratch_release(ShapeScratch& sc)
 {
     for (auto& e : sc.ev) if (e) cudaEventDestroy(e);
     if (sc.stream) cudaStreamDestroy(sc.stream);
-    cudaFree(sc.dcounts); cudaFree(sc.doffsets); cudaFree(sc.dhits);
     cudaFreeHost(sc.hoffsets);
     cudaFreeHost(sc.hcounts);
     sc = ShapeScratch{};

@@ -85,10 +85,10 @@ struct DNgpuVolume {
 
 
 // The draw's blocks: 16 x 8 pixels (a warp 16 x 2, whose rays stay together and whose rows are whole 32-byte sectors
-// of the image), 32 warps per SM (64 registers, 16 bytes of spills).  us per 1080p draw of the 64x32x64 map, 257x143
-// draw, edited 720p frame, 234x149 draw through glass: 309, 12.4, 192, 42; blocks of 8 x 32 335, 13.1, 197, 47; 8 x 8
-// 308, 13.1, 191, 48; 32 x 4 332, 12.9, 195, 40; 16 x 2 294, 12.9, 191, 47; 28 warps per SM 341, 12.4, 197, 42; 40 warps
-// 311, 12.3, 194, 42.
+// of the image), 32 warps per SM (64 registers, 12 bytes of spills).  us per 1080p draw of the 64x32x64 map, 257x143
+// draw, edited 720p frame, 234x149 draw through glass: 283, 11.4, 154, 35; blocks of 8 x 16 288, 11.6, 157, 39; 8 x 8
+// 283, 11.8, 156, 39; 32 x 4 302, 11.3, 157, 33; 16 x 4 284, 11.2, 156, 36; 28 warps per SM 291, 11.4, 156, 35; 24 warps
+// 312, 11.4, 160, 35.
 #ifndef DN_DRAW_WARPS
 #define DN_DRAW_WARPS 32
 #endif
@@ -352,48 +352,63 @@ __device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Mater
     using namespace dn;
     const dn_draw_params& p = a.p;
     cnt = Counters{0, 0, 0, 0, 0};
-    uint32_t primary = 0;
-    if (x < p.width && y < p.height) {
+    const bool inside = x < p.width && y < p.height;
+    const uint32_t limW = p.truncate16 ? (p.width / 16u) * 16u : p.width;
+    const uint32_t limH = p.truncate16 ? (p.height / 16u) * 16u : p.height;
+    const bool seen = x < limW && y < limH;         // the pixel is drawn
+    bool cast = false;                              // its ray meets the map
+    f3 rayPos = mk(p.origin[0], p.origin[1], p.origin[2]), rayDir = rayPos, inv = rayPos;
+    const f3 orgRayPos = rayPos;
+    float maxDepth = -1.0f;     // raster depth as a distance from the camera (voxelDraw.comp:86-101); negative: not tested
+    if (seen) {
+        const float sx = (float)x / (float)p.width * 2.0f - 1.0f;
+        const float sy = (float)y / (float)p.height * 2.0f - 1.0f;
+        const float (*M)[4] = p.dirMat;
+        f3 rd = mk(M[0][0] * sx + M[1][0] * sy + M[2][0] * 0.0f + M[3][0] * 1.0f,
+                   M[0][1] * sx + M[1][1] * sy + M[2][1] * 0.0f + M[3][1] * 1.0f,
+                   M[0][2] * sx + M[1][2] * sy + M[2][2] * 0.0f + M[3][2] * 1.0f);
+        rayDir = adds(normalize(rd), EPS);
+        inv = mk(1.0f / rayDir.x, 1.0f / rayDir.y, 1.0f / rayDir.z);
+        if (p.compose) {
+            float d;
+            raster_sample<1, 1>(p.rasterDepth, p.rasterDepthW, p.rasterDepthH, (float)x / (float)p.rasterColorW,
+                                (float)y / (float)p.rasterColorH, &d);
+            maxDepth = d * 2.0f - 1.0f;
+            if (maxDepth < 1.0f) {
+                const float (*P)[4] = p.invProj;
+                float vs[4];
+#pragma unroll
+                for (int r = 0; r < 4; r++) vs[r] = P[0][r] * sx + P[1][r] * sy + P[2][r] * maxDepth + P[3][r] * 1.0f;
+                const float wv = vs[3];
+                const f3 vsp = mk(vs[0] / wv, vs[1] / wv, vs[2] / wv);
+                maxDepth = sqrtf(dot(vsp, vsp));
+            } else {
+                maxDepth = -1.0f;
+            }
+        }
+        const f3 mapMax = mk((float)a.m.sx, (float)a.m.sy, (float)a.m.sz);
+        // intersect_AABB, voxelShared.comp:261-273
+        f3 tMin = mul(sub(mk(0.0f, 0.0f, 0.0f), rayPos), inv);
+        f3 tMax = mul(sub(mapMax, rayPos), inv);
+        f3 t1 = mk(gmin(tMin.x, tMax.x), gmin(tMin.y, tMax.y), gmin(tMin.z, tMax.z));
+        f3 t2 = mk(gmax(tMin.x, tMax.x), gmax(tMin.y, tMax.y), gmax(tMin.z, tMax.z));
+        float tNear = gmax(gmax(t1.x, t1.y), t1.z);
+        float tFar = gmin(gmin(t2.x, t2.y), t2.z);
+        cast = !(tNear > tFar || tFar < 0.0f);
+        if (cast && tNear > 0.0f) rayPos = add(rayPos, muls(rayDir, tNear + EPS));
+    }
+    f3 hitNormal;
+    f3 cadd; float cmul; PrimaryHit hi;
+    const bool found = trace_primary<FAR>(cast, a.m, mats, mk(p.sunStrength[0], p.sunStrength[1], p.sunStrength[2]), orgRayPos, rayPos,
+                                          rayDir, inv, maxDepth, hitNormal, cadd, cmul, hi, cnt);
+    if (inside) {
         const uint64_t pix = (uint64_t)y * p.width + x;
         uint32_t hitIdx = 0xFFFFFFFFu;
         uint8_t face = 6;
-        float4 out;
-        const uint32_t limW = p.truncate16 ? (p.width / 16u) * 16u : p.width;
-        const uint32_t limH = p.truncate16 ? (p.height / 16u) * 16u : p.height;
-        if (x >= limW || y >= limH) {
-            out = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
-        } else {
-            const float sx = (float)x / (float)p.width * 2.0f - 1.0f;
-            const float sy = (float)y / (float)p.height * 2.0f - 1.0f;
-            f3 rayPos = mk(p.origin[0], p.origin[1], p.origin[2]);
-            const f3 orgRayPos = rayPos;
-            const float (*M)[4] = p.dirMat;
-            f3 rd = mk(M[0][0] * sx + M[1][0] * sy + M[2][0] * 0.0f + M[3][0] * 1.0f,
-                       M[0][1] * sx + M[1][1] * sy + M[2][1] * 0.0f + M[3][1] * 1.0f,
-                       M[0][2] * sx + M[1][2] * sy + M[2][2] * 0.0f + M[3][2] * 1.0f);
-            f3 rayDir = adds(normalize(rd), EPS);
-            f3 inv = mk(1.0f / rayDir.x, 1.0f / rayDir.y, 1.0f / rayDir.z);
-            // raster depth as a distance from the camera (voxelDraw.comp:86-101); negative: not tested
-            float maxDepth = -1.0f;
-            float texS = 0.0f, texT = 0.0f;
-            if (p.compose) {
-                texS = (float)x / (float)p.rasterColorW;
-                texT = (float)y / (float)p.rasterColorH;
-                float d;
-                raster_sample<1, 1>(p.rasterDepth, p.rasterDepthW, p.rasterDepthH, texS, texT, &d);
-                maxDepth = d * 2.0f - 1.0f;
-                if (maxDepth < 1.0f) {
-                    const float (*P)[4] = p.invProj;
-                    float vs[4];
-#pragma unroll
-                    for (int r = 0; r < 4; r++) vs[r] = P[0][r] * sx + P[1][r] * sy + P[2][r] * maxDepth + P[3][r] * 1.0f;
-                    const float wv = vs[3];
-                    const f3 vsp = mk(vs[0] / wv, vs[1] / wv, vs[2] / wv);
-                    maxDepth = sqrtf(dot(vsp, vsp));
-                } else {
-                    maxDepth = -1.0f;
-                }
-            }
+        float4 out = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+        if (seen) {
+            f3 fc;
+            float depth = -1.0f;
             // background_color (voxelDraw.comp:24-30): the sky, or the raster colour where a depth is tested
             auto background = [&](f3 dir) -> f3 {
                 if (maxDepth < 0.0f) {
@@ -401,69 +416,54 @@ __device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Mater
                     return mk(powf(s.x, 2.2f), powf(s.y, 2.2f), powf(s.z, 2.2f));
                 }
                 float rc[3];
-                raster_sample<4, 3>(p.rasterColor, p.rasterColorW, p.rasterColorH, texS, texT, rc);
+                raster_sample<4, 3>(p.rasterColor, p.rasterColorW, p.rasterColorH, (float)x / (float)p.rasterColorW,
+                                (float)y / (float)p.rasterColorH, rc);
                 return mk(rc[0], rc[1], rc[2]);
             };
-            const f3 mapMax = mk((float)a.m.sx, (float)a.m.sy, (float)a.m.sz);
-            // intersect_AABB, voxelShared.comp:261-273
-            f3 tMin = mul(sub(mk(0.0f, 0.0f, 0.0f), rayPos), inv);
-            f3 tMax = mul(sub(mapMax, rayPos), inv);
-            f3 t1 = mk(gmin(tMin.x, tMax.x), gmin(tMin.y, tMax.y), gmin(tMin.z, tMax.z));
-            f3 t2 = mk(gmax(tMin.x, tMax.x), gmax(tMin.y, tMax.y), gmax(tMin.z, tMax.z));
-            float tNear = gmax(gmax(t1.x, t1.y), t1.z);
-            float tFar = gmin(gmin(t2.x, t2.y), t2.z);
-            f3 fc;
-            float depth = -1.0f;
-            if (tNear > tFar || tFar < 0.0f) {
-                fc = background(rayDir);
-            } else {
-                if (tNear > 0.0f) rayPos = add(rayPos, muls(rayDir, tNear + EPS));
-                f3 hitNormal;
-                f3 cadd; float cmul; PrimaryHit hi;
-                primary = 1;
-                if (trace_primary<FAR>(a.m, mats, mk(p.sunStrength[0], p.sunStrength[1], p.sunStrength[2]), orgRayPos, rayPos, rayDir,
-                                  inv, maxDepth, hitNormal, cadd, cmul, hi, cnt)) {
-                    i3 mp{f2i(floorf(rayPos.x)), f2i(floorf(rayPos.y)), f2i(floorf(rayPos.z))};
-                    if (in_map(a.m, mp)) {
-                        uint8_t* vp = &a.m.tvis[map_index(a.m, mp)];
-                        if (*vp == 0) *vp = 1;
-                    }
-                    f3 dv = sub(rayPos, orgRayPos);
-                    depth = sqrtf(dot(dv, dv));
-                    if (maxDepth > 0.0f && depth > maxDepth) {
-                        // the rasterised scene is in front of the voxel (voxelDraw.comp:127-131): the pixel shows
-                        // it, so no voxel is reported as hit
-                        fc = add(muls(background(rayDir), cmul), cadd);
-                        depth = maxDepth;
-                    } else {
-                        // voxel_color, voxelDraw.comp:32-61
-                        Voxel fv;
-                        decompress(a.m, hi.voxel, fv);
-                        const Material& mt = mats[fv.material];
-                        f3 sp = muls(fv.spec, mt.specular);
-                        f3 df = muls(fv.diff, 1.0f - mt.specular);
-                        switch (p.viewMode) {
-                        case 0: {
-                            f3 solid = mt.emissive ? muls(fv.albedo, p.emissiveStrength) : add(mul(df, fv.albedo), sp);
-                            fc = add(muls(solid, cmul), cadd);
-                            break;
-                        }
-                        case 1: fc = fv.albedo; break;
-                        case 2: fc = mt.emissive ? fv.albedo : df; break;
-                        case 3: fc = mt.emissive ? fv.albedo : sp; break;
-                        case 4: fc = vabs(fv.normal); break;
-                        case 5: fc = vabs(hitNormal); break;
-                        default: fc = mk(0.0f, 0.0f, 0.0f); break;
-                        }
-                        const uint32_t gx = (uint32_t)hi.cell.x * 8u + (hi.local & 7u), gy = (uint32_t)hi.cell.y * 8u + ((hi.local >> 3) & 7u),
-                                       gz = (uint32_t)hi.cell.z * 8u + (hi.local >> 6);
-                        hitIdx = gx + (a.m.sx * 8u) * (gy + (a.m.sy * 8u) * gz);
-                        if (hitNormal.x > 0.0f) face = 0; else if (hitNormal.x < 0.0f) face = 1;
-                        else if (hitNormal.y > 0.0f) face = 2; else if (hitNormal.y < 0.0f) face = 3;
-                        else if (hitNormal.z > 0.0f) face = 4; else if (hitNormal.z < 0.0f) face = 5;
-                    }
-                } else {
+            if (found) {
+                i3 mp{f2i(floorf(rayPos.x)), f2i(floorf(rayPos.y)), f2i(floorf(rayPos.z))};
+                if (in_map(a.m, mp)) {
+                    uint8_t* vp = &a.m.tvis[map_index(a.m, mp)];
+                    if (*vp == 0) *vp = 1;
+                }
+                f3 dv = sub(rayPos, orgRayPos);
+                depth = sqrtf(dot(dv, dv));
+                if (maxDepth > 0.0f && depth > maxDepth) {
+                    // the rasterised scene is in front of the voxel (voxelDraw.comp:127-131): the pixel shows
+                    // it, so no voxel is reported as hit
                     fc = add(muls(background(rayDir), cmul), cadd);
+                    depth = maxDepth;
+                } else {
+                    // voxel_color, voxelDraw.comp:32-61
+                    Voxel fv;
+                    decompress(a.m, hi.voxel, fv);
+                    const Material& mt = mats[fv.material];
+                    f3 sp = muls(fv.spec, mt.specular);
+                    f3 df = muls(fv.diff, 1.0f - mt.specular);
+                    switch (p.viewMode) {
+                    case 0: {
+                        f3 solid = mt.emissive ? muls(fv.albedo, p.emissiveStrength) : add(mul(df, fv.albedo), sp);
+                        fc = add(muls(solid, cmul), cadd);
+                        break;
+                    }
+                    case 1: fc = fv.albedo; break;
+                    case 2: fc = mt.emissive ? fv.albedo : df; break;
+                    case 3: fc = mt.emissive ? fv.albedo : sp; break;
+                    case 4: fc = vabs(fv.normal); break;
+                    case 5: fc = vabs(hitNormal); break;
+                    default: fc = mk(0.0f, 0.0f, 0.0f); break;
+                    }
+                    const uint32_t gx = (uint32_t)hi.cell.x * 8u + (hi.local & 7u), gy = (uint32_t)hi.cell.y * 8u + ((hi.local >> 3) & 7u),
+                                   gz = (uint32_t)hi.cell.z * 8u + (hi.local >> 6);
+                    hitIdx = gx + (a.m.sx * 8u) * (gy + (a.m.sy * 8u) * gz);
+                    if (hitNormal.x > 0.0f) face = 0; else if (hitNormal.x < 0.0f) face = 1;
+                    else if (hitNormal.y > 0.0f) face = 2; else if (hitNormal.y < 0.0f) face = 3;
+                    else if (hitNormal.z > 0.0f) face = 4; else if (hitNormal.z < 0.0f) face = 5;
+                }
+            } else {
+                fc = background(rayDir);
+                if (cast) {
+                    fc = add(muls(fc, cmul), cadd);
                     depth = maxDepth;
                 }
             }
@@ -473,7 +473,7 @@ __device__ __forceinline__ uint32_t draw_pixel(const DrawMap& a, const dn::Mater
         if (a.hit) a.hit[pix] = hitIdx;
         if (a.face) a.face[pix] = face;
     }
-    return primary;
+    return cast ? 1u : 0u;
 }
 
 // -------------------------------------------------------------- sync

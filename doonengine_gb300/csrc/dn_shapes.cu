@@ -11,8 +11,8 @@
  *   host:                   exclusive prefix over the chunks;
  *   pass 2 (k_shape_write): each edited voxel's record at its chunk's offset plus its rank among the
  *                           chunk's edited voxels in voxel order z, y, x (warp ballots + a block scan).
- * Both read and write pinned host memory: a call moves nothing but its edits, and three copies with their waits cost
- * more than that (sphere of radius 8: 74 -> 54 us; 12: 120 -> 100; 24, 8 MB of edits: 540 either way).
+ * Counts and offsets are in pinned host memory, and so are the edits of all but large shapes: copies with their waits
+ * cost more than the kernels' accesses (sphere of radius 8: 74 -> 54 us; 12, 7200 edits: 120 -> 100).
  * A shape over few chunks takes one pass (k_shape_once) that writes each chunk's records at 512 times its number, and the
  * host closes the gaps: such a call is all latency, and this is one launch and one wait instead of two of each.
  * The host side (voxelShapes.c of this library) applies the list to the CPU map with the reference's
@@ -228,7 +228,8 @@ extern "C" void dn_cuda_shape_stats(uint64_t* voxels, double* deviceMs, int rese
 namespace {
 
 // Per-thread buffers of the evaluation, grown as needed and kept between calls (a shape call then costs
-// one launch or two, no allocation): pinned offsets, counts and hits, a stream and four timing events.  A shape call made from inside a transform function while the
+// one launch or two, no allocation): pinned offsets, counts and hits, device hits of
+// large shapes, a stream and four timing events.  A shape call made from inside a transform function while the
 // thread's buffers are still lent out (between dn_cuda_shape_eval and dn_cuda_shape_free) uses buffers
 // of its own for that call.  The buffers are not freed at thread exit.
 struct ShapeScratch {
@@ -239,8 +240,22 @@ struct ShapeScratch {
     uint64_t* hoffsets; size_t nHOffsets;
     uint32_t* hcounts; size_t nHCounts;
     dn_shape_hit* hhits; size_t nHHits;
+    dn_shape_hit* dhits; size_t nHits;
 };
 thread_local ShapeScratch t_scratch = {};
+
+template <class T> int grow_device(T*& p, size_t& cap, size_t need)
+{
+    if (need <= cap && p) return DN_CUDA_OK;
+    if (p) cudaFree(p);
+    p = nullptr;
+    cap = 0;
+    const size_t n = need < 1024 ? 1024 : need + need / 2;
+    COUNT_ALLOC();
+    CK(cudaMalloc((void**)&p, n * sizeof(T)));
+    cap = n;
+    return DN_CUDA_OK;
+}
 
 template <class T> int grow_pinned(T*& p, size_t& cap, size_t need)
 {
@@ -269,6 +284,12 @@ int scratch_ready(ShapeScratch& sc)
 // Frames that place or cut a sphere and relight it, us, before -> after: 639x400 (24x7x8 chunks) 135 -> 123, 101x64
 // (24x4x5) 95 -> 67, 720p with spheres of up to 11 voxels radius (27 to 64 chunks) 165 -> 161.
 const int64_t SHAPE_ONCE_CHUNKS = 32;
+
+// At most this many edits are written straight to the host.  Shapes larger than that are evaluated faster than the link to
+// the host takes their edits, so the second pass writes device memory and one copy follows: the same time for a call
+// (sphere of radius 24, 58000 edits, 540 us either way), and the passes' own time, which dn_cuda_shape_stats reports, is
+// a third (16 shapes of up to 48 voxels half extent 0.41 ms, 1.13 with direct writes; 0.44 with a limit of 32768 edits).
+const uint64_t SHAPE_DIRECT_EDITS = 8192;
 
 // the evaluation on sc; hits land in sc.hhits (pinned)
 int shape_eval_on(ShapeScratch& sc, const ShapeArgs& proto, int64_t nchunks, uint32_t* counts, uint64_t* total)
@@ -317,16 +338,19 @@ int shape_eval_on(ShapeScratch& sc, const ShapeArgs& proto, int64_t nchunks, uin
     uint64_t sum = 0;
     for (int64_t i = 0; i < nchunks; i++) { sc.hoffsets[i] = sum; sum += counts[i]; }
     if (sum) {
+        const bool direct = sum <= SHAPE_DIRECT_EDITS;
         rc = grow_pinned(sc.hhits, sc.nHHits, (size_t)sum);
+        if (!rc && !direct) rc = grow_device(sc.dhits, sc.nHits, (size_t)sum);
         if (rc) return rc;
         a.offsets = sc.hoffsets;
-        a.hits = sc.hhits;
+        a.hits = direct ? sc.hhits : sc.dhits;
         a.capacity = sum;
         COUNT_LAUNCH();
         CK(cudaEventRecord(sc.ev[2], sc.stream));
         k_shape_write<<<(unsigned)nchunks, 512, 0, sc.stream>>>(a);
         CK(cudaGetLastError());
         CK(cudaEventRecord(sc.ev[3], sc.stream));
+        if (!direct) CK(cudaMemcpyAsync(sc.hhits, sc.dhits, (size_t)sum * sizeof(dn_shape_hit), cudaMemcpyDeviceToHost, sc.stream));
         CK(cudaStreamSynchronize(sc.stream));
         cudaEventElapsedTime(&msWrite, sc.ev[2], sc.ev[3]);
     } else if (!sc.hhits) {
@@ -343,6 +367,7 @@ void scratch_release(ShapeScratch& sc)
 {
     for (auto& e : sc.ev) if (e) cudaEventDestroy(e);
     if (sc.stream) cudaStreamDestroy(sc.stream);
+    cudaFree(sc.dhits);
     cudaFreeHost(sc.hoffsets);
     cudaFreeHost(sc.hcounts);
     sc = ShapeScratch{};

@@ -62,7 +62,7 @@ struct DNgpuBatch {
     BatchLightArgs lastLight;
     bool lastLightValid;
     uint32_t lastSegs;          // the packet build the last frame's maps can take (its segments; 0: ray streams only)
-    bool lastFar;
+    bool lastFar, lastSide;
     std::vector<std::pair<DNgpuVolume*, uint64_t>> lastLightGens;
 };
 
@@ -178,13 +178,14 @@ __global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* 
 }
 
 // the diffuse paths of the voxels k_light_packet_batch lit, as per-lane path streams over every map's queue
+template <bool SIDE>
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse_batch(const __grid_constant__ BatchLightArgs a)
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
     __shared__ uint8_t order[128];
-    if (*a.mixed) path_loop<true, true>(nullptr, &a, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
-    else path_loop<true, false>(nullptr, &a, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
+    if (*a.mixed) path_loop<true, true, SIDE>(nullptr, &a, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
+    else path_loop<true, false, SIDE>(nullptr, &a, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
 }
 
 __global__ void k_commit_batch(const BatchLightMap* l, const uint32_t* reqStart, uint32_t nl)
@@ -232,7 +233,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     b->tuning.streamBatch = b->tuning.kernel == 2u ? g_packetBatch : g_streamBatch;
     b->tuning.blocksPerSM = DN_STREAM_MIN_BLOCKS; b->tuning.useGraph = 1;
     b->tuning.poolRays = PK_POOL_FAN; b->tuning.diffuseBatch = g_pathBatch;
-    b->lastSegs = 0; b->lastFar = false;
+    b->lastSegs = 0; b->lastFar = b->lastSide = false;
     b->graph = nullptr;
     b->lastLightValid = false;
     int rc = DN_CUDA_OK;
@@ -261,7 +262,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM2, k_light_packet_batch<PK_POOL_FAN, 2>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMAlt, k_light_packet_batch<PK_POOL_ALT, 2>, 128, 0);
         b->maxBlocksPacketAlt = perSMAlt < 1 ? 1 : perSMAlt;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM3, k_light_diffuse_batch, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM3, k_light_diffuse_batch<true>, 128, 0);
         if (e != cudaSuccess) rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "occupancy: %s", cudaGetErrorString(e));
         b->maxBlocksPerSM = perSM < 1 ? 1 : perSM;
         b->maxBlocksPacket = perSM2 < 1 ? 1 : perSM2;
@@ -358,12 +359,13 @@ struct FramePlan {
     uint32_t drawBlocks, syncBlocks;
     bool hostImages;
     uint32_t packets;           // lighting as warp packets (dn_light_packet.cuh): the build's segments, or 0
+    bool side;                  // a lit map has more than one diffuse path per voxel
     bool far;                   // a map of the frame is far: the kernels' FAR forms, ray streams for lighting
 };
 
 // packets: the segments of the build of dn_light_packet.cuh to run (every map's specBounceLimit within its limit), 0
 // for the ray streams
-static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, uint32_t packets, bool far)
+static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, uint32_t packets, bool far, bool side)
 {
     COUNT_LAUNCH();
     k_mark_opaque_batch<<<la.nmaps * MARK_BLOCKS, 256, 0, s>>>(la.maps, la.mixed);
@@ -382,7 +384,9 @@ static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, 
         BatchLightArgs ld = la;
         ld.batch = b->tuning.diffuseBatch;
         COUNT_LAUNCH();
-        k_light_diffuse_batch<<<(unsigned)(g_numSMs * b->maxBlocksDiffuse), 128, 0, s>>>(ld);
+        const unsigned blocks = (unsigned)(g_numSMs * b->maxBlocksDiffuse);
+        if (side) k_light_diffuse_batch<true><<<blocks, 128, 0, s>>>(ld);
+        else k_light_diffuse_batch<false><<<blocks, 128, 0, s>>>(ld);
         CK(cudaGetLastError());
     }
     return DN_CUDA_OK;
@@ -447,7 +451,7 @@ static int issue_frame(DNgpuBatch* b, const dn_batch_item* items, uint32_t n, co
         la.mixed = b->workCounter + 2;
         la.stats = b->bst->lstats;
         la.batch = b->tuning.streamBatch;
-        int rc = issue_light(b, la, s, f.packets, f.far);
+        int rc = issue_light(b, la, s, f.packets, f.far, f.side);
         if (rc) return rc;
         COUNT_LAUNCH();
         k_commit_batch<<<(unsigned)(g_numSMs * 4), 256, 0, s>>>(la.maps, la.reqStart, t.nl);
@@ -519,7 +523,10 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
     for (uint32_t i = 0; i < n; i++) f.far = f.far || map_far(items[i].map);
     f.packets = b->tuning.kernel == 2u && maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far ? packet_segments(maxSpec) : 0u;
     b->lastSegs = maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far ? packet_segments(maxSpec) : 0u;
+    f.side = false;
+    for (uint32_t i = 0; i < n; i++) f.side = f.side || ((items[i].phases & DN_BATCH_LIGHT) && items[i].light.numDiffuse > 1u);
     b->lastFar = f.far;
+    b->lastSide = f.side;
     if (f.t.size > b->tabCap) {
         // growing waits for the stream, frees pinned memory (which waits for the device) and renews the
         // graph, a stall of up to two frames: the first table is large enough for about 370 maps per frame
@@ -552,7 +559,7 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
     std::vector<uint64_t> key;
     key.reserve(4 + (size_t)n * 10);
     key.push_back(n); key.push_back(b->tabGen); key.push_back(b->tuning.streamBatch); key.push_back(b->tuning.blocksPerSM);
-    key.push_back(b->tuning.kernel); key.push_back(((uint64_t)f.packets << 1) | (f.far ? 1u : 0u));
+    key.push_back(b->tuning.kernel); key.push_back(((uint64_t)f.packets << 2) | (f.side ? 2u : 0u) | (f.far ? 1u : 0u));
     for (uint32_t i = 0; i < n; i++) {
         const dn_batch_item& it = items[i];
         DNgpuVolume* g = it.map;
@@ -782,7 +789,7 @@ extern "C" int dn_cuda_batch_autotune(DNgpuBatch* b, dn_batch_tuning* chosen)
             cudaError_t e = cudaMemsetAsync(b->workCounter, 0, 12, b->stream);
             if (e == cudaSuccess) e = cudaEventRecord(e0, b->stream);
             if (e != cudaSuccess) { rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "autotune: %s", cudaGetErrorString(e)); break; }
-            rc = issue_light(b, la, b->stream, t.kernel == 2u ? b->lastSegs : 0u, b->lastFar);
+            rc = issue_light(b, la, b->stream, t.kernel == 2u ? b->lastSegs : 0u, b->lastFar, b->lastSide);
             if (rc) break;
             e = cudaEventRecord(e1, b->stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);

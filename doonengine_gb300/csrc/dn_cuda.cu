@@ -697,13 +697,15 @@ __global__ void __launch_bounds__(128, packet_blocks(SEGS)) k_light_packet(const
 }
 
 // the diffuse paths of the voxels k_light_packet lit (dn_light_path.cuh)
+// SIDE: voxels have several paths
+template <bool SIDE>
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const __grid_constant__ StreamArgs a)
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
     __shared__ uint8_t order[128];
-    if (*a.mixed) path_loop<false, true>(&a, nullptr, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
-    else path_loop<false, false>(&a, nullptr, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
+    if (*a.mixed) path_loop<false, true, SIDE>(&a, nullptr, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
+    else path_loop<false, false, SIDE>(&a, nullptr, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
 }
 
 // launches the lighting kernel g_lightKernel selects (1 ray streams, 2 warp packets followed by the
@@ -732,7 +734,7 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materi
     g->lightTurn ^= 1u;
     if (g_lightKernel == 2 && a.p.specBounceLimit <= PK_MAX_SPEC_SEGMENTS && !map_far(g)) {
         static const int packets2 = resident(k_light_packet<PK_POOL_FAN, 2>), packets4 = resident(k_light_packet<64, 4>),
-                         packets8 = resident(k_light_packet<64, 8>), paths = resident(k_light_diffuse);
+                         packets8 = resident(k_light_packet<64, 8>), paths = resident(k_light_diffuse<false>), sidePaths = resident(k_light_diffuse<true>);
         a.batch = g_packetBatch;
         COUNT_LAUNCH();
         switch (packet_segments(a.p.specBounceLimit)) {
@@ -743,7 +745,8 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materi
         CK(cudaGetLastError());
         a.batch = g_pathBatch;
         COUNT_LAUNCH();
-        k_light_diffuse<<<g->numSMs * paths, 128, 0, g->stream>>>(a);
+        if (a.p.numDiffuse > 1u) k_light_diffuse<true><<<g->numSMs * sidePaths, 128, 0, g->stream>>>(a);
+        else k_light_diffuse<false><<<g->numSMs * paths, 128, 0, g->stream>>>(a);
     } else {
         static const int streams = resident(k_light_stream<false>), farStreams = resident(k_light_stream<true>);
         a.batch = g_streamBatch;

@@ -125,3 +125,49 @@ def test_batched_generators_match_plain(gpu_ready):
         batch.close()
         for x in images + plain + batched:
             x.close()
+
+
+@pytest.mark.parametrize("paths", [2, 3, 31, 32, 33])
+@pytest.mark.parametrize("bounces", [0, 4])
+def test_paths_side_by_side_match_oracle(gpu_ready, paths, bounces):
+    """small launches give each of a voxel's paths a lane (up to 32 paths, at least one bounce)"""
+    pair = Pair("tiny", K=3, map=(3, 2, 3), shapes=3)
+    try:
+        pair.vol.s.diffuseBounceLimit = bounces
+        for m in range(0, 14, 3):
+            pair.vol.set_material(m, opacity=0.5, refract=1.2)
+        mirrors(pair.vol)
+        for _ in range(3):
+            pair.draw()
+            pair.sync()
+            _, differ = pair.light(num_diffuse=paths)
+            assert differ == 0
+        check_counters(pair)
+    finally:
+        pair.close()
+
+
+def test_batched_path_counts_match_plain(gpu_ready):
+    """maps with different numbers of paths in one batch, and a repeated composition whose count changes"""
+    dn.init()
+    plain, batched = ([configs.build_volume("tiny", map=(2, 2, 1 + i), shapes=2, seed=80 + i)[0] for i in range(4)] for _ in range(2))
+    images = [dn.Image(64, 48) for _ in plain]
+    batch = dn.Batch(batched)
+    try:
+        for frame in range(6):
+            counts = (1, 1, 1, 1) if frame in (2, 5) else (1, 3, 40, 2)
+            for v, im, c in zip(plain, images, counts):
+                v.draw(im, *v.view_proj(0.75))
+                v.sync()
+                v.update_lighting(c, 1000, 1.0 + frame)
+            batch.run([dn.Batch.item(v, im, *v.view_proj(0.75), sync=(2, 1), light=(c, 1000, 1.0 + frame))
+                       for v, im, c in zip(batched, images, counts)])
+            assert batch.finish()
+            for a, b in zip(plain, batched):
+                assert a.finish()
+                for x, y in zip(a.export_lighting(), b.export_lighting()):
+                    assert np.array_equal(x, y)
+    finally:
+        batch.close()
+        for x in images + plain + batched:
+            x.close()

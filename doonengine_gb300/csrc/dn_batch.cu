@@ -58,10 +58,11 @@ struct DNgpuBatch {
     std::vector<uint64_t> lastKey;
     std::vector<uint64_t> graphKey;
     cudaGraphExec_t graph;
-    // the lighting launch of the last frame (autotuning re-runs it) and the generations of its maps
+    // the lighting launch of the last frame (autotuning re-runs it; valid while the table on the device is that
+    // frame's, so not after a frame without lighting) and the generations of its maps
     BatchLightArgs lastLight;
     bool lastLightValid;
-    uint32_t lastSegs;          // the packet build the last frame's maps can take (its segments; 0: ray streams only)
+    uint32_t lastSegs;          // the packet build that frame's maps can take (its segments; 0: ray streams only)
     bool lastFar, lastSide;
     std::vector<std::pair<DNgpuVolume*, uint64_t>> lastLightGens;
 };
@@ -358,7 +359,8 @@ struct FramePlan {
     TableLayout t;
     uint32_t drawBlocks, syncBlocks;
     bool hostImages;
-    uint32_t packets;           // lighting as warp packets (dn_light_packet.cuh): the build's segments, or 0
+    uint32_t segs;              // the packet build (dn_light_packet.cuh) the lit maps can take: its segments, or 0
+    uint32_t packets;           // the one lighting runs: segs, or 0 where the tuning asks for the ray streams
     bool side;                  // a lit map has more than one diffuse path per voxel
     bool far;                   // a map of the frame is far: the kernels' FAR forms, ray streams for lighting
 };
@@ -457,6 +459,7 @@ static int issue_frame(DNgpuBatch* b, const dn_batch_item* items, uint32_t n, co
         k_commit_batch<<<(unsigned)(g_numSMs * 4), 256, 0, s>>>(la.maps, la.reqStart, t.nl);
         CK(cudaGetLastError());
         b->lastLight = la;
+        b->lastSegs = f.segs; b->lastFar = f.far; b->lastSide = f.side;
         b->lastLightValid = true;
         b->lastLightGens.clear();
         for (uint32_t i = 0; i < n; i++)
@@ -521,12 +524,12 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
         if ((items[i].phases & DN_BATCH_LIGHT) && items[i].light.specBounceLimit > maxSpec) maxSpec = items[i].light.specBounceLimit;
     f.far = false;
     for (uint32_t i = 0; i < n; i++) f.far = f.far || map_far(items[i].map);
-    f.packets = b->tuning.kernel == 2u && maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far ? packet_segments(maxSpec) : 0u;
-    b->lastSegs = maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far ? packet_segments(maxSpec) : 0u;
+    f.segs = maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far ? packet_segments(maxSpec) : 0u;
+    f.packets = b->tuning.kernel == 2u ? f.segs : 0u;
     f.side = false;
     for (uint32_t i = 0; i < n; i++) f.side = f.side || ((items[i].phases & DN_BATCH_LIGHT) && items[i].light.numDiffuse > 1u);
-    b->lastFar = f.far;
-    b->lastSide = f.side;
+    // from here on the table may change
+    b->lastLightValid = false;
     if (f.t.size > b->tabCap) {
         // growing waits for the stream, frees pinned memory (which waits for the device) and renews the
         // graph, a stall of up to two frames: the first table is large enough for about 370 maps per frame
@@ -621,7 +624,11 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
 
     const bool repeat = b->tuning.useGraph && key == b->lastKey;
     b->lastKey = key;
-    if (!repeat) return issue_frame(b, items, n, f, false);
+    if (!repeat) {
+        const int rc = issue_frame(b, items, n, f, false);
+        if (rc) b->lastKey.clear();
+        return rc;
+    }
     if (!b->graph || b->graphKey != key) {
         if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
         b->graphKey.clear();
@@ -642,6 +649,7 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
     const unsigned long long k = (f.t.ns ? 2u : 0u) + (f.t.nd ? 1u : 0u) + ((f.t.nl || f.t.ns) ? 1u : 0u) + (f.t.nl ? 2u : 0u);
     __atomic_fetch_add(&g_launches, k, __ATOMIC_RELAXED);
     CK(cudaGraphLaunch(b->graph, b->stream));
+    b->lastLightValid = f.t.nl != 0u;   // lastLight is that of the frame before, which this one repeats
     return DN_CUDA_OK;
 }
 

@@ -1,0 +1,51 @@
+"""The tuning of a batch (dn_cuda_batch_set_tuning, dn_cuda_batch_autotune) across frames of different kinds."""
+import pytest
+
+import doonengine_gb300 as dn
+from doonengine_gb300 import configs
+
+pytestmark = pytest.mark.gpu
+
+
+class Maps:
+    """a batch of small maps, each with an image"""
+
+    def __init__(self, n=3, **settings):
+        dn.init()
+        self.vols = [configs.build_volume("tiny", map=(3 + i, 3, 4), shapes=3, seed=30 + i)[0] for i in range(n)]
+        for v in self.vols:
+            for k, x in settings.items():
+                setattr(v.s, k, x)
+        self.images = [dn.Image(64, 48) for _ in self.vols]
+        self.batch = dn.Batch(self.vols)
+        self.time = 0.5
+
+    def frame(self, light=True, paths=1):
+        self.time += 0.25
+        self.batch.run([dn.Batch.item(v, im, *v.view_proj(0.75), sync=(2, 1) if light else None,
+                                      light=(paths, 1000, self.time) if light else None)
+                        for v, im in zip(self.vols, self.images)])
+        assert self.batch.finish(), dn.load().dn_cuda_last_error().decode()
+
+    def close(self):
+        self.batch.close()
+        for x in self.images + self.vols:
+            x.close()
+
+
+def test_autotune_needs_a_lit_last_frame(gpu_ready):
+    """the launch that autotuning runs again reads the frame's table, which a frame without lighting has replaced"""
+    maps = Maps()
+    try:
+        for k in range(3):          # the first two frames are issued, the third is a replayed graph
+            for _ in range(k + 1):
+                maps.frame()
+            maps.batch.autotune()
+            for _ in range(k + 1):
+                maps.frame(light=False)
+            with pytest.raises(RuntimeError):
+                maps.batch.autotune()
+        maps.frame()
+        maps.batch.autotune()
+    finally:
+        maps.close()

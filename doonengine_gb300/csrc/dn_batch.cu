@@ -697,6 +697,7 @@ extern "C" int dn_cuda_batch_finish(DNgpuBatch* b)
     for (uint32_t i = 0; i < n; i++) {
         DNgpuVolume* g = res[i];
         memcpy(g->hst->w, &b->hgather[4 * i], sizeof(g->hst->w));
+        if (g->hst->w[ST_REQ] > g->reqCap) g->hst->w[ST_REQ] = (uint32_t)g->reqCap;   // an overflowed list holds no more
         if (g->hst->w[ST_ERR]) { if (!bad) { first = i; flags = g->hst->w[ST_ERR]; } bad++; }
     }
     if (bad) return dn_set_err(DN_CUDA_ERR_KERNEL, "kernel error flags 0x%x on resident member %u (%u members flagged)", flags, first, bad);

@@ -49,3 +49,27 @@ def test_autotune_needs_a_lit_last_frame(gpu_ready):
         maps.batch.autotune()
     finally:
         maps.close()
+
+
+def test_overflowed_list_counts_alike(gpu_ready):
+    """more requests than a member's list holds: the batch and the map alone report what the list holds"""
+    dn.init()
+    vol, _ = configs.build_volume("small", map=(16, 12, 16), seed=11, mean=0.26, amp=0.14, shapes=40, shape_max=18, K=1)
+    vol.s.lightingRequestCap = 1 << 30      # the host takes the device's list for long enough and never grows it
+    img = dn.Image(320, 180)
+    batch = dn.Batch([vol])
+    try:
+        for i in range(10):
+            vol.draw(img, *vol.view_proj(180 / 320))
+            vol.sync()
+            vol.update_lighting(1, 1000, 1.0 + i)
+        vol.draw(img, *vol.view_proj(180 / 320))
+        vol.sync()
+        assert not batch.finish()           # the overflow is reported
+        assert vol.s.numLightingRequests == 1024
+        vol.finish()                        # (an error is reported once)
+        assert vol.s.numLightingRequests == 1024
+    finally:
+        batch.close()
+        img.close()
+        vol.close()

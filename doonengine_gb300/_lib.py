@@ -324,6 +324,7 @@ _SIGS = [
     ("dn_cuda_batch_stats", c_int, [c_void_p, c_int, c_void_p]),
     ("dn_cuda_batch_reset_stats", c_int, [c_void_p]),
     ("dn_cuda_batch_stream", c_void_p, [c_void_p]),
+    ("dn_cuda_batch_captures", c_uint64, [c_void_p]),
     ("dn_cuda_batch_get_tuning", c_int, [c_void_p, POINTER(DnBatchTuning)]),
     ("dn_cuda_batch_set_tuning", c_int, [c_void_p, POINTER(DnBatchTuning)]),
     ("dn_cuda_batch_autotune", c_int, [c_void_p, POINTER(DnBatchTuning)]),

@@ -58,6 +58,7 @@ struct DNgpuBatch {
     std::vector<uint64_t> lastKey;
     std::vector<uint64_t> graphKey;
     cudaGraphExec_t graph;
+    uint64_t captures;          // graphs made so far
     // the lighting launch of the last frame (autotuning re-runs it; valid while the table on the device is that
     // frame's, so not after a frame without lighting) and the generations of its maps
     BatchLightArgs lastLight;
@@ -235,7 +236,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     b->tuning.blocksPerSM = DN_STREAM_MIN_BLOCKS; b->tuning.useGraph = 1;
     b->tuning.poolRays = PK_POOL_FAN; b->tuning.diffuseBatch = g_pathBatch;
     b->lastSegs = 0; b->lastFar = b->lastSide = false;
-    b->graph = nullptr;
+    b->graph = nullptr; b->captures = 0;
     b->lastLightValid = false;
     int rc = DN_CUDA_OK;
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
@@ -562,7 +563,8 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
     std::vector<uint64_t> key;
     key.reserve(4 + (size_t)n * 10);
     key.push_back(n); key.push_back(b->tabGen); key.push_back(b->tuning.streamBatch); key.push_back(b->tuning.blocksPerSM);
-    key.push_back(b->tuning.kernel); key.push_back(((uint64_t)f.packets << 2) | (f.side ? 2u : 0u) | (f.far ? 1u : 0u));
+    key.push_back(b->tuning.kernel); key.push_back(((uint64_t)b->tuning.poolRays << 32) | b->tuning.diffuseBatch);
+    key.push_back(((uint64_t)f.packets << 2) | (f.side ? 2u : 0u) | (f.far ? 1u : 0u));
     for (uint32_t i = 0; i < n; i++) {
         const dn_batch_item& it = items[i];
         DNgpuVolume* g = it.map;
@@ -644,6 +646,7 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) { b->graph = nullptr; return dn_set_err(DN_CUDA_ERR_LAUNCH, "graph instantiate: %s", cudaGetErrorString(e)); }
         b->graphKey = key;
+        b->captures++;
     }
     // the graph's kernels: reset and compact (sync), draw, prep, light and commit
     const unsigned long long k = (f.t.ns ? 2u : 0u) + (f.t.nd ? 1u : 0u) + ((f.t.nl || f.t.ns) ? 1u : 0u) + (f.t.nl ? 2u : 0u);
@@ -724,6 +727,8 @@ extern "C" int dn_cuda_batch_reset_stats(DNgpuBatch* b)
     CK(cudaMemsetAsync(b->bst->stats, 0, sizeof(b->bst->stats) + sizeof(b->bst->lstats), b->stream));
     return DN_CUDA_OK;
 }
+
+extern "C" uint64_t dn_cuda_batch_captures(DNgpuBatch* b) { return b ? b->captures : 0u; }
 
 extern "C" void* dn_cuda_batch_stream(DNgpuBatch* b) { return b ? (void*)b->stream : nullptr; }
 

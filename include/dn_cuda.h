@@ -248,6 +248,8 @@ int dn_cuda_batch_finish(struct DNgpuBatch* b);
 int dn_cuda_batch_stats(struct DNgpuBatch* b, int kind, dn_stats* out);
 int dn_cuda_batch_reset_stats(struct DNgpuBatch* b);
 void* dn_cuda_batch_stream(struct DNgpuBatch* b);
+/* graphs the batch has captured so far: one for each run of frames that repeat under one tuning */
+uint64_t dn_cuda_batch_captures(struct DNgpuBatch* b);
 int dn_cuda_batch_get_tuning(struct DNgpuBatch* b, dn_batch_tuning* out);
 int dn_cuda_batch_set_tuning(struct DNgpuBatch* b, const dn_batch_tuning* t);
 /* Times the lighting launch of the last batched frame under each candidate tuning, keeps the fastest and

@@ -73,3 +73,21 @@ def test_overflowed_list_counts_alike(gpu_ready):
         batch.close()
         img.close()
         vol.close()
+
+
+@pytest.mark.parametrize("change", [dict(poolRays=64), dict(diffuseBatch=7), dict(streamBatch=9), dict(blocksPerSM=1)])
+def test_tuning_change_renews_the_graph(gpu_ready, change):
+    """a repeated frame is replayed as a graph; a setting that the launches in it hold needs another"""
+    maps = Maps()
+    captures = lambda: maps.batch.lib.dn_cuda_batch_captures(maps.batch._gpu())
+    try:
+        maps.batch.set_tuning(poolRays=128, diffuseBatch=20, streamBatch=16, blocksPerSM=2, useGraph=1)
+        for _ in range(4):
+            maps.frame()
+        assert captures() == 1
+        maps.batch.set_tuning(**change)
+        for _ in range(4):
+            maps.frame()
+        assert captures() == 2
+    finally:
+        maps.close()

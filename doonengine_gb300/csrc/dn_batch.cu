@@ -59,6 +59,7 @@ struct DNgpuBatch {
     std::vector<uint64_t> graphKey;
     cudaGraphExec_t graph;
     uint64_t captures;          // graphs made so far
+    unsigned long long graphLaunches;   // kernels in the graph
     // the lighting launch of the last frame (autotuning re-runs it; valid while the table on the device is that
     // frame's, so not after a frame without lighting) and the generations of its maps
     BatchLightArgs lastLight;
@@ -236,7 +237,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     b->tuning.blocksPerSM = DN_STREAM_MIN_BLOCKS; b->tuning.useGraph = 1;
     b->tuning.poolRays = PK_POOL_FAN; b->tuning.diffuseBatch = g_pathBatch;
     b->lastSegs = 0; b->lastFar = b->lastSide = false;
-    b->graph = nullptr; b->captures = 0;
+    b->graph = nullptr; b->captures = 0; b->graphLaunches = 0;
     b->lastLightValid = false;
     int rc = DN_CUDA_OK;
     cudaError_t e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
@@ -635,11 +636,13 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
         if (b->graph) { cudaGraphExecDestroy(b->graph); b->graph = nullptr; }
         b->graphKey.clear();
         CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        const unsigned long long before = g_launches;
+        const unsigned long long before = t_launches;
         int rc = issue_frame(b, items, n, f, true);
         cudaGraph_t graph = nullptr;
         cudaError_t e = cudaStreamEndCapture(b->stream, &graph);
-        __atomic_store_n(&g_launches, before, __ATOMIC_RELAXED);   // captured launches run when the graph does
+        // captured launches run when the graph does
+        b->graphLaunches = t_launches - before;
+        __atomic_fetch_sub(&g_launches, b->graphLaunches, __ATOMIC_RELAXED);
         if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
         if (e != cudaSuccess) return dn_set_err(DN_CUDA_ERR_LAUNCH, "stream capture: %s", cudaGetErrorString(e));
         e = cudaGraphInstantiate(&b->graph, graph, 0);
@@ -648,9 +651,7 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
         b->graphKey = key;
         b->captures++;
     }
-    // the graph's kernels: reset and compact (sync), draw, prep, light and commit
-    const unsigned long long k = (f.t.ns ? 2u : 0u) + (f.t.nd ? 1u : 0u) + ((f.t.nl || f.t.ns) ? 1u : 0u) + (f.t.nl ? 2u : 0u);
-    __atomic_fetch_add(&g_launches, k, __ATOMIC_RELAXED);
+    __atomic_fetch_add(&g_launches, b->graphLaunches, __ATOMIC_RELAXED);
     CK(cudaGraphLaunch(b->graph, b->stream));
     b->lastLightValid = f.t.nl != 0u;   // lastLight is that of the frame before, which this one repeats
     return DN_CUDA_OK;

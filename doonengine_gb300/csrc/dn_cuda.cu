@@ -82,6 +82,7 @@ static cudaStream_t g_copyStream = nullptr;      // evictions
 static cudaStream_t g_restoreStream = nullptr;   // restores
 static int g_copyStreamDevice = -1;
 unsigned long long g_launches = 0;
+thread_local unsigned long long t_launches = 0;
 unsigned long long g_allocs = 0;
 static unsigned long long g_generation = 0;
 

@@ -100,11 +100,12 @@ struct DNgpuVolume {
 extern int g_device;
 extern int g_numSMs;
 extern unsigned long long g_launches;   // kernels launched by this library (all threads)
+extern thread_local unsigned long long t_launches;   // those the calling thread launched or captured
 extern int g_lightKernel;               // 1 per-lane ray streams, 2 warp packets (default)
 extern uint32_t g_pathBatch;            // the same for diffuse paths
 extern uint32_t g_streamBatch;          // lanes that wait before per-segment work runs (1..32), ray streams
 extern uint32_t g_packetBatch;          // the same threshold for the packet kernel's ray pools
-#define COUNT_LAUNCH() __atomic_fetch_add(&g_launches, 1ull, __ATOMIC_RELAXED)
+#define COUNT_LAUNCH() (t_launches++, __atomic_fetch_add(&g_launches, 1ull, __ATOMIC_RELAXED))
 extern unsigned long long g_allocs;     // device and pinned allocations made by this library (all threads)
 #define COUNT_ALLOC() __atomic_fetch_add(&g_allocs, 1ull, __ATOMIC_RELAXED)
 

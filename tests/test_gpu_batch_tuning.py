@@ -91,3 +91,23 @@ def test_tuning_change_renews_the_graph(gpu_ready, change):
         assert captures() == 2
     finally:
         maps.close()
+
+
+@pytest.mark.parametrize("settings", [{}, {"specBounceLimit": 9}])     # packets and diffuse paths, ray streams
+@pytest.mark.parametrize("light", [True, False])
+def test_replayed_frame_counts_its_launches(gpu_ready, light, settings):
+    """a frame counts the same kernels whether it is issued or replayed as a graph"""
+    maps = Maps(**settings)
+    count = maps.batch.lib.dn_cuda_launch_count
+    try:
+        for _ in range(6):      # the maps load
+            maps.frame(light)
+        counts = []
+        for graph in (1, 0):
+            maps.batch.set_tuning(useGraph=graph)
+            before = count()
+            maps.frame(light)
+            counts.append(count() - before)
+        assert counts[0] == counts[1] > 0, counts
+    finally:
+        maps.close()

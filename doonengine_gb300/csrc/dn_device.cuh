@@ -58,8 +58,14 @@ __device__ __forceinline__ f3 refract(f3 I, f3 N, float eta)
     float s = eta * d + sqrtf(k);
     return sub(muls(I, eta), muls(N, s));
 }
-// float -> int32 towards zero with saturation, NaN -> 0: what PTX's cvt.rzi.s32.f32 does
-__device__ __forceinline__ int32_t f2i(float x) { return __float2int_rz(x); }
+// float -> int32 towards zero with saturation, NaN -> 0: PTX defines cvt.rzi.s32.f32 so for every float (C's cast and
+// __float2int_rz are undefined outside the range, which det_sin of a large argument and positions far off reach)
+__device__ __forceinline__ int32_t f2i(float x)
+{
+    int32_t i;
+    asm("cvt.rzi.s32.f32 %0, %1;" : "=r"(i) : "f"(x));
+    return i;
+}
 
 // ---------------------------------------------------------------- RNG (D5)
 

@@ -123,7 +123,7 @@ constexpr uint32_t CODE_BITS = 0x4B400000u;   // CODE_BASE's bits
 template <bool FAR>
 __device__ __forceinline__ f3 cell_code(f3 fl)
 {
-    if constexpr (FAR) return mk(__int_as_float((int32_t)fl.x), __int_as_float((int32_t)fl.y), __int_as_float((int32_t)fl.z));
+    if constexpr (FAR) return mk(__int_as_float(f2i(fl.x)), __int_as_float(f2i(fl.y)), __int_as_float(f2i(fl.z)));
     return mk(__fmaf_rn(2.0f, fl.x, CODE_BASE), CODE_BASE + fl.y, CODE_BASE + fl.z);
 }
 // the coordinates of a coded cell

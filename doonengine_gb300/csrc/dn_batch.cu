@@ -161,12 +161,12 @@ __global__ void __launch_bounds__(128, DN_STREAM_MIN_BLOCKS) k_light_stream_batc
 
 // POOL: rays per fan kind per pool (the rays a warp pulls from a request group at a time); the autotuner
 // picks PK_POOL_FAN or PK_POOL_ALT (dn_batch_tuning.poolRays)
-template <uint32_t POOL, uint32_t SEGS>
+template <uint32_t POOL, uint32_t SEGS, bool FAR>
 __global__ void __launch_bounds__(128, packet_blocks(SEGS)) k_light_packet_batch(const __grid_constant__ BatchLightArgs a)
 {
     __shared__ PacketWarpT<POOL, SEGS> warps[4];
-    if (*a.mixed) packet_loop<true, POOL, SEGS, true>(nullptr, &a, warps[threadIdx.x >> 5]);
-    else packet_loop<true, POOL, SEGS, false>(nullptr, &a, warps[threadIdx.x >> 5]);
+    if (FAR || *a.mixed) packet_loop<true, POOL, SEGS, true, FAR>(nullptr, &a, warps[threadIdx.x >> 5]);
+    else if constexpr (!FAR) packet_loop<true, POOL, SEGS, false, false>(nullptr, &a, warps[threadIdx.x >> 5]);
 }
 
 // the opaque-chunk marks (mark_opaque_cells) of every map of a lighting launch: MARK_BLOCKS blocks per map
@@ -181,14 +181,15 @@ __global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* 
 }
 
 // the diffuse paths of the voxels k_light_packet_batch lit, as per-lane path streams over every map's queue
-template <bool SIDE>
+template <bool SIDE, bool FAR>
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse_batch(const __grid_constant__ BatchLightArgs a)
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
     __shared__ uint8_t order[128];
-    if (*a.mixed) path_loop<true, true, SIDE>(nullptr, &a, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
-    else path_loop<true, false, SIDE>(nullptr, &a, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
+    uint8_t* const mine = order + (threadIdx.x & ~31u);
+    if (FAR || *a.mixed) path_loop<true, true, SIDE, FAR>(nullptr, &a, jobs[threadIdx.x], tint, mine);
+    else if constexpr (!FAR) path_loop<true, false, SIDE, false>(nullptr, &a, jobs[threadIdx.x], tint, mine);
 }
 
 __global__ void k_commit_batch(const BatchLightMap* l, const uint32_t* reqStart, uint32_t nl)
@@ -262,10 +263,10 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
         int perSM = 0, perSM2 = 0, perSM3 = 0;
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k_light_stream_batch<false>, 128, 0);
         int perSMAlt = 0;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM2, k_light_packet_batch<PK_POOL_FAN, 2>, 128, 0);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMAlt, k_light_packet_batch<PK_POOL_ALT, 2>, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM2, k_light_packet_batch<PK_POOL_FAN, 2, false>, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMAlt, k_light_packet_batch<PK_POOL_ALT, 2, false>, 128, 0);
         b->maxBlocksPacketAlt = perSMAlt < 1 ? 1 : perSMAlt;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM3, k_light_diffuse_batch<true>, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM3, k_light_diffuse_batch<true, false>, 128, 0);
         if (e != cudaSuccess) rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "occupancy: %s", cudaGetErrorString(e));
         b->maxBlocksPerSM = perSM < 1 ? 1 : perSM;
         b->maxBlocksPacket = perSM2 < 1 ? 1 : perSM2;
@@ -364,7 +365,7 @@ struct FramePlan {
     uint32_t segs;              // the packet build (dn_light_packet.cuh) the lit maps can take: its segments, or 0
     uint32_t packets;           // the one lighting runs: segs, or 0 where the tuning asks for the ray streams
     bool side;                  // a lit map has more than one diffuse path per voxel
-    bool far;                   // a map of the frame is far: the kernels' FAR forms, ray streams for lighting
+    bool far;                   // a map of the frame is far: the kernels' FAR forms for all
 };
 
 // packets: the segments of the build of dn_light_packet.cuh to run (every map's specBounceLimit within its limit), 0
@@ -376,10 +377,11 @@ static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, 
     CK(cudaGetLastError());
     COUNT_LAUNCH();
     const unsigned grid = (unsigned)(g_numSMs * (int)b->tuning.blocksPerSM);
-    if (packets == 4u) k_light_packet_batch<64, 4><<<grid, 128, 0, s>>>(la);
-    else if (packets == 8u) k_light_packet_batch<64, 8><<<grid, 128, 0, s>>>(la);
-    else if (packets && b->tuning.poolRays == PK_POOL_ALT) k_light_packet_batch<PK_POOL_ALT, 2><<<grid, 128, 0, s>>>(la);
-    else if (packets) k_light_packet_batch<PK_POOL_FAN, 2><<<grid, 128, 0, s>>>(la);
+    if (packets && far) k_light_packet_batch<PK_POOL_FAN, 2, true><<<grid, 128, 0, s>>>(la);
+    else if (packets == 4u) k_light_packet_batch<64, 4, false><<<grid, 128, 0, s>>>(la);
+    else if (packets == 8u) k_light_packet_batch<64, 8, false><<<grid, 128, 0, s>>>(la);
+    else if (packets && b->tuning.poolRays == PK_POOL_ALT) k_light_packet_batch<PK_POOL_ALT, 2, false><<<grid, 128, 0, s>>>(la);
+    else if (packets) k_light_packet_batch<PK_POOL_FAN, 2, false><<<grid, 128, 0, s>>>(la);
     else if (far) k_light_stream_batch<true><<<grid, 128, 0, s>>>(la);
     else k_light_stream_batch<false><<<grid, 128, 0, s>>>(la);
     CK(cudaGetLastError());
@@ -389,8 +391,9 @@ static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, 
         ld.batch = b->tuning.diffuseBatch;
         COUNT_LAUNCH();
         const unsigned blocks = (unsigned)(g_numSMs * b->maxBlocksDiffuse);
-        if (side) k_light_diffuse_batch<true><<<blocks, 128, 0, s>>>(ld);
-        else k_light_diffuse_batch<false><<<blocks, 128, 0, s>>>(ld);
+        if (far) k_light_diffuse_batch<false, true><<<blocks, 128, 0, s>>>(ld);
+        else if (side) k_light_diffuse_batch<true, false><<<blocks, 128, 0, s>>>(ld);
+        else k_light_diffuse_batch<false, false><<<blocks, 128, 0, s>>>(ld);
         CK(cudaGetLastError());
     }
     return DN_CUDA_OK;
@@ -526,7 +529,7 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
         if ((items[i].phases & DN_BATCH_LIGHT) && items[i].light.specBounceLimit > maxSpec) maxSpec = items[i].light.specBounceLimit;
     f.far = false;
     for (uint32_t i = 0; i < n; i++) f.far = f.far || map_far(items[i].map);
-    f.segs = maxSpec <= PK_MAX_SPEC_SEGMENTS && !f.far ? packet_segments(maxSpec) : 0u;
+    f.segs = packet_build(maxSpec, f.far);
     f.packets = b->tuning.kernel == 2u ? f.segs : 0u;
     f.side = false;
     for (uint32_t i = 0; i < n; i++) f.side = f.side || ((items[i].phases & DN_BATCH_LIGHT) && items[i].light.numDiffuse > 1u);
@@ -790,7 +793,7 @@ extern "C" int dn_cuda_batch_autotune(DNgpuBatch* b, dn_batch_tuning* chosen)
     }
     const dn_batch_tuning keep = b->tuning;
     dn_batch_tuning best = keep;
-    // packets are possible when every lit map's specBounceLimit allows them and no map is far
+    // packets are possible when there is a build for the frame (packet_build)
     const bool packetsOk = b->lastSegs != 0u;
     float bestMs = 3.4e38f;
     int rc = DN_CUDA_OK;

@@ -687,31 +687,32 @@ __global__ void __launch_bounds__(256) k_light_prep(const __grid_constant__ DevM
 }
 
 // The lighting launch with specular and shadow fans traced as warp packets (dn_light_packet.cuh).
-template <uint32_t POOL, uint32_t SEGS>
+// FAR: see dn_walk.cuh; its builds always run the loops with see-through voxels, which are right for opaque maps too
+template <uint32_t POOL, uint32_t SEGS, bool FAR>
 __global__ void __launch_bounds__(128, packet_blocks(SEGS)) k_light_packet(const __grid_constant__ StreamArgs a)
 {
     // shared memory holds only the four warps' pools (25 KB per block with 128-ray pools): 7 blocks take 175 KB, the
     // rest of the SM's 256 KB is L1 for the map's masks and voxels; the tables are read from a.gtab
     __shared__ PacketWarpT<POOL, SEGS> warps[4];
-    if (*a.mixed) packet_loop<false, POOL, SEGS, true>(&a, nullptr, warps[threadIdx.x >> 5]);
-    else packet_loop<false, POOL, SEGS, false>(&a, nullptr, warps[threadIdx.x >> 5]);
+    if (FAR || *a.mixed) packet_loop<false, POOL, SEGS, true, FAR>(&a, nullptr, warps[threadIdx.x >> 5]);
+    else if constexpr (!FAR) packet_loop<false, POOL, SEGS, false, false>(&a, nullptr, warps[threadIdx.x >> 5]);
 }
 
 // the diffuse paths of the voxels k_light_packet lit (dn_light_path.cuh)
 // SIDE: voxels have several paths
-template <bool SIDE>
+template <bool SIDE, bool FAR>
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const __grid_constant__ StreamArgs a)
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
     __shared__ uint8_t order[128];
-    if (*a.mixed) path_loop<false, true, SIDE>(&a, nullptr, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
-    else path_loop<false, false, SIDE>(&a, nullptr, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
+    uint8_t* const mine = order + (threadIdx.x & ~31u);
+    if (FAR || *a.mixed) path_loop<false, true, SIDE, FAR>(&a, nullptr, jobs[threadIdx.x], tint, mine);
+    else if constexpr (!FAR) path_loop<false, false, SIDE, false>(&a, nullptr, jobs[threadIdx.x], tint, mine);
 }
 
 // launches the lighting kernel g_lightKernel selects (1 ray streams, 2 warp packets followed by the
-// diffuse-path kernel; packets need specBounceLimit <= PK_MAX_SPEC_SEGMENTS and a map that is not
-// far, and fall back to streams otherwise) with its batch threshold
+// diffuse-path kernel where packet_build has one, streams otherwise) with its batch threshold
 static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materials)
 {
     // resident blocks per SM, the same on every device this library is built for
@@ -733,27 +734,38 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materi
     a.gtab = g->dtab;
     a.mixed = &g->st->mixed[g->lightTurn];
     g->lightTurn ^= 1u;
-    if (g_lightKernel == 2 && a.p.specBounceLimit <= PK_MAX_SPEC_SEGMENTS && !map_far(g)) {
-        static const int packets2 = resident(k_light_packet<PK_POOL_FAN, 2>), packets4 = resident(k_light_packet<64, 4>),
-                         packets8 = resident(k_light_packet<64, 8>), paths = resident(k_light_diffuse<false>), sidePaths = resident(k_light_diffuse<true>);
-        a.batch = g_packetBatch;
+    const bool far = map_far(g);
+    const uint32_t segs = g_lightKernel == 2 ? packet_build(a.p.specBounceLimit, far) : 0u;
+    auto launch = [&](auto* k, int blocks) {
         COUNT_LAUNCH();
-        switch (packet_segments(a.p.specBounceLimit)) {
-        case 2: k_light_packet<PK_POOL_FAN, 2><<<g->numSMs * packets2, 128, 0, g->stream>>>(a); break;
-        case 4: k_light_packet<64, 4><<<g->numSMs * packets4, 128, 0, g->stream>>>(a); break;
-        default: k_light_packet<64, 8><<<g->numSMs * packets8, 128, 0, g->stream>>>(a); break;
+        k<<<g->numSMs * blocks, 128, 0, g->stream>>>(a);
+    };
+    if (segs && far) {
+        static const int packets = resident(k_light_packet<PK_POOL_FAN, 2, true>), paths = resident(k_light_diffuse<false, true>);
+        a.batch = g_packetBatch;
+        launch(k_light_packet<PK_POOL_FAN, 2, true>, packets);
+        CK(cudaGetLastError());
+        a.batch = g_pathBatch;
+        launch(k_light_diffuse<false, true>, paths);
+    } else if (segs) {
+        static const int packets2 = resident(k_light_packet<PK_POOL_FAN, 2, false>), packets4 = resident(k_light_packet<64, 4, false>),
+                         packets8 = resident(k_light_packet<64, 8, false>), paths = resident(k_light_diffuse<false, false>),
+                         sidePaths = resident(k_light_diffuse<true, false>);
+        a.batch = g_packetBatch;
+        switch (segs) {
+        case 2: launch(k_light_packet<PK_POOL_FAN, 2, false>, packets2); break;
+        case 4: launch(k_light_packet<64, 4, false>, packets4); break;
+        default: launch(k_light_packet<64, 8, false>, packets8); break;
         }
         CK(cudaGetLastError());
         a.batch = g_pathBatch;
-        COUNT_LAUNCH();
-        if (a.p.numDiffuse > 1u) k_light_diffuse<true><<<g->numSMs * sidePaths, 128, 0, g->stream>>>(a);
-        else k_light_diffuse<false><<<g->numSMs * paths, 128, 0, g->stream>>>(a);
+        if (a.p.numDiffuse > 1u) launch(k_light_diffuse<true, false>, sidePaths);
+        else launch(k_light_diffuse<false, false>, paths);
     } else {
         static const int streams = resident(k_light_stream<false>), farStreams = resident(k_light_stream<true>);
         a.batch = g_streamBatch;
-        COUNT_LAUNCH();
-        if (map_far(g)) k_light_stream<true><<<g->numSMs * farStreams, 128, 0, g->stream>>>(a);
-        else k_light_stream<false><<<g->numSMs * streams, 128, 0, g->stream>>>(a);
+        if (far) launch(k_light_stream<true>, farStreams);
+        else launch(k_light_stream<false>, streams);
     }
     CK(cudaGetLastError());
     return DN_CUDA_OK;

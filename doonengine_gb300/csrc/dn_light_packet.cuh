@@ -50,6 +50,14 @@ __host__ __device__ constexpr uint32_t packet_segments(uint32_t specBounceLimit)
     return specBounceLimit <= 2u ? 2u : specBounceLimit <= 4u ? 4u : 8u;
 }
 
+// the build a launch takes: its segments, or 0 for the ray streams.  far: a map of it is far (dn_walk.cuh); there is one
+// far build, for the reference's limit and below (a lighting update of a 1x2x262200 map, us: K = 16 89, ray streams 189;
+// K = 64 119, 630; batched with four 16x12x16 maps, which the far build then lights too, 1352 a frame, 7300)
+__host__ __device__ constexpr uint32_t packet_build(uint32_t specBounceLimit, bool far)
+{
+    return specBounceLimit <= (far ? 2u : PK_MAX_SPEC_SEGMENTS) ? packet_segments(specBounceLimit) : 0u;
+}
+
 // resident blocks the register allocation of a build must allow (8-segment pools take 34 KB per block)
 constexpr int packet_blocks(uint32_t segs) { return segs <= 4u ? DN_PACKET_MIN_BLOCKS : 6; }
 
@@ -179,7 +187,7 @@ __device__ __forceinline__ bool packet_unit(uint32_t u, uint32_t nreq, uint32_t&
 // have one, so no lane waits for the slowest ray of a fan; each ray's contributions go to shared memory, and when
 // the pool is empty every voxel's sums are formed in the reference's order and written (its diffuse paths run in
 // k_light_diffuse, which reads the direct light left in the voxel's diffuse slot).
-template <bool MANY, uint32_t POOL, uint32_t SEGS, bool TINTED>
+template <bool MANY, uint32_t POOL, uint32_t SEGS, bool TINTED, bool FAR>
 __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLightArgs* many, PacketWarpT<POOL, SEGS>& W)
 {
     static_assert(SEGS >= 2u && POOL >= 64u, "a slot holds a direction and its reciprocal, a pool one voxel's rays");
@@ -291,7 +299,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                             inv = mk(sinv[k][0], sinv[k][1], sinv[k][2]);
                         }
                         c.rays++;
-                        ray_begin<false, TINTED>(s, m, W.v[vi].pos0, d, inv, false, c, W.tint, lane);
+                        ray_begin<FAR, TINTED>(s, m, W.v[vi].pos0, d, inv, false, c, W.tint, lane);
                     }
                     next = min(next + (uint32_t)__popc(need), total);
                 }
@@ -302,7 +310,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                 for (;;) {
                     const unsigned st = __ballot_sync(0xFFFFFFFFu, ray_stepping(s));
                     if (!st || (uint32_t)__popc(live & ~st) >= batch) break;
-                    if (ray_stepping(s)) walk_round<false, TINTED>(s, m, mats, p.sunStrength, c, W.tint, lane);
+                    if (ray_stepping(s)) walk_round<FAR, TINTED>(s, m, mats, p.sunStrength, c, W.tint, lane);
                 }
                 // shade the ended segments
                 if (s.mode == RM_IDLE || ray_stepping(s)) continue;
@@ -330,7 +338,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                 bool more = false, add_ = true;
                 f3 sc;
                 if (hit) {
-                    const f3 hpos = ray_hit_position<false>(s);
+                    const f3 hpos = ray_hit_position<FAR>(s);
                     Voxel hv;
                     decompress(m, ray_hit_index(s, m), hv);
                     const i3 hp{f2i(hpos.x), f2i(hpos.y), f2i(hpos.z)};
@@ -359,7 +367,7 @@ __device__ __forceinline__ void packet_loop(const StreamArgs* one, const BatchLi
                                 W.con[up + 1u][q] = mult.y * (hv.albedo.y * cmul * hm.specular);
                                 W.con[up + 2u][q] = mult.z * (hv.albedo.z * cmul * hm.specular);
                                 const f3 nd = reflect(s.dir, hv.normal);
-                                ray_begin<false, TINTED>(s, m, hpos, nd, rcp3(nd), true, c, W.tint, lane);
+                                ray_begin<FAR, TINTED>(s, m, hpos, nd, rcp3(nd), true, c, W.tint, lane);
                                 s.flags |= ((SEGS == 2u ? 1u : b + 1u) << RF_BOUNCES) | (hm.reflectType == 1u ? RF_SKY : 0u);
                                 c.rays++;
                             }

@@ -163,7 +163,7 @@ __device__ __forceinline__ f3 warp_sphere_points(bool need, bool sine, const Pat
 // voxel forms its sum.  us per pass, before -> after: four updates of a 16x12x16 map with 4 paths per voxel 4840 -> 4395,
 // 23x11x37 map with 2 paths 418 -> 402, six maps of 9x12x7 with 3 paths batched 372 -> 280; a limit of one voxel per lane
 // 4874, 421, 280.  Launches whose voxels have one path take the build without it (glass map 2 % faster than with).
-template <bool MANY, bool TINTED, bool SIDE>
+template <bool MANY, bool TINTED, bool SIDE, bool FAR>
 __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLightArgs* many, PathJob& j, TintT<128>& tint,
                                           uint8_t* order)
 {
@@ -214,7 +214,7 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
                 float cmul;
                 ray_tint<TINTED>(s, tint, col, cadd, cmul);
                 if (s.mode == RM_HIT) {
-                    org = ray_hit_position<false>(s);
+                    org = ray_hit_position<FAR>(s);
                     const uint2 w = __ldg(&M().vox[ray_hit_index(s, M())]);
                     const f3 albedo = mk((float)((w.y >> 24) & 0xFF) * INV255, (float)((w.y >> 16) & 0xFF) * INV255,
                                          (float)((w.y >> 8) & 0xFF) * INV255);
@@ -348,11 +348,11 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
             if (begin) {
                 f3 d = normalize(point ? add(base, rs) : base);
                 if (!lobe) d = adds(d, EPS);
-                ray_begin<false, TINTED>(s, M(), org, d, rcp3(d), start, c, tint, col);
+                ray_begin<FAR, TINTED>(s, M(), org, d, rcp3(d), start, c, tint, col);
                 c.rays++;
             }
         }
-        if (ray_stepping(s)) walk_round<false, TINTED>(s, M(), MATS(), P().sunStrength, c, tint, col);
+        if (ray_stepping(s)) walk_round<FAR, TINTED>(s, M(), MATS(), P().sunStrength, c, tint, col);
     }
     flush_counters(MANY ? many->stats : one->stats, c, 0, 0);
 }

@@ -54,6 +54,7 @@ struct DNgpuBatch {
     int maxBlocksPerSM;         // of the ray-stream kernel
     int maxBlocksPacket;        // of the packet kernel with PK_POOL_FAN-ray pools
     int maxBlocksPacketAlt;     // of the packet kernel with the other pool size (PK_POOL_ALT)
+    int maxBlocksPacket4, maxBlocksPacket8;   // of its builds for 4 and 8 specular segments
     int maxBlocksDiffuse;       // of the diffuse-path kernel that follows it
     std::vector<uint64_t> lastKey;
     std::vector<uint64_t> graphKey;
@@ -266,6 +267,11 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM2, k_light_packet_batch<PK_POOL_FAN, 2, false>, 128, 0);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSMAlt, k_light_packet_batch<PK_POOL_ALT, 2, false>, 128, 0);
         b->maxBlocksPacketAlt = perSMAlt < 1 ? 1 : perSMAlt;
+        int perSM4 = 0, perSM8 = 0;
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM4, k_light_packet_batch<64, 4, false>, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM8, k_light_packet_batch<64, 8, false>, 128, 0);
+        b->maxBlocksPacket4 = perSM4 < 1 ? 1 : perSM4;
+        b->maxBlocksPacket8 = perSM8 < 1 ? 1 : perSM8;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM3, k_light_diffuse_batch<true, false>, 128, 0);
         if (e != cudaSuccess) rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "occupancy: %s", cudaGetErrorString(e));
         b->maxBlocksPerSM = perSM < 1 ? 1 : perSM;
@@ -368,6 +374,14 @@ struct FramePlan {
     bool far;                   // a map of the frame is far: the kernels' FAR forms for all
 };
 
+// resident blocks per SM of the packet build of segs segments; only that of 2 segments has the second pool size
+static int packet_limit(const DNgpuBatch* b, uint32_t segs, bool far, uint32_t poolRays)
+{
+    if (segs == 4u) return b->maxBlocksPacket4;
+    if (segs == 8u) return b->maxBlocksPacket8;
+    return far || poolRays == PK_POOL_FAN ? b->maxBlocksPacket : b->maxBlocksPacketAlt;
+}
+
 // packets: the segments of the build of dn_light_packet.cuh to run (every map's specBounceLimit within its limit), 0
 // for the ray streams
 static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, uint32_t packets, bool far, bool side)
@@ -376,7 +390,9 @@ static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, 
     k_mark_opaque_batch<<<la.nmaps * MARK_BLOCKS, 256, 0, s>>>(la.maps, la.mixed);
     CK(cudaGetLastError());
     COUNT_LAUNCH();
-    const unsigned grid = (unsigned)(g_numSMs * (int)b->tuning.blocksPerSM);
+    int perSM = (int)b->tuning.blocksPerSM;
+    if (packets) perSM = std::min(perSM, packet_limit(b, packets, far, b->tuning.poolRays));
+    const unsigned grid = (unsigned)(g_numSMs * perSM);
     if (packets && far) k_light_packet_batch<PK_POOL_FAN, 2, true><<<grid, 128, 0, s>>>(la);
     else if (packets == 4u) k_light_packet_batch<64, 4, false><<<grid, 128, 0, s>>>(la);
     else if (packets == 8u) k_light_packet_batch<64, 8, false><<<grid, 128, 0, s>>>(la);
@@ -825,26 +841,24 @@ extern "C" int dn_cuda_batch_autotune(DNgpuBatch* b, dn_batch_tuning* chosen)
         dn_batch_tuning t = best;
         t.kernel = 3u - t.kernel;
         t.streamBatch = t.kernel == 2u ? g_packetBatch : g_streamBatch;
-        t.blocksPerSM = (uint32_t)(t.kernel == 2u ? b->maxBlocksPacket : b->maxBlocksPerSM);
+        t.blocksPerSM = (uint32_t)(t.kernel == 2u ? packet_limit(b, b->lastSegs, b->lastFar, t.poolRays) : b->maxBlocksPerSM);
         if (!rc && (t.kernel == 1u || packetsOk)) trial(t);
     }
     const uint32_t batches[] = {4u, 8u, 12u, 16u, 20u, 24u, 28u, 32u};
     for (uint32_t sb : batches) { dn_batch_tuning t = best; t.streamBatch = sb; if (!rc) trial(t); }
     if (best.kernel == 2u && packetsOk) {
-        // rays a warp pulls per pool, then the diffuse kernel's refill threshold
-        {
+        // rays a warp pulls per pool where the build has two sizes, then the diffuse kernel's refill threshold
+        if (b->lastSegs == 2u && !b->lastFar) {
             dn_batch_tuning t = best;
             t.poolRays = best.poolRays == PK_POOL_FAN ? PK_POOL_ALT : PK_POOL_FAN;
-            const uint32_t mx = (uint32_t)(t.poolRays == PK_POOL_FAN ? b->maxBlocksPacket : b->maxBlocksPacketAlt);
+            const uint32_t mx = (uint32_t)packet_limit(b, 2u, false, t.poolRays);
             if (t.blocksPerSM > mx) t.blocksPerSM = mx;
             if (!rc) trial(t);
         }
         const uint32_t dbatches[] = {8u, 12u, 16u, 20u, 24u, 28u};
         for (uint32_t db : dbatches) { dn_batch_tuning t = best; t.diffuseBatch = db; if (!rc) trial(t); }
     }
-    const uint32_t bpsMax = (uint32_t)(best.kernel == 2u ? (best.poolRays == PK_POOL_FAN ? b->maxBlocksPacket
-                                                                                    : b->maxBlocksPacketAlt)
-                                                       : b->maxBlocksPerSM);
+    const uint32_t bpsMax = (uint32_t)(best.kernel == 2u ? packet_limit(b, b->lastSegs, b->lastFar, best.poolRays) : b->maxBlocksPerSM);
     for (uint32_t bps = 2; bps <= bpsMax && bps <= 8; bps++) {
         dn_batch_tuning t = best; t.blocksPerSM = bps; if (!rc) trial(t);
     }

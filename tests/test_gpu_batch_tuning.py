@@ -111,3 +111,18 @@ def test_replayed_frame_counts_its_launches(gpu_ready, light, settings):
         assert counts[0] == counts[1] > 0, counts
     finally:
         maps.close()
+
+
+@pytest.mark.parametrize("limit", [4, 8])
+def test_autotune_keeps_a_pool_size_that_has_no_effect(gpu_ready, limit):
+    """only the packet build of two segments has two pool sizes; for the others a trial of the second times the same
+    kernel again, and would be chosen by chance"""
+    maps = Maps(specBounceLimit=limit)
+    try:
+        for pool in (128, 64):
+            for _ in range(6):
+                maps.batch.set_tuning(poolRays=pool, kernel=2, streamBatch=16, blocksPerSM=2)
+                maps.frame()
+                assert maps.batch.autotune()["poolRays"] == pool
+    finally:
+        maps.close()

@@ -66,7 +66,8 @@ struct DNgpuBatch {
     BatchLightArgs lastLight;
     bool lastLightValid;
     uint32_t lastSegs;          // the packet build that frame's maps can take (its segments; 0: ray streams only)
-    bool lastFar, lastSide;
+    bool lastFar;
+    uint32_t lastSide;
     std::vector<std::pair<DNgpuVolume*, uint64_t>> lastLightGens;
 };
 
@@ -111,8 +112,10 @@ __global__ void __launch_bounds__(256) k_compact_batch(const CompactArgs* s, con
 // blocks [0, nl): shadow directions of light map blockIdx.x.  Block nl: clamp the request count of every
 // synced map to its capacity (the list's words behind it were not written), then the exclusive prefix of the light
 // maps' counts into reqStart[0..nl] and a zero work counter.
+// sideLanes: the lanes of the diffuse launch if it may run paths side by side, else 0: the exclusive prefix of the maps'
+// windows into winStart[0..nl] where it does.
 __global__ void k_batch_prep(BatchLightMap* l, uint32_t nl, const CompactArgs* s, uint32_t ns, uint32_t* reqStart,
-                             uint32_t* workCounter)
+                             uint32_t* winStart, uint32_t sideLanes, uint32_t* workCounter)
 {
     if (blockIdx.x < nl) {
         BatchLightMap& e = l[blockIdx.x];
@@ -123,33 +126,40 @@ __global__ void k_batch_prep(BatchLightMap* l, uint32_t nl, const CompactArgs* s
         uint32_t* c = &s[i].st->w[ST_REQ];
         if (*c > s[i].reqCap) *c = (uint32_t)s[i].reqCap;
     }
+    if (threadIdx.x == 0) workCounter[0] = workCounter[1] = workCounter[2] = 0;
     __shared__ uint32_t warpSum[32];
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) { carry = 0; workCounter[0] = workCounter[1] = workCounter[2] = 0; }
-    __syncthreads();
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    for (uint32_t base = 0; base < nl; base += blockDim.x) {
-        const uint32_t i = base + threadIdx.x;
-        uint32_t v = 0;
-        if (i < nl) {
-            v = *l[i].nreqPtr;
-            if (v > l[i].reqCap) v = (uint32_t)l[i].reqCap;
+    // exclusive prefix of value(i) over the maps into start[0..nl]; the whole block calls it and gets the sum
+    auto prefix = [&](uint32_t* start, auto value) {
+        uint32_t carry = 0;
+        for (uint32_t base = 0; base < nl; base += blockDim.x) {
+            const uint32_t i = base + threadIdx.x;
+            const uint32_t v = i < nl ? value(i) : 0u;
+            uint32_t incl = v;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if ((int)lane >= o) incl += t;
+            }
+            if (lane == 31u) warpSum[warp] = incl;
+            __syncthreads();
+            uint32_t before = carry;
+            for (uint32_t w = 0; w < warp; w++) before += warpSum[w];
+            if (i < nl) start[i] = before + incl - v;
+            for (uint32_t w = 0; w < blockDim.x / 32u; w++) carry += warpSum[w];
+            __syncthreads();
         }
-        uint32_t incl = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if ((int)lane >= o) incl += t;
-        }
-        if (lane == 31u) warpSum[warp] = incl;
-        __syncthreads();
-        uint32_t before = carry;
-        for (uint32_t w = 0; w < warp; w++) before += warpSum[w];
-        if (i < nl) reqStart[i] = before + incl - v;
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry = before + incl;
-        __syncthreads();
+        if (threadIdx.x == 0) start[nl] = carry;
+        return carry;
+    };
+    auto requests = [&](uint32_t i) {
+        const uint32_t v = *l[i].nreqPtr;
+        return v > l[i].reqCap ? (uint32_t)l[i].reqCap : v;
+    };
+    const uint32_t nreq = prefix(reqStart, requests);
+    if (sideLanes && paths_side_by_side(nreq, sideLanes)) {
+        const uint32_t parts = window_parts(nreq, sideLanes / 32u);
+        prefix(winStart, [&](uint32_t i) { return requests(i) << share_parts(parts, path_share(l[i].p)); });
     }
-    if (threadIdx.x == 0) reqStart[nl] = carry;
 }
 
 template <bool FAR>
@@ -182,15 +192,13 @@ __global__ void __launch_bounds__(256) k_mark_opaque_batch(const BatchLightMap* 
 }
 
 // the diffuse paths of the voxels k_light_packet_batch lit, as per-lane path streams over every map's queue
-template <bool SIDE, bool FAR>
+template <uint32_t SIDE, bool FAR>
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse_batch(const __grid_constant__ BatchLightArgs a)
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
     __shared__ uint8_t order[128];
-    uint8_t* const mine = order + (threadIdx.x & ~31u);
-    if (FAR || *a.mixed) path_loop<true, true, SIDE, FAR>(nullptr, &a, jobs[threadIdx.x], tint, mine);
-    else if constexpr (!FAR) path_loop<true, false, SIDE, false>(nullptr, &a, jobs[threadIdx.x], tint, mine);
+    path_launch<true, SIDE, FAR>(nullptr, &a, *a.mixed != 0u, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
 }
 
 __global__ void k_commit_batch(const BatchLightMap* l, const uint32_t* reqStart, uint32_t nl)
@@ -238,7 +246,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
     b->tuning.streamBatch = b->tuning.kernel == 2u ? g_packetBatch : g_streamBatch;
     b->tuning.blocksPerSM = DN_STREAM_MIN_BLOCKS; b->tuning.useGraph = 1;
     b->tuning.poolRays = PK_POOL_FAN; b->tuning.diffuseBatch = g_pathBatch;
-    b->lastSegs = 0; b->lastFar = b->lastSide = false;
+    b->lastSegs = 0; b->lastFar = false; b->lastSide = 0;
     b->graph = nullptr; b->captures = 0; b->graphLaunches = 0;
     b->lastLightValid = false;
     int rc = DN_CUDA_OK;
@@ -272,7 +280,7 @@ extern "C" int dn_cuda_batch_create(DNgpuBatch** out)
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM8, k_light_packet_batch<64, 8, false>, 128, 0);
         b->maxBlocksPacket4 = perSM4 < 1 ? 1 : perSM4;
         b->maxBlocksPacket8 = perSM8 < 1 ? 1 : perSM8;
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM3, k_light_diffuse_batch<true, false>, 128, 0);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM3, k_light_diffuse_batch<2, false>, 128, 0);
         if (e != cudaSuccess) rc = dn_set_err(DN_CUDA_ERR_LAUNCH, "occupancy: %s", cudaGetErrorString(e));
         b->maxBlocksPerSM = perSM < 1 ? 1 : perSM;
         b->maxBlocksPacket = perSM2 < 1 ? 1 : perSM2;
@@ -345,7 +353,7 @@ extern "C" void dn_cuda_batch_destroy(DNgpuBatch* b)
 // byte offsets of the sections of a frame's table
 struct TableLayout {
     uint32_t nm, nd, ns, nl;
-    size_t oMats, oDraw, oSync, oLight, oReqStart, oDrawStart, oSyncStart, size;
+    size_t oMats, oDraw, oSync, oLight, oReqStart, oWinStart, oDrawStart, oSyncStart, size;
 };
 
 static TableLayout layout(uint32_t nm, uint32_t nd, uint32_t ns, uint32_t nl)
@@ -358,6 +366,7 @@ static TableLayout layout(uint32_t nm, uint32_t nd, uint32_t ns, uint32_t nl)
     t.oSync = o; o = align256(o + (size_t)ns * sizeof(CompactArgs));
     t.oLight = o; o = align256(o + (size_t)nl * sizeof(BatchLightMap));
     t.oReqStart = o; o = align256(o + (size_t)(nl + 1) * 4);
+    t.oWinStart = o; o = align256(o + (size_t)(nl + 1) * 4);
     t.oDrawStart = o; o = align256(o + (size_t)(nd + 1) * 4);
     t.oSyncStart = o; o = align256(o + (size_t)(ns + 1) * 4);
     t.size = o;
@@ -370,7 +379,7 @@ struct FramePlan {
     bool hostImages;
     uint32_t segs;              // the packet build (dn_light_packet.cuh) the lit maps can take: its segments, or 0
     uint32_t packets;           // the one lighting runs: segs, or 0 where the tuning asks for the ray streams
-    bool side;                  // a lit map has more than one diffuse path per voxel
+    uint32_t side;              // the diffuse kernel's SIDE: the largest that a lit map asks for (path_side)
     bool far;                   // a map of the frame is far: the kernels' FAR forms for all
 };
 
@@ -384,7 +393,7 @@ static int packet_limit(const DNgpuBatch* b, uint32_t segs, bool far, uint32_t p
 
 // packets: the segments of the build of dn_light_packet.cuh to run (every map's specBounceLimit within its limit), 0
 // for the ray streams
-static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, uint32_t packets, bool far, bool side)
+static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, uint32_t packets, bool far, uint32_t side)
 {
     COUNT_LAUNCH();
     k_mark_opaque_batch<<<la.nmaps * MARK_BLOCKS, 256, 0, s>>>(la.maps, la.mixed);
@@ -407,9 +416,10 @@ static int issue_light(DNgpuBatch* b, const BatchLightArgs& la, cudaStream_t s, 
         ld.batch = b->tuning.diffuseBatch;
         COUNT_LAUNCH();
         const unsigned blocks = (unsigned)(g_numSMs * b->maxBlocksDiffuse);
-        if (far) k_light_diffuse_batch<false, true><<<blocks, 128, 0, s>>>(ld);
-        else if (side) k_light_diffuse_batch<true, false><<<blocks, 128, 0, s>>>(ld);
-        else k_light_diffuse_batch<false, false><<<blocks, 128, 0, s>>>(ld);
+        if (far) k_light_diffuse_batch<0, true><<<blocks, 128, 0, s>>>(ld);
+        else if (side == 2u) k_light_diffuse_batch<2, false><<<blocks, 128, 0, s>>>(ld);
+        else if (side) k_light_diffuse_batch<1, false><<<blocks, 128, 0, s>>>(ld);
+        else k_light_diffuse_batch<0, false><<<blocks, 128, 0, s>>>(ld);
         CK(cudaGetLastError());
     }
     return DN_CUDA_OK;
@@ -462,13 +472,15 @@ static int issue_frame(DNgpuBatch* b, const dn_batch_item* items, uint32_t n, co
     if (t.nl || t.ns) {
         COUNT_LAUNCH();
         k_batch_prep<<<t.nl + 1, 128, 0, s>>>((BatchLightMap*)(d + t.oLight), t.nl, syncs, t.ns,
-                                              (uint32_t*)(d + t.oReqStart), b->workCounter);
+                                              (uint32_t*)(d + t.oReqStart), (uint32_t*)(d + t.oWinStart),
+                                              f.side ? (uint32_t)(g_numSMs * b->maxBlocksDiffuse) * 128u : 0u, b->workCounter);
         CK(cudaGetLastError());
     }
     if (t.nl) {
         BatchLightArgs la;
         la.maps = (BatchLightMap*)(d + t.oLight);
         la.reqStart = (const uint32_t*)(d + t.oReqStart);
+        la.winStart = (const uint32_t*)(d + t.oWinStart);
         la.nmaps = t.nl;
         la.workCounter = b->workCounter;
         la.mixed = b->workCounter + 2;
@@ -547,8 +559,9 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
     for (uint32_t i = 0; i < n; i++) f.far = f.far || map_far(items[i].map);
     f.segs = packet_build(maxSpec, f.far);
     f.packets = b->tuning.kernel == 2u ? f.segs : 0u;
-    f.side = false;
-    for (uint32_t i = 0; i < n; i++) f.side = f.side || ((items[i].phases & DN_BATCH_LIGHT) && items[i].light.numDiffuse > 1u);
+    f.side = 0;
+    for (uint32_t i = 0; i < n && !f.far; i++)
+        if (items[i].phases & DN_BATCH_LIGHT) f.side = std::max(f.side, path_side(items[i].light));
     // from here on the table may change
     b->lastLightValid = false;
     if (f.t.size > b->tabCap) {
@@ -584,7 +597,7 @@ extern "C" int dn_cuda_batch_frame(DNgpuBatch* b, const dn_batch_item* items, ui
     key.reserve(4 + (size_t)n * 10);
     key.push_back(n); key.push_back(b->tabGen); key.push_back(b->tuning.streamBatch); key.push_back(b->tuning.blocksPerSM);
     key.push_back(b->tuning.kernel); key.push_back(((uint64_t)b->tuning.poolRays << 32) | b->tuning.diffuseBatch);
-    key.push_back(((uint64_t)f.packets << 2) | (f.side ? 2u : 0u) | (f.far ? 1u : 0u));
+    key.push_back(((uint64_t)f.packets << 3) | (f.side << 1) | (f.far ? 1u : 0u));
     for (uint32_t i = 0; i < n; i++) {
         const dn_batch_item& it = items[i];
         DNgpuVolume* g = it.map;

@@ -699,16 +699,13 @@ __global__ void __launch_bounds__(128, packet_blocks(SEGS)) k_light_packet(const
 }
 
 // the diffuse paths of the voxels k_light_packet lit (dn_light_path.cuh)
-// SIDE: voxels have several paths
-template <bool SIDE, bool FAR>
+template <uint32_t SIDE, bool FAR>
 __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const __grid_constant__ StreamArgs a)
 {
     __shared__ PathJob jobs[128];
     __shared__ TintT<128> tint;
     __shared__ uint8_t order[128];
-    uint8_t* const mine = order + (threadIdx.x & ~31u);
-    if (FAR || *a.mixed) path_loop<false, true, SIDE, FAR>(&a, nullptr, jobs[threadIdx.x], tint, mine);
-    else if constexpr (!FAR) path_loop<false, false, SIDE, false>(&a, nullptr, jobs[threadIdx.x], tint, mine);
+    path_launch<false, SIDE, FAR>(&a, nullptr, *a.mixed != 0u, jobs[threadIdx.x], tint, order + (threadIdx.x & ~31u));
 }
 
 // launches the lighting kernel g_lightKernel selects (1 ray streams, 2 warp packets followed by the
@@ -741,16 +738,16 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materi
         k<<<g->numSMs * blocks, 128, 0, g->stream>>>(a);
     };
     if (segs && far) {
-        static const int packets = resident(k_light_packet<PK_POOL_FAN, 2, true>), paths = resident(k_light_diffuse<false, true>);
+        static const int packets = resident(k_light_packet<PK_POOL_FAN, 2, true>), paths = resident(k_light_diffuse<0, true>);
         a.batch = g_packetBatch;
         launch(k_light_packet<PK_POOL_FAN, 2, true>, packets);
         CK(cudaGetLastError());
         a.batch = g_pathBatch;
-        launch(k_light_diffuse<false, true>, paths);
+        launch(k_light_diffuse<0, true>, paths);
     } else if (segs) {
         static const int packets2 = resident(k_light_packet<PK_POOL_FAN, 2, false>), packets4 = resident(k_light_packet<64, 4, false>),
-                         packets8 = resident(k_light_packet<64, 8, false>), paths = resident(k_light_diffuse<false, false>),
-                         sidePaths = resident(k_light_diffuse<true, false>);
+                         packets8 = resident(k_light_packet<64, 8, false>), paths = resident(k_light_diffuse<0, false>),
+                         paths1 = resident(k_light_diffuse<1, false>), paths2 = resident(k_light_diffuse<2, false>);
         a.batch = g_packetBatch;
         switch (segs) {
         case 2: launch(k_light_packet<PK_POOL_FAN, 2, false>, packets2); break;
@@ -759,8 +756,11 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materi
         }
         CK(cudaGetLastError());
         a.batch = g_pathBatch;
-        if (a.p.numDiffuse > 1u) launch(k_light_diffuse<true, false>, sidePaths);
-        else launch(k_light_diffuse<false, false>, paths);
+        switch (path_side(a.p)) {
+        case 0: launch(k_light_diffuse<0, false>, paths); break;
+        case 1: launch(k_light_diffuse<1, false>, paths1); break;
+        default: launch(k_light_diffuse<2, false>, paths2); break;
+        }
     } else {
         static const int streams = resident(k_light_stream<false>), farStreams = resident(k_light_stream<true>);
         a.batch = g_streamBatch;

@@ -30,7 +30,7 @@ struct PathJob {
     f3 pos0, tnormal, direct;
     f3 acc, carry, normal;       // the voxel's sum; the path's colour so far; the normal the next direction starts from
     uint32_t material;           // of the last hit
-    uint32_t key, vidx, req, vlane;   // vlane: bits 0-4; above bit 8 how many lanes share the voxel, a path each
+    uint32_t key, vidx, req, vlane;   // vlane: bits 0-4; bit 9: the lane has one path of the voxel, others the rest
     float indirect;              // weight of the lighting so far (0: the voxel's first sample)
     uint32_t b, i;               // bounce, path
     uint32_t draw;               // what the next direction's sphere point is drawn with (path_base)
@@ -61,7 +61,7 @@ __device__ __forceinline__ bool path_setup(PathJob& j, uint32_t req, uint32_t vl
     const ChunkRec* rc = &m.rec[tw & SLOT_MASK];
     if ((tw >> 30) != 2u || vn >= __ldg(&rc->nvox) || !select_voxel(rc, vn, cp, li)) return false;
     const i3 mp{__ldg(&rc->pos[0]), __ldg(&rc->pos[1]), __ldg(&rc->pos[2])};
-    j.req = req; j.vlane = vlane | 256u;
+    j.req = req; j.vlane = vlane;
     j.vidx = __ldg(&rc->voxBase) + vn;
     const uint2 w = __ldg(&m.vox[j.vidx]);
     if (!(mats[w.x >> 24].specular < 1.0f)) return false;
@@ -155,32 +155,68 @@ __device__ __forceinline__ f3 warp_sphere_points(bool need, bool sine, const Pat
     return point;
 }
 
+// the map whose range of a queue holds r: starts[map] <= r < starts[map + 1]
+__device__ __forceinline__ uint32_t window_map(const uint32_t* starts, uint32_t nmaps, uint32_t r)
+{
+    uint32_t lo = 0, hi = nmaps;
+    while (hi - lo > 1u) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (__ldg(&starts[mid]) <= r) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// Paths side by side (SIDE).  In a launch of at most two voxels per lane (counted in whole groups, of which about two
+// thirds hold voxels) a lane's paths, one after the other, would be the launch's length while other lanes have nothing to
+// do; there a voxel takes several lanes, a path each, and when the paths of all a warp's voxels have ended one lane per
+// voxel adds them up in order.  How many lanes: all its paths up to 32; 16 for more, which then takes several passes with
+// the sum carried on (16 and not 32: 33 paths are 3 passes of two voxels at a time instead of 2 passes of one).  Each
+// window of the queue is taken by its own map's rule, so maps with one path keep a lane per voxel beside others.
+// SIDE 0: a lane per voxel; 1: no map of the launch has more than 32 paths; 2: passes too (they cost the others 2.7 %).
+// us per lighting update, a lane per voxel -> side by side: 3x2x3 map (0.002 voxels per lane) 4 paths 76 -> 47, 32 353 ->
+// 57, 64 673 -> 103; 12x8x12 (0.55) 4 397 -> 278, 17 1035 -> 630, 33 1804 -> 857; 22x12x22 (1.84) 2 599 -> 569, 17 1979 ->
+// 1959, 32 3338 -> 2240, 33 3418 -> 2685.  Batched frames: twelve 5x4x6 maps, 32 paths on one and 1 on the others, 1360 ->
+// 447, with 33 on all 2181 -> 1517; a 3x2x3 map with 4, 16 or 64 paths beside two 14x9x14 maps with one, 294, 507, 1345 ->
+// 284, 290, 330.  The line lies at two voxels per lane because up to there no number of paths loses; above it those that
+// leave lanes of a warp without a path do (28x12x28, 2.8: 17 paths 2757 -> 3088, 32 4570 -> 3554), and below it all would
+// lose by a lower line (18x12x18, 1.25: 4 paths 479, a lane per voxel 603).
+__host__ __device__ __forceinline__ uint32_t path_share(const dn_light_params& p)
+{
+    return p.numDiffuse < 2u || p.diffuseBounceLimit == 0u ? 1u : p.numDiffuse <= 32u ? p.numDiffuse : 16u;
+}
+__device__ __forceinline__ bool paths_side_by_side(uint32_t nreq, uint32_t lanes) { return nreq <= lanes / 16u; }
+
+// a map's windows are 2^-result of a request group: as parts for all maps (window_parts), smaller where a window's paths
+// would fill a warp more than once
+__device__ __forceinline__ uint32_t share_parts(uint32_t parts, uint32_t share)
+{
+    while (parts < 5u && (32u >> parts) * share > 32u) parts++;
+    return parts;
+}
+
 // The persistent loop of the launch: one map (one) or a queue over the requests of many maps (many), each lane then
-// reading its voxel's map through that map's entry of the device table.
-// SIDE: a voxel may have several paths.  In a launch of at most two voxels per lane (counted in whole groups, of which
-// about two thirds hold voxels) a lane's paths, one after the other, would be the launch's length while other lanes have
-// nothing to do; there each path gets a lane of its own, and when all paths of a warp's window have ended one lane per
-// voxel forms its sum.  us per pass, before -> after: four updates of a 16x12x16 map with 4 paths per voxel 4840 -> 4395,
-// 23x11x37 map with 2 paths 418 -> 402, six maps of 9x12x7 with 3 paths batched 372 -> 280; a limit of one voxel per lane
-// 4874, 421, 280.  Launches whose voxels have one path take the build without it (glass map 2 % faster than with).
-template <bool MANY, bool TINTED, bool SIDE, bool FAR>
-__device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLightArgs* many, PathJob& j, TintT<128>& tint,
-                                          uint8_t* order)
+// reading its voxel's map through that map's entry of the device table.  FAR: maps above FAR_SUM chunks (dn_walk.cuh).
+template <bool MANY, bool TINTED, uint32_t SIDE, bool FAR>
+__device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLightArgs* many, uint32_t nreq, PathJob& j,
+                                          TintT<128>& tint, uint8_t* order)
 {
     const uint32_t lane = lane_id_s(), col = threadIdx.x;
     const uint32_t batch = MANY ? many->batch : one->batch;
-    uint32_t nreq = 0;
-    if constexpr (MANY) nreq = *(volatile const uint32_t*)&many->reqStart[many->nmaps];
-    else nreq = *(volatile const uint32_t*)one->nreqPtr;
     uint32_t* const counter = (MANY ? many->workCounter : one->workCounter) + 1;
     uint32_t winMap = 0, winReq = 0, winNext = 32, winEnd = 32;   // warp-uniform voxel window: map, request, next voxel, end
-    const bool split = SIDE && nreq * 32u <= 2u * gridDim.x * blockDim.x;
-    uint32_t parts = window_parts(nreq);
-    if (split) {
-        // a window's paths fill a warp once
-        const uint32_t paths = MANY ? many->maps[0].p.numDiffuse : one->p.numDiffuse;
-        while (parts < 5u && (32u >> parts) * min(paths, 32u) > 32u) parts++;
-    }
+    const uint32_t allParts = window_parts(nreq, gridDim.x * (blockDim.x / 32u));
+    // the queue: windows of the maps one after the other
+    const uint32_t* const starts = MANY ? (SIDE != 0u ? many->winStart : many->reqStart) : nullptr;
+    auto mapParams = [&](uint32_t map) -> const dn_light_params& { if constexpr (MANY) return many->maps[map].p; else return one->p; };
+    uint32_t winShare = 1, parts = allParts;   // SIDE > 0: the lanes a voxel of the window takes, and the window's part of a group
+    if constexpr (!MANY && SIDE != 0u) { winShare = path_share(one->p); parts = share_parts(allParts, winShare); }
+    uint32_t nwin = nreq << parts;
+    if constexpr (MANY && SIDE != 0u) nwin = *(volatile const uint32_t*)&many->winStart[many->nmaps];
+    // whether the window's voxels take several lanes (one map: all windows' do)
+    auto shared = [&]() { return SIDE != 0u && (!MANY || winShare > 1u); };
+    bool team = false;                 // the warp's lanes are on such voxels
+    uint32_t first = 0;                // the first path of their pass (SIDE 2)
+    uint32_t role = 0;                 // the lane's path in its voxel's pass, from 1 on; 0: none
     bool exhausted = false;
     const BatchLightMap* le = nullptr;
     if constexpr (MANY) le = &many->maps[0];
@@ -191,15 +227,15 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
     Ray s;
     s.mode = RM_IDLE;
     bool own = false, done = false;    // the lane has a voxel; no voxel is left for it
-    uint32_t lead = 0;                 // lanes, from this one, whose paths are this lane's voxel's
     Counters c{0, 0, 0, 0, 0};
     for (;;) {
         const unsigned waiting = __ballot_sync(0xFFFFFFFFu, !ray_stepping(s) && !done);
         const unsigned stepping = __ballot_sync(0xFFFFFFFFu, ray_stepping(s));
         if ((waiting | stepping) == 0u) break;
         bool go = stepping == 0u;
-        if (split) {
-            // lanes whose path is done wait for their voxel's others: the threshold is a share of the lanes at work
+        if (shared() && (!MANY || team || winNext < winEnd)) {
+            // lanes whose path is done wait for their voxel's others, or for the lanes that finish before the warp turns to
+            // the window's voxels: the threshold is a share of the lanes at work
             const unsigned work = __ballot_sync(0xFFFFFFFFu, own);
             go = go || (uint32_t)__popc(work & ~stepping) * 32u >= batch * (uint32_t)__popc(work);
         } else {
@@ -243,7 +279,7 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
                 }
                 s.mode = RM_IDLE;
                 if (!start) {
-                    if (SIDE && j.vlane >= 512u) {
+                    if (SIDE != 0u && j.vlane >= 512u) {
                         own = false;
                     } else {
                         j.acc = add(j.acc, j.direct);
@@ -255,53 +291,70 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
                     }
                 }
             }
-            if (split && __ballot_sync(0xFFFFFFFFu, own) == 0u) {
-                // the sums of the voxels whose paths were traced side by side, in the reference's order.  (A path adds at
-                // most one contribution; one without adds zero, which changes no sum.)
+            if (SIDE != 0u && team && __ballot_sync(0xFFFFFFFFu, own) == 0u) {
+                // a pass has ended: its paths are added to the voxels' sums in the reference's order.  (A path adds at most
+                // one contribution; one without adds zero, which changes no sum.)  The sum is carried where the voxel's
+                // second lane keeps the direct light, which only the first one needs.
+                uint32_t paths = winShare;
+                if constexpr (SIDE == 2u) paths = mapParams(winMap).numDiffuse;
                 __syncwarp();
-                if (lead) {
+                if (role == 1u) {
                     f3 acc = mk(0.0f, 0.0f, 0.0f);
+                    if (SIDE == 2u && first) acc = (&j)[1].direct;
                     const f3 amb = mk(P().ambient[0], P().ambient[1], P().ambient[2]);
-                    for (uint32_t i = 0; i < lead; i++) acc = add(add(add(acc, amb), (&j)[i].acc), j.direct);
-                    j.acc = acc;
-                    path_write(j, M(), P(), OUT());
-                    lead = 0;
+                    const uint32_t n = SIDE == 2u ? min(winShare, paths - first) : winShare;
+                    for (uint32_t i = 0; i < n; i++) acc = add(add(add(acc, amb), (&j)[i].acc), j.direct);
+                    if (SIDE == 2u && first + winShare < paths) {
+                        (&j)[1].direct = acc;
+                    } else {
+                        j.acc = acc;
+                        path_write(j, M(), P(), OUT());
+                    }
                 }
                 __syncwarp();
+                team = false;
+                if constexpr (SIDE == 2u) {
+                    first += winShare;
+                    team = first < paths;
+                    if (team && role) {
+                        j.acc = mk(0.0f, 0.0f, 0.0f);
+                        j.i = first + role - 1u;
+                        own = j.i < paths;
+                    }
+                }
+                if (!team) role = 0;
             }
             // voxels for the lanes without one
             for (;;) {
                 const unsigned need = __ballot_sync(0xFFFFFFFFu, !own && !done);
-                if (need == 0u || (split && need != 0xFFFFFFFFu)) break;
+                if (need == 0u || (SIDE != 0u && team)) break;
                 if (winNext >= winEnd) {
                     uint32_t r = 0;
                     if (!exhausted && lane == 0) r = atomicAdd(counter, 1u);
                     r = __shfl_sync(0xFFFFFFFFu, r, 0);
-                    if (exhausted || r >= nreq << parts) {
+                    if (exhausted || r >= nwin) {
                         exhausted = true;
                         if (!own) done = true;
                         break;
                     }
+                    if constexpr (MANY && SIDE != 0u) {
+                        winMap = window_map(starts, many->nmaps, r);
+                        r -= __ldg(&starts[winMap]);
+                        winShare = path_share(mapParams(winMap));
+                        parts = share_parts(allParts, winShare);
+                    }
                     winNext = (r & ((1u << parts) - 1u)) << (5u - parts);
                     winEnd = winNext + (32u >> parts);
                     r >>= parts;
-                    winReq = r;
-                    if constexpr (MANY) {
-                        // the map whose request range holds r: reqStart[map] <= r < reqStart[map + 1]
-                        uint32_t lo = 0, hi = many->nmaps;
-                        while (hi - lo > 1u) {
-                            const uint32_t mid = (lo + hi) >> 1;
-                            if (__ldg(&many->reqStart[mid]) <= r) lo = mid; else hi = mid;
-                        }
-                        winMap = lo;
-                        winReq = r - __ldg(&many->reqStart[lo]);
+                    if constexpr (MANY && SIDE == 0u) {
+                        winMap = window_map(starts, many->nmaps, r);
+                        r -= __ldg(&starts[winMap]);
                     }
+                    winReq = r;
                 }
-                if (split) {
-                    // the next voxels, each on as many lanes as it has paths
-                    const dn_light_params& p = MANY ? many->maps[winMap].p : one->p;
-                    const uint32_t share = p.numDiffuse >= 2u && p.numDiffuse <= 32u && p.diffuseBounceLimit ? p.numDiffuse : 1u;
-                    const uint32_t nvox = min(32u / share, winEnd - winNext), v = lane / share;
+                if (shared()) {
+                    if (need != 0xFFFFFFFFu) break;   // the lanes at work finish first
+                    const uint32_t nvox = min(32u / winShare, winEnd - winNext), v = lane / winShare;
                     if (v < nvox) {
                         if constexpr (MANY) {
                             le = &many->maps[winMap];
@@ -309,13 +362,15 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
                         } else {
                             own = path_setup(j, winReq, winNext + v, one->m, one->p, MATS(), one->reqs, one->nsamples, one->out);
                         }
-                        if (own && share > 1u) {
-                            j.i = lane - v * share;
-                            j.vlane = (j.vlane & 31u) | share << 8;
-                            lead = j.i == 0u ? share : 0u;
+                        if (own) {
+                            role = lane - v * winShare + 1u;
+                            j.i = role - 1u;
+                            j.vlane |= 512u;
                         }
                     }
                     winNext += nvox;
+                    first = 0;
+                    team = __ballot_sync(0xFFFFFFFFu, own) != 0u;
                     continue;
                 }
                 const uint32_t rank = __popc(need & ((1u << lane) - 1u));
@@ -336,7 +391,7 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
             f3 base = mk(0.0f, 0.0f, 0.0f);
             if (begin) {
                 if (!start) {
-                    if (!SIDE || j.vlane < 512u) j.acc = add(j.acc, mk(P().ambient[0], P().ambient[1], P().ambient[2]));
+                    if (SIDE == 0u || j.vlane < 512u) j.acc = add(j.acc, mk(P().ambient[0], P().ambient[1], P().ambient[2]));
                     j.carry = mk(1.0f, 1.0f, 1.0f);
                     j.normal = adds(j.tnormal, EPS);
                     j.b = 0;
@@ -355,6 +410,29 @@ __device__ __forceinline__ void path_loop(const StreamArgs* one, const BatchLigh
         if (ray_stepping(s)) walk_round<FAR, TINTED>(s, M(), MATS(), P().sunStrength, c, tint, col);
     }
     flush_counters(MANY ? many->stats : one->stats, c, 0, 0);
+}
+
+// the SIDE a map asks for
+__host__ __device__ __forceinline__ uint32_t path_side(const dn_light_params& p)
+{
+    return path_share(p) == 1u ? 0u : p.numDiffuse <= 32u ? 1u : 2u;
+}
+
+// the loop a launch runs: with paths side by side or a lane per voxel
+template <bool MANY, uint32_t SIDE, bool FAR>
+__device__ __forceinline__ void path_launch(const StreamArgs* one, const BatchLightArgs* many, bool tinted, PathJob& j,
+                                            TintT<128>& tint, uint8_t* order)
+{
+    const uint32_t nreq = MANY ? *(volatile const uint32_t*)&many->reqStart[many->nmaps] : *(volatile const uint32_t*)one->nreqPtr;
+    if constexpr (SIDE != 0u) {
+        if (paths_side_by_side(nreq, gridDim.x * blockDim.x)) {
+            if (tinted) path_loop<MANY, true, SIDE, FAR>(one, many, nreq, j, tint, order);
+            else path_loop<MANY, false, SIDE, FAR>(one, many, nreq, j, tint, order);
+            return;
+        }
+    }
+    if (FAR || tinted) path_loop<MANY, true, 0, FAR>(one, many, nreq, j, tint, order);
+    else if constexpr (!FAR) path_loop<MANY, false, 0, false>(one, many, nreq, j, tint, order);
 }
 
 } // namespace dn

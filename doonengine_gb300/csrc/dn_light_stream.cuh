@@ -365,6 +365,7 @@ struct BatchLightMap {
 struct BatchLightArgs {
     BatchLightMap* maps;
     const uint32_t* reqStart;   // [nmaps + 1]: first request of each map in the launch's queue
+    const uint32_t* winStart;   // [nmaps + 1]: first window of each map where paths run side by side (dn_light_path.cuh)
     uint32_t nmaps;
     uint32_t* workCounter;
     unsigned long long* stats;
@@ -388,10 +389,10 @@ __device__ __forceinline__ void shadow_dir(const dn_light_params& p, int k, floa
 
 // A warp's window into the queue is a whole request group, or a part of one (2^-result) when the launch has fewer
 // groups than warps: its few voxels then run on all SMs, and one waits for fewer others.
-__device__ __forceinline__ uint32_t window_parts(uint32_t nreq)
+__device__ __forceinline__ uint32_t window_parts(uint32_t nreq, uint32_t warps)
 {
     uint32_t parts = 0;
-    while (parts < 5u && (nreq << (parts + 1u)) <= gridDim.x * (blockDim.x / 32u)) parts++;
+    while (parts < 5u && (nreq << (parts + 1u)) <= warps) parts++;
     return parts;
 }
 
@@ -411,7 +412,7 @@ __device__ __forceinline__ void stream_loop(const StreamArgs* one, const BatchLi
     else nreq = *(volatile const uint32_t*)one->nreqPtr;
     uint32_t* const counter = MANY ? many->workCounter : one->workCounter;
     uint32_t winMap = 0, winReq = 0, winNext = 32, winEnd = 32;   // warp-uniform voxel window: map, request, next voxel, end
-    const uint32_t parts = window_parts(nreq);
+    const uint32_t parts = window_parts(nreq, gridDim.x * (blockDim.x / 32u));
     bool exhausted = false;
     j.phase = PH_FETCH;
     j.map = 0;

@@ -712,11 +712,6 @@ __global__ void __launch_bounds__(128, DN_DIFF_MIN_BLOCKS) k_light_diffuse(const
 // diffuse-path kernel where packet_build has one, streams otherwise) with its batch threshold
 static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materials)
 {
-    // resident blocks per SM, the same on every device this library is built for
-    auto resident = [](auto* k) {
-        int n = 0;
-        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, 128, 0) == cudaSuccess && n > 0 ? n : 1;
-    };
     {
         MaterialTable table;            // on the stack: a launch argument, copied at the launch
         memcpy(table.m, materials, sizeof(table.m));
@@ -733,42 +728,39 @@ static int launch_light(DNgpuVolume* g, StreamArgs& a, const dn_material* materi
     g->lightTurn ^= 1u;
     const bool far = map_far(g);
     const uint32_t segs = g_lightKernel == 2 ? packet_build(a.p.specBounceLimit, far) : 0u;
-    auto launch = [&](auto* k, int blocks) {
+    // kept: the kernel's resident blocks per SM, the same on every device this library is built for; 0 until asked
+    auto launch = [&](auto* k, int& kept) -> int {
+        int blocks = __atomic_load_n(&kept, __ATOMIC_RELAXED);
+        if (!blocks) {
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, 128, 0));
+            if (blocks < 1) blocks = 1;
+            __atomic_store_n(&kept, blocks, __ATOMIC_RELAXED);
+        }
         COUNT_LAUNCH();
         k<<<g->numSMs * blocks, 128, 0, g->stream>>>(a);
+        CK(cudaGetLastError());
+        return DN_CUDA_OK;
     };
-    if (segs && far) {
-        static const int packets = resident(k_light_packet<PK_POOL_FAN, 2, true>), paths = resident(k_light_diffuse<0, true>);
-        a.batch = g_packetBatch;
-        launch(k_light_packet<PK_POOL_FAN, 2, true>, packets);
-        CK(cudaGetLastError());
-        a.batch = g_pathBatch;
-        launch(k_light_diffuse<0, true>, paths);
-    } else if (segs) {
-        static const int packets2 = resident(k_light_packet<PK_POOL_FAN, 2, false>), packets4 = resident(k_light_packet<64, 4, false>),
-                         packets8 = resident(k_light_packet<64, 8, false>), paths = resident(k_light_diffuse<0, false>),
-                         paths1 = resident(k_light_diffuse<1, false>), paths2 = resident(k_light_diffuse<2, false>);
-        a.batch = g_packetBatch;
-        switch (segs) {
-        case 2: launch(k_light_packet<PK_POOL_FAN, 2, false>, packets2); break;
-        case 4: launch(k_light_packet<64, 4, false>, packets4); break;
-        default: launch(k_light_packet<64, 8, false>, packets8); break;
-        }
-        CK(cudaGetLastError());
-        a.batch = g_pathBatch;
-        switch (path_side(a.p)) {
-        case 0: launch(k_light_diffuse<0, false>, paths); break;
-        case 1: launch(k_light_diffuse<1, false>, paths1); break;
-        default: launch(k_light_diffuse<2, false>, paths2); break;
-        }
-    } else {
-        static const int streams = resident(k_light_stream<false>), farStreams = resident(k_light_stream<true>);
+    if (!segs) {
+        static int streams, farStreams;
         a.batch = g_streamBatch;
-        if (far) launch(k_light_stream<true>, farStreams);
-        else launch(k_light_stream<false>, streams);
+        return far ? launch(k_light_stream<true>, farStreams) : launch(k_light_stream<false>, streams);
     }
-    CK(cudaGetLastError());
-    return DN_CUDA_OK;
+    static int packets2, packets4, packets8, farPackets, paths0, paths1, paths2, farPaths;
+    a.batch = g_packetBatch;
+    int rc;
+    if (far) rc = launch(k_light_packet<PK_POOL_FAN, 2, true>, farPackets);
+    else if (segs == 2u) rc = launch(k_light_packet<PK_POOL_FAN, 2, false>, packets2);
+    else if (segs == 4u) rc = launch(k_light_packet<64, 4, false>, packets4);
+    else rc = launch(k_light_packet<64, 8, false>, packets8);
+    if (rc) return rc;
+    a.batch = g_pathBatch;
+    if (far) return launch(k_light_diffuse<0, true>, farPaths);
+    switch (path_side(a.p)) {
+    case 0: return launch(k_light_diffuse<0, false>, paths0);
+    case 1: return launch(k_light_diffuse<1, false>, paths1);
+    default: return launch(k_light_diffuse<2, false>, paths2);
+    }
 }
 
 // D1/D2: commit the new lighting after the whole launch, then count the sample

@@ -5,10 +5,12 @@
  *   1. one host-to-device copy of the frame's table (per-map parameters, image pointers, materials);
  *   2. k_batch_reset: zero the request counters of the maps whose per-tile pass runs;
  *   3. k_draw_batch: every pixel of every image (blocks of 16x8 pixels; a block belongs to one map);
- *   4. k_compact_batch: the per-tile sync pass over every tile of every map (blocks of 256 tiles);
+ *   4. k_compact_batch: the per-tile sync pass over every tile of every map (blocks of 256 walk-grid cells);
  *   5. k_batch_prep: clamp the request counts, lay the maps' request lists end to end as one queue (an
- *      exclusive prefix over the counts) and compute each map's shadow directions;
- *   6. k_light_stream_batch: the persistent lighting loop (dn_light_stream.cuh) over the whole queue;
+ *      exclusive prefix over the counts, and over the maps' windows where paths run side by side) and
+ *      compute each map's shadow directions; k_mark_opaque_batch: the opaque-chunk marks;
+ *   6. k_light_packet_batch and k_light_diffuse_batch (or k_light_stream_batch): the persistent lighting
+ *      loops over the whole queue;
  *   7. k_commit_batch: commit every map's new lighting.
  * Host-memory images are copied back on a second stream that overlaps steps 4-7.  A frame whose
  * composition repeats is captured once and replayed as a CUDA graph.

@@ -1311,7 +1311,7 @@ static int launch_draw(DNgpuVolume* g, const dn_draw_params* p, const dn_materia
                    by = (uint32_t)(((uint64_t)p->height + DN_DRAW_BY - 1) / DN_DRAW_BY), bz = (by + 65534u) / 65535u;
     const dim3 grid(bx, (by + bz - 1u) / bz, bz);
     COUNT_LAUNCH();
-    // an image whose warps are all resident at 24 per SM takes the build for 24 (74 registers, no spills): a 257x143
+    // an image whose warps are all resident at 24 per SM takes the build for 24 (77 registers, no spills): a 257x143
     // draw 13.1 us against 14.0
     if (map_far(g)) k_draw<true, DN_DRAW_WARPS><<<grid, block, 0, g->stream>>>(*a);
     else if ((uint64_t)bx * by * (DN_DRAW_BX * DN_DRAW_BY / 32u) <= 24u * (uint64_t)g->numSMs) k_draw<false, 24><<<grid, block, 0, g->stream>>>(*a);

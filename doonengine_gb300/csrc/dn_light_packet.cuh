@@ -24,7 +24,7 @@
  * Bound by issue and by load latency at 28 warps per SM.  Between segments a lane keeps only its ray's number:
  * what a bounce needs besides (multiplier, sky flag) is in the ray's shared-memory slot and two flag bits, and
  * the light of see-through voxels is in shared memory for the rays that meet one (TintT), so the kernel takes
- * 70 registers instead of 80.  Measured with the directions formed by full warps, the table-free sums (a lane
+ * 71 registers (72 for many maps) instead of 80.  Measured with the directions formed by full warps, the table-free sums (a lane
  * per component) and the three unit sizes, us per frame or call, before -> after: 64x32x64 map at 1080p, K = 32:
  * 14200 -> 12240; 16x16x16 at 640x360, K = 16: 661 -> 507; glass 2970 -> 2597; twelve maps batched
  * 15230 -> 12010; eight maps served 2259 -> 1459.
@@ -35,7 +35,7 @@
 namespace dn {
 
 #ifndef DN_PACKET_MIN_BLOCKS
-// 7 blocks of 4 warps per SM (70 registers).  The 64x32x64 map, us per frame: 12440; 6 blocks 12800, 8 (64
+// 7 blocks of 4 warps per SM (71 registers; 72 for many maps, with 60 bytes of spills).  The 64x32x64 map, us per frame: 12440; 6 blocks 12800, 8 (64
 // registers, spills, little L1 left) 12990
 #define DN_PACKET_MIN_BLOCKS 7
 #endif
@@ -156,7 +156,7 @@ __device__ __forceinline__ void packet_setup(PacketVoxel& pv, uint32_t req, uint
 
 // Unit u of a queue of nreq request groups: voxels [first, first + count) of group r; false when there is none.  The
 // queue is five stretches, of units of 16, 8, 4, 2 and 1 voxels.  (Formed again for every unit: kept over the loop,
-// the stretches' bounds cost the many-map kernel spills.)
+// the stretches' bounds cost the many-map kernel more spills than the 60 bytes it has.)
 __device__ __forceinline__ bool packet_unit(uint32_t u, uint32_t nreq, uint32_t& r, uint32_t& first, uint32_t& count)
 {
     const uint32_t warps = gridDim.x * (blockDim.x / 32u);

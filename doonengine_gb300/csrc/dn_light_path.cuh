@@ -3,8 +3,9 @@
  *
  * The packet kernel (dn_light_packet.cuh) leaves each voxel's direct light in its diffuse output slot; this kernel
  * traces the voxel's numDiffuse paths of up to diffuseBounceLimit segments, forms the running average and replaces
- * the slot.  Every lane owns one voxel and walks its paths in the reference's order; a lane whose voxel is done takes
- * the next one of its warp's window, so that a long path holds no other lane.  The paths of a warp have nothing in
+ * the slot.  Every lane owns one voxel and walks its paths in the reference's order (launches of few voxels: see
+ * path_share); a lane whose voxel is done takes the next one of its warp's window, so that a long path holds no other
+ * lane.  The paths of a warp have nothing in
  * common, so the walk's rounds run with about a third of the lanes, and what a segment's end needs runs for all
  * waiting lanes at once when `batch` of them wait (or none is left stepping).
  *
@@ -18,7 +19,7 @@
 #pragma once
 #include "dn_light_stream.cuh"
 
-// 7 blocks of 4 warps per SM (67 and 71 registers); 6 and 8 within 1 %
+// 7 blocks of 4 warps per SM (68 registers, 71 and 72 with paths side by side); 6 and 8 within 1 %
 #ifndef DN_DIFF_MIN_BLOCKS
 #define DN_DIFF_MIN_BLOCKS 7
 #endif

@@ -280,9 +280,10 @@ int scratch_ready(ShapeScratch& sc)
     return DN_CUDA_OK;
 }
 
-// Shapes over at most this many chunks take one pass: the records of 32 chunks are at most 256 KB to move on the host.
-// Frames that place or cut a sphere and relight it, us, before -> after: 639x400 (24x7x8 chunks) 135 -> 123, 101x64
-// (24x4x5) 95 -> 67, 720p with spheres of up to 11 voxels radius (27 to 64 chunks) 165 -> 161.
+// Shapes over at most this many chunks take one pass: it saves a launch and a wait, and costs the host a move of the
+// records that lie behind gaps.  us per call, two passes -> one: spheres over 8 chunks 36 -> 22, 27 chunks 58 -> 46, 45
+// chunks 64 -> 58, 64 chunks 104 -> 96, 94 chunks 228 -> 222, 170 chunks 319 -> 318, 216 chunks 573 -> 589.  The line lies at 32:
+// above it one pass gains 0 to 9 % of a call up to about 170 chunks, for 8 KB of pinned records per chunk and thread.
 const int64_t SHAPE_ONCE_CHUNKS = 32;
 
 // At most this many edits are written straight to the host.  Shapes larger than that are evaluated faster than the link to
